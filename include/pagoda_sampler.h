@@ -183,7 +183,7 @@ PGS_API const char *pgs_static_last_error(void);
  * reference, candidate probabilities use the exact expf, and the f32 left-fold sum of
  * temperature_softmax (sampler.rs:99-113) agrees with the reference's to about 1e-6 relative,
  * so a top-p or CDF decision can differ only when it sits that close to its boundary.  With
- * `on` != 0 every row takes the general kernel, which reproduces that sum -- and therefore
+ * `on` != 0 every row takes the wide kernel, which reproduces that sum -- and therefore
  * every token id -- bit for bit, at a fraction of the speed.  (Environment: PGS_EXACT=1.) */
 PGS_API int pgs_set_exact(pgs_handle *h, int on);
 

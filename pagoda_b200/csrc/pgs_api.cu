@@ -15,6 +15,7 @@
 #include "pgs_args.cuh"
 #include "pgs_stream.cuh"
 #include "pgs_tp.cuh"
+#include "pgs_wide.cuh"
 
 namespace pgs {
 cudaError_t configure_general();
@@ -26,6 +27,8 @@ cudaError_t configure_stream();
 cudaError_t stream_ctas_per_sm(int* out);
 cudaError_t launch_stream(const RowArgs& a, const StreamLaunch& sl, uint32_t grid, uint32_t csize, cudaStream_t stream);
 cudaError_t stream_max_clusters(int csize, int* out);
+cudaError_t configure_wide();
+cudaError_t launch_wide(const RowArgs& a, const WideLaunch& l, uint32_t slots, uint32_t grid, cudaStream_t stream);
 struct ScoreArgs {
     const float* logits;
     unsigned long long row_stride;
@@ -70,11 +73,15 @@ struct pgs_handle {
     unsigned char* aux_host = nullptr;   // pinned
     unsigned char* aux_dev = nullptr;
     size_t aux_bytes = 0;
-    // rows the row kernel hands on to the general kernel (work list)
+    // rows that the row kernel hands on (work list)
     uint32_t* work_rows = nullptr;
     uint32_t* work_count = nullptr;   // [2]
     uint32_t* tp_done = nullptr;      // CTAs finished in the current peer-store push
     int exact = 0;
+    // wide kernel: its workspace (one block of device memory)
+    unsigned char* wide_ws = nullptr;
+    pgs::WideLaunch wide = {};
+    uint32_t wide_vocab = 0;          // longest row the workspace holds
     // streaming row kernel: id -> count slots, shared memory and CTAs per SM, the gate's counter
     uint32_t stream_hash = 0, stream_cohort = 0;
     int max_clusters[4] = {0, 0, 0, 0};   // resident clusters of 1 (unused), 2, 4, 8 CTAs of the row kernel
@@ -133,6 +140,55 @@ uint32_t pow2_at_least(uint32_t v, uint32_t lo) {
 }
 }  // namespace
 
+namespace {
+// The wide kernel's workspace, sized for W_CHUNK rows (fewer when the handle has fewer) of the handle's vocabulary.
+int wide_workspace(pgs_handle* h) {
+    using namespace pgs;
+    const size_t rows = h->slots < (uint32_t)W_CHUNK ? h->slots : (uint32_t)W_CHUNK;
+    const uint32_t vocab = h->max_vocab < (uint32_t)W_MAX_VOCAB ? h->max_vocab : (uint32_t)W_MAX_VOCAB;
+    const uint32_t regions = (vocab + W_REGION - 1) / W_REGION;
+    WideLaunch& l = h->wide;
+    l.reg_stride = regions; l.rs_stride = regions + 1u;
+    size_t used = 0;
+    auto take = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~size_t(255); return at; };
+    const size_t o_sync = take(64), o_left = take(4), zeroed = used;
+    const size_t o_rows = take((size_t)h->max_rows * 4), o_row = take(rows * sizeof(WideRow)), o_reg = take(rows * regions * sizeof(float2));
+    const size_t o_seg = take(rows * regions * sizeof(uint2)), o_pre = take(rows * regions * 4), o_rs = take(rows * (regions + 1u) * 4);
+    const size_t o_eid = take(rows * (W_MAX_HIST + 32) * 4), o_exn = take(rows * (W_MAX_HIST + 32) * 4);
+    const size_t o_hist = take(rows * W_BUCKETS * 4);
+    const size_t o_terms = take(rows * (size_t)W_TERMS * W_REGION * 4);
+    PGS_CUDA(nullptr, cudaMalloc(&h->wide_ws, used));
+    PGS_CUDA(nullptr, cudaMemsetAsync(h->wide_ws, 0, zeroed, h->stream));
+    unsigned char* p = h->wide_ws;
+    l.sync = (uint32_t*)(p + o_sync); l.left_count = (uint32_t*)(p + o_left); l.left_rows = (uint32_t*)(p + o_rows);
+    l.row = (WideRow*)(p + o_row); l.reg = (float2*)(p + o_reg); l.seg = (uint2*)(p + o_seg); l.pre = (float*)(p + o_pre);
+    l.rs = (uint32_t*)(p + o_rs); l.ent_id = (uint32_t*)(p + o_eid); l.ent_xn = (float*)(p + o_exn); l.hist = (uint32_t*)(p + o_hist);
+    l.list = h->sl_key; l.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
+    l.terms = (float*)(p + o_terms);
+    h->wide_vocab = vocab;
+    return PGS_OK;
+}
+
+// Every step of a handle uses the same scratch, lists and counters: a step on another stream than the one before waits for
+// that one to finish on the device.
+int order_steps(pgs_handle* h, cudaStream_t stream) {
+    if (stream != h->last_stream) {
+        PGS_CUDA(h, cudaEventRecord(h->ev_step, h->last_stream));
+        PGS_CUDA(h, cudaStreamWaitEvent(stream, h->ev_step, 0));
+        h->last_stream = stream;
+    }
+    return PGS_OK;
+}
+
+// CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid
+// barriers cost more with more CTAs).
+uint32_t wide_grid(const pgs_handle* h, uint32_t rows, uint32_t vocab) {
+    const uint64_t share = ((uint64_t)rows * ((vocab + pgs::W_REGION - 1) / pgs::W_REGION) + 7u) / 8u;
+    const uint64_t want = share > rows ? share : rows;
+    return want < (uint64_t)h->sm_count ? (uint32_t)want : (uint32_t)h->sm_count;
+}
+}  // namespace
+
 extern "C" const char* pgs_last_error(const pgs_handle* h) { return h ? h->err : g_create_error; }
 
 static int destroy_impl(pgs_handle* h) {
@@ -147,7 +203,7 @@ static int destroy_impl(pgs_handle* h) {
     cudaFree(h->sx); cudaFree(h->sl_id); cudaFree(h->sl_p); cudaFree(h->sl_key);
     cudaFree(h->sh_key); cudaFree(h->sh_cnt); cudaFree(h->tables_dev);
     cudaFree(h->logits_stage); cudaFree(h->aux_dev); cudaFree(h->work_rows); cudaFree(h->work_count); cudaFree(h->tp_done); cudaFree(h->prof);
-    cudaFree(h->p1_done); cudaFree(h->faulted);
+    cudaFree(h->p1_done); cudaFree(h->faulted); cudaFree(h->wide_ws);
     if (h->aux_host) cudaFreeHost(h->aux_host);
     if (h->ev_step) cudaEventDestroy(h->ev_step);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -187,6 +243,7 @@ extern "C" int pgs_create(int device, uint32_t max_rows, uint32_t max_vocab, uin
         PGS_CUDA(nullptr, pgs::configure_general());
         PGS_CUDA(nullptr, pgs::configure_tp());
         PGS_CUDA(nullptr, pgs::configure_score());
+        PGS_CUDA(nullptr, pgs::configure_wide());
         PGS_CUDA(nullptr, cudaMalloc(&h->work_rows, (size_t)max_rows * sizeof(uint32_t)));
         PGS_CUDA(nullptr, cudaMalloc(&h->work_count, 2 * sizeof(uint32_t)));
         PGS_CUDA(nullptr, cudaMemsetAsync(h->work_count, 0, 2 * sizeof(uint32_t), h->stream));
@@ -198,7 +255,7 @@ extern "C" int pgs_create(int device, uint32_t max_rows, uint32_t max_vocab, uin
         PGS_CUDA(nullptr, cudaMemsetAsync(h->faulted, 0, 2 * sizeof(unsigned long long), h->stream));
         h->tp_timeouts = h->faulted + 1;
         h->stream_hash = pow2_at_least(2 * (max_history ? max_history : 1), 64);
-        if (h->stream_hash > (uint32_t)pgs::S_MAX_HASH) h->stream_hash = pgs::S_MAX_HASH;   // longer histories take the general kernel
+        if (h->stream_hash > (uint32_t)pgs::S_MAX_HASH) h->stream_hash = pgs::S_MAX_HASH;   // longer histories go on the work list
         h->stream_smem = pgs::stream_smem_bytes();
         PGS_CUDA(nullptr, pgs::configure_stream());
         PGS_CUDA(nullptr, pgs::stream_ctas_per_sm(&h->stream_ctas));
@@ -232,6 +289,8 @@ extern "C" int pgs_create(int device, uint32_t max_rows, uint32_t max_vocab, uin
         PGS_CUDA(nullptr, cudaMalloc(&h->sh_cnt, s * h->hash_cap * sizeof(uint32_t)));
         PGS_CUDA(nullptr, cudaMalloc(&h->tables_dev, sizeof h->tables_host));
         PGS_CUDA(nullptr, cudaMemsetAsync(h->tables_dev, 0, sizeof h->tables_host, h->stream));
+        const int rc_wide = wide_workspace(h);
+        if (rc_wide != PGS_OK) return rc_wide;
         // aux staging: per-row parameter and output arrays of a host-resident batch
         h->aux_bytes = (size_t)max_rows * 128 + (size_t)max_rows * max_history * 4 + 4096;
         PGS_CUDA(nullptr, cudaMalloc(&h->aux_dev, h->aux_bytes));
@@ -323,22 +382,20 @@ extern "C" int pgs_mask_table_free(pgs_handle* h, int32_t table_id) {
 
 namespace {
 
-// One step: the streaming row kernel serves every row it can and lists the others, which the general kernel then
-// processes.  In exact mode every row takes the
-// general kernel.
+// One step: the streaming row kernel serves every row it can and lists the others, which the wide kernel then processes.
+// In exact mode, and where no row is 16-byte aligned, every row goes to the wide kernel at once.
 int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
     const uint32_t rows = a.rows;
     const uint32_t grid = rows < h->slots ? rows : h->slots;
     a.faulted = h->faulted;
-    // Every step of a handle uses the same scratch, lists and counters: a step on another stream than the one before
-    // waits for that one to finish on the device.
-    if (stream != h->last_stream) {
-        PGS_CUDA(h, cudaEventRecord(h->ev_step, h->last_stream));
-        PGS_CUDA(h, cudaStreamWaitEvent(stream, h->ev_step, 0));
-        h->last_stream = stream;
-    }
-    if (h->exact || a.vocab > (uint32_t)pgs::S_MAX_VOCAB) {
-        PGS_CUDA(h, pgs::launch_general(a, grid, stream));
+    const int rc = order_steps(h, stream);
+    if (rc != PGS_OK) return rc;
+    const bool wide = !a.tp_records && a.vocab <= h->wide_vocab;   // (shard records and longer rows: the general kernel)
+    const uint32_t per = a.dtype == 0 ? 4u : 8u;
+    const bool aligned = ((uintptr_t)a.logits & 15u) == 0u && a.row_stride % per == 0u && a.vocab % per == 0u;
+    if (h->exact || a.vocab > (uint32_t)pgs::S_MAX_VOCAB || (wide && !aligned)) {
+        if (wide) PGS_CUDA(h, pgs::launch_wide(a, h->wide, h->slots, wide_grid(h, rows, a.vocab), stream));
+        else PGS_CUDA(h, pgs::launch_general(a, grid, stream));
         h->counters.kernel_launches += 1;
         return PGS_OK;
     }
@@ -362,7 +419,8 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
     pgs::RowArgs wl = a;
     wl.work_rows = h->work_rows;
     wl.work_count = h->work_count;
-    PGS_CUDA(h, pgs::launch_general(wl, grid < 32u ? grid : 32u, stream));
+    if (wide) PGS_CUDA(h, pgs::launch_wide(wl, h->wide, h->slots, wide_grid(h, rows, a.vocab), stream));
+    else PGS_CUDA(h, pgs::launch_general(wl, grid < 32u ? grid : 32u, stream));
     h->counters.kernel_launches += 2;
     return PGS_OK;
 }
@@ -797,9 +855,21 @@ extern "C" int pgs_log_softmax(pgs_handle* h, const float* logits, uint32_t rows
         return fail(h, PGS_ERR_INVALID, "pgs_log_softmax: need logits, row_stride >= vocab and an output");
     if (rows == 0) return PGS_OK;
     DeviceGuard g(h->device);
-    pgs::ScoreArgs a{logits, row_stride, rows, vocab, ids, out_gather, out_full, status};
-    const uint32_t grid = rows < (uint32_t)h->sm_count ? rows : (uint32_t)h->sm_count;
-    PGS_CUDA(h, pgs::launch_log_softmax(a, grid, cuda_stream ? (cudaStream_t)cuda_stream : h->stream));
+    cudaStream_t stream = cuda_stream ? (cudaStream_t)cuda_stream : h->stream;
+    if (vocab <= h->wide_vocab) {
+        const int rc = order_steps(h, stream);
+        if (rc != PGS_OK) return rc;
+        pgs::RowArgs a;
+        memset(&a, 0, sizeof a);
+        a.logits = logits; a.rows = rows; a.vocab = vocab; a.row_stride = row_stride; a.status = status; a.eos = -1;
+        pgs::WideLaunch l = h->wide;
+        l.score = 1u; l.ids = ids; l.out_gather = out_gather; l.out_full = out_full;
+        PGS_CUDA(h, pgs::launch_wide(a, l, h->slots, wide_grid(h, rows, vocab), stream));
+    } else {   // longer rows than the handle was made for: one CTA per row, no workspace
+        pgs::ScoreArgs a{logits, row_stride, rows, vocab, ids, out_gather, out_full, status};
+        const uint32_t grid = rows < (uint32_t)h->sm_count ? rows : (uint32_t)h->sm_count;
+        PGS_CUDA(h, pgs::launch_log_softmax(a, grid, stream));
+    }
     h->counters.kernel_launches += 1;
     return PGS_OK;
 }

@@ -19,7 +19,7 @@ constexpr int F_QUAD = 256;        // lists up to this length are ranked by coun
 // Working arrays of the finish, in shared memory: each holds CAP entries (CAP a power of two >= 512, the
 // longest list the owner hands in).
 template <int CAP>
-struct FinishArraysT {
+struct alignas(16) FinishArraysT {
     unsigned long long key[CAP];   // sort keys
     uint32_t sid[CAP];             // ids ascending
     float sp[CAP];                 // probabilities in id order (zeroed when dropped)
@@ -151,16 +151,14 @@ __device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint3
 
 
 // Candidates of one row -> token.  Called by every thread of a CTA of T threads (T >= F_QUAD, a multiple of 32)
-// with a barrier in front; cand_id / cand_x: the row's n <= F_MCAP candidates in any order (shared memory outside
-// of `f`); V: the full vocabulary size (the CDF walk falls through to V - 1, sampler.rs:54).  Ends with the row's
+// with a barrier in front; cand_id: the row's n <= F_MCAP candidates in any order, prob(j) their probabilities (memory
+// outside of `f`); V: the full vocabulary size (the CDF walk falls through to V - 1, sampler.rs:54).  Ends with the row's
 // outputs written; the caller needs a barrier before it reuses `f` or the candidate arrays.
-template <int T, class FA>
-__device__ __forceinline__ void cta_finish(FA& f, const unsigned long long* exp_tab, const RowArgs& a, uint32_t row,
-                                           uint32_t V, const uint32_t* cand_id, const float* cand_x, uint32_t n, float m, float t,
-                                           float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
+template <int T, class FA, class P>
+__device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32_t row, uint32_t V, const uint32_t* cand_id, P prob, uint32_t n,
+                                                 float m, float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
     static_assert(T >= F_QUAD && T % 32 == 0, "one thread per candidate of a short list");
     const int tid = threadIdx.x;
-    const bool norm = S > 1e-9f;
     if (tid == 0) f.n_live = 0u;
     if (n <= (uint32_t)F_QUAD) {
         // short list: every candidate counts the candidates in front of it, by id and by (probability descending,
@@ -169,8 +167,7 @@ __device__ __forceinline__ void cta_finish(FA& f, const unsigned long long* exp_
         float my_p = 0.0f;
         if ((uint32_t)tid < n) {
             my_id = cand_id[tid];
-            const float e = softmax_num(cand_x[tid], m, t, exp_tab);   // exact expf
-            my_p = norm ? fdiv(e, S) : e;
+            my_p = prob((uint32_t)tid);
             f.key[tid] = ((unsigned long long)f2u(my_p) << 32) | (unsigned long long)(0xffffffffu - my_id);   // p >= 0
         }
         __syncthreads();
@@ -192,8 +189,7 @@ __device__ __forceinline__ void cta_finish(FA& f, const unsigned long long* exp_
         for (uint32_t j = tid; j < npad; j += T) {
             unsigned long long k = ~0ull;   // the padding sorts to the end
             if (j < n) {
-                const float e = softmax_num(cand_x[j], m, t, exp_tab);
-                k = ((unsigned long long)cand_id[j] << 32) | f2u(norm ? fdiv(e, S) : e);
+                k = ((unsigned long long)cand_id[j] << 32) | f2u(prob(j));
             }
             f.key[j] = k;
         }
@@ -210,6 +206,18 @@ __device__ __forceinline__ void cta_finish(FA& f, const unsigned long long* exp_
         }
     }
     cta_finish_ranked<T, FA>(f, a, row, V, n, m, S, top_k, top_p, u01, amax, status);
+}
+
+// The same with the candidates' logits: exact probabilities exp((x - m) / t) / S.
+template <int T, class FA>
+__device__ __forceinline__ void cta_finish(FA& f, const unsigned long long* exp_tab, const RowArgs& a, uint32_t row,
+                                           uint32_t V, const uint32_t* cand_id, const float* cand_x, uint32_t n, float m, float t,
+                                           float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
+    const bool norm = S > 1e-9f;
+    cta_finish_probs<T>(f, a, row, V, cand_id, [&](uint32_t j) {
+        const float e = softmax_num(cand_x[j], m, t, exp_tab);   // exact expf
+        return norm ? fdiv(e, S) : e;
+    }, n, m, S, top_k, top_p, u01, amax, status);
 }
 
 }  // namespace pgs

@@ -41,7 +41,7 @@
 // Fidelity of this path: argmax, masks, penalties and candidate sets follow the reference bit for bit
 // (pagoda/src/engine.rs:1286-1314, pagoda/src/sampler.rs:28-150); candidate numerators use the exact expf.
 // Rows this kernel does not serve (top-k off or > 1024, more candidates than its buffers, histories beyond its
-// id -> count table, rows that are not 16-byte aligned) are appended to a work list for the general row kernel.
+// id -> count table, rows that are not 16-byte aligned) are appended to a work list for the wide kernel.
 #include <cuda_runtime.h>
 
 #include <cooperative_groups.h>
@@ -75,7 +75,7 @@ struct SRowCtl {
     float temp, freq, pres, rep, top_p, u01;
     float sc, sc_lo;        // log2(e) / max(temp, 1e-9) as a two-float sum
     uint32_t top_k, gflags, h0, nh;
-    uint32_t kind;          // 0 serve, 1 bad parameters, 2 defer to the general kernel
+    uint32_t kind;          // 0 serve, 1 bad parameters, 2 leave to the work list
 };
 
 // What the pass loops need to know about the row they work on.
@@ -952,7 +952,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 for (uint32_t k = 0; k < csize; k++) am_all = umin(am_all, sm.xam[k]);
                 amax = any ? am_all : 0u;
             }
-            if (defer_row) {   // (cluster mode only) a CTA could not index the history: the general kernel takes the row
+            if (defer_row) {   // (cluster mode only) a CTA could not index the history: the work list takes the row
                 if (writer) sl.work_rows[atomicAdd(sl.work_count, 1u)] = row;
                 continue;
             }

@@ -1,0 +1,1325 @@
+// Wide kernel: all SMs work on every listed row, bit-exact with the reference's serial folds.  It serves the exact mode, the
+// rows that the streaming kernel cannot (top-k off or > 1024, rows that are not 16-byte aligned, long candidate lists) and
+// log-softmax scoring.
+//
+// A launch is a sequence of phases with a grid barrier between two of them.  In "region" phases the warps of the grid share
+// all regions (512 consecutive logits) of all rows; in "row" phases a CTA does what is left of a row:
+//
+//   row     parameters; distinct history ids and what the penalties make of them
+//   region  sanity, mask, penalties; maximum and plain sum of the softmax numerators relative to it
+//   row     row maximum, argmax; estimate of the reference's running f32 sum at every region
+//   region  exact numerators; their increments of the running sum, in ulps of its binade
+//   row     the f32 left fold, exactly (see fold below)                                  -> S
+//   region  histogram of the probabilities                                               (rows with top-k or top-p)
+//   row     the bucket in which top-k and top-p end
+//   region  probabilities from that bucket upwards into a list, grouped by bucket
+//   row     short list: top-k, top-p, total and draw (pgs_finish.cuh).  Long list: the top-p fold over the buckets
+//   region  increments of the running total over the kept probabilities                  (what has no short list)
+//   row     total and inverse-CDF pick
+//
+// The fold (pagoda/src/sampler.rs:42, :99-113, :136-144): while the running value stays inside one binade, adding a
+// non-negative term is an integer addition in ulps which depends on the running value only where the term ends exactly on
+// half an ulp.  A region (or bucket) without such a tie whose running value provably stays inside one binade is one
+// integer, whatever the order; the few others are added in order, each lane of a warp a run of terms that is summarised by
+// its increments from an even and from an odd start (as in pgs_block.cuh).  Every summary is checked against the exact
+// running value before it is used, so the result is bit-identical to the serial fold.
+#include <cuda_runtime.h>
+
+#include "pgs_args.cuh"
+#include "pgs_block.cuh"
+#include "pgs_finish.cuh"
+#include "pgs_general.cuh"
+#include "pgs_wide.cuh"
+
+namespace pgs {
+
+constexpr int WNW = W_NT / 32;
+constexpr int WL = W_REGION / 32;        // logits per lane and region
+constexpr uint32_t W_NIL = 0xffffffffu;
+
+// 32 runs of terms, one per lane, ready to be added to a running value: lanes whose runs are estimated to begin in one
+// binade form a group, and each lane holds the increments from the group's first lane up to and including its own, for an
+// even and for an odd running value there.
+struct Runs {
+    uint32_t k;         // bits of the estimated binade's lower end (0: none)
+    uint32_t c0, c1;    // SEQ_SAT: leaves the binade
+    uint32_t head;      // first lane of the group; bit 31: nothing but zeros in this lane's run
+};
+
+struct alignas(16) WideSmem {
+    RowArgs a;                           // the launch's arguments, for the phases, which are functions of their own
+    WideLaunch l;
+    WideRow row;
+    unsigned long long exp_tab[32];
+    uint32_t red_u[WNW], red_v[WNW];
+    float red_f[WNW];
+    double red_d[WNW];
+    uint32_t last, found, n_serial, ok;
+    uint32_t rank, size, target;         // of the CTA among those that take part; arrivals at the barrier behind this one
+    float R;
+    float stage[WNW][W_REGION];          // per warp: a region in id order
+    float spare[W_REGION];
+    Runs runs[WNW][32];
+    uint32_t serial[W_MAX_REGIONS];      // segments that are added term by term
+    union {
+        struct {
+            uint2 seg[W_MAX_REGIONS];
+            float pre[W_MAX_REGIONS];
+            float start[W_MAX_REGIONS];  // exact running value at the segment's start
+        };
+        uint32_t hash[4 * W_MAX_HIST];   // ids, then counts
+        struct {
+            uint32_t bn[W_BUCKETS];      // long list: increments per bucket
+            float bs[W_BUCKETS];         // plain sums, then estimates of the running value
+            unsigned long long sort[W_SORT];
+        };
+        struct {
+            FinishArrays fin;
+            uint32_t cand_id[F_MCAP];
+            float cand_p[F_MCAP];
+        };
+        GeneralSmem general;
+    };
+};
+static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
+
+// ------------------------------------------------------------------------------------------------ grid barrier
+
+// The CTAs that take part are those that run when the first of them closes the list (at most one per SM fits; usually all
+// of the grid, but where another stream's kernel keeps SMs busy the launch does not depend on the rest, which leave at
+// once).  So a barrier never waits for a CTA that has not started, and the launch needs no cooperative attribute, which
+// costs 3 us and keeps the work-list pass from being set up early.  Waits have a limit all the same; when one runs out the
+// launch gives up.
+__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, uint32_t limit) {
+    for (uint32_t i = 0; (int32_t)(*(const volatile uint32_t*)p - target) < 0; i++) {
+        if (i > limit) return false;
+        __nanosleep(40);
+    }
+    return true;
+}
+constexpr uint32_t W_CLOSED = 0x80000000u;   // in sync[5], above the number of CTAs that have joined
+
+// Joins the launch; false: too late.
+__device__ __forceinline__ bool grid_join(WideSmem& sm, const WideLaunch& l) {
+    if (threadIdx.x == 0) sm.rank = atomicAdd(l.sync + 5, 1u);
+    __syncthreads();
+    return !(sm.rank & W_CLOSED);
+}
+
+__device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bool good = true;
+        __threadfence();
+        atomicAdd(l.sync, 1u);
+        if (sm.target == 0u) {   // the first barrier: how many take part?
+            if (sm.rank == 0u) {
+                wait_for(l.sync + 5, gridDim.x, 64u);
+                *(volatile uint32_t*)(l.sync + 6) = atomicOr(l.sync + 5, W_CLOSED);
+            } else good = wait_for(l.sync + 6, 1u, 1u << 23);
+            sm.size = *(volatile uint32_t*)(l.sync + 6);
+        }
+        sm.target += sm.size;
+        good = good && wait_for(l.sync, sm.target, 1u << 23);
+        if (!good) atomicAdd(l.sync + 1, 1u);
+        __threadfence();
+        sm.ok = good;
+    }
+    __syncthreads();
+    return sm.ok != 0u;
+}
+
+// ------------------------------------------------------------------------------------------------ a warp's region
+
+template <bool BF16, bool VEC> struct WLay {
+    static constexpr int ESZ = BF16 ? 2 : 4;
+    static constexpr int GE = VEC ? 16 / ESZ : 1;   // consecutive logits of a group
+    static constexpr int G = WL / GE;
+    static constexpr int GS = 32 * GE;
+    __device__ static __forceinline__ uint32_t off(uint32_t lane, uint32_t j) { return (j / GE) * GS + lane * GE + j % GE; }
+};
+
+// the lane's raw logits of region r (nv: logits of the region; zeros behind them)
+template <bool BF16, bool VEC>
+__device__ __forceinline__ void wload(float (&x)[WL], const char* rowp, uint32_t r, uint32_t nv) {
+    using L = WLay<BF16, VEC>;
+    const uint32_t lane = threadIdx.x & 31;
+    const char* p = rowp + (size_t)r * W_REGION * L::ESZ;
+#pragma unroll
+    for (int h = 0; h < L::G; h++) {
+        const uint32_t o = h * L::GS + lane * L::GE;
+        const bool in = o < nv;
+        if constexpr (VEC && !BF16) {
+            const float4 v = in ? __ldcg(reinterpret_cast<const float4*>(p + o * 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            x[4 * h] = v.x; x[4 * h + 1] = v.y; x[4 * h + 2] = v.z; x[4 * h + 3] = v.w;
+        } else if constexpr (VEC) {
+            const uint4 v = in ? __ldcg(reinterpret_cast<const uint4*>(p + o * 2)) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t u4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                x[h * 8 + 2 * u] = __uint_as_float(u4[u] << 16);
+                x[h * 8 + 2 * u + 1] = __uint_as_float(u4[u] & 0xffff0000u);
+            }
+        } else if constexpr (BF16) x[h] = in ? __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(p) + o) << 16) : 0.0f;
+        else x[h] = in ? __ldcg(reinterpret_cast<const float*>(p) + o) : 0.0f;
+    }
+}
+
+// raw -> processed logits: mask, history entries (values after penalties, mask and EOS fix), end of the row
+template <bool BF16, bool VEC>
+__device__ __forceinline__ void wprocess(float* buf, float (&x)[WL], const WideLaunch& l, uint32_t slot, const uint32_t* mw, uint32_t entries,
+                                         uint32_t r, uint32_t nv) {
+    using L = WLay<BF16, VEC>;
+    const uint32_t lane = threadIdx.x & 31;
+    if (mw) {   // warp-uniform
+        const uint32_t word = lane < 16u && lane * 32u < nv ? __ldg(mw + (size_t)r * (W_REGION / 32) + lane) : 0u;
+#pragma unroll
+        for (int h = 0; h < L::G; h++) {
+            const uint32_t o = h * L::GS + lane * L::GE, bits = __shfl_sync(FULL, word, o >> 5) >> (o & 31u);
+#pragma unroll
+            for (int c = 0; c < L::GE; c++)
+                if (!((bits >> c) & 1u)) x[h * L::GE + c] = -INFINITY;
+        }
+    }
+    if (nv < (uint32_t)W_REGION) {
+#pragma unroll
+        for (int j = 0; j < WL; j++)
+            if (L::off(lane, j) >= nv) x[j] = -INFINITY;
+    }
+    if (entries) {
+        const uint32_t* rs = l.rs + (size_t)slot * l.rs_stride + r;
+        const uint32_t e0 = __ldcg(rs), e1 = __ldcg(rs + 1);
+        if (e0 < e1) {
+#pragma unroll
+            for (int j = 0; j < WL; j++) buf[L::off(lane, j)] = x[j];
+            __syncwarp();
+            for (uint32_t e = e0 + lane; e < e1; e += 32)
+                buf[__ldcg(l.ent_id + (size_t)slot * (W_MAX_HIST + 32) + e) - r * W_REGION] = __ldcg(l.ent_xn + (size_t)slot * (W_MAX_HIST + 32) + e);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < WL; j++) x[j] = buf[L::off(lane, j)];
+            __syncwarp();
+        }
+    }
+}
+
+// the terms of a fold: softmax numerators (S <= 0), or the probabilities that are kept
+struct Terms {
+    float m, t, S;           // S > 0: probabilities, numerator / S when that is above the reference's epsilon
+    bool filter;
+    float p_thr;
+    uint32_t id_thr;
+};
+__device__ __forceinline__ float term_of(float x, uint32_t id, const Terms& f, const unsigned long long* tab) {
+    float v = softmax_num(x, f.m, f.t, tab);
+    if (f.S >= 0.0f) {
+        if (f.S > 1e-9f) v = fdiv(v, f.S);
+        if (f.filter && !(v > f.p_thr || (v == f.p_thr && id <= f.id_thr))) v = 0.0f;
+    }
+    return v;
+}
+
+// the terms of region r, from memory
+template <bool BF16, bool VEC>
+__device__ __forceinline__ void wterms(const unsigned long long* tab, float* buf, float (&x)[WL], const WideLaunch& l, const WideRow& w, uint32_t slot,
+                                       uint32_t V, uint32_t r, const Terms& f) {
+    using L = WLay<BF16, VEC>;
+    const uint32_t lane = threadIdx.x & 31, nv = min(V - r * W_REGION, (uint32_t)W_REGION);
+    wload<BF16, VEC>(x, w.rowp, r, nv);
+    wprocess<BF16, VEC>(buf, x, l, slot, w.mw, w.entries, r, nv);
+#pragma unroll
+    for (int j = 0; j < WL; j++) x[j] = term_of(x[j], r * W_REGION + L::off(lane, j), f, tab);
+}
+
+// ------------------------------------------------------------------------------------------------ the exact fold
+
+// Increments of the running value over this warp's terms (each lane's share), in ulps of the binade whose lower end has
+// the bits `kb`: one integer whatever the order.  {0, 0}: has to be added term by term (no binade given, a term too large
+// for it, or one that ends on half an ulp).  {0, 1}: nothing but zeros.
+__device__ __forceinline__ uint2 increments(const float (&x)[WL], uint32_t kb) {
+    float top = 0.0f;
+#pragma unroll
+    for (int j = 0; j < WL; j++) top = fmaxf(top, x[j]);
+    if (__all_sync(FULL, top == 0.0f)) return make_uint2(0u, 1u);
+    const float b0 = u2f(kb), b1 = u2f(kb + 1u);
+    uint32_t n = 0u, tie = 0u;
+#pragma unroll
+    for (int j = 0; j < WL; j++) {
+        const uint32_t i0 = f2u(fadd(b0, x[j])) - kb, i1 = f2u(fadd(b1, x[j])) - (kb + 1u);
+        n += i0;
+        tie |= i0 ^ i1;
+    }
+    const bool bad = kb == 0u || tie != 0u || !(top < b0) || n >= 0x01000000u;
+    if (__any_sync(FULL, bad)) return make_uint2(0u, 0u);
+    return make_uint2(__reduce_add_sync(FULL, n), kb);   // (the table keeps the sum below 2^24 ulps)
+}
+
+// v: this lane's run; R0: estimate of the running value at the first lane's run
+__device__ __forceinline__ Runs make_runs(const float (&v)[WL], float R0) {
+    const uint32_t lane = threadIdx.x & 31;
+    float c = 0.0f;
+#pragma unroll
+    for (int j = 0; j < WL; j++) c += v[j];
+    float inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    Runs s;
+    s.k = f2u(R0 + (inc - c)) & 0x7f800000u;
+    if (s.k == 0x7f800000u) s.k = 0u;
+    s.c0 = s.c1 = SEQ_SAT;
+    if (c == 0.0f) s.c0 = s.c1 = 0u;
+    else if (s.k) {
+        float a0 = u2f(s.k), a1 = u2f(s.k + 1u);
+#pragma unroll
+        for (int j = 0; j < WL; j++) { a0 = fadd(a0, v[j]); a1 = fadd(a1, v[j]); }
+        if ((f2u(a0) & 0x7f800000u) == s.k) s.c0 = f2u(a0) - s.k;
+        if ((f2u(a1) & 0x7f800000u) == s.k) s.c1 = f2u(a1) - (s.k + 1u);
+    }
+    const uint32_t before = __shfl_up_sync(FULL, s.k, 1);
+    const unsigned heads = __ballot_sync(FULL, lane == 0u || before != s.k);
+    s.head = 31u - __clz((int)(heads & (0xffffffffu >> (31u - lane))));
+    // compose(left, right)(p) = left_p + right_{(p + left_p) & 1}, inside the group
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t l0 = __shfl_up_sync(FULL, s.c0, o), l1 = __shfl_up_sync(FULL, s.c1, o);
+        if (lane >= s.head + (uint32_t)o) {
+            const uint32_t n0 = l0 + ((l0 & 1u) ? s.c1 : s.c0), n1 = l1 + (((l1 + 1u) & 1u) ? s.c1 : s.c0);
+            s.c0 = (l0 >= SEQ_SAT || n0 >= SEQ_SAT) ? SEQ_SAT : n0;
+            s.c1 = (l1 >= SEQ_SAT || n1 >= SEQ_SAT) ? SEQ_SAT : n1;
+        }
+    }
+    if (c == 0.0f) s.head |= 0x80000000u;
+    return s;
+}
+
+// Adds the runs to the exact running value R; one warp, the same result in all lanes.
+__device__ __forceinline__ float add_runs(float R, const Runs& s, const float (&v)[WL]) {
+    const uint32_t lane = threadIdx.x & 31, head = s.head & 31u;
+    uint32_t pos = 0u;
+#pragma unroll 1
+    while (pos < 32u) {
+        const uint32_t rb = f2u(R), d = (rb & 1u) ? s.c1 : s.c0;
+        // the group that begins here, as far as the running value stays in its binade
+        const bool fits = lane >= pos && head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u;
+        const unsigned ok = __ballot_sync(FULL, fits) >> pos;
+        uint32_t n = ~ok ? __ffs((int)~ok) - 1u : 32u;
+        if (n) {
+            if (n > 32u - pos) n = 32u - pos;
+            R = u2f(rb + __shfl_sync(FULL, d, (int)(pos + n - 1u)));
+            pos += n;
+            continue;
+        }
+        // zeros change nothing; otherwise the running value changes binade in this run, or the estimate missed it
+        const unsigned zero = __ballot_sync(FULL, (s.head >> 31) != 0u) >> pos;
+        if (zero & 1u) { pos += ~zero ? __ffs((int)~zero) - 1u : 32u; continue; }
+        float r = R;
+        if (lane == pos) {
+#pragma unroll
+            for (int j = 0; j < WL; j++) r = fadd(r, v[j]);
+        }
+        R = __shfl_sync(FULL, r, (int)pos);
+        pos++;
+    }
+    return R;
+}
+
+// the warp's terms, as a region holds them, into id order: lane k gets the terms k * WL ..
+template <class L>
+__device__ __forceinline__ void to_runs(float* buf, float (&v)[WL], const float (&x)[WL]) {
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < WL; j++) buf[L::off(lane, j)] = x[j];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < WL; j++) v[j] = buf[lane * WL + j];
+}
+
+// The exact left fold of a row's terms from the segments that the grid left in l.seg (estimates of the running value in
+// l.pre); the CTA.  Leaves the running value at every region's start in sm.start.
+template <bool BF16, bool VEC>
+__device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_t slot, uint32_t V, const Terms f) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_regions = (V + W_REGION - 1) / W_REGION;
+    const WideRow& row = sm.row;
+    __syncthreads();
+    if (tid == 0) sm.n_serial = 0u;
+    for (uint32_t r = tid; r < n_regions; r += W_NT) {
+        sm.seg[r] = __ldcg(l.seg + (size_t)slot * l.reg_stride + r);
+        sm.pre[r] = __ldcg(l.pre + (size_t)slot * l.reg_stride + r);
+    }
+    __syncthreads();
+    // segments to be added term by term, in order (one warp: there are few)
+    if (w == 0) {
+        uint32_t n = 0u;
+        for (uint32_t r0 = 0; r0 < n_regions; r0 += 32) {
+            const bool s = r0 + lane < n_regions && sm.seg[r0 + lane].y == 0u;
+            const unsigned b = __ballot_sync(FULL, s);
+            if (s) sm.serial[n + __popc(b & ((1u << lane) - 1u))] = r0 + lane;
+            n += __popc(b);
+        }
+        if (lane == 0) sm.n_serial = n;
+    }
+    __syncthreads();
+    const uint32_t n_serial = sm.n_serial;
+    float R = 0.0f;        // warp 0
+    uint32_t pos = 0u;
+    for (uint32_t b = 0; b < n_serial || b == 0u; b += WNW) {
+        if (b + w < n_serial) {
+            const uint32_t r = sm.serial[b + w], at = sm.seg[r].x;
+            float v[WL];
+            if (at) {   // the region phase has left the terms
+                const float4* t = reinterpret_cast<const float4*>(l.terms + ((size_t)slot * W_TERMS + at - 1u) * W_REGION) + lane * (WL / 4);
+#pragma unroll
+                for (int j = 0; j < WL / 4; j++) {
+                    const float4 q = __ldcg(t + j);
+                    v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+                }
+            } else {
+                float x[WL];
+                wterms<BF16, VEC>(sm.exp_tab, sm.stage[w], x, l, row, slot, V, r, f);
+                to_runs<WLay<BF16, VEC>>(sm.stage[w], v, x);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < WL; j++) sm.stage[w][j * 32 + lane] = v[j];
+            sm.runs[w][lane] = make_runs(v, sm.pre[r]);
+        }
+        __syncthreads();
+        if (w == 0) {
+            const uint32_t n = min(n_serial - min(b, n_serial), (uint32_t)WNW);
+            for (uint32_t q = 0; q <= n; q++) {
+                const uint32_t stop = q < n ? sm.serial[b + q] : b + WNW >= n_serial ? n_regions : pos;
+                while (pos < stop) {   // whole segments up to the next one that is not
+                    const uint2 sg = pos + lane < stop ? sm.seg[pos + lane] : make_uint2(0u, 1u);
+                    const uint32_t rb = f2u(R);
+                    const unsigned not_ok = ~__ballot_sync(FULL, sg.y == 1u || sg.y == (rb & 0x7f800000u));
+                    uint32_t cnt = not_ok ? __ffs((int)not_ok) - 1u : 32u;
+                    uint32_t inc = lane < cnt ? sg.x : 0u;
+                    const uint32_t own = inc;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                        if (lane >= (uint32_t)o) inc += t;
+                    }
+                    const unsigned over = __ballot_sync(FULL, (rb & 0x007fffffu) + inc >= 0x00800000u && own != 0u);
+                    if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
+                    if (cnt) {
+                        if (lane < cnt && pos + lane < stop) sm.start[pos + lane] = u2f(rb + inc - own);
+                        R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
+                        pos = min(pos + cnt, stop);
+                    } else {   // the estimate was not good enough for this one
+                        float x[WL], v[WL];
+                        wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, row, slot, V, pos, f);
+                        to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
+                        if (lane == 0) sm.start[pos] = R;
+                        R = add_runs(R, make_runs(v, R), v);
+                        pos++;
+                    }
+                }
+                if (q < n) {
+                    float v[WL];
+#pragma unroll
+                    for (int j = 0; j < WL; j++) v[j] = sm.stage[q][j * 32 + lane];
+                    if (lane == 0) sm.start[pos] = R;
+                    R = add_runs(R, sm.runs[q][lane], v);
+                    pos++;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) sm.R = R;
+    __syncthreads();
+    return sm.R;
+}
+
+// binade of a segment whose plain sum P begins at the estimate `pre` of the running value, 0 when it may change there.  The
+// plain sums overestimate the running value by up to a few 1e-4 (the small terms it drops).
+__device__ __forceinline__ uint32_t safe_binade(float pre, float P, float slack) {
+    const float lo = pre * (1.0f - slack), hi = (pre + P) * (1.0f + slack);
+    const uint32_t kb = f2u(lo) & 0x7f800000u;
+    return kb != 0u && kb == (f2u(hi) & 0x7f800000u) && hi < INFINITY && P * (1.0f + slack) < 0.999f * u2f(kb) ? kb : 0u;
+}
+
+// exclusive scan over the CTA (plain adds: estimates only); one barrier in front, one behind
+__device__ __forceinline__ float wscan_f32(WideSmem& sm, float v, float* total) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    __syncthreads();
+    if (lane == 31) sm.red_f[w] = inc;
+    __syncthreads();
+    const float x = sm.red_f[lane];
+    float xi = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(FULL, xi, o);
+        if (lane >= (uint32_t)o) xi += t;
+    }
+    *total = __shfl_sync(FULL, xi, 31);
+    return __shfl_sync(FULL, xi - x, (int)w) + (inc - v);
+}
+
+// Table of a row's regions from their plain sums P(r): estimates and binades for the next region phase.
+template <class F>
+__device__ __forceinline__ void make_table(WideSmem& sm, const WideLaunch& l, uint32_t slot, uint32_t n_regions, float slack, F P) {
+    float carry = 0.0f;
+    for (uint32_t r0 = 0; r0 < n_regions; r0 += W_NT) {
+        const uint32_t r = r0 + threadIdx.x;
+        const float p = r < n_regions ? P(r) : 0.0f;
+        float tot;
+        const float pre = carry + wscan_f32(sm, p, &tot);
+        if (r < n_regions) {
+            l.pre[(size_t)slot * l.reg_stride + r] = pre;
+            l.seg[(size_t)slot * l.reg_stride + r] = make_uint2(0u, safe_binade(pre, p, slack));
+        }
+        carry += tot;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ row phases
+
+__device__ __forceinline__ void wresult(const RowArgs& a, uint32_t row, uint32_t token, int status, int drew) {
+    a.token[row] = token;
+    a.status[row] = status;
+    if (a.drew) a.drew[row] = (uint8_t)drew;
+}
+// outcome of a row that draws nothing
+__device__ __forceinline__ void wresult_plain(const RowArgs& a, uint32_t row, int status, uint32_t amax, float m) {
+    wresult(a, row, amax, status, 0);
+    if (a.argmax) a.argmax[row] = amax;
+    if (a.row_max) a.row_max[row] = m;
+    if (a.sumexp) a.sumexp[row] = 0.0f;
+    if (a.total) a.total[row] = 0.0f;
+    if (a.n_kept) a.n_kept[row] = 0u;
+}
+__device__ __forceinline__ void wleave(const WideLaunch& l, uint32_t row) { l.left_rows[atomicAdd(l.left_count, 1u)] = row; }
+
+__device__ __forceinline__ void row_in(WideSmem& sm, const WideLaunch& l, uint32_t slot) {
+    __syncthreads();
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(l.row + slot);
+    if (threadIdx.x < sizeof(WideRow) / 4) reinterpret_cast<uint32_t*>(&sm.row)[threadIdx.x] = __ldcg(from + threadIdx.x);
+    __syncthreads();
+}
+__device__ __forceinline__ void row_out(WideSmem& sm, const WideLaunch& l, uint32_t slot) {
+    __syncthreads();
+    if (threadIdx.x < sizeof(WideRow) / 4)
+        reinterpret_cast<uint32_t*>(l.row + slot)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&sm.row)[threadIdx.x];
+}
+
+// Parameters (same rules as the other kernels), and the distinct history ids of the row grouped by region with the values
+// the chain sees there.
+template <bool BF16>
+__device__ __noinline__ void open_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot, uint32_t row) {
+    const uint32_t tid = threadIdx.x, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    __syncthreads();
+    if (tid == 0) {
+        WideRow& c = sm.row;
+        c.row = row;
+        c.rowp = (const char*)a.logits + (size_t)row * a.row_stride * (BF16 ? 2 : 4);
+        c.temp = l.score ? 1.0f : a.temperature ? a.temperature[row] : 0.0f;
+        c.top_k = a.top_k ? a.top_k[row] : 0u;
+        c.top_p = a.top_p ? a.top_p[row] : 1.0f;
+        c.freq = a.freq ? a.freq[row] : 0.0f;
+        c.pres = a.pres ? a.pres[row] : 0.0f;
+        c.rep = a.rep ? a.rep[row] : 1.0f;
+        c.u01 = a.uniform ? a.uniform[row] : 0.0f;
+        c.t = fmaxf(c.temp, 1e-9f);
+        bool bad = !finite_f(c.temp) || !finite_f(c.top_p) || !finite_f(c.freq) || !finite_f(c.pres) || !finite_f(c.rep) || !(c.rep > 0.0f) ||
+                   !finite_f(c.u01);
+        c.mw = nullptr;
+        c.gflags = 0u;
+        const int32_t mt = a.mask_table ? a.mask_table[row] : -1;
+        if (mt >= 0) {
+            const int32_t ms = a.mask_state ? a.mask_state[row] : 0;
+            if (mt >= MAX_TABLES || !a.tables[mt].live || ms < 0 || (uint32_t)ms >= a.tables[mt].n_states ||
+                (unsigned long long)a.tables[mt].words_per_state * 32ull < V) bad = true;
+            else {
+                c.mw = a.tables[mt].words + (size_t)ms * a.tables[mt].words_per_state;
+                c.gflags = a.tables[mt].flags[ms];
+            }
+        }
+        c.h0 = a.hist_offsets ? a.hist_offsets[row] : 0u;
+        const uint32_t h1 = a.hist_offsets ? a.hist_offsets[row + 1] : 0u;
+        c.nh = 0u;
+        if (h1 < c.h0 || h1 - c.h0 > a.max_history || (h1 > c.h0 && !a.hist_ids)) bad = true; else c.nh = h1 - c.h0;
+        if ((fabsf(c.freq) < 1e-6f && fabsf(c.pres) < 1e-6f) && c.rep == 1.0f) c.nh = 0u;
+        c.entries = 0u;
+        c.nonfinite = 0u;
+        c.n_terms = 0u;
+        c.state = WS_FIRST;
+        c.n_list = 0u; c.n_kept = 0u; c.p_thr = -1.0f; c.id_thr = 0u; c.cut = 0u; c.m = -INFINITY; c.S = 0.0f; c.amax = 0u;
+        if (bad) { wresult_plain(a, row, ROW_BAD_PARAM, 0u, -INFINITY); c.state = WS_DONE; }
+        else if (c.nh > (uint32_t)W_MAX_HIST) { wleave(l, row); c.state = WS_DONE; }
+    }
+    __syncthreads();
+    const WideRow& c = sm.row;
+    const bool fix = (c.gflags & 1u) && c.mw && a.eos >= 0 && (uint32_t)a.eos < V;   // engine.rs:1307-1312
+    if (c.state == WS_FIRST && (c.nh || fix)) {
+        uint32_t* rcnt = sm.serial;   // ids per region, then the scatter cursor
+        uint32_t H = 64;
+        while (H < 2u * (c.nh + 1u) && H < 2u * W_MAX_HIST) H <<= 1;
+        uint32_t *hkey = sm.hash, *hcnt = sm.hash + H;
+        for (uint32_t s = tid; s < 2u * H; s += W_NT) sm.hash[s] = s < H ? W_NIL : 0u;
+        for (uint32_t r = tid; r < n_regions; r += W_NT) rcnt[r] = 0u;
+        __syncthreads();
+        for (uint32_t j = tid; j < c.nh + (fix ? 1u : 0u); j += W_NT) {
+            const bool is_fix = j == c.nh;
+            const uint32_t id = is_fix ? (uint32_t)a.eos : __ldg(a.hist_ids + c.h0 + j);
+            if (id >= V) continue;   // engine.rs:1562
+            uint32_t s = (id * 2654435761u) & (H - 1u);
+            for (uint32_t probe = 0; probe < H; probe++) {
+                const uint32_t prev = atomicCAS(&hkey[s], W_NIL, id);
+                if (prev == W_NIL) atomicAdd(&rcnt[id / W_REGION], 1u);
+                if (prev == W_NIL || prev == id) { if (!is_fix) atomicAdd(&hcnt[s], 1u); break; }
+                s = (s + 1u) & (H - 1u);
+            }
+        }
+        __syncthreads();
+        uint32_t carry = 0u;
+        for (uint32_t r0 = 0; r0 < n_regions; r0 += W_NT) {
+            const uint32_t r = r0 + tid, lane = tid & 31, w = tid >> 5;
+            const uint32_t v = r < n_regions ? rcnt[r] : 0u;
+            uint32_t inc = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= (uint32_t)o) inc += t;
+            }
+            if (lane == 31) sm.red_u[w] = inc;
+            __syncthreads();
+            const uint32_t x = sm.red_u[lane];
+            const uint32_t before = carry + __reduce_add_sync(FULL, lane < w ? x : 0u) + inc - v;
+            carry += __reduce_add_sync(FULL, x);
+            if (r < n_regions) { l.rs[(size_t)slot * l.rs_stride + r] = before; rcnt[r] = before; }
+            __syncthreads();
+        }
+        if (tid == 0) { l.rs[(size_t)slot * l.rs_stride + n_regions] = carry; sm.row.entries = carry; }
+        const bool do_fp = !(fabsf(c.freq) < 1e-6f && fabsf(c.pres) < 1e-6f), do_pres = fabsf(c.pres) > 1e-6f, do_rep = c.rep != 1.0f;
+        for (uint32_t s = tid; s < H; s += W_NT) {
+            const uint32_t id = hkey[s];
+            if (id == W_NIL) continue;
+            float v = BF16 ? __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(c.rowp) + id) << 16)
+                           : __ldcg(reinterpret_cast<const float*>(c.rowp) + id);
+            const bool allowed = !c.mw || ((__ldg(c.mw + (id >> 5)) >> (id & 31u)) & 1u);
+            const uint32_t n = hcnt[s];
+            if (n) {
+                if (do_rep) v = v > 0.0f ? fdiv(v, c.rep) : fmul(v, c.rep);
+                if (do_fp) {
+                    v = fsub(v, fmul(c.freq, (float)n));
+                    if (do_pres) v = fsub(v, c.pres);
+                }
+            }
+            if (!allowed || !finite_f(v)) v = -INFINITY;   // an overflowed penalty counts as masked
+            if (fix && id == (uint32_t)a.eos && !finite_f(v)) v = 0.0f;
+            const uint32_t at = atomicAdd(&rcnt[id / W_REGION], 1u);
+            l.ent_id[(size_t)slot * (W_MAX_HIST + 32) + at] = id;
+            l.ent_xn[(size_t)slot * (W_MAX_HIST + 32) + at] = v;
+        }
+    }
+    if (c.state == WS_FIRST)
+        for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) l.hist[(size_t)slot * W_BUCKETS + b] = 0u;
+    row_out(sm, l, slot);
+}
+
+// Row maximum, argmax, and the table for the fold of the numerators.
+template <bool BF16, bool VEC>
+__device__ __noinline__ void maximum_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    row_in(sm, l, slot);
+    if (sm.row.state != WS_FIRST) return;
+    uint32_t k = 0u, rr = W_NIL;
+    for (uint32_t r = tid; r < n_regions; r += W_NT) {
+        const float2 v = __ldcg(l.reg + (size_t)slot * l.reg_stride + r);
+        sm.pre[r] = v.x; sm.start[r] = v.y;
+        const uint32_t kr = order_key(v.x);
+        if (kr > k) { k = kr; rr = r; }
+    }
+    const uint32_t wk = __reduce_max_sync(FULL, k), wr = __reduce_min_sync(FULL, k == wk ? rr : W_NIL);
+    if (lane == 0) { sm.red_u[w] = wk; sm.red_v[w] = wr; }
+    __syncthreads();
+    const uint32_t kk = sm.red_u[lane], gkey = __reduce_max_sync(FULL, kk);
+    const uint32_t rstar = __reduce_min_sync(FULL, kk == gkey ? sm.red_v[lane] : W_NIL);
+    const bool any = gkey != 0u;
+    const float m = any ? key_to_float(gkey) : -INFINITY;
+    if (w == 0 && any && !sm.row.nonfinite) {   // the lowest id that holds the maximum
+        float x[WL];
+        const uint32_t nv = min(V - rstar * W_REGION, (uint32_t)W_REGION);
+        wload<BF16, VEC>(x, sm.row.rowp, rstar, nv);
+        wprocess<BF16, VEC>(sm.spare, x, l, slot, sm.row.mw, sm.row.entries, rstar, nv);
+        uint32_t o = W_NIL;
+#pragma unroll
+        for (int j = WL - 1; j >= 0; j--)
+            if (x[j] == m) o = WLay<BF16, VEC>::off(lane, j);   // (a lane's logits are in id order)
+        o = __reduce_min_sync(FULL, o);
+        if (lane == 0) sm.row.amax = rstar * W_REGION + o;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        WideRow& c = sm.row;
+        c.m = m;
+        c.state = WS_DONE;
+        if (l.score) {
+            if (a.status) a.status[c.row] = c.nonfinite ? ROW_NONFINITE : ROW_OK;
+            if (c.nonfinite || !any) { if (l.out_gather) l.out_gather[c.row] = NAN; }   // the reference does not define scores for such rows
+            else c.state = WS_SUM;
+        } else if (c.nonfinite) {
+            wresult_plain(a, c.row, ROW_NONFINITE, 0u, -INFINITY);
+            if (a.faulted) atomicAdd(a.faulted, 1ull);
+        } else if (c.gflags & 2u) wresult_plain(a, c.row, ROW_DEAD, 0u, -INFINITY);
+        else if (c.temp < 1e-5f || !any) wresult_plain(a, c.row, any ? ROW_OK : ROW_EMPTY, any ? c.amax : 0u, m);
+        else c.state = WS_SUM;
+    }
+    __syncthreads();
+    if (sm.row.state == WS_SUM) {
+        const float sc = 1.44269504f / sm.row.t;
+        make_table(sm, l, slot, n_regions, 0.001953125f + 1e-7f * fabsf(m * sc), [&](uint32_t r) {
+            return sm.start[r] > 0.0f ? sm.start[r] * ex2_approx_ftz((sm.pre[r] - m) * sc) : 0.0f;
+        });
+    }
+    row_out(sm, l, slot);
+}
+
+__device__ __forceinline__ uint32_t bucket_of(float p) {
+    const int b = (int)(f2u(p) >> 15) - (87 << 8);
+    return b < 0 ? 0u : min((uint32_t)b, (uint32_t)W_BUCKETS - 1u);
+}
+__device__ __forceinline__ float bucket_floor(uint32_t b) { return b ? u2f((b + (87u << 8)) << 15) : 0.0f; }
+
+// The sum of the numerators; rows with top-k or top-p go on to the selection, others to the total.
+template <bool BF16, bool VEC>
+__device__ __noinline__ void sum_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+    const uint32_t V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    row_in(sm, l, slot);
+    if (sm.row.state != WS_SUM) return;
+    Terms f;
+    f.m = sm.row.m; f.t = sm.row.t; f.S = -1.0f; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+    const float S = resolve<BF16, VEC>(sm, l, slot, V, f);
+    if (threadIdx.x == 0) sm.row.n_terms = 0u;
+    const bool use_k = sm.row.top_k != 0u && sm.row.top_k < V, use_p = !(sm.row.top_p >= 1.0f);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        WideRow& c = sm.row;
+        c.S = S;
+        if (l.score) {   // sampler.rs:73-87
+            c.total = fmaxf(__double2float_rn(log((double)S)), 1.17549435e-38f);
+            c.state = l.out_full ? WS_TOTAL : WS_DONE;
+            if (l.ids && l.out_gather) {
+                const uint32_t id = l.ids[c.row];
+                float v = NAN;
+                if (id < V) {
+                    const float e = pgs_expf_tab(fsub(reinterpret_cast<const float*>(c.rowp)[id], c.m), sm.exp_tab);
+                    v = fsub(__double2float_rn(log((double)e)), c.total);
+                }
+                l.out_gather[c.row] = v;
+            }
+        } else c.state = use_k || use_p ? WS_SELECT : WS_TOTAL;
+        if (c.state == WS_SELECT) atomicAdd(l.sync + 2, 1u);
+        if (c.state == WS_TOTAL) atomicAdd(l.sync + 3, 1u);
+    }
+    __syncthreads();
+    if (sm.row.state == WS_TOTAL && !l.score) {
+        const float q = S > 1e-9f ? 1.0f / S : 1.0f;
+        make_table(sm, l, slot, n_regions, 0.001953125f, [&](uint32_t r) { return ((r + 1u < n_regions ? sm.start[r + 1u] : S) - sm.start[r]) * q; });
+    }
+    row_out(sm, l, slot);
+}
+
+// The lowest bucket that can matter: the one with the k-th largest probability, or the one in which the top-p fold ends (a
+// lower bound of the mass above it exceeds top-p by more than the fold can lose).  List positions for the buckets above.
+__device__ __noinline__ void select_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+    constexpr int PER = (W_BUCKETS + W_NT - 1) / W_NT;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab;
+    row_in(sm, l, slot);
+    if (sm.row.state != WS_SELECT) return;
+    uint32_t* hist = l.hist + (size_t)slot * W_BUCKETS;
+    const uint32_t k = sm.row.top_k;
+    const bool use_k = k != 0u && k < V, use_p = !(sm.row.top_p >= 1.0f);
+    uint32_t n[PER], own = 0u;
+    float mass = 0.0f;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+        n[u] = b >= 0 ? __ldcg(hist + b) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+        own += n[u];
+        if (b > 0) mass += (float)n[u] * bucket_floor(b);
+    }
+    if (tid == 0) { sm.last = 0u; sm.found = 0u; }
+    float all;
+    float above_mass = wscan_f32(sm, mass, &all);
+    uint32_t inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    if (lane == 31) sm.red_u[w] = inc;
+    __syncthreads();
+    const uint32_t x = sm.red_u[lane];
+    const uint32_t before = __reduce_add_sync(FULL, lane < w ? x : 0u) + inc - own;
+    const float goal = sm.row.top_p * 1.002f;
+    {
+        uint32_t above = before;
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+            if (b > 0) {
+                if (use_k && above < k && k <= above + n[u]) atomicMax(&sm.last, (uint32_t)b);
+                const float next = above_mass + (float)n[u] * bucket_floor(b);
+                if (use_p && above_mass < goal && next >= goal) atomicMax(&sm.found, (uint32_t)b);
+                above_mass = next;
+            }
+            above += n[u];
+        }
+    }
+    __syncthreads();
+    const uint32_t cut = umax(sm.last, sm.found);
+    {
+        uint32_t above = before;
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+            if (b >= (int)cut) {
+                hist[b] = above;
+                if (b == (int)cut) sm.row.n_list = above + n[u];
+            }
+            above += n[u];
+        }
+    }
+    if (tid == 0) sm.row.cut = cut | (use_k && sm.last == cut ? 0x80000000u : 0u);   // top bit: top-k ends in the cut bucket
+    row_out(sm, l, slot);
+}
+
+// bucket b of the row's list as sorted keys (probability descending, id ascending) in sm.sort; false when it is too long
+__device__ __forceinline__ bool sort_bucket(WideSmem& sm, const WideLaunch& l, uint32_t slot, uint32_t at, uint32_t n) {
+    if (n > (uint32_t)W_SORT) return false;
+    uint32_t pad = 32u;
+    while (pad < n) pad <<= 1;
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < pad; j += W_NT) {
+        unsigned long long key = ~0ull;
+        if (j < n) {
+            const unsigned long long v = __ldcg(l.list + (size_t)slot * l.list_stride + at + j);
+            key = ((unsigned long long)(~(uint32_t)(v >> 32)) << 32) | (uint32_t)v;
+        }
+        sm.sort[j] = key;
+    }
+    cta_bitonic_sort<W_NT>(sm.sort, pad);
+    return true;
+}
+
+// Top-k and top-p on the list.  A short list is finished here; a long one leaves the last kept (probability, id) and the
+// table for the fold of the kept probabilities.
+__device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    row_in(sm, l, slot);
+    if (sm.row.state != WS_SELECT) return;
+    const uint32_t n = sm.row.n_list, k = sm.row.top_k, cut = sm.row.cut & 0x7fffffffu, row = sm.row.row;
+    const bool use_k = k != 0u && k < V, use_p = !(sm.row.top_p >= 1.0f), k_ends = sm.row.cut != cut;
+    const unsigned long long* list = l.list + (size_t)slot * l.list_stride;
+    if (n <= (uint32_t)F_MCAP) {
+        for (uint32_t j = tid; j < n; j += W_NT) {
+            const unsigned long long v = __ldcg(list + j);
+            sm.cand_id[j] = (uint32_t)v; sm.cand_p[j] = u2f((uint32_t)(v >> 32));
+        }
+        __syncthreads();
+        cta_finish_probs<W_NT>(sm.fin, a, row, V, sm.cand_id, [&](uint32_t j) { return sm.cand_p[j]; }, n, sm.row.m, sm.row.S, use_k ? k : 0u,
+                               sm.row.top_p, sm.row.u01, sm.row.amax, ROW_OK);
+        __syncthreads();
+        if (tid == 0) sm.row.state = WS_DONE;
+        row_out(sm, l, slot);
+        return;
+    }
+    const uint32_t* hist = l.hist + (size_t)slot * W_BUCKETS;   // where bucket b ends in the list; it begins where b + 1 ends
+    float thr_k = 0.0f;
+    bool leave = false;
+    uint32_t n_live = n;
+    if (k_ends && k <= n) {
+        const uint32_t at = cut + 1u < (uint32_t)W_BUCKETS ? __ldcg(hist + cut + 1u) : 0u, nb = n - at;
+        leave = !sort_bucket(sm, l, slot, at, nb);
+        if (!leave) {
+            thr_k = u2f(~(uint32_t)(sm.sort[k - at - 1u] >> 32));
+            uint32_t mine = 0u;
+            for (uint32_t j = tid; j < nb; j += W_NT) mine += u2f(~(uint32_t)(sm.sort[j] >> 32)) >= thr_k;
+            mine = __reduce_add_sync(FULL, mine);
+            if (lane == 0) sm.red_u[w] = mine;
+            __syncthreads();
+            n_live = at + __reduce_add_sync(FULL, sm.red_u[lane]);
+        }
+    }
+    float p_thr = thr_k;
+    uint32_t id_thr = 0xffffffffu, n_kept = n_live;
+    if (use_p && !leave) {
+        __syncthreads();
+        for (uint32_t b = cut + tid; b < (uint32_t)W_BUCKETS; b += W_NT) { sm.bn[b] = 0u; sm.bs[b] = 0.0f; }
+        __syncthreads();
+        for (uint32_t j = tid; j < n; j += W_NT) {
+            const float p = u2f((uint32_t)(__ldcg(list + j) >> 32));
+            if (p >= thr_k) atomicAdd(&sm.bs[bucket_of(p)], p);
+        }
+        __syncthreads();
+        {   // plain sums -> the binade of the running value at each bucket
+            constexpr int PER = (W_BUCKETS + W_NT - 1) / W_NT;
+            float own = 0.0f, P[PER];
+#pragma unroll
+            for (int u = 0; u < PER; u++) {
+                const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+                P[u] = b >= (int)cut ? sm.bs[b] : 0.0f;
+                own += P[u];
+            }
+            float all;
+            float pre = wscan_f32(sm, own, &all);
+#pragma unroll
+            for (int u = 0; u < PER; u++) {
+                const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
+                if (b >= (int)cut) sm.bs[b] = u2f(safe_binade(pre, P[u], 0.001953125f));
+                pre += P[u];
+            }
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < n; j += W_NT) {
+            const float p = u2f((uint32_t)(__ldcg(list + j) >> 32));
+            if (!(p >= thr_k)) continue;
+            const uint32_t b = bucket_of(p), kb = f2u(sm.bs[b]);
+            if (kb == 0u) continue;
+            const uint32_t i0 = f2u(fadd(u2f(kb), p)) - kb, i1 = f2u(fadd(u2f(kb + 1u), p)) - (kb + 1u);
+            if (i0 != i1 || !(p < u2f(kb))) sm.bs[b] = 0.0f;   // to be added one by one
+            else atomicAdd(&sm.bn[b], i0);
+        }
+        // the fold over the buckets, highest first: warp 0 adds whole buckets until it meets one that is not, or the one in
+        // which top-p is reached; the CTA sorts that bucket and warp 0 adds its entries in order
+        float R = 0.0f;                              // warp 0
+        int b = W_BUCKETS - 1;
+        bool found = false;
+        for (;;) {
+            __syncthreads();
+            if (w == 0) {
+                bool stop = false;
+                while (b >= (int)cut && !stop) {
+                    const int mine = b - (int)lane;
+                    const uint32_t end = mine >= (int)cut ? __ldcg(hist + mine) : 0u;
+                    const uint32_t at = mine >= (int)cut && mine + 1 < W_BUCKETS ? __ldcg(hist + mine + 1) : 0u;
+                    const bool empty = mine < (int)cut || end == at;
+                    const uint32_t kb = empty ? 1u : f2u(sm.bs[mine]), rb = f2u(R);
+                    uint32_t inc = empty ? 0u : sm.bn[mine];
+                    const uint32_t own = inc;
+                    const unsigned bad = __ballot_sync(FULL, !(empty || (kb != 0u && kb == (rb & 0x7f800000u))));
+                    uint32_t cnt = bad ? __ffs((int)bad) - 1u : 32u;
+                    if (lane >= cnt) inc = 0u;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                        if (lane >= (uint32_t)o) inc += t;
+                    }
+                    // (the running value only grows: it reaches top-p in the first bucket behind which it has)
+                    const unsigned over = __ballot_sync(FULL, !empty && lane < cnt && ((rb & 0x007fffffu) + inc >= 0x00800000u || (own != 0u && u2f(rb + inc) >= sm.row.top_p)));
+                    if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
+                    if (cnt) R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
+                    b -= (int)cnt;
+                    stop = cnt < 32u;
+                }
+                if (lane == 0) sm.last = b >= (int)cut ? (uint32_t)b : W_NIL;
+            }
+            __syncthreads();
+            const uint32_t sb = sm.last;
+            if (sb == W_NIL) break;
+            const uint32_t end = __ldcg(hist + sb), at = sb + 1u < (uint32_t)W_BUCKETS ? __ldcg(hist + sb + 1u) : 0u, nb = end - at;
+            if (!sort_bucket(sm, l, slot, at, nb)) { leave = true; break; }
+            if (w == 0) {
+                uint32_t hit = W_NIL;
+                for (uint32_t j0 = 0; j0 < nb && hit == W_NIL; j0 += W_REGION) {
+                    float v[WL];
+#pragma unroll
+                    for (int j = 0; j < WL; j++) {
+                        const uint32_t q = j0 + lane * WL + j;
+                        const float p = q < nb ? u2f(~(uint32_t)(sm.sort[q] >> 32)) : 0.0f;
+                        v[j] = p >= thr_k ? p : 0.0f;
+                    }
+                    const float R1 = add_runs(R, make_runs(v, R), v);
+                    if (R1 >= sm.row.top_p) {   // in here: one lane looks for the entry
+                        if (lane == 0) {
+                            float r = R;
+                            uint32_t q = j0;
+                            for (; q < nb && q < j0 + W_REGION; q++) {
+                                const float p = u2f(~(uint32_t)(sm.sort[q] >> 32));
+                                r = fadd(r, p >= thr_k ? p : 0.0f);
+                                if (r >= sm.row.top_p) break;
+                            }
+                            hit = q;
+                        }
+                        hit = __shfl_sync(FULL, hit, 0);
+                    }
+                    R = R1;
+                }
+                if (lane == 0) sm.found = hit;
+            }
+            __syncthreads();
+            if (sm.found != W_NIL) {
+                found = true;
+                p_thr = u2f(~(uint32_t)(sm.sort[sm.found] >> 32));
+                id_thr = (uint32_t)sm.sort[sm.found];
+                n_kept = at + sm.found + 1u;
+                break;
+            }
+            b--;
+        }
+        // top-p was not reached although the list ends where it should have been: the list is too short for this row
+        if (!found && !leave && cut != 0u && !k_ends) leave = true;
+    }
+    __syncthreads();
+    if (leave) {
+        if (tid == 0) { wleave(l, row); sm.row.state = WS_DONE; }
+        row_out(sm, l, slot);
+        return;
+    }
+    for (uint32_t r = tid; r < n_regions; r += W_NT) sm.start[r] = 0.0f;
+    __syncthreads();
+    for (uint32_t j = tid; j < n; j += W_NT) {
+        const unsigned long long v = __ldcg(list + j);
+        const float p = u2f((uint32_t)(v >> 32));
+        if (p > p_thr || (p == p_thr && (uint32_t)v <= id_thr)) atomicAdd(&sm.start[(uint32_t)v / W_REGION], p);
+    }
+    __syncthreads();
+    make_table(sm, l, slot, n_regions, 0.001953125f, [&](uint32_t r) { return sm.start[r]; });
+    if (tid == 0) {
+        WideRow& c = sm.row;
+        c.p_thr = p_thr; c.id_thr = id_thr; c.n_kept = n_kept;
+        c.state = WS_TOTAL;
+        atomicAdd(l.sync + 3, 1u);
+    }
+    row_out(sm, l, slot);
+}
+
+__device__ __forceinline__ Terms kept_terms(const WideRow& c, uint32_t V) {
+    Terms f;
+    f.m = c.m; f.t = c.t; f.S = c.S;
+    f.filter = (c.top_k != 0u && c.top_k < V) || !(c.top_p >= 1.0f);
+    f.p_thr = c.p_thr; f.id_thr = c.id_thr;
+    return f;
+}
+
+// Total of the kept probabilities and the inverse-CDF pick.
+template <bool BF16, bool VEC>
+__device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    row_in(sm, l, slot);
+    if (sm.row.state != WS_TOTAL) return;
+    const Terms f = kept_terms(sm.row, V);
+    const float total = resolve<BF16, VEC>(sm, l, slot, V, f);
+    const float target = fmul(sm.row.u01, total);
+    if (tid == 0) sm.found = W_NIL;
+    __syncthreads();
+    if (total > 1e-9f)
+        for (uint32_t r = tid; r < n_regions; r += W_NT)
+            if (target < (r + 1u < n_regions ? sm.start[r + 1u] : total)) atomicMin(&sm.found, r);
+    __syncthreads();
+    const uint32_t row = sm.row.row, r = sm.found;
+    uint32_t token = sm.row.amax;
+    if (total > 1e-9f) token = V - 1u;   // (also when no running value exceeds the target, sampler.rs:54)
+    if (w == 0) {
+        if (r != W_NIL) {   // the running value exceeds the target in this region: one lane looks for the id
+            float x[WL], v[WL];
+            wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, sm.row, slot, V, r, f);
+            to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
+            if (lane == 0) {
+                float acc = sm.start[r];
+                const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
+                for (uint32_t j = 0; j < nv; j++) {
+                    acc = fadd(acc, sm.spare[j]);
+                    if (target < acc) { token = r * W_REGION + j; break; }
+                }
+            }
+        }
+        if (lane == 0) {
+            wresult(a, row, token, ROW_OK, total > 1e-9f ? 1 : 0);
+            if (a.argmax) a.argmax[row] = sm.row.amax;
+            if (a.row_max) a.row_max[row] = sm.row.m;
+            if (a.sumexp) a.sumexp[row] = sm.row.S;
+            if (a.total) a.total[row] = total;
+        }
+    }
+    if (a.n_kept || a.dump_ids || a.dump_probs) {   // diagnostics: the kept set in id order
+        uint32_t done = 0u;
+        for (uint32_t r0 = 0; r0 < n_regions; r0 += WNW) {
+            __syncthreads();
+            float x[WL], v[WL];
+            uint32_t n = 0u;
+            if (r0 + w < n_regions) {
+                wterms<BF16, VEC>(sm.exp_tab, sm.stage[w], x, l, sm.row, slot, V, r0 + w, f);
+                to_runs<WLay<BF16, VEC>>(sm.stage[w], v, x);
+#pragma unroll
+                for (int j = 0; j < WL; j++) n += v[j] > 0.0f;
+            }
+            uint32_t inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= (uint32_t)o) inc += t;
+            }
+            if (lane == 31) sm.red_u[w] = inc;
+            __syncthreads();
+            const uint32_t c = sm.red_u[lane];
+            uint32_t at = done + __reduce_add_sync(FULL, lane < w ? c : 0u) + inc - n;
+            done += __reduce_add_sync(FULL, c);
+            if (n) {
+#pragma unroll
+                for (int j = 0; j < WL; j++)
+                    if (v[j] > 0.0f) {
+                        if (at < a.dump_cap) {
+                            if (a.dump_ids) a.dump_ids[(size_t)row * a.dump_cap + at] = (r0 + w) * W_REGION + lane * WL + j;
+                            if (a.dump_probs) a.dump_probs[(size_t)row * a.dump_cap + at] = v[j];
+                        }
+                        at++;
+                    }
+            }
+        }
+        if (tid == 0 && a.n_kept) a.n_kept[row] = done;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ region phases
+
+enum : int { WP_FIRST = 0, WP_SUM, WP_HIST, WP_LIST, WP_TOTAL, WP_FULL };
+
+// One region phase: the warps of the grid take the regions of all rows of the chunk in turn (the histogram: sixteen regions
+// of a row per half of a CTA's warps, so that most counting happens in shared memory).
+template <bool BF16, bool VEC, int PHASE>
+__device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
+    using L = WLay<BF16, VEC>;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    float* buf = sm.stage[w];
+    for (uint32_t i = w * sm.size + sm.rank; i < n_rows * n_regions; i += sm.size * WNW) {
+        const uint32_t slot = i / n_regions, r = i - slot * n_regions, nv = min(V - r * W_REGION, (uint32_t)W_REGION);
+        const WideRow* rp = l.row + slot;
+        const uint32_t state = __ldcg(&rp->state);
+        WideRow c;
+        c.rowp = (const char*)__ldcg((const unsigned long long*)&rp->rowp);
+        c.mw = (const uint32_t*)__ldcg((const unsigned long long*)&rp->mw);
+        c.entries = __ldcg(&rp->entries);
+        float x[WL];
+        if (PHASE == WP_FIRST) {
+            if (state != WS_FIRST) continue;
+            wload<BF16, VEC>(x, c.rowp, r, nv);
+            uint32_t bad = 0u;
+#pragma unroll
+            for (int j = 0; j < WL; j++) bad |= !finite_f(x[j]);
+            wprocess<BF16, VEC>(buf, x, l, slot, c.mw, c.entries, r, nv);
+            float top = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < WL; j++) top = fmaxf(top, x[j]);
+            uint32_t key = f2u(top);
+            key = __reduce_max_sync(FULL, key ^ (((uint32_t)((int32_t)key >> 31)) | 0x80000000u));   // monotone; -inf lowest
+            const float wm = u2f((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), sc = 1.44269504f / __ldcg(&rp->t);
+            float s = 0.0f;
+            if (wm > -INFINITY) {
+#pragma unroll
+                for (int j = 0; j < WL; j++) s += ex2_approx_ftz((x[j] - wm) * sc);
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+            bad = __any_sync(FULL, bad);
+            if (lane == 0) {
+                l.reg[(size_t)slot * l.reg_stride + r] = make_float2(wm, s);
+                if (bad) l.row[slot].nonfinite = 1u;
+            }
+            continue;
+        }
+        if (state != (PHASE == WP_SUM ? WS_SUM : PHASE == WP_LIST ? WS_SELECT : WS_TOTAL)) continue;
+        c.m = __ldcg(&rp->m); c.t = __ldcg(&rp->t); c.S = __ldcg(&rp->S);
+        if (PHASE == WP_FULL) {   // the whole log-softmax vector
+            const float log_sum = __ldcg(&rp->total);
+            const uint32_t row = __ldcg(&rp->row);
+            wload<BF16, VEC>(x, c.rowp, r, nv);
+#pragma unroll
+            for (int j = 0; j < WL; j++) {
+                const uint32_t o = L::off(lane, j);
+                const float e = pgs_expf_tab(fsub(x[j], c.m), sm.exp_tab);
+                if (o < nv) l.out_full[(size_t)row * V + r * W_REGION + o] = fsub(__double2float_rn(log((double)e)), log_sum);
+            }
+            continue;
+        }
+        Terms f;
+        f.m = c.m; f.t = c.t; f.S = PHASE == WP_SUM ? -1.0f : c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+        if (PHASE == WP_TOTAL) {
+            c.top_k = __ldcg(&rp->top_k); c.top_p = __ldcg(&rp->top_p); c.p_thr = __ldcg(&rp->p_thr); c.id_thr = __ldcg(&rp->id_thr);
+            f = kept_terms(c, V);
+        }
+        wterms<BF16, VEC>(sm.exp_tab, buf, x, l, c, slot, V, r, f);
+        if (PHASE == WP_SUM || PHASE == WP_TOTAL) {
+            uint2* seg = l.seg + (size_t)slot * l.reg_stride + r;
+            uint2 out = increments(x, __ldcg(&seg->y));
+            if (out.y == 0u) {   // to be added term by term: the terms are left in id order, as far as there is room
+                if (lane == 0) out.x = atomicAdd(&l.row[slot].n_terms, 1u) + 1u;
+                out.x = __shfl_sync(FULL, out.x, 0);
+                if (out.x > (uint32_t)W_TERMS) out.x = 0u;
+                else {
+                    float* t = l.terms + ((size_t)slot * W_TERMS + out.x - 1u) * W_REGION;
+#pragma unroll
+                    for (int j = 0; j < WL; j++) t[L::off(lane, j)] = x[j];
+                }
+            }
+            if (lane == 0) *seg = out;
+        } else {   // WP_LIST
+            const uint32_t cut = __ldcg(&rp->cut) & 0x7fffffffu;
+#pragma unroll
+            for (int j = 0; j < WL; j++)
+                if (x[j] > 0.0f && bucket_of(x[j]) >= cut) {
+                    const uint32_t at = atomicAdd(l.hist + (size_t)slot * W_BUCKETS + bucket_of(x[j]), 1u);
+                    l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
+                }
+        }
+    }
+}
+
+template <bool BF16, bool VEC>
+__device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
+    const uint32_t tid = threadIdx.x, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
+    const uint32_t tiles = (n_regions + WNW - 1) / WNW;
+    for (uint32_t i = sm.rank; i < n_rows * tiles; i += sm.size) {   // CTA-uniform
+        const uint32_t slot = i / tiles, r = (i - slot * tiles) * WNW + w;
+        const WideRow* rp = l.row + slot;
+        if (__ldcg(&rp->state) != WS_SELECT) continue;
+        for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) sm.bn[b] = 0u;
+        __syncthreads();
+        if (r < n_regions) {
+            WideRow c;
+            c.rowp = (const char*)__ldcg((const unsigned long long*)&rp->rowp);
+            c.mw = (const uint32_t*)__ldcg((const unsigned long long*)&rp->mw);
+            c.entries = __ldcg(&rp->entries);
+            Terms f;
+            f.m = __ldcg(&rp->m); f.t = __ldcg(&rp->t); f.S = __ldcg(&rp->S); f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+            float x[WL];
+            wterms<BF16, VEC>(sm.exp_tab, sm.stage[w], x, l, c, slot, V, r, f);
+#pragma unroll
+            for (int j = 0; j < WL; j++) if (x[j] > 0.0f) atomicAdd(&sm.bn[bucket_of(x[j])], 1u);
+        }
+        __syncthreads();
+        for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT)
+            if (sm.bn[b]) atomicAdd(l.hist + (size_t)slot * W_BUCKETS + b, sm.bn[b]);
+        __syncthreads();
+    }
+}
+
+__device__ __noinline__ void leftover(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slots) {
+    const uint32_t n = *(volatile uint32_t*)l.left_count;
+    slots = min(slots, sm.size);
+    if (n == 0u || sm.rank >= slots) return;
+    __syncthreads();
+    if (threadIdx.x < 32u) sm.general.exp_tab[threadIdx.x] = kExp2TableDev[threadIdx.x];
+    __syncthreads();
+    general_rows(a, sm.general, sm.rank, slots, n, l.left_rows);
+}
+
+template <bool BF16, bool VEC>
+__global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const WideLaunch l_, uint32_t slots) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    WideSmem& sm = *reinterpret_cast<WideSmem*>(smem_raw);
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
+    const uint32_t tid = threadIdx.x;
+    if (a_.work_rows) cudaGridDependencySynchronize();   // launched ahead of the end of the kernel that fills the list
+    const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
+    if (n_work == 0u) return;   // the usual case of the work-list pass
+    if (tid == 0) { sm.a = a_; sm.target = 0u; }
+    if (tid == 32u) sm.l = l_;
+    if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
+    __syncthreads();
+    bool ok = grid_join(sm, l);
+    for (uint32_t c0 = 0; c0 < n_work && ok; c0 += W_CHUNK) {
+        const uint32_t n = min(n_work - c0, (uint32_t)W_CHUNK);
+        const auto open = [&](uint32_t s) { open_row<BF16>(sm, a, l, s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
+        uint32_t s = sm.rank;
+        if (c0 == 0u) {   // (how many take part is not known yet)
+            if (s < n) open(s);
+            if (!(ok = grid_sync(sm, l))) break;
+            s += sm.size;
+        }
+        if (c0 || sm.size < n) {
+            for (; s < n; s += sm.size) open(s);
+            if (!(ok = grid_sync(sm, l))) break;
+        }
+        region_phase<BF16, VEC, WP_FIRST>(sm, a, l, n);
+        if (!(ok = grid_sync(sm, l))) break;
+        for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(sm, a, l, s);
+        if (sm.rank == 0u && tid == 0) { l.sync[2] = 0u; l.sync[3] = 0u; }
+        if (!(ok = grid_sync(sm, l))) break;
+        region_phase<BF16, VEC, WP_SUM>(sm, a, l, n);
+        if (!(ok = grid_sync(sm, l))) break;
+        for (uint32_t s = sm.rank; s < n; s += sm.size) sum_row<BF16, VEC>(sm, a, l, s);
+        if (!(ok = grid_sync(sm, l))) break;
+        if (l.score) {
+            if (l.out_full) region_phase<BF16, VEC, WP_FULL>(sm, a, l, n);
+        } else {
+            if (*(volatile uint32_t*)(l.sync + 2)) {   // (the same for all CTAs)
+                hist_phase<BF16, VEC>(sm, a, l, n);
+                if (!(ok = grid_sync(sm, l))) break;
+                for (uint32_t s = sm.rank; s < n; s += sm.size) select_row(sm, a, l, s);
+                if (!(ok = grid_sync(sm, l))) break;
+                region_phase<BF16, VEC, WP_LIST>(sm, a, l, n);
+                if (!(ok = grid_sync(sm, l))) break;
+                for (uint32_t s = sm.rank; s < n; s += sm.size) choose_row(sm, a, l, s);
+                if (!(ok = grid_sync(sm, l))) break;
+            }
+            if (*(volatile uint32_t*)(l.sync + 3)) {
+                region_phase<BF16, VEC, WP_TOTAL>(sm, a, l, n);
+                if (!(ok = grid_sync(sm, l))) break;
+                for (uint32_t s = sm.rank; s < n; s += sm.size) total_row<BF16, VEC>(sm, a, l, s);
+            }
+        }
+        if (!(ok = grid_sync(sm, l))) break;   // the chunk's workspace is free
+    }
+    if (ok && !l.score) leftover(sm, a, l, slots);
+    // the last CTA of the grid to leave resets the counters and empties the lists
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(l.sync + 4, 1u) == gridDim.x - 1u) {
+            l.sync[0] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
+            *l.left_count = 0u;
+            if (a.work_rows) *a.work_count = 0u;
+        }
+    }
+}
+
+template <bool BF16, bool VEC>
+static cudaError_t wide_configure_one() {
+    return cudaFuncSetAttribute(wide_kernel<BF16, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WideSmem));
+}
+
+cudaError_t configure_wide() {
+    cudaError_t e = wide_configure_one<false, true>();
+    if (e == cudaSuccess) e = wide_configure_one<true, true>();
+    if (e == cudaSuccess) e = wide_configure_one<false, false>();
+    if (e == cudaSuccess) e = wide_configure_one<true, false>();
+    return e;
+}
+
+// `grid` CTAs, at most one per SM; a.work_rows: the work-list pass behind another kernel (programmatic stream serialization)
+cudaError_t launch_wide(const RowArgs& a, const WideLaunch& l, uint32_t slots, uint32_t grid, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(W_NT, 1, 1);
+    cfg.dynamicSmemBytes = sizeof(WideSmem);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = a.work_rows ? 1 : 0;
+    const uint32_t ge = a.dtype ? 8u : 4u;
+    const bool vec = ((uintptr_t)a.logits & 15u) == 0u && a.row_stride % ge == 0u && a.vocab % ge == 0u;
+    if (vec) return a.dtype ? cudaLaunchKernelEx(&cfg, wide_kernel<true, true>, a, l, slots) : cudaLaunchKernelEx(&cfg, wide_kernel<false, true>, a, l, slots);
+    return a.dtype ? cudaLaunchKernelEx(&cfg, wide_kernel<true, false>, a, l, slots) : cudaLaunchKernelEx(&cfg, wide_kernel<false, false>, a, l, slots);
+}
+
+}  // namespace pgs

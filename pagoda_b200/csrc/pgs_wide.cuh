@@ -1,0 +1,60 @@
+// Workspace and launch block of the wide kernel (pgs_wide.cu), shared with the host launcher.
+#pragma once
+
+#include <stdint.h>
+
+#include "pgs_args.cuh"
+
+namespace pgs {
+
+constexpr int W_NT = 1024;              // threads per CTA, one CTA per SM
+constexpr int W_REGION = 512;           // consecutive logits of one warp
+constexpr int W_MAX_VOCAB = 1 << 20;
+constexpr int W_MAX_REGIONS = W_MAX_VOCAB / W_REGION;
+constexpr int W_MAX_HIST = 2048;
+constexpr int W_CHUNK = 64;             // rows in flight together: what the workspace is sized for
+constexpr int W_BUCKETS = 41 * 256;     // probabilities by exponent (2^-40 .. 1) and eight mantissa bits
+constexpr int W_TERMS = 64;             // segments of a row whose terms the region phase leaves for the fold
+constexpr int W_SORT = 4096;            // entries of a bucket that one CTA sorts
+
+// One row of the chunk.
+struct WideRow {
+    const char* rowp;
+    const uint32_t* mw;
+    float temp, t, freq, pres, rep, top_p, u01;
+    uint32_t top_k, gflags, h0, nh, row;
+    uint32_t entries;        // history entries (and EOS fix) of the row, grouped by region
+    uint32_t nonfinite;      // set by the first pass
+    uint32_t state;          // WS_*
+    float m, S, total;
+    uint32_t amax;
+    uint32_t cut, n_list;    // entries in buckets >= cut
+    uint32_t n_terms;        // segments whose terms are in WideLaunch::terms
+    float p_thr;             // kept: p > p_thr, or p == p_thr and id <= id_thr
+    uint32_t id_thr, n_kept;
+};
+enum : uint32_t { WS_FIRST = 0u, WS_SUM = 1u, WS_SELECT = 2u, WS_TOTAL = 3u, WS_DONE = 4u };
+
+struct WideLaunch {
+    WideRow* row;               // [W_CHUNK]
+    float2* reg;                // [W_CHUNK][n_regions]: a region's maximum, its plain sum
+    uint2* seg;                 // [W_CHUNK][n_regions]: increments in ulps, binade (0: add term by term)
+    float* pre;                 // [W_CHUNK][n_regions]: estimate of the running value at the region's start
+    float* terms;               // [W_CHUNK][W_TERMS][W_REGION]: terms of segments that are added one by one
+    uint32_t* ent_id;           // [W_CHUNK][W_MAX_HIST + 32]
+    float* ent_xn;
+    uint32_t* rs;               // [W_CHUNK][n_regions + 1]
+    uint32_t* hist;             // [W_CHUNK][W_BUCKETS]: counts, then list positions
+    unsigned long long* list;   // [W_CHUNK][list_stride] (the general kernel's sort buffer): probability bits and id
+    uint32_t* sync;             // [0] barrier arrivals, [1] lost waits, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    uint32_t reg_stride, rs_stride, list_stride;
+    uint32_t* left_rows;        // rows left to the general kernel
+    uint32_t* left_count;
+    // log-softmax scoring in place of sampling (score != 0)
+    uint32_t score;
+    const uint32_t* ids;
+    float* out_gather;
+    float* out_full;
+};
+
+}  // namespace pgs
