@@ -419,7 +419,13 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
     pgs::RowArgs wl = a;
     wl.work_rows = h->work_rows;
     wl.work_count = h->work_count;
-    if (wide) PGS_CUDA(h, pgs::launch_wide(wl, h->wide, h->slots, wide_grid(h, rows, a.vocab), stream));
+    if (wide) {
+        // A CTA of the wide kernel fits on no SM that still runs the row kernel.  Where a small batch leaves most SMs free,
+        // the pass takes only those, and is in place before the rows are done.
+        const uint32_t busy = rows * csize, want = wide_grid(h, rows, a.vocab), sms = (uint32_t)h->sm_count;
+        const uint32_t room = csize > 1u && busy <= sms / 2u ? sms - busy : sms;
+        PGS_CUDA(h, pgs::launch_wide(wl, h->wide, h->slots, want < room ? want : room, stream));
+    }
     else PGS_CUDA(h, pgs::launch_general(wl, grid < 32u ? grid : 32u, stream));
     h->counters.kernel_launches += 2;
     return PGS_OK;

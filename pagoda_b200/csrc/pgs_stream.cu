@@ -686,6 +686,9 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
     if (CL) { crank = cg::this_cluster().block_rank(); csize = cg::this_cluster().num_blocks(); }
     const uint32_t first_row = CL ? blockIdx.x / csize : blockIdx.x, row_step = CL ? gridDim.x / csize : gridDim.x;
     const uint32_t tail_owner = n_full % csize;   // the CTA that takes the ragged piece
+    // set up while the kernel before this one drains; the pass over the work list is set up in the same way behind this one
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     if (tid == PREP_TID && first_row < a.rows) sprepare_row<BF16>(a, sl, first_row, sm.ctl[0]);
     long long tick_ = clock64();
     uint32_t it = 0;
@@ -1165,22 +1168,23 @@ cudaError_t stream_max_clusters(int csize, int* out) {
 
 // csize == 1: one CTA per row, `grid` CTAs.  csize > 1: `grid` clusters of csize CTAs, one cluster per row at a time.
 cudaError_t launch_stream(const RowArgs& a, const StreamLaunch& sl, uint32_t grid, uint32_t csize, cudaStream_t stream) {
-    if (csize <= 1u) {
-        if (a.dtype == 0) stream_row_kernel<false, false><<<grid, SNT, sizeof(StreamSmem), stream>>>(a, sl);
-        else stream_row_kernel<true, false><<<grid, SNT, sizeof(StreamSmem), stream>>>(a, sl);
-        return cudaGetLastError();
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid * csize, 1, 1);
     cfg.blockDim = dim3(SNT, 1, 1);
     cfg.dynamicSmemBytes = sizeof(StreamSmem);
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    if (a.dtype == 0) return cudaLaunchKernelEx(&cfg, stream_row_kernel<false, true>, a, sl);
-    return cudaLaunchKernelEx(&cfg, stream_row_kernel<true, true>, a, sl);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = csize; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = csize > 1u ? 2 : 1;
+    if (csize > 1u) {
+        if (a.dtype == 0) return cudaLaunchKernelEx(&cfg, stream_row_kernel<false, true>, a, sl);
+        return cudaLaunchKernelEx(&cfg, stream_row_kernel<true, true>, a, sl);
+    }
+    if (a.dtype == 0) return cudaLaunchKernelEx(&cfg, stream_row_kernel<false, false>, a, sl);
+    return cudaLaunchKernelEx(&cfg, stream_row_kernel<true, false>, a, sl);
 }
 
 }  // namespace pgs
