@@ -16,10 +16,11 @@ namespace pgs {
 constexpr int F_MCAP = 2048;       // longest candidate list (a power of two)
 constexpr int F_QUAD = 256;        // lists up to this length are ranked by counting, longer ones by sorting
 
-// Working arrays of the finish, in shared memory: each holds CAP entries (CAP a power of two >= 512, the
-// longest list the owner hands in).
+// Working arrays of the finish, in shared memory: each holds CAP entries (CAP a power of two, at least the CTA's threads:
+// the longest list the owner hands in).
 template <int CAP>
 struct alignas(16) FinishArraysT {
+    static constexpr int CAPACITY = CAP;
     unsigned long long key[CAP];   // sort keys
     uint32_t sid[CAP];             // ids ascending
     float sp[CAP];                 // probabilities in id order (zeroed when dropped)
@@ -72,52 +73,93 @@ __device__ __forceinline__ int warp_find(const float* pre, int n, int mode, floa
     return -1;
 }
 
-// Ascending bitonic sort of n_pad (a power of two) 64-bit keys in shared memory by a CTA of T threads.
-template <int T>
-__device__ __forceinline__ void cta_bitonic_sort(unsigned long long* keys, uint32_t n_pad) {
-    const uint32_t tid = threadIdx.x;
-    __syncthreads();
-    for (uint32_t k = 2; k <= n_pad; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = tid; i < n_pad / 2; i += T) {   // the i-th pair of this step
-                const uint32_t lo = ((i & ~(j - 1u)) << 1) | (i & (j - 1u)), hi = lo | j;
-                const unsigned long long a = keys[lo], b = keys[hi];
-                const bool up = (lo & k) == 0u;
-                if ((a > b) == up) { keys[lo] = b; keys[hi] = a; }
+// How many of the n ranked probabilities the top-p walk keeps (sampler.rs:130-150); one warp.  One lane adds, and stops
+// where top-p is reached.
+__device__ __forceinline__ uint32_t warp_top_p(const float* p, uint32_t n, float top_p) {
+    uint32_t keep = n;
+    if (!(top_p >= 1.0f) && (threadIdx.x & 31) == 0) {
+        float acc = 0.0f;
+#pragma unroll 1
+        for (uint32_t j0 = 0; j0 < n; j0 += 8) {
+            const float4 lo4 = *reinterpret_cast<const float4*>(p + j0), hi4 = *reinterpret_cast<const float4*>(p + j0 + 4);
+            const float x[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+            float pre[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) pre[u] = acc = fadd(acc, x[u]);
+            if (acc >= top_p || j0 + 8 >= n) {   // (the running value never falls, but entries behind n are not probabilities)
+#pragma unroll
+                for (int u = 7; u >= 0; u--)
+                    if (j0 + u < n && pre[u] >= top_p) keep = j0 + u + 1;
+                if (keep < n) break;
             }
+        }
+    }
+    return __shfl_sync(FULL, keep, 0);
+}
+
+// Ascending bitonic sort of T * E 64-bit keys by a CTA of T threads: thread t holds the elements t * E .. t * E + E - 1.
+// Partners in one thread or one warp are compared in registers; only what crosses warps goes through `buf` (shared memory,
+// T * E keys) and barriers: ten exchanges whatever the length up to 2048 keys of 512 threads, where a sort that keeps the
+// keys in shared memory has 66 steps with a barrier each (2048 candidates, both sorts of a row: 62 us, now 9).
+template <int T, int E>
+__device__ __forceinline__ void cta_sort(unsigned long long (&v)[E], unsigned long long* buf) {
+    const uint32_t tid = threadIdx.x;
+    const auto keep = [&](unsigned long long& mine, unsigned long long other, uint32_t i, uint32_t j, uint32_t k) {
+        const bool lower = (i & j) == 0u, up = (i & k) == 0u;
+        if ((other < mine) == (lower == up)) mine = other;   // (keys are distinct, or equal ones are alike)
+    };
+#pragma unroll 1
+    for (uint32_t k = 2; k <= (uint32_t)(T * E); k <<= 1) {
+        uint32_t j = k >> 1;
+#pragma unroll 1
+        for (; j >= 32u * E; j >>= 1) {
+#pragma unroll
+            for (int e = 0; e < E; e++) buf[e * T + tid] = v[e];
             __syncthreads();
+#pragma unroll
+            for (int e = 0; e < E; e++) keep(v[e], buf[e * T + (tid ^ (j / E))], tid * E + e, j, k);
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (; j >= (uint32_t)E; j >>= 1) {
+#pragma unroll
+            for (int e = 0; e < E; e++) keep(v[e], __shfl_xor_sync(FULL, v[e], (int)(j / E)), tid * E + e, j, k);
+        }
+#pragma unroll
+        for (int jj = E / 2; jj >= 1; jj >>= 1) {
+            if ((uint32_t)jj >= k) continue;
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                if (!(e & jj)) {
+                    const bool up = ((tid * E + e) & k) == 0u;
+                    const unsigned long long x = v[e], y = v[e | jj];
+                    if ((x > y) == up) { v[e] = y; v[e | jj] = x; }
+                }
         }
     }
 }
+// The same for n <= LIMIT keys in shared memory (`keys`: room for the next power of two, at least T), in place; the keys
+// behind n are overwritten with ones that sort to the end.  Barriers in front and behind.
+template <int T, int LIMIT, int E = 1>
+__device__ __forceinline__ void cta_sort_shared(unsigned long long* keys, uint32_t n) {
+    if constexpr (T * E < LIMIT)
+        if (n > (uint32_t)(T * E)) { cta_sort_shared<T, LIMIT, 2 * E>(keys, n); return; }
+    unsigned long long v[E];
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] = threadIdx.x * E + e < n ? keys[threadIdx.x * E + e] : ~0ull;
+    __syncthreads();
+    cta_sort<T, E>(v, keys);
+#pragma unroll
+    for (int e = 0; e < E; e++) keys[threadIdx.x * E + e] = v[e];
+    __syncthreads();
+}
 
-// Second half of the finish, from ranked candidates: f.sid / f.sp hold the n candidates in id order, f.rp / f.rpos
-// the same by (probability descending, id ascending), f.n_live is zero.  Called by every thread; ends with the row's
-// outputs written.
-template <int T, class FA>
-__device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, float m,
-                                                  float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
-    const int tid = threadIdx.x, lane = tid & 31;
-    __syncthreads();
-    {   // top-k: every tie at the k-th probability survives; entries with zero probability never matter
-        const float thr = (top_k != 0u && top_k <= n) ? f.rp[top_k - 1] : 0.0f;
-        for (uint32_t j = tid; j < n; j += T) {
-            const bool live = f.rp[j] >= thr && f.rp[j] > 0.0f;
-            const bool next_live = j + 1 < n && f.rp[j + 1] >= thr && f.rp[j + 1] > 0.0f;
-            if (live && !next_live) f.n_live = j + 1;
-        }
-    }
-    __syncthreads();
-    if (tid >= 32) return;
-    // one warp: top-p walk in ranked order, then total and inverse-CDF pick in id order
-    const uint32_t n_live = f.n_live;
-    uint32_t keep = n_live;
-    if (!(top_p >= 1.0f) && n_live > 0) {
-        warp_prefix(f.rp, (int)n_live, f.fp);
-        const int found = warp_find(f.fp, (int)n_live, SEQ_FIND_GE, top_p);
-        if (found >= 0) keep = (uint32_t)found + 1;
-    }
-    for (uint32_t j = keep + lane; j < n; j += 32) f.sp[f.rpos[j]] = 0.0f;
-    __syncwarp();
+// Total and inverse-CDF pick of the n entries in f.sid / f.sp (id order), and the row's outputs; one warp.
+template <class FA>
+__device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, float m, float S, float u01, uint32_t amax,
+                                            int status) {
+    const int lane = threadIdx.x & 31;
     const float total = warp_prefix(f.sp, (int)n, f.fp);
     int pick = -1;
     if (total > 1e-9f) pick = warp_find(f.fp, (int)n, SEQ_FIND_GT, fmul(u01, total));
@@ -149,6 +191,36 @@ __device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint3
     }
 }
 
+// Entries that survive top-k, from ranked probabilities f.rp: every tie at the k-th probability survives; entries with zero
+// probability never matter.  f.n_live is zero.  Every thread; barriers in front and behind.
+template <int T, class FA>
+__device__ __forceinline__ uint32_t cta_top_k(FA& f, uint32_t n, uint32_t top_k) {
+    const int tid = threadIdx.x;
+    __syncthreads();
+    const float thr = (top_k != 0u && top_k <= n) ? f.rp[top_k - 1] : 0.0f;
+    for (uint32_t j = tid; j < n; j += T) {
+        const bool live = f.rp[j] >= thr && f.rp[j] > 0.0f;
+        const bool next_live = j + 1 < n && f.rp[j + 1] >= thr && f.rp[j + 1] > 0.0f;
+        if (live && !next_live) f.n_live = j + 1;
+    }
+    __syncthreads();
+    return f.n_live;
+}
+
+// Second half of the finish, from ranked candidates: f.sid / f.sp hold the n candidates in id order, f.rp / f.rpos
+// the same by (probability descending, id ascending), f.n_live is zero.  Called by every thread; ends with the row's
+// outputs written.
+template <int T, class FA>
+__device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, float m,
+                                                  float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t n_live = cta_top_k<T>(f, n, top_k);
+    if (threadIdx.x >= 32) return;
+    const uint32_t keep = warp_top_p(f.rp, n_live, top_p);
+    for (uint32_t j = keep + lane; j < n; j += 32) f.sp[f.rpos[j]] = 0.0f;
+    __syncwarp();
+    warp_finish(f, a, row, V, n, m, S, u01, amax, status);
+}
 
 // Candidates of one row -> token.  Called by every thread of a CTA of T threads (T >= F_QUAD, a multiple of 32)
 // with a barrier in front; cand_id: the row's n <= F_MCAP candidates in any order, prob(j) their probabilities (memory
@@ -183,27 +255,39 @@ __device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32
             f.sid[r_id] = my_id; f.sp[r_id] = my_p; f.rp[r_p] = my_p; f.rpos[r_p] = r_id;
         }
     } else {
-        // long list: sorted by id, then by (probability, position) -- two sorts of 64-bit keys
-        uint32_t npad = 512;
-        while (npad < n) npad <<= 1;
-        for (uint32_t j = tid; j < npad; j += T) {
-            unsigned long long k = ~0ull;   // the padding sorts to the end
-            if (j < n) {
-                k = ((unsigned long long)cand_id[j] << 32) | f2u(prob(j));
-            }
-            f.key[j] = k;
-        }
-        cta_bitonic_sort<T>(f.key, npad);
-        for (uint32_t j = tid; j < n; j += T) { f.sid[j] = (uint32_t)(f.key[j] >> 32); f.sp[j] = u2f((uint32_t)f.key[j]); }
-        __syncthreads();
-        for (uint32_t j = tid; j < npad; j += T)   // ascending by (p, position descending) = rank descending; padding first
-            f.key[j] = j < n ? ((unsigned long long)f2u(f.sp[j]) << 32) | (0xffffffffu - j) : 0ull;
-        cta_bitonic_sort<T>(f.key, npad);
+        // long list: sorted by (probability descending, id ascending); what top-k and top-p leave is put into id order, by
+        // counting where it has become short
+        for (uint32_t j = tid; j < n; j += T) f.key[j] = ((unsigned long long)~f2u(prob(j)) << 32) | cand_id[j];
+        cta_sort_shared<T, FA::CAPACITY>(f.key, n);
         for (uint32_t r = tid; r < n; r += T) {
-            const unsigned long long k = f.key[npad - 1u - r];
-            f.rp[r] = u2f((uint32_t)(k >> 32));
-            f.rpos[r] = 0xffffffffu - (uint32_t)k;
+            const unsigned long long k = f.key[r];
+            f.rp[r] = u2f(~(uint32_t)(k >> 32));
+            f.rpos[r] = (uint32_t)k;   // (the id here)
         }
+        const uint32_t n_live = cta_top_k<T>(f, n, top_k);
+        if (tid < 32) {
+            const uint32_t keep = warp_top_p(f.rp, n_live, top_p);
+            if (tid == 0) f.n_live = keep;
+        }
+        __syncthreads();
+        const uint32_t keep = f.n_live;
+        if (keep <= (uint32_t)F_QUAD) {
+            if ((uint32_t)tid < keep) {
+                const uint32_t id = f.rpos[tid];
+                uint32_t at = 0;
+#pragma unroll 8
+                for (uint32_t o = 0; o < keep; o++) at += f.rpos[o] < id;
+                f.sid[at] = id; f.sp[at] = f.rp[tid];
+            }
+            __syncthreads();
+        } else {
+            for (uint32_t r = tid; r < keep; r += T) f.key[r] = ((unsigned long long)f.rpos[r] << 32) | f2u(f.rp[r]);
+            cta_sort_shared<T, FA::CAPACITY>(f.key, keep);
+            for (uint32_t r = tid; r < keep; r += T) { f.sid[r] = (uint32_t)(f.key[r] >> 32); f.sp[r] = u2f((uint32_t)f.key[r]); }
+            __syncthreads();
+        }
+        if (tid < 32) warp_finish(f, a, row, V, keep, m, S, u01, amax, status);
+        return;
     }
     cta_finish_ranked<T, FA>(f, a, row, V, n, m, S, top_k, top_p, u01, amax, status);
 }

@@ -63,8 +63,10 @@ constexpr int S_NCELL = 4;               // running maxima per thread (piece num
 constexpr int S_CELLS = S_NCELL * SNT;   // per-thread maxima that bound the top-k threshold
 constexpr int S_NB = 1024;               // buckets of their histogram
 constexpr int S_BPT = S_NB / SNT;        // buckets per thread
-constexpr int S_RPT = S_MAX_REGIONS / SNT;   // regions per thread in the CTA-wide walks over regions
+constexpr int S_ENT = S_MAX_HASH / 2 + 1;   // distinct history ids, and the EOS fix
+constexpr int S_WORDS = S_MAX_VOCAB / 32;
 constexpr uint32_t S_NIL = 0xffffffffu;
+constexpr uint32_t ENT_MASKED = 0x80000000u, ENT_EOS = 0x40000000u;   // beside an entry's count
 static_assert(SNW <= 32, "warp slots are combined by one warp");
 
 // Everything the kernel needs to know about a row, read and validated by one thread while the CTA still works
@@ -79,13 +81,11 @@ struct SRowCtl {
 };
 
 // What the pass loops need to know about the row they work on.
-enum : uint32_t { PF_PEN = 1u, PF_REP = 2u, PF_FP = 4u, PF_PRES = 8u };
+enum : uint32_t { PF_REP = 1u, PF_FP = 2u, PF_PRES = 4u };
 struct PassArgs {
     const char* rowp;
-    const uint32_t* mw;
     float sc, sc_lo, c_hi, c_lo, cut_f, freq, pres, rep;
     uint32_t V, n_full, n_regions, flags;
-    uint32_t eos_piece, eos_tid, eos_sub;
     // a row shared by the CTAs of a cluster: this CTA works on the pieces q0, q0 + qstep, ...; the candidates of all of
     // them are collected by the first CTA (pointers into its shared memory)
     uint32_t q0, qstep;
@@ -107,41 +107,46 @@ struct StreamSmem {
     // the first CTA's copy (xs, xam)
     uint32_t xk[8], xlo[8], xfin[8], xflag[8], xam[8];
     double xs[8];
-    uint32_t cand_id[F_MCAP];
-    float cand_x[F_MCAP];
     long long prof_acc[16];
-    // Two lives of one area: the tables of a row while it streams, and the arrays of the finish once its
-    // candidates are known (nothing of the first is needed by then).
-    union {
+    // Three lives of one area: the id -> count table while the entries are set up, the tables of a row while it streams, and
+    // the arrays of the finish once its candidates are known (nothing of the tables is needed by then).
+    union alignas(16) {
         struct {
-            uint32_t hist[S_NB];
-            float cell[S_CELLS];             // [S_NCELL][SNT]
-            float t_am[SNT], t_max[SNT];     // per-thread results of pass 1 over the whole pieces
-            uint32_t t_q[SNT];
-            // per warp region of the row (512 consecutive logits): pass 1 leaves the warp's maximum and the plain sum
-            // of its numerators relative to it; then the binade's lower end the fold has there (0 = fold this region the
-            // careful way) and the estimate of the running value at its start.  While the history is indexed, reg_a
-            // counts the distinct history ids per region.
-            float reg_a[S_MAX_REGIONS], reg_b[S_MAX_REGIONS];
-            float reg_t[S_MAX_REGIONS];      // a logit below this adds exactly nothing to the fold in this region
-            // distinct history ids grouped by region: those of region r are the entries rs[r] .. rs[r + 1]
-            uint16_t rs[S_MAX_REGIONS + 2];
-            uint32_t pmask[S_MAX_REGIONS / 32];   // bit r: region r holds history ids
-            uint16_t pid[S_MAX_HASH / 2];    // position inside the region
-            uint32_t pval[S_MAX_HASH / 2];   // count, then (after pass 1) the bits of the penalised logit
-            // id -> count table while the history is indexed (hkey[H], hcnt[H]), then per-warp staging of a piece
-            // while penalties are applied to it (SNW x S_REGION floats)
-            union alignas(16) {
-                uint32_t hash[2 * S_MAX_HASH];
-                float stage[SNW * S_REGION];
-            } u;
+            uint32_t cand_id[F_MCAP];
+            float cand_x[F_MCAP];
+            union {
+                struct {
+                    uint32_t hist[S_NB];
+                    float cell[S_CELLS];             // [S_NCELL][SNT]
+                    float t_am[SNT], t_max[SNT];   // per-thread results of pass 1 over the whole pieces
+                    uint32_t t_q[SNT];
+                    // per warp region of the row (512 consecutive logits): pass 1 leaves the warp's maximum and the plain
+                    // sum of its numerators relative to it; then the binade's lower end the fold has there (0 = fold this
+                    // region the careful way) and the estimate of the running value at its start.  While the entries are
+                    // set up, reg_a counts them per region.
+                    float reg_a[S_MAX_REGIONS], reg_b[S_MAX_REGIONS];
+                    // a logit below this adds exactly nothing to the fold in this region; before, the plain sum of the
+                    // region's entries relative to the CTA's maximum
+                    float reg_t[S_MAX_REGIONS];
+                    // The row's entries: the distinct history ids and the EOS fix, those of region r at rs[r] .. rs[r + 1].
+                    // The passes leave their logits out (the bits are clear); pass 1 copies them to ent_raw, and one thread
+                    // per entry adds what the chain sees there to what the passes find.
+                    uint16_t rs[S_MAX_REGIONS + 2];
+                    uint32_t ent_id[S_ENT];
+                    float ent_x[S_ENT];              // before pass 1 is over: the count; ENT_MASKED, ENT_EOS
+                    uint32_t ent_raw[S_ENT];         // the word that holds the raw logit
+                    uint32_t bits[S_WORDS];          // one bit per logit: allowed, and no entry
+                };
+                FinishArrays fin;
+                unsigned long long tpkey[SNT];   // vocabulary-sharded mode: one candidate per thread while a record is ranked
+            };
         };
-        FinishArrays fin;
-        unsigned long long tpkey[SNT];   // vocabulary-sharded mode: one candidate per thread while a record is ranked
+        uint32_t hash[2 * S_MAX_HASH];           // hkey[H], hcnt[H]: ends before reg_a
     };
 };
 
 static_assert(sizeof(StreamSmem) <= 113 * 1024, "two CTAs per SM");
+static_assert(offsetof(StreamSmem, hash) + sizeof(StreamSmem::hash) <= offsetof(StreamSmem, reg_a), "entries are set up while the table stands");
 
 #define PGS_STICK(slot)                                             \
     do {                                                            \
@@ -353,79 +358,69 @@ __device__ __forceinline__ void raw_unpack(float (&x)[S_EPT], const Raw<BF16>& r
     }
 }
 
-// Raw logits of piece q -> the logits the chain sees: penalties (through the warp's staging area: the owner of a
-// history id is whichever lane holds it), grammar mask / end of row, EOS fix.  PASS 1 computes the penalised
-// values and leaves them where the counts were; PASS 2 takes them from there.
-template <bool BF16, bool MASK, bool TAIL, int PASS>
-__device__ __forceinline__ void fix_x(StreamSmem& sm, float (&x)[S_EPT], uint32_t q) {
+// Raw logits of piece q -> the logits of the pass: -inf where the row's bits say so (BITS: grammar mask, entries, end of
+// the row) or behind the end of the row.  The bits come from shared memory, four logits (bf16: eight) of a lane to the
+// load.  (Read from the mask table a piece at a time, every group of the piece waited for L2: 128 masked rows of 151936
+// took 100 us, with the bits 51.)
+template <bool BF16, bool BITS, bool TAIL>
+__device__ __forceinline__ void fix_x(const StreamSmem& sm, float (&x)[S_EPT], uint32_t q) {
     constexpr int G = Geo<BF16>::G, GE = Geo<BF16>::GE, GS = Geo<BF16>::GS;
-    const PassArgs& pa = sm.pa;
+    if (!BITS && !TAIL) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t region = q * SNW + (uint32_t)w;
-    if ((pa.flags & PF_PEN) && ((sm.pmask[region >> 5] >> (region & 31u)) & 1u)) {   // warp-uniform
-        float* stg = sm.u.stage + w * S_REGION;
-        const uint32_t c0 = sm.rs[region], c1 = sm.rs[region + 1];
+    const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
+    const uint32_t shift = ((uint32_t)lane * GE) & 31u;
 #pragma unroll
-        for (int j = 0; j < S_EPT; j += 4)
-            *reinterpret_cast<float4*>(stg + (j / GE) * GS + lane * GE + (j % GE)) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
-        __syncwarp();
-#pragma unroll 1
-        for (uint32_t i = c0 + lane; i < c1; i += 32) {
-            const uint32_t off = sm.pid[i];
-            if (PASS == 1) {
-                float v = stg[off];
-                if (pa.flags & PF_REP) v = v > 0.0f ? fdiv(v, pa.rep) : fmul(v, pa.rep);
-                if (pa.flags & PF_FP) {
-                    v = fsub(v, fmul(pa.freq, (float)sm.pval[i]));
-                    if (pa.flags & PF_PRES) v = fsub(v, pa.pres);
-                }
-                v = finite_f(v) ? v : -INFINITY;   // an overflowed penalty counts as masked
-                stg[off] = v;
-                sm.pval[i] = f2u(v);
-            } else {
-                stg[off] = u2f(sm.pval[i]);
-            }
-        }
-        __syncwarp();
+    for (int h = 0; h < G; h++) {
+        const uint32_t idx = e0 + h * GS;
+        uint32_t bits = 0xffffffffu;
+        if (BITS) bits = sm.bits[idx >> 5] >> shift;
+        else if (idx >= sm.pa.V) bits = 0u;
 #pragma unroll
-        for (int j = 0; j < S_EPT; j += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(stg + (j / GE) * GS + lane * GE + (j % GE));
-            x[j] = v.x; x[j + 1] = v.y; x[j + 2] = v.z; x[j + 3] = v.w;
-        }
-        __syncwarp();   // the next piece's staging must not overtake these reads
+        for (int c = 0; c < GE; c++)
+            if (!((bits >> c) & 1u)) x[h * GE + c] = -INFINITY;
     }
-    if (MASK || TAIL) {
-        const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
-        const uint32_t mshift = ((uint32_t)lane * GE) & 31u;
-#pragma unroll
-        for (int h = 0; h < G; h++) {
-            const uint32_t idx = e0 + h * GS;
-            uint32_t bits = 0xffffffffu;
-            if (MASK) bits = (!TAIL || idx < pa.V) ? __ldg(pa.mw + (idx >> 5)) >> mshift : 0u;
-            else if (idx >= pa.V) bits = 0u;
-#pragma unroll
-            for (int c = 0; c < GE; c++)
-                if (!((bits >> c) & 1u)) x[h * GE + c] = -INFINITY;
+}
+
+// What the chain sees at an entry: penalties, mask, EOS fix on the raw logit.
+__device__ __forceinline__ float entry_value(const PassArgs& pa, float v, uint32_t c) {
+    const uint32_t n = c & ~(ENT_MASKED | ENT_EOS);
+    if (n) {
+        if (pa.flags & PF_REP) v = v > 0.0f ? fdiv(v, pa.rep) : fmul(v, pa.rep);
+        if (pa.flags & PF_FP) {
+            v = fsub(v, fmul(pa.freq, (float)n));
+            if (pa.flags & PF_PRES) v = fsub(v, pa.pres);
         }
-        if (MASK && q == pa.eos_piece && threadIdx.x == pa.eos_tid) {   // the EOS fix (engine.rs:1307-1312)
-#pragma unroll
-            for (int j = 0; j < S_EPT; j++)
-                if ((uint32_t)j == pa.eos_sub && !finite_f(x[j])) x[j] = 0.0f;
-        }
+    }
+    if ((c & ENT_MASKED) || !finite_f(v)) v = (c & ENT_EOS) ? 0.0f : -INFINITY;   // an overflowed penalty counts as masked
+    return v;
+}
+// The raw logits of the region's entries into ent_raw, asynchronously: the region's own loads bring the same lines, and
+// nothing in the pass waits for these.  (Waited for in the pass, to be part of its maxima and sums, they made pass 1 over
+// 256 rows take 30 us in place of 21; found through a staging area 33 us; gathered before the pass 21 us and 4 us more in
+// front of it.)
+template <bool BF16>
+__device__ __forceinline__ void copy_entries(StreamSmem& sm, uint32_t region) {
+    const uint32_t e1 = sm.rs[region + 1];
+    for (uint32_t e = sm.rs[region] + (threadIdx.x & 31u); e < e1; e += 32u) {
+        const uint32_t id = sm.ent_id[e];
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(&sm.ent_raw[e])),
+                     "l"(sm.pa.rowp + (size_t)(BF16 ? id >> 1 : id) * 4u) : "memory");
     }
 }
 
 // pass 1 on one piece
-template <bool BF16, bool MASK, bool TAIL, bool STOCH>
+template <bool BF16, bool BITS, bool TAIL, bool STOCH>
 __device__ __forceinline__ void p1_piece(StreamSmem& sm, const Raw<BF16>& raw, uint32_t q, float& am, float& tmx, uint32_t& tqx) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t region = q * SNW + (uint32_t)w;
+    if (BITS) copy_entries<BF16>(sm, region);
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
     am = absmax_ept_nan(am, x);   // max |raw logit|, NaN-propagating: the sanity check
-    fix_x<BF16, MASK, TAIL, 1>(sm, x, q);
+    fix_x<BF16, BITS, TAIL>(sm, x, q);
     const float pm = max_ept(x);
     if (pm >= tmx) { tmx = pm; tqx = q; }   // pieces arrive in descending order: an equal maximum here has the lower id
     if (STOCH) {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         const float sc = sm.pa.sc;
         // one of the per-thread maxima that bound the top-k threshold
         const uint32_t ci = (q % S_NCELL) * SNT + threadIdx.x;
@@ -447,7 +442,6 @@ __device__ __forceinline__ void p1_piece(StreamSmem& sm, const Raw<BF16>& raw, u
         // all-masked region has NaN here, which converts to 0
         const uint32_t ws = __reduce_add_sync(FULL, __float2uint_rn(((p0 + p1) + (p2 + p3)) * 1048576.0f));
         if (lane == 0) {
-            const uint32_t region = q * SNW + (uint32_t)w;
             sm.reg_a[region] = wm; sm.reg_b[region] = (float)ws * (1.0f / 1048576.0f);
         }
     }
@@ -465,29 +459,56 @@ struct FoldAcc {
     }
 };
 
+template <bool CL>
+__device__ __forceinline__ void add_candidate(StreamSmem& sm, uint32_t id, float x) {
+    uint32_t* n = CL ? sm.pa.cand_n_p : &sm.cand_n;
+    const uint32_t at = atomicAdd(n, 1u);
+    if (at >= (uint32_t)F_MCAP) return;
+    (CL ? sm.pa.cand_id_p : sm.cand_id)[at] = id;
+    (CL ? sm.pa.cand_x_p : sm.cand_x)[at] = x;
+}
+
+// the logarithm (base 2) of a numerator
+template <bool BF16>
+__device__ __forceinline__ float exponent_of(const PassArgs& pa, float x) {
+    if (BF16) return __fmaf_rn(x, pa.sc, pa.c_hi) + __fmaf_rn(x, pa.sc_lo, pa.c_lo);
+    return __fmaf_rn(x, pa.sc, pa.c_hi) + pa.c_lo;
+}
+
+// The entries' part of pass 2: candidates, and what they add to the fold where it stands in their region.  (In a region
+// that is folded the careful way they are added at its start: a rounding there is half an ulp of the running value at most.)
+template <bool BF16, bool CL>
+__device__ __forceinline__ void p2_entries(StreamSmem& sm, uint32_t n_ent) {
+    if (threadIdx.x / 32u * 32u >= n_ent) return;   // warp-uniform
+    double td = 0.0;
+    for (uint32_t e = threadIdx.x; e < n_ent; e += SNT) {
+        const float x = sm.ent_x[e];
+        const uint32_t id = sm.ent_id[e], region = id / S_REGION;
+        if (x >= sm.pa.cut_f) add_candidate<CL>(sm, id, x);
+        const float v = ex2_approx_ftz(exponent_of<BF16>(sm.pa, x)), base = sm.reg_a[region];
+        if (base != 0.0f) td += (double)(f2u(fadd(base, v)) - f2u(base)) * ((double)base * 1.1920928955078125e-07);
+        else { const float R0 = sm.reg_b[region]; td += (double)fsub(fadd(R0, v), R0); }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) td += __shfl_xor_sync(FULL, td, o);
+    if ((threadIdx.x & 31u) == 0u) sm.wacc[threadIdx.x >> 5] += td;
+}
+
 // pass 2 on one piece
-template <bool BF16, bool MASK, bool TAIL, bool CL = false>
+template <bool BF16, bool BITS, bool TAIL, bool CL = false>
 __device__ __forceinline__ void p2_piece(StreamSmem& sm, const Raw<BF16>& raw, uint32_t q, FoldAcc& fa) {
     constexpr int G = Geo<BF16>::G, GE = Geo<BF16>::GE;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float sc = sm.pa.sc, c_hi = sm.pa.c_hi, c_lo = sm.pa.c_lo, cut_f = sm.pa.cut_f;
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
-    fix_x<BF16, MASK, TAIL, 2>(sm, x, q);
+    fix_x<BF16, BITS, TAIL>(sm, x, q);
     const float pm = max_ept(x);
     if (pm >= cut_f) {
         const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
 #pragma unroll
         for (int j = 0; j < S_EPT; j++)
-            if (x[j] >= cut_f) {
-                if (CL) {
-                    const uint32_t at = atomicAdd(sm.pa.cand_n_p, 1u);
-                    if (at < (uint32_t)F_MCAP) { sm.pa.cand_id_p[at] = elem_id<BF16>(e0, j); sm.pa.cand_x_p[at] = x[j]; }
-                } else {
-                    const uint32_t at = atomicAdd(&sm.cand_n, 1u);
-                    if (at < (uint32_t)F_MCAP) { sm.cand_id[at] = elem_id<BF16>(e0, j); sm.cand_x[at] = x[j]; }
-                }
-            }
+            if (x[j] >= cut_f) add_candidate<CL>(sm, elem_id<BF16>(e0, j), x[j]);
     }
     const uint32_t region = q * SNW + (uint32_t)w;
     if (TAIL && region >= sm.pa.n_regions) return;   // warp-uniform: past the end of the row
@@ -574,7 +595,7 @@ __device__ __forceinline__ void prefetch_piece(const char* warp_piece) {
 }
 
 // pass 1 over the whole pieces n_full-1 .. 0; the thread's results go to sm.t_*[tid]
-template <bool BF16, bool MASK, bool STOCH, bool CL>
+template <bool BF16, bool BITS, bool STOCH, bool CL>
 __device__ __noinline__ void pass1_whole(StreamSmem& sm) {
     constexpr int PB = S_PIECE * (BF16 ? 2 : 4);
     const uint32_t lane_e0 = (threadIdx.x >> 5) * S_REGION + (threadIdx.x & 31) * Geo<BF16>::GE;
@@ -594,7 +615,7 @@ __device__ __noinline__ void pass1_whole(StreamSmem& sm) {
                 if (q - 2 * qs >= q0) prefetch_piece<BF16>(wp - 2 * step);
                 Raw<BF16> b;
                 raw_load<BF16>(b, p);
-                p1_piece<BF16, MASK, false, STOCH>(sm, b, (uint32_t)q, am, tmx, tqx);
+                p1_piece<BF16, BITS, false, STOCH>(sm, b, (uint32_t)q, am, tmx, tqx);
             }
         }
         sm.t_am[threadIdx.x] = am; sm.t_max[threadIdx.x] = tmx; sm.t_q[threadIdx.x] = tqx;
@@ -611,13 +632,13 @@ __device__ __noinline__ void pass1_whole(StreamSmem& sm) {
         if (q >= (uint32_t)PGS_PF_DIST) prefetch_piece<BF16>(wp - (size_t)PGS_PF_DIST * PB);
         Raw<BF16> b;
         raw_load<BF16>(b, p);
-        p1_piece<BF16, MASK, false, STOCH>(sm, b, q, am, tmx, tqx);
+        p1_piece<BF16, BITS, false, STOCH>(sm, b, q, am, tmx, tqx);
     }
     sm.t_am[threadIdx.x] = am; sm.t_max[threadIdx.x] = tmx; sm.t_q[threadIdx.x] = tqx;
 }
 
 // pass 2 over the whole pieces 0 .. n_full-1; the warp's share of the fold is added to sm.wacc[w]
-template <bool BF16, bool MASK, bool CL>
+template <bool BF16, bool BITS, bool CL>
 __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
     constexpr int PB = S_PIECE * (BF16 ? 2 : 4);
     const uint32_t lane_e0 = (threadIdx.x >> 5) * S_REGION + (threadIdx.x & 31) * Geo<BF16>::GE;
@@ -636,7 +657,7 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
             if (q + 2u * qs < n) prefetch_piece<BF16>(wp + 2 * step);
             Raw<BF16> b;
             raw_load<BF16>(b, p);
-            p2_piece<BF16, MASK, false, true>(sm, b, q, fa);
+            p2_piece<BF16, BITS, false, true>(sm, b, q, fa);
         }
         fa.flush();
         if ((threadIdx.x & 31) == 0) sm.wacc[threadIdx.x >> 5] += fa.accd;
@@ -650,7 +671,7 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
         if (q + (uint32_t)PGS_PF_DIST < n) prefetch_piece<BF16>(wp + (size_t)PGS_PF_DIST * PB);
         Raw<BF16> b;
         raw_load<BF16>(b, p);
-        p2_piece<BF16, MASK, false>(sm, b, q, fa);
+        p2_piece<BF16, BITS, false>(sm, b, q, fa);
     }
     fa.flush();
     if ((threadIdx.x & 31) == 0) sm.wacc[threadIdx.x >> 5] += fa.accd;
@@ -664,13 +685,13 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
 template <bool BF16, bool CL>
 __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, const StreamLaunch sl) {
     namespace cg = cooperative_groups;
-    constexpr int GE = Geo<BF16>::GE, GS = Geo<BF16>::GS;
+    constexpr int GE = Geo<BF16>::GE;
     constexpr int ESZ = BF16 ? 2 : 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StreamSmem& sm = *reinterpret_cast<StreamSmem*>(smem_raw);
     const uint32_t H = sl.hash_slots;
-    uint32_t* hkey = sm.u.hash;
-    uint32_t* hcnt = sm.u.hash + H;
+    uint32_t* hkey = sm.hash;
+    uint32_t* hcnt = sm.hash + H;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const uint32_t V = a.vocab;
     const uint32_t n_full = V / S_PIECE;                        // whole pieces
@@ -725,13 +746,14 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         const float sc = ctl.sc;
         const bool greedy = temp < 1e-5f;
         const bool has_mask = ctl.mw != nullptr;
-        const bool do_fp = !(fabsf(ctl.freq) < 1e-6f && fabsf(ctl.pres) < 1e-6f);
+        const bool do_fp = !(fabsf(ctl.freq) < 1e-6f && fabsf(ctl.pres) < 1e-6f), do_pres = fabsf(ctl.pres) > 1e-6f;
         const bool do_rep = ctl.rep != 1.0f;
         const bool pen = nh > 0 && (do_fp || do_rep);
+        const bool fix = has_mask && (gflags & 1u) && a.eos >= 0 && (uint32_t)a.eos < V;   // engine.rs:1307-1312
+        const bool has_bits = has_mask || pen;
         if (tid == 0) {   // what the pass loops read
             PassArgs& pa = sm.pa;
-            pa.rowp = rowp; pa.mw = ctl.mw; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
-            pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep;
+            pa.rowp = rowp; pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
             pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions;
             pa.q0 = crank; pa.qstep = csize;
             pa.cand_n_p = &sm.cand_n; pa.cand_id_p = sm.cand_id; pa.cand_x_p = sm.cand_x;
@@ -741,17 +763,14 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 pa.cand_id_p = cluster.map_shared_rank(sm.cand_id, 0);
                 pa.cand_x_p = cluster.map_shared_rank(sm.cand_x, 0);
             }
-            pa.flags = (pen ? PF_PEN : 0u) | (do_rep ? PF_REP : 0u) | (do_fp ? PF_FP : 0u) | (fabsf(ctl.pres) > 1e-6f ? PF_PRES : 0u);
-            // the EOS fix touches one logit: where it sits in the piece / thread / register layout
-            pa.eos_piece = 0xffffffffu; pa.eos_tid = 0u; pa.eos_sub = 0u;
-            if (has_mask && (gflags & 1u) && a.eos >= 0 && (uint32_t)a.eos < V) {
-                const uint32_t r = (uint32_t)a.eos % S_PIECE, p = r % S_REGION;
-                pa.eos_piece = (uint32_t)a.eos / S_PIECE;
-                pa.eos_tid = (r / S_REGION) * 32u + (p % GS) / GE;
-                pa.eos_sub = (p / GS) * GE + p % GE;
-            }
+            pa.flags = (do_rep ? PF_REP : 0u) | (do_fp ? PF_FP : 0u) | (do_pres ? PF_PRES : 0u);
         }
 
+        // the history ids of the thread
+        constexpr int HPT = S_MAX_HASH / 2 / SNT;
+        uint32_t hid[HPT];
+#pragma unroll
+        for (int u = 0; u < HPT; u++) hid[u] = pen && (uint32_t)(tid + u * SNT) < nh ? __ldg(a.hist_ids + h0 + tid + u * SNT) : S_NIL;
         // the pieces the first pass starts with are requested now, so that they arrive while the history is indexed
         if (n_full > 0u) {
             constexpr int PB = S_PIECE * ESZ;
@@ -763,94 +782,108 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 if (qlast >= qs + crank) prefetch_piece<BF16>(wp - (size_t)qs * PB);
             }
         }
-        // ---- history: distinct ids with their counts, grouped by the warp region they fall into
+        // ---- entries (distinct history ids with what the penalties make of them; the EOS fix) and the row's bits
         bool defer_row = false;
-        if (pen) {
-            uint32_t* rcnt = reinterpret_cast<uint32_t*>(sm.reg_a);   // distinct ids per region, then the scatter cursor
-            // the first id of every thread is requested before the tables are cleared
-            const uint32_t hid0 = (uint32_t)tid < nh ? __ldg(a.hist_ids + h0 + tid) : S_NIL;
-#pragma unroll 1
-            for (uint32_t s = tid; s < H; s += SNT) { hkey[s] = S_NIL; hcnt[s] = 0u; }
-#pragma unroll 1
-            for (uint32_t r = tid; r < n_regions; r += SNT) rcnt[r] = 0u;
-#pragma unroll 1
-            for (uint32_t r = tid; r < (uint32_t)(S_MAX_REGIONS / 32); r += SNT) sm.pmask[r] = 0u;
-            __syncthreads();
-            int spilled = 0;
-#pragma unroll 1
-            for (uint32_t j = tid; j < nh; j += SNT) {
-                const uint32_t id = (j == (uint32_t)tid ? hid0 : __ldg(a.hist_ids + h0 + j)) - a.id_base;   // ids below a shard wrap around
-                if (id >= V) continue;   // engine.rs:1562
-                uint32_t s = (id * 2654435761u) & (H - 1u);
-                bool placed = false;
-#pragma unroll 1
-                for (int probe = 0; probe < 128; probe++) {
-                    const uint32_t prev = atomicCAS(&hkey[s], S_NIL, id);
-                    if (prev == S_NIL) {
-                        atomicAdd(&rcnt[id / S_REGION], 1u);
-                        atomicOr(&sm.pmask[id / (S_REGION * 32)], 1u << ((id / S_REGION) & 31u));
-                    }
-                    if (prev == S_NIL || prev == id) { atomicAdd(&hcnt[s], 1u); placed = true; break; }
-                    s = (s + 1u) & (H - 1u);
+        uint32_t n_ent = 0u;
+        if (has_bits) {
+#pragma unroll
+            for (int u = 0; u < HPT; u++) {
+                if (hid[u] != S_NIL) hid[u] -= a.id_base;   // ids below a shard wrap around
+                // engine.rs:1562; CL: another CTA's piece
+                if (hid[u] >= V || (CL && (hid[u] / S_PIECE) % csize != crank)) hid[u] = S_NIL;
+            }
+            uint32_t* rcnt = reinterpret_cast<uint32_t*>(sm.reg_a);
+            {
+                const uint32_t whole = V / 32u, words = ((V + S_PIECE - 1) / S_PIECE) * (S_PIECE / 32);
+                const uint32_t* mw = ctl.mw;
+#pragma unroll 4
+                for (uint32_t k = tid; k < words; k += SNT) {
+                    uint32_t b = k < whole ? 0xffffffffu : k == whole ? (1u << (V & 31u)) - 1u : 0u;
+                    if (has_mask && b) b &= __ldg(mw + k);
+                    sm.bits[k] = b;
                 }
-                if (!placed) spilled = 1;
             }
-            spilled = __syncthreads_or(spilled);
-            if (spilled && !CL) {   // CTA-uniform
-                if (writer) { sl.work_rows[atomicAdd(sl.work_count, 1u)] = row; atomicAdd(sl.p1_done, 1u); }
-                continue;
-            }
-            // (A cluster must meet at its barriers whatever one of its CTAs finds here: the CTA goes through the first
-            // pass without penalties and says so in the exchange behind it, where all CTAs give the row up together.)
-            if (CL && spilled) { defer_row = true; if (tid == 0) sm.pa.flags = 0u; }
-            if (!spilled) {
-            // exclusive scan of the counts in region order; thread t owns the regions t * rpt ..
-            const uint32_t rpt = (n_regions + SNT - 1) / SNT;   // <= S_RPT
-            uint32_t cnt[S_RPT], own = 0u;
-#pragma unroll
-            for (int j = 0; j < S_RPT; j++) {
-                const uint32_t r = (uint32_t)tid * rpt + j;
-                cnt[j] = ((uint32_t)j < rpt && r < n_regions) ? rcnt[r] : 0u;
-                own += cnt[j];
-            }
-            uint32_t total;
-            uint32_t before = sblock_excl_scan_u32(own, &total, sm.scan_u);
-#pragma unroll
-            for (int j = 0; j < S_RPT; j++) {
-                const uint32_t r = (uint32_t)tid * rpt + j;
-                if ((uint32_t)j < rpt && r < n_regions) { sm.rs[r] = (uint16_t)before; rcnt[r] = before; }
-                before += cnt[j];
-            }
-            if (tid == 0) sm.rs[n_regions] = (uint16_t)total;
-            __syncthreads();
+            static_assert(S_MAX_REGIONS <= SNT, "one thread per region");
+            if (tid < S_MAX_REGIONS) { rcnt[tid] = 0u; sm.rs[tid] = 0; sm.reg_t[tid] = 0.0f; }
+            if (tid < 2) sm.rs[S_MAX_REGIONS + tid] = 0;
+            if (pen || fix) {
 #pragma unroll 1
-            for (uint32_t s = tid; s < H; s += SNT) {
-                const uint32_t id = hkey[s];
-                if (id == S_NIL) continue;
-                const uint32_t at = atomicAdd(&rcnt[id / S_REGION], 1u);
-                sm.pid[at] = (uint16_t)(id % S_REGION);
-                sm.pval[at] = hcnt[s];
-            }
+                for (uint32_t s = tid; s < 2u * H; s += SNT) sm.hash[s] = s < H ? S_NIL : 0u;
+                __syncthreads();
+                // the thread that meets an id first owns its entry
+                bool spilled = false;
+                const auto insert = [&](uint32_t id, uint32_t n) {   // the id's slot | 2^31 where it is not new
+                    const uint32_t mul = id * 2654435761u;
+                    uint32_t s = (mul ^ (mul >> 15)) & (H - 1u);
+#pragma unroll 1
+                    for (int probe = 0; probe < 128; probe++) {
+                        const uint32_t prev = atomicCAS(&hkey[s], S_NIL, id);
+                        if (prev == S_NIL || prev == id) {
+                            if (prev == S_NIL) {
+                                const uint32_t bit = 1u << (id & 31u);
+                                if (!(atomicAnd(&sm.bits[id >> 5], ~bit) & bit)) n |= ENT_MASKED;
+                                if (fix && id == (uint32_t)a.eos) n |= ENT_EOS;
+                                atomicAdd(&rcnt[id / S_REGION], 1u);
+                            }
+                            atomicAdd(&hcnt[s], n);
+                            return prev == S_NIL ? s : s | 0x80000000u;
+                        }
+                        s = (s + 1u) & (H - 1u);
+                    }
+                    spilled = true;
+                    return S_NIL;
+                };
+                uint32_t slot[HPT];
+#pragma unroll
+                for (int u = 0; u < HPT; u++) slot[u] = hid[u] != S_NIL ? insert(hid[u], 1u) : S_NIL;
+                uint32_t eos_slot = S_NIL;
+                if (tid == 0 && fix && (!CL || ((uint32_t)a.eos / S_PIECE) % csize == crank)) eos_slot = insert((uint32_t)a.eos, 0u);
+                if (__syncthreads_or(spilled)) {
+                    if (!CL) {   // CTA-uniform
+                        if (writer) { sl.work_rows[atomicAdd(sl.work_count, 1u)] = row; atomicAdd(sl.p1_done, 1u); }
+                        continue;
+                    }
+                    // A cluster must meet at its barriers whatever one of its CTAs finds here: the CTA goes through the
+                    // first pass without entries and says so in the exchange behind it, where all CTAs give the row up
+                    // together.
+                    defer_row = true;
+                } else {
+                    const uint32_t own = tid < S_MAX_REGIONS ? rcnt[tid] : 0u;
+                    const uint32_t before = sblock_excl_scan_u32(own, &n_ent, sm.scan_u);
+                    if (tid < S_MAX_REGIONS) { sm.rs[tid] = (uint16_t)before; rcnt[tid] = before; }
+                    if (tid < 2) sm.rs[S_MAX_REGIONS + tid] = (uint16_t)n_ent;
+                    __syncthreads();
+                    const auto entry = [&](uint32_t id, uint32_t s) {
+                        if (s & 0x80000000u) return;
+                        const uint32_t at = atomicAdd(&rcnt[id / S_REGION], 1u);
+                        sm.ent_id[at] = id;
+                        sm.ent_x[at] = u2f(hcnt[s]);
+                    };
+#pragma unroll
+                    for (int u = 0; u < HPT; u++) entry(hid[u], slot[u]);
+                    if (tid == 0 && fix) entry((uint32_t)a.eos, eos_slot);
+                }
+                __syncthreads();
             }
         }
 #pragma unroll
         for (int c = 0; c < S_NCELL; c++) sm.cell[c * SNT + tid] = -INFINITY;
-        __syncthreads();   // the id -> count table is dead from here on (its space is the staging area); PassArgs are set
+        __syncthreads();   // PassArgs, entries and bits are set
         PGS_STICK(1);   // history indexed
 
         // ================================================================ pass 1 (HBM, last piece first)
         float am = 0.0f;            // max |raw logit|
-        float tmx = -INFINITY;      // the thread's running maximum, and the lowest piece that holds it
+        float tmx = -INFINITY;      // the thread's running maximum without entries, and the lowest piece that holds it
         uint32_t tqx = 0u;
         const bool my_tail = has_tail && (!CL || tail_owner == crank);
         if (my_tail) {
             Raw<BF16> raw;
             raw_load_tail<BF16>(raw, rowp + ((size_t)n_full * S_PIECE + lane_e0) * ESZ, n_full * S_PIECE + lane_e0, V);
-            if (has_mask) { if (greedy) p1_piece<BF16, true, true, false>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, true, true, true>(sm, raw, n_full, am, tmx, tqx); }
+            if (has_bits) { if (greedy) p1_piece<BF16, true, true, false>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, true, true, true>(sm, raw, n_full, am, tmx, tqx); }
             else { if (greedy) p1_piece<BF16, false, true, false>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, false, true, true>(sm, raw, n_full, am, tmx, tqx); }
         }
         if (n_full > 0u) {
-            if (has_mask) { if (greedy) pass1_whole<BF16, true, false, CL>(sm); else pass1_whole<BF16, true, true, CL>(sm); }
+            if (has_bits) { if (greedy) pass1_whole<BF16, true, false, CL>(sm); else pass1_whole<BF16, true, true, CL>(sm); }
             else { if (greedy) pass1_whole<BF16, false, false, CL>(sm); else pass1_whole<BF16, false, true, CL>(sm); }
             am = absmax3_nan(am, sm.t_am[tid], 0.0f);
             if (sm.t_max[tid] >= tmx) { tmx = sm.t_max[tid]; tqx = sm.t_q[tid]; }   // the whole pieces come before the ragged one
@@ -858,6 +891,19 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         PGS_STICK(2);   // pass 1
 
         // ---- row maximum, sanity, and the material for the top-k bound
+        float emx = -INFINITY;      // the largest of the thread's entries
+        if (n_ent) {   // CTA-uniform
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            for (uint32_t e = tid, c = 0; e < n_ent; e += SNT, c++) {
+                const uint32_t raw = sm.ent_raw[e];
+                const float v = entry_value(sm.pa, u2f(!BF16 ? raw : (sm.ent_id[e] & 1u) ? raw & 0xffff0000u : raw << 16), f2u(sm.ent_x[e]));
+                sm.ent_x[e] = v;
+                emx = fmaxf(emx, v);
+                float& cell = sm.cell[c % S_NCELL * SNT + tid];   // (any cell: a logit counts in one)
+                if (v > cell) cell = v;
+            }
+        }
         {
             uint32_t lo = 0xffffffffu, fin = 0u;
             if (!greedy) {
@@ -869,7 +915,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                     fin++;
                 }
             }
-            const uint32_t wk = __reduce_max_sync(FULL, order_key(tmx));
+            const uint32_t wk = __reduce_max_sync(FULL, order_key(fmaxf(tmx, emx)));
             const uint32_t wlo = __reduce_min_sync(FULL, lo);
             const uint32_t wfin = __reduce_add_sync(FULL, fin);
             const uint32_t wbad = __any_sync(FULL, !(am < INFINITY)) ? 1u : 0u;
@@ -883,6 +929,10 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         uint32_t lo_key = __reduce_min_sync(FULL, lane < SNW ? sm.red_lo[lane] : 0xffffffffu);
         uint32_t n_fin = __reduce_add_sync(FULL, lane < SNW ? sm.red_fin[lane] : 0u);
         bool nonfinite = __any_sync(FULL, lane < SNW && sm.red_flag[lane] != 0u);
+        const float lm = key_to_float(gkey);   // (of no interest without one)
+        if (!greedy && gkey)
+            for (uint32_t e = tid; e < n_ent; e += SNT)
+                if (sm.ent_x[e] > -INFINITY) atomicAdd(&sm.reg_t[sm.ent_id[e] / S_REGION], ex2_approx_ftz((sm.ent_x[e] - lm) * sc));
         if (CL) {
             // First barrier: every CTA of the cluster is through its first pass, so nobody still uses the space of the
             // region table for its history counts, and everybody is done with the row before.  Then every CTA hands its
@@ -894,7 +944,12 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 for (uint32_t r = tid; r < n_regions; r += SNT) {
                     const uint32_t q = r / SNW;
                     if ((q < n_full ? q % csize : tail_owner) != crank) continue;
-                    const float ra = sm.reg_a[r], rb = sm.reg_b[r];
+                    float ra = sm.reg_a[r], rb = sm.reg_b[r];
+                    if (has_bits && sm.reg_t[r] > 0.0f) {   // with the entries, from now on relative to this CTA's maximum
+                        rb = (rb > 0.0f ? rb * ex2_approx_ftz((ra - lm) * sc) : 0.0f) + sm.reg_t[r];
+                        ra = lm;
+                        sm.reg_a[r] = ra; sm.reg_b[r] = rb;
+                    }
                     for (uint32_t k = 0; k < csize; k++) {
                         if (k == crank) continue;
                         *cluster.map_shared_rank(&sm.reg_a[r], k) = ra;
@@ -932,7 +987,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 raw_load_tail<BF16>(raw, rowp + ((size_t)q * S_PIECE + lane_e0) * ESZ, q * S_PIECE + lane_e0, V);
                 float x[S_EPT];
                 raw_unpack<BF16>(x, raw);
-                if (has_mask) fix_x<BF16, true, true, 2>(sm, x, q); else fix_x<BF16, false, true, 2>(sm, x, q);
+                if (has_bits) fix_x<BF16, true, true>(sm, x, q); else fix_x<BF16, false, true>(sm, x, q);
                 const bool mine = ((pending >> lane) & 1u) && tqx == q;
                 if (mine) {
                     int j0 = 0;
@@ -942,6 +997,8 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 }
                 pending &= ~__ballot_sync(FULL, mine);
             }
+            for (uint32_t e = tid; e < n_ent; e += SNT)
+                if (sm.ent_x[e] == m) atomicMin(&sm.amax, sm.ent_id[e]);
             __syncthreads();
         }
         uint32_t amax = any ? sm.amax : 0u;
@@ -1050,6 +1107,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 const uint32_t r = r0 + (uint32_t)tid;
                 float P = 0.0f;
                 if (r < n_regions && sm.reg_b[r] > 0.0f) P = sm.reg_b[r] * ex2_approx_ftz((sm.reg_a[r] - m) * sc);
+                if (!CL && has_bits && r < n_regions) P += sm.reg_t[r];
                 float tot;
                 const float pre = carry + sblock_excl_scan_f32(P, &tot, sm.scan_f);
                 if (r < n_regions) {
@@ -1080,17 +1138,18 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         PGS_STICK(3);   // fold table
 
         // ================================================================ pass 2 (L2, first piece first)
+        p2_entries<BF16, CL>(sm, n_ent);
         if (my_tail) {
             Raw<BF16> raw;
             raw_load_tail<BF16>(raw, rowp + ((size_t)n_full * S_PIECE + lane_e0) * ESZ, n_full * S_PIECE + lane_e0, V);
             FoldAcc fa;
             fa.accd = 0.0; fa.cur_n = 0ull; fa.cur_bb = 0u;
-            if (has_mask) p2_piece<BF16, true, true, CL>(sm, raw, n_full, fa); else p2_piece<BF16, false, true, CL>(sm, raw, n_full, fa);
+            if (has_bits) p2_piece<BF16, true, true, CL>(sm, raw, n_full, fa); else p2_piece<BF16, false, true, CL>(sm, raw, n_full, fa);
             fa.flush();
             if (lane == 0) sm.wacc[w] += fa.accd;
         }
         if (n_full > 0u) {
-            if (has_mask) pass2_whole<BF16, true, CL>(sm); else pass2_whole<BF16, false, CL>(sm);
+            if (has_bits) pass2_whole<BF16, true, CL>(sm); else pass2_whole<BF16, false, CL>(sm);
         }
         __syncthreads();   // the candidate list and the warps' shares are complete
         PGS_STICK(4);   // pass 2

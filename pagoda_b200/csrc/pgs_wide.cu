@@ -804,18 +804,12 @@ __device__ __noinline__ void select_row(WideSmem& sm, const RowArgs& a, const Wi
 // bucket b of the row's list as sorted keys (probability descending, id ascending) in sm.sort; false when it is too long
 __device__ __forceinline__ bool sort_bucket(WideSmem& sm, const WideLaunch& l, uint32_t slot, uint32_t at, uint32_t n) {
     if (n > (uint32_t)W_SORT) return false;
-    uint32_t pad = 32u;
-    while (pad < n) pad <<= 1;
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < pad; j += W_NT) {
-        unsigned long long key = ~0ull;
-        if (j < n) {
-            const unsigned long long v = __ldcg(l.list + (size_t)slot * l.list_stride + at + j);
-            key = ((unsigned long long)(~(uint32_t)(v >> 32)) << 32) | (uint32_t)v;
-        }
-        sm.sort[j] = key;
+    for (uint32_t j = threadIdx.x; j < n; j += W_NT) {
+        const unsigned long long v = __ldcg(l.list + (size_t)slot * l.list_stride + at + j);
+        sm.sort[j] = ((unsigned long long)(~(uint32_t)(v >> 32)) << 32) | (uint32_t)v;
     }
-    cta_bitonic_sort<W_NT>(sm.sort, pad);
+    cta_sort_shared<W_NT, W_SORT>(sm.sort, n);
     return true;
 }
 

@@ -1,0 +1,36 @@
+"""The streaming kernel against the oracle where its branches change: candidate lists around the lengths of the sort,
+histories that crowd one 512-logit region or fill the table, masks that end inside a word, a bf16 row of odd groups."""
+import numpy as np
+import pytest
+
+from .util import assert_close, run_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("vocab, top_k, history, crowd, masked, bf16", [
+    (8200, 255, 40, 512, False, False), (8192, 257, 2048, 8192, True, False), (40016, 511, 300, 300, True, True),
+    (32776, 513, 700, 32776, False, True), (151936, 1024, 1, 1, True, False), (262144, 1000, 2047, 1024, False, False),
+    (262152, 64, 8, 64, True, True)])
+def test_stream_edges(oracle, vocab, top_k, history, crowd, masked, bf16):
+    import pagoda_b200
+    from pagoda_b200 import synth
+    rows = 6
+    rng = np.random.default_rng(vocab + top_k)
+    x = synth.normal_f32(11 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    x[:, rng.integers(0, vocab, 40)] += 6.0
+    kw = {}
+    if masked:
+        words = rng.integers(0, 1 << 32, (3, (vocab + 31) // 32), dtype=np.uint64).astype(np.uint32)
+        kw = dict(mask_words=words, state_flags=np.array([0, 1, 0], np.uint32),
+                  mask_state=np.array([0, 1, 2, -1, 1, 0], np.int32), eos_token_id=vocab - 1)
+    w = synth.Workload(
+        "edges", (x.view(np.uint32) >> 16).astype(np.uint16) if bf16 else x, np.resize(np.float32([0.7, 1.3, 0.0]), rows),
+        np.full(rows, top_k, np.uint32), np.resize(np.float32([1.0, 0.9]), rows), np.full(rows, 0.2, np.float32),
+        np.full(rows, 0.1, np.float32), np.full(rows, 1.1, np.float32), np.arange(rows + 1, dtype=np.uint32) * history,
+        rng.integers(0, crowd, rows * history).astype(np.uint32), synth.uniform_f32(5, rows), **kw)
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=history)
+    try:
+        assert_close(*run_both(s, oracle, w), "edges")
+    finally:
+        s.close()
