@@ -152,7 +152,7 @@ int wide_workspace(pgs_handle* h) {
     size_t used = 0;
     auto take = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~size_t(255); return at; };
     const size_t o_sync = take(64), o_left = take(4), zeroed = used;
-    const size_t o_rows = take((size_t)h->max_rows * 4), o_row = take(rows * sizeof(WideRow)), o_reg = take(rows * regions * sizeof(float2));
+    const size_t o_rows = take((size_t)h->max_rows * 4), o_row = take(rows * sizeof(WideRow)), o_reg = take(rows * regions * sizeof(float2)), o_cell = take(rows * regions * sizeof(float4));
     const size_t o_seg = take(rows * regions * sizeof(uint2)), o_pre = take(rows * regions * 4), o_rs = take(rows * (regions + 1u) * 4);
     const size_t o_eid = take(rows * (W_MAX_HIST + 32) * 4), o_exn = take(rows * (W_MAX_HIST + 32) * 4);
     const size_t o_hist = take(rows * W_BUCKETS * 4);
@@ -161,7 +161,7 @@ int wide_workspace(pgs_handle* h) {
     PGS_CUDA(nullptr, cudaMemsetAsync(h->wide_ws, 0, zeroed, h->stream));
     unsigned char* p = h->wide_ws;
     l.sync = (uint32_t*)(p + o_sync); l.left_count = (uint32_t*)(p + o_left); l.left_rows = (uint32_t*)(p + o_rows);
-    l.row = (WideRow*)(p + o_row); l.reg = (float2*)(p + o_reg); l.seg = (uint2*)(p + o_seg); l.pre = (float*)(p + o_pre);
+    l.row = (WideRow*)(p + o_row); l.reg = (float2*)(p + o_reg); l.cell = (float4*)(p + o_cell); l.seg = (uint2*)(p + o_seg); l.pre = (float*)(p + o_pre);
     l.rs = (uint32_t*)(p + o_rs); l.ent_id = (uint32_t*)(p + o_eid); l.ent_xn = (float*)(p + o_exn); l.hist = (uint32_t*)(p + o_hist);
     l.list = h->sl_key; l.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
     l.terms = (float*)(p + o_terms);

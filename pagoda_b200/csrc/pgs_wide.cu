@@ -36,6 +36,8 @@ namespace pgs {
 constexpr int WNW = W_NT / 32;
 constexpr int WL = W_REGION / 32;        // logits per lane and region
 constexpr uint32_t W_NIL = 0xffffffffu;
+constexpr uint32_t F_KMAX = F_MCAP / 2;  // top-k up to which the second pass lists the candidates
+constexpr uint32_t W_DUAL = 2u;          // beside a segment's binade: it may also be the next one
 
 // 32 runs of terms, one per lane, ready to be added to a running value: lanes whose runs are estimated to begin in one
 // binade form a group, and each lane holds the increments from the group's first lane up to and including its own, for an
@@ -50,6 +52,7 @@ struct alignas(16) WideSmem {
     RowArgs a;                           // the launch's arguments, for the phases, which are functions of their own
     WideLaunch l;
     WideRow row;
+    WideRow rows[W_CHUNK];               // region phases: the chunk's rows
     unsigned long long exp_tab[32];
     uint32_t red_u[WNW], red_v[WNW];
     float red_f[WNW];
@@ -234,24 +237,64 @@ __device__ __forceinline__ void wterms(const unsigned long long* tab, float* buf
 // ------------------------------------------------------------------------------------------------ the exact fold
 
 // Increments of the running value over this warp's terms (each lane's share), in ulps of the binade whose lower end has
-// the bits `kb`: one integer whatever the order.  {0, 0}: has to be added term by term (no binade given, a term too large
-// for it, or one that ends on half an ulp).  {0, 1}: nothing but zeros.
-__device__ __forceinline__ uint2 increments(const float (&x)[WL], uint32_t kb) {
-    float top = 0.0f;
-#pragma unroll
-    for (int j = 0; j < WL; j++) top = fmaxf(top, x[j]);
-    if (__all_sync(FULL, top == 0.0f)) return make_uint2(0u, 1u);
-    const float b0 = u2f(kb), b1 = u2f(kb + 1u);
-    uint32_t n = 0u, tie = 0u;
+// the bits `kb`: one integer whatever the order.  W_TIE: has to be added term by term (a term too large for the binade, or
+// one that ends on half an ulp).
+constexpr uint32_t W_TIE = 0xffffffffu;
+__device__ __forceinline__ bool increment(float x, uint32_t kb, uint32_t& n) {
+    const uint32_t i0 = f2u(fadd(u2f(kb), x)) - kb, i1 = f2u(fadd(u2f(kb + 1u), x)) - (kb + 1u);
+    n += i0;
+    return i0 == i1 && x < u2f(kb);
+}
+
+// What the approximate terms need to know: with d = x - max (exact as the reference's), log2 of a term in ulps is
+// d * c + k0 - log2(ulp).
+struct Approx {
+    float c, k0;
+};
+__device__ __forceinline__ Approx approx_of(const Terms& f) {
+    Approx q;
+    q.c = 1.44269504f / f.t;
+    q.k0 = f.S > 1e-9f ? -(float)log2((double)f.S) : 0.0f;
+    return q;
+}
+// The increment of a term is its value in ulps, rounded: the hardware's exp2 decides that unless it lands close to half an
+// ulp.  The error of its argument is a few 2^-24 of |d * c| and |k|, that of the exp2 below 2^-21; the margin is four times
+// as wide.  Nearly all terms are far below the running value, so that about one of a region's 512 is in doubt and takes the
+// exact exponential, which costs ten times as much (64 rows of 151936: 25 us for all of them).
+template <bool BF16, bool VEC>
+__device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id0, const Terms& f, const Approx& q, uint32_t kb, const unsigned long long* tab) {
+    const float k = q.k0 - (float)((int)(kb >> 23) - 127 - 23), eps = (2.0f * fabsf(k) + 2.0f * fabsf(q.k0) + 12.0f) * 2.384185791015625e-07f;
+    const float p_lim = f.filter ? f.p_thr / u2f(kb) * 8388608.0f : 0.0f, slack = 4.0f * eps * p_lim;   // the threshold in ulps
+    uint32_t n = 0u, doubt = 0u;
 #pragma unroll
     for (int j = 0; j < WL; j++) {
-        const uint32_t i0 = f2u(fadd(b0, x[j])) - kb, i1 = f2u(fadd(b1, x[j])) - (kb + 1u);
-        n += i0;
-        tie |= i0 ^ i1;
+        const float v = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, k));   // (-inf -> 0)
+        const float r = fadd(v, 8388608.0f);                                  // (beyond 2^23: in doubt)
+        bool open = !(__fmaf_rn(v, eps, fabsf(fsub(v, fsub(r, 8388608.0f)))) < 0.5f);
+        uint32_t i = f2u(r) - 0x4b000000u;
+        if (f.filter) {   // warp-uniform
+            open = open && !(v < p_lim - slack);
+            open = open || fabsf(v - p_lim) <= slack;
+            if (v < p_lim) i = 0u;
+        }
+        if (open) doubt |= 1u << j; else n += i;
     }
-    const bool bad = kb == 0u || tie != 0u || !(top < b0) || n >= 0x01000000u;
-    if (__any_sync(FULL, bad)) return make_uint2(0u, 0u);
-    return make_uint2(__reduce_add_sync(FULL, n), kb);   // (the table keeps the sum below 2^24 ulps)
+    bool good = true;
+    while (__any_sync(FULL, doubt != 0u)) {
+        if (doubt) {
+            const int j = __ffs((int)doubt) - 1;
+            float xj = x[0];
+#pragma unroll
+            for (int u = 1; u < WL; u++) if (u == j) xj = x[u];
+            uint32_t o = 0u;
+#pragma unroll
+            for (int u = 0; u < WL; u++) if (u == j) o = WLay<BF16, VEC>::off(threadIdx.x & 31u, u);
+            good &= increment(term_of(xj, id0 + o, f, tab), kb, n);
+            doubt &= doubt - 1u;
+        }
+    }
+    if (__any_sync(FULL, !good || n >= 0x01000000u)) return W_TIE;
+    return __reduce_add_sync(FULL, n);   // (the table keeps the sum below 2^24 ulps)
 }
 
 // v: this lane's run; R0: estimate of the running value at the first lane's run
@@ -393,9 +436,11 @@ __device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_
             for (uint32_t q = 0; q <= n; q++) {
                 const uint32_t stop = q < n ? sm.serial[b + q] : b + WNW >= n_serial ? n_regions : pos;
                 while (pos < stop) {   // whole segments up to the next one that is not
-                    const uint2 sg = pos + lane < stop ? sm.seg[pos + lane] : make_uint2(0u, 1u);
-                    const uint32_t rb = f2u(R);
-                    const unsigned not_ok = ~__ballot_sync(FULL, sg.y == 1u || sg.y == (rb & 0x7f800000u));
+                    uint2 sg = pos + lane < stop ? sm.seg[pos + lane] : make_uint2(0u, 1u);
+                    const uint32_t rb = f2u(R), kb = rb & 0x7f800000u;
+                    if ((sg.y & W_DUAL) && kb == sg.y - W_DUAL + 0x00800000u) sg = make_uint2(f2u(sm.pre[pos + lane]), kb);
+                    sg.y &= ~W_DUAL;
+                    const unsigned not_ok = ~__ballot_sync(FULL, sg.y == 1u || sg.y == kb);
                     uint32_t cnt = not_ok ? __ffs((int)not_ok) - 1u : 32u;
                     uint32_t inc = lane < cnt ? sg.x : 0u;
                     const uint32_t own = inc;
@@ -436,12 +481,22 @@ __device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_
     return sm.R;
 }
 
-// binade of a segment whose plain sum P begins at the estimate `pre` of the running value, 0 when it may change there.  The
-// plain sums overestimate the running value by up to a few 1e-4 (the small terms it drops).
-__device__ __forceinline__ uint32_t safe_binade(float pre, float P, float slack) {
+// Table entry of a segment whose plain sum P begins at the estimate `pre` of the running value: the binade that the running
+// value stays in; that binade | W_DUAL when it may also be in the next one throughout (the estimate is close to the border);
+// 0 when it is expected to change there.  The plain sums overestimate the running value by up to a few 1e-4 (the small terms
+// it drops), hence the slack.
+__device__ __forceinline__ uint32_t binade(float v) { return f2u(v) & 0x7f800000u; }
+__device__ __forceinline__ uint32_t segment_binade(float pre, float P, float slack) {
     const float lo = pre * (1.0f - slack), hi = (pre + P) * (1.0f + slack);
-    const uint32_t kb = f2u(lo) & 0x7f800000u;
-    return kb != 0u && kb == (f2u(hi) & 0x7f800000u) && hi < INFINITY && P * (1.0f + slack) < 0.999f * u2f(kb) ? kb : 0u;
+    const uint32_t kb = binade(lo);
+    if (kb == 0u || !(hi < INFINITY) || !(P * (1.0f + slack) < 0.999f * u2f(kb))) return 0u;
+    if (kb == binade(hi)) return kb;
+    return kb + 0x00800000u == binade(hi) && binade(pre) == binade(pre + P) ? kb | W_DUAL : 0u;
+}
+// the same for one binade only
+__device__ __forceinline__ uint32_t safe_binade(float pre, float P, float slack) {
+    const uint32_t kb = segment_binade(pre, P, slack);
+    return kb & W_DUAL ? 0u : kb;
 }
 
 // exclusive scan over the CTA (plain adds: estimates only); one barrier in front, one behind
@@ -478,7 +533,7 @@ __device__ __forceinline__ void make_table(WideSmem& sm, const WideLaunch& l, ui
         const float pre = carry + wscan_f32(sm, p, &tot);
         if (r < n_regions) {
             l.pre[(size_t)slot * l.reg_stride + r] = pre;
-            l.seg[(size_t)slot * l.reg_stride + r] = make_uint2(0u, safe_binade(pre, p, slack));
+            l.seg[(size_t)slot * l.reg_stride + r] = make_uint2(0u, segment_binade(pre, p, slack));
         }
         carry += tot;
     }
@@ -508,6 +563,12 @@ __device__ __forceinline__ void row_in(WideSmem& sm, const WideLaunch& l, uint32
     if (threadIdx.x < sizeof(WideRow) / 4) reinterpret_cast<uint32_t*>(&sm.row)[threadIdx.x] = __ldcg(from + threadIdx.x);
     __syncthreads();
 }
+// the chunk's rows, for a region phase; a barrier behind
+__device__ __forceinline__ void rows_in(WideSmem& sm, const WideLaunch& l, uint32_t n_rows) {
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(l.row);
+    for (uint32_t i = threadIdx.x; i < n_rows * (uint32_t)(sizeof(WideRow) / 4); i += W_NT) reinterpret_cast<uint32_t*>(sm.rows)[i] = __ldcg(from + i);
+    __syncthreads();
+}
 __device__ __forceinline__ void row_out(WideSmem& sm, const WideLaunch& l, uint32_t slot) {
     __syncthreads();
     if (threadIdx.x < sizeof(WideRow) / 4)
@@ -520,44 +581,50 @@ template <bool BF16>
 __device__ __noinline__ void open_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot, uint32_t row) {
     const uint32_t tid = threadIdx.x, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     __syncthreads();
-    if (tid == 0) {
+    uint32_t param = 0u;
+    if (tid < 32) {   // one parameter per lane, so that their latencies overlap
+        const void* from[11] = {a.temperature, a.top_k, a.top_p, a.freq, a.pres, a.rep, a.uniform, a.mask_table, a.mask_state, a.hist_offsets, a.hist_offsets};
+        const void* p = nullptr;
+#pragma unroll
+        for (int u = 0; u < 11; u++) if (tid == (uint32_t)u) p = from[u];
+        param = tid == 2u || tid == 5u ? f2u(1.0f) : tid == 7u ? 0xffffffffu : 0u;   // top-p and repetition off, no mask
+        if (p) param = static_cast<const uint32_t*>(p)[row + (tid == 10u ? 1u : 0u)];
+    }
+    const auto get = [&](int u) { return __shfl_sync(FULL, param, u); };
+    if (tid < 32) {
         WideRow& c = sm.row;
-        c.row = row;
-        c.rowp = (const char*)a.logits + (size_t)row * a.row_stride * (BF16 ? 2 : 4);
-        c.temp = l.score ? 1.0f : a.temperature ? a.temperature[row] : 0.0f;
-        c.top_k = a.top_k ? a.top_k[row] : 0u;
-        c.top_p = a.top_p ? a.top_p[row] : 1.0f;
-        c.freq = a.freq ? a.freq[row] : 0.0f;
-        c.pres = a.pres ? a.pres[row] : 0.0f;
-        c.rep = a.rep ? a.rep[row] : 1.0f;
-        c.u01 = a.uniform ? a.uniform[row] : 0.0f;
-        c.t = fmaxf(c.temp, 1e-9f);
-        bool bad = !finite_f(c.temp) || !finite_f(c.top_p) || !finite_f(c.freq) || !finite_f(c.pres) || !finite_f(c.rep) || !(c.rep > 0.0f) ||
-                   !finite_f(c.u01);
-        c.mw = nullptr;
-        c.gflags = 0u;
-        const int32_t mt = a.mask_table ? a.mask_table[row] : -1;
-        if (mt >= 0) {
-            const int32_t ms = a.mask_state ? a.mask_state[row] : 0;
-            if (mt >= MAX_TABLES || !a.tables[mt].live || ms < 0 || (uint32_t)ms >= a.tables[mt].n_states ||
-                (unsigned long long)a.tables[mt].words_per_state * 32ull < V) bad = true;
-            else {
-                c.mw = a.tables[mt].words + (size_t)ms * a.tables[mt].words_per_state;
-                c.gflags = a.tables[mt].flags[ms];
+        const float temp = l.score ? 1.0f : u2f(get(0)), top_p = u2f(get(2)), freq = u2f(get(3)), pres = u2f(get(4)), rep = u2f(get(5)), u01 = u2f(get(6));
+        const uint32_t top_k = get(1), h0 = get(9), h1 = get(10);
+        const int32_t mt = (int32_t)get(7), ms = (int32_t)get(8);
+        if (tid == 0) {
+            c.row = row;
+            c.rowp = (const char*)a.logits + (size_t)row * a.row_stride * (BF16 ? 2 : 4);
+            c.temp = temp; c.top_k = top_k; c.top_p = top_p; c.freq = freq; c.pres = pres; c.rep = rep; c.u01 = u01;
+            c.t = fmaxf(c.temp, 1e-9f);
+            bool bad = !finite_f(c.temp) || !finite_f(c.top_p) || !finite_f(c.freq) || !finite_f(c.pres) || !finite_f(c.rep) || !(c.rep > 0.0f) ||
+                       !finite_f(c.u01);
+            c.mw = nullptr;
+            c.gflags = 0u;
+            if (mt >= 0) {
+                if (mt >= MAX_TABLES || !a.tables[mt].live || ms < 0 || (uint32_t)ms >= a.tables[mt].n_states ||
+                    (unsigned long long)a.tables[mt].words_per_state * 32ull < V) bad = true;
+                else {
+                    c.mw = a.tables[mt].words + (size_t)ms * a.tables[mt].words_per_state;
+                    c.gflags = a.tables[mt].flags[ms];
+                }
             }
+            c.h0 = h0;
+            c.nh = 0u;
+            if (h1 < c.h0 || h1 - c.h0 > a.max_history || (h1 > c.h0 && !a.hist_ids)) bad = true; else c.nh = h1 - c.h0;
+            if ((fabsf(c.freq) < 1e-6f && fabsf(c.pres) < 1e-6f) && c.rep == 1.0f) c.nh = 0u;
+            c.entries = 0u;
+            c.nonfinite = 0u;
+            c.n_terms = 0u;
+            c.state = WS_FIRST;
+            c.n_list = 0u; c.cut_x = INFINITY; c.n_kept = 0u; c.p_thr = -1.0f; c.id_thr = 0u; c.cut = 0u; c.m = -INFINITY; c.S = 0.0f; c.amax = 0u;
+            if (bad) { wresult_plain(a, row, ROW_BAD_PARAM, 0u, -INFINITY); c.state = WS_DONE; }
+            else if (c.nh > (uint32_t)W_MAX_HIST) { wleave(l, row); c.state = WS_DONE; }
         }
-        c.h0 = a.hist_offsets ? a.hist_offsets[row] : 0u;
-        const uint32_t h1 = a.hist_offsets ? a.hist_offsets[row + 1] : 0u;
-        c.nh = 0u;
-        if (h1 < c.h0 || h1 - c.h0 > a.max_history || (h1 > c.h0 && !a.hist_ids)) bad = true; else c.nh = h1 - c.h0;
-        if ((fabsf(c.freq) < 1e-6f && fabsf(c.pres) < 1e-6f) && c.rep == 1.0f) c.nh = 0u;
-        c.entries = 0u;
-        c.nonfinite = 0u;
-        c.n_terms = 0u;
-        c.state = WS_FIRST;
-        c.n_list = 0u; c.n_kept = 0u; c.p_thr = -1.0f; c.id_thr = 0u; c.cut = 0u; c.m = -INFINITY; c.S = 0.0f; c.amax = 0u;
-        if (bad) { wresult_plain(a, row, ROW_BAD_PARAM, 0u, -INFINITY); c.state = WS_DONE; }
-        else if (c.nh > (uint32_t)W_MAX_HIST) { wleave(l, row); c.state = WS_DONE; }
     }
     __syncthreads();
     const WideRow& c = sm.row;
@@ -624,8 +691,6 @@ __device__ __noinline__ void open_row(WideSmem& sm, const RowArgs& a, const Wide
             l.ent_xn[(size_t)slot * (W_MAX_HIST + 32) + at] = v;
         }
     }
-    if (c.state == WS_FIRST)
-        for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) l.hist[(size_t)slot * W_BUCKETS + b] = 0u;
     row_out(sm, l, slot);
 }
 
@@ -678,6 +743,52 @@ __device__ __noinline__ void maximum_row(WideSmem& sm, const RowArgs& a, const W
         else c.state = WS_SUM;
     }
     __syncthreads();
+    if (sm.row.state == WS_SUM && sm.row.cut_x == INFINITY && !l.score && sm.row.top_k != 0u && sm.row.top_k < V && sm.row.top_k <= (uint32_t)F_KMAX) {
+        // A row with a short top-k: the k-th largest of the parts' maxima is reached by at least k logits, so everything
+        // from a little below it on (for ties) is a superset of the top-k set, and nearly always a small one.  As in the
+        // streaming kernel: buckets of equal width between the smallest finite maximum and the largest.
+        const uint32_t k = sm.row.top_k, n_cells = 4u * n_regions;
+        const float* cell = reinterpret_cast<const float*>(l.cell + (size_t)slot * l.reg_stride);
+        uint32_t lo = W_NIL, fin = 0u;
+        float mine[8];
+        static_assert(4 * W_MAX_REGIONS == 8 * W_NT && W_NT == 1024, "eight maxima and one bucket per thread");
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const uint32_t i = tid + u * W_NT;
+            mine[u] = i < n_cells ? __ldcg(cell + i) : -INFINITY;
+            const uint32_t key = order_key(mine[u]);
+            if (key) { lo = umin(lo, key); fin++; }
+        }
+        lo = __reduce_min_sync(FULL, lo); fin = __reduce_add_sync(FULL, fin);
+        if (lane == 0) { sm.red_u[w] = lo; sm.red_v[w] = fin; }
+        if (tid == 0) sm.last = 0u;
+        __syncthreads();
+        lo = __reduce_min_sync(FULL, sm.red_u[lane]); fin = __reduce_add_sync(FULL, sm.red_v[lane]);
+        if (fin >= k) {   // CTA-uniform
+            const float lo_v = key_to_float(lo), scb = m > lo_v ? 1023.0f / (m - lo_v) : 0.0f;
+            uint32_t* bucket = sm.serial;   // (1024 of them)
+            bucket[tid] = 0u;
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (finite_f(mine[u])) atomicAdd(&bucket[min(1023u, (uint32_t)((mine[u] - lo_v) * scb))], 1u);
+            __syncthreads();
+            const uint32_t own = bucket[1023u - tid];
+            uint32_t inc = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= (uint32_t)o) inc += t;
+            }
+            if (lane == 31) sm.red_u[w] = inc;
+            __syncthreads();
+            const uint32_t x = sm.red_u[lane], above = __reduce_add_sync(FULL, lane < w ? x : 0u) + inc - own;
+            if (above < k && k <= above + own) sm.last = 1023u - tid;
+            __syncthreads();
+            const float bound = sm.last >= 1u && scb > 0.0f ? lo_v + ((float)sm.last - 1.0f) / scb : lo_v;
+            if (tid == 0) sm.row.cut_x = bound - 4.8e-7f * (fabsf(m - bound) + 4.0f * sm.row.t) - 4.8e-7f * (fabsf(bound) + fabsf(m));
+        }
+    }
     if (sm.row.state == WS_SUM) {
         const float sc = 1.44269504f / sm.row.t;
         make_table(sm, l, slot, n_regions, 0.001953125f + 1e-7f * fabsf(m * sc), [&](uint32_t r) {
@@ -720,11 +831,25 @@ __device__ __noinline__ void sum_row(WideSmem& sm, const RowArgs& a, const WideL
                 }
                 l.out_gather[c.row] = v;
             }
-        } else c.state = use_k || use_p ? WS_SELECT : WS_TOTAL;
+        } else c.state = c.cut_x < INFINITY && c.n_list <= (uint32_t)F_MCAP ? WS_DONE : use_k || use_p ? WS_SELECT : WS_TOTAL;
         if (c.state == WS_SELECT) atomicAdd(l.sync + 2, 1u);
         if (c.state == WS_TOTAL) atomicAdd(l.sync + 3, 1u);
     }
     __syncthreads();
+    if (sm.row.state == WS_DONE && !l.score) {   // the second pass has found the candidates
+        const uint32_t n = sm.row.n_list;
+        for (uint32_t j = threadIdx.x; j < n; j += W_NT) {
+            const unsigned long long v = __ldcg(l.list + (size_t)slot * l.list_stride + j);
+            sm.cand_id[j] = (uint32_t)v; sm.cand_p[j] = u2f((uint32_t)(v >> 32));
+        }
+        __syncthreads();
+        cta_finish<W_NT>(sm.fin, sm.exp_tab, a, sm.row.row, V, sm.cand_id, sm.cand_p, n, sm.row.m, sm.row.t, S, sm.row.top_k, sm.row.top_p,
+                         sm.row.u01, sm.row.amax, ROW_OK);
+    }
+    if (sm.row.state == WS_SELECT) {
+        for (uint32_t b = threadIdx.x; b < (uint32_t)W_BUCKETS; b += W_NT) l.hist[(size_t)slot * W_BUCKETS + b] = 0u;
+        if (threadIdx.x == 0) sm.row.n_list = 0u;
+    }
     if (sm.row.state == WS_TOTAL && !l.score) {
         const float q = S > 1e-9f ? 1.0f / S : 1.0f;
         make_table(sm, l, slot, n_regions, 0.001953125f, [&](uint32_t r) { return ((r + 1u < n_regions ? sm.start[r + 1u] : S) - sm.start[r]) * q; });
@@ -893,21 +1018,28 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
         }
         // the fold over the buckets, highest first: warp 0 adds whole buckets until it meets one that is not, or the one in
         // which top-p is reached; the CTA sorts that bucket and warp 0 adds its entries in order
+        uint32_t* ends = reinterpret_cast<uint32_t*>(&sm.stage[0][0]);   // where a bucket ends in the list
+        static_assert(sizeof(sm.stage) >= W_BUCKETS * 4, "one word per bucket");
+        for (uint32_t b = cut + tid; b < (uint32_t)W_BUCKETS; b += W_NT) ends[b] = __ldcg(hist + b);
         float R = 0.0f;                              // warp 0
         int b = W_BUCKETS - 1;
         bool found = false;
         for (;;) {
             __syncthreads();
             if (w == 0) {
-                bool stop = false;
-                while (b >= (int)cut && !stop) {
-                    const int mine = b - (int)lane;
-                    const uint32_t end = mine >= (int)cut ? __ldcg(hist + mine) : 0u;
-                    const uint32_t at = mine >= (int)cut && mine + 1 < W_BUCKETS ? __ldcg(hist + mine + 1) : 0u;
-                    const bool empty = mine < (int)cut || end == at;
-                    const uint32_t kb = empty ? 1u : f2u(sm.bs[mine]), rb = f2u(R);
-                    uint32_t inc = empty ? 0u : sm.bn[mine];
-                    const uint32_t own = inc;
+                // (four buckets per lane, one where that does not do)
+                for (int per = 4; b >= (int)cut;) {
+                    uint32_t own = 0u, kb = 1u;
+                    for (int u = 0; u < per; u++) {
+                        const int mine = b - (int)lane * per - u;
+                        if (mine < (int)cut || ends[mine] == (mine + 1 < W_BUCKETS ? ends[mine + 1] : 0u)) continue;   // empty
+                        const uint32_t k1 = f2u(sm.bs[mine]);
+                        kb = kb == 1u || kb == k1 ? k1 : 0u;
+                        own += sm.bn[mine];
+                    }
+                    const bool empty = kb == 1u;
+                    const uint32_t rb = f2u(R);
+                    uint32_t inc = own;
                     const unsigned bad = __ballot_sync(FULL, !(empty || (kb != 0u && kb == (rb & 0x7f800000u))));
                     uint32_t cnt = bad ? __ffs((int)bad) - 1u : 32u;
                     if (lane >= cnt) inc = 0u;
@@ -920,15 +1052,17 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
                     const unsigned over = __ballot_sync(FULL, !empty && lane < cnt && ((rb & 0x007fffffu) + inc >= 0x00800000u || (own != 0u && u2f(rb + inc) >= sm.row.top_p)));
                     if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
                     if (cnt) R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
-                    b -= (int)cnt;
-                    stop = cnt < 32u;
+                    b -= (int)cnt * per;
+                    if (cnt == 32u) continue;
+                    if (per == 1) break;
+                    per = 1;
                 }
                 if (lane == 0) sm.last = b >= (int)cut ? (uint32_t)b : W_NIL;
             }
             __syncthreads();
             const uint32_t sb = sm.last;
             if (sb == W_NIL) break;
-            const uint32_t end = __ldcg(hist + sb), at = sb + 1u < (uint32_t)W_BUCKETS ? __ldcg(hist + sb + 1u) : 0u, nb = end - at;
+            const uint32_t end = ends[sb], at = sb + 1u < (uint32_t)W_BUCKETS ? ends[sb + 1u] : 0u, nb = end - at;
             if (!sort_bucket(sm, l, slot, at, nb)) { leave = true; break; }
             if (w == 0) {
                 uint32_t hit = W_NIL;
@@ -1093,14 +1227,11 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
     using L = WLay<BF16, VEC>;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     float* buf = sm.stage[w];
+    rows_in(sm, l, n_rows);
     for (uint32_t i = w * sm.size + sm.rank; i < n_rows * n_regions; i += sm.size * WNW) {
         const uint32_t slot = i / n_regions, r = i - slot * n_regions, nv = min(V - r * W_REGION, (uint32_t)W_REGION);
-        const WideRow* rp = l.row + slot;
-        const uint32_t state = __ldcg(&rp->state);
-        WideRow c;
-        c.rowp = (const char*)__ldcg((const unsigned long long*)&rp->rowp);
-        c.mw = (const uint32_t*)__ldcg((const unsigned long long*)&rp->mw);
-        c.entries = __ldcg(&rp->entries);
+        const WideRow& c = sm.rows[slot];
+        const uint32_t state = c.state;
         float x[WL];
         if (PHASE == WP_FIRST) {
             if (state != WS_FIRST) continue;
@@ -1112,9 +1243,13 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
             float top = -INFINITY;
 #pragma unroll
             for (int j = 0; j < WL; j++) top = fmaxf(top, x[j]);
+            float part = top;   // of eight lanes
+#pragma unroll
+            for (int o = 4; o; o >>= 1) part = fmaxf(part, __shfl_xor_sync(FULL, part, o));
+            if ((lane & 7u) == 0u) reinterpret_cast<float*>(l.cell + (size_t)slot * l.reg_stride + r)[lane >> 3] = part;
             uint32_t key = f2u(top);
             key = __reduce_max_sync(FULL, key ^ (((uint32_t)((int32_t)key >> 31)) | 0x80000000u));   // monotone; -inf lowest
-            const float wm = u2f((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), sc = 1.44269504f / __ldcg(&rp->t);
+            const float wm = u2f((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), sc = 1.44269504f / c.t;
             float s = 0.0f;
             if (wm > -INFINITY) {
 #pragma unroll
@@ -1130,10 +1265,9 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
             continue;
         }
         if (state != (PHASE == WP_SUM ? WS_SUM : PHASE == WP_LIST ? WS_SELECT : WS_TOTAL)) continue;
-        c.m = __ldcg(&rp->m); c.t = __ldcg(&rp->t); c.S = __ldcg(&rp->S);
         if (PHASE == WP_FULL) {   // the whole log-softmax vector
-            const float log_sum = __ldcg(&rp->total);
-            const uint32_t row = __ldcg(&rp->row);
+            const float log_sum = c.total;
+            const uint32_t row = c.row;
             wload<BF16, VEC>(x, c.rowp, r, nv);
 #pragma unroll
             for (int j = 0; j < WL; j++) {
@@ -1145,15 +1279,41 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
         }
         Terms f;
         f.m = c.m; f.t = c.t; f.S = PHASE == WP_SUM ? -1.0f : c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
-        if (PHASE == WP_TOTAL) {
-            c.top_k = __ldcg(&rp->top_k); c.top_p = __ldcg(&rp->top_p); c.p_thr = __ldcg(&rp->p_thr); c.id_thr = __ldcg(&rp->id_thr);
-            f = kept_terms(c, V);
+        if (PHASE == WP_TOTAL) f = kept_terms(c, V);
+        wload<BF16, VEC>(x, c.rowp, r, nv);
+        uint2* seg = l.seg + (size_t)slot * l.reg_stride + r;
+        uint2 out = make_uint2(0u, PHASE == WP_LIST ? 0u : __ldcg(&seg->y));
+        wprocess<BF16, VEC>(buf, x, l, slot, c.mw, c.entries, r, nv);
+        if (PHASE == WP_SUM) {
+            const float cut = c.cut_x;
+#pragma unroll
+            for (int j = 0; j < WL; j++)
+                if (x[j] >= cut) {   // (rare)
+                    const uint32_t at = atomicAdd(&l.row[slot].n_list, 1u);
+                    if (at < (uint32_t)F_MCAP) l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
+                }
         }
-        wterms<BF16, VEC>(sm.exp_tab, buf, x, l, c, slot, V, r, f);
         if (PHASE == WP_SUM || PHASE == WP_TOTAL) {
-            uint2* seg = l.seg + (size_t)slot * l.reg_stride + r;
-            uint2 out = increments(x, __ldcg(&seg->y));
+            const uint32_t kb = out.y & ~W_DUAL;
+            if (kb) {
+                const Approx q = approx_of(f);
+                out.x = increments<BF16, VEC>(x, r * W_REGION, f, q, kb, sm.exp_tab);
+                uint32_t n1 = 0u;
+                if (out.x != W_TIE && (out.y & W_DUAL)) n1 = increments<BF16, VEC>(x, r * W_REGION, f, q, kb + 0x00800000u, sm.exp_tab);
+                if (out.x == W_TIE || n1 == W_TIE) out.y = 0u;
+                else if ((out.y & W_DUAL) && lane == 0) l.pre[(size_t)slot * l.reg_stride + r] = u2f(n1);
+            }
             if (out.y == 0u) {   // to be added term by term: the terms are left in id order, as far as there is room
+                bool zeros = true;
+#pragma unroll
+                for (int j = 0; j < WL; j++) {
+                    x[j] = term_of(x[j], r * W_REGION + L::off(lane, j), f, sm.exp_tab);
+                    zeros &= x[j] == 0.0f;
+                }
+                if (__all_sync(FULL, zeros)) {   // nothing but zeros
+                    if (lane == 0) *seg = make_uint2(0u, 1u);
+                    continue;
+                }
                 if (lane == 0) out.x = atomicAdd(&l.row[slot].n_terms, 1u) + 1u;
                 out.x = __shfl_sync(FULL, out.x, 0);
                 if (out.x > (uint32_t)W_TERMS) out.x = 0u;
@@ -1165,7 +1325,9 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
             }
             if (lane == 0) *seg = out;
         } else {   // WP_LIST
-            const uint32_t cut = __ldcg(&rp->cut) & 0x7fffffffu;
+            const uint32_t cut = c.cut & 0x7fffffffu;
+#pragma unroll
+            for (int j = 0; j < WL; j++) x[j] = term_of(x[j], r * W_REGION + L::off(lane, j), f, sm.exp_tab);
 #pragma unroll
             for (int j = 0; j < WL; j++)
                 if (x[j] > 0.0f && bucket_of(x[j]) >= cut) {
@@ -1180,23 +1342,29 @@ template <bool BF16, bool VEC>
 __device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
     const uint32_t tid = threadIdx.x, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     const uint32_t tiles = (n_regions + WNW - 1) / WNW;
+    rows_in(sm, l, n_rows);
     for (uint32_t i = sm.rank; i < n_rows * tiles; i += sm.size) {   // CTA-uniform
         const uint32_t slot = i / tiles, r = (i - slot * tiles) * WNW + w;
-        const WideRow* rp = l.row + slot;
-        if (__ldcg(&rp->state) != WS_SELECT) continue;
+        const WideRow& c = sm.rows[slot];
+        if (c.state != WS_SELECT) continue;
         for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) sm.bn[b] = 0u;
         __syncthreads();
         if (r < n_regions) {
-            WideRow c;
-            c.rowp = (const char*)__ldcg((const unsigned long long*)&rp->rowp);
-            c.mw = (const uint32_t*)__ldcg((const unsigned long long*)&rp->mw);
-            c.entries = __ldcg(&rp->entries);
             Terms f;
-            f.m = __ldcg(&rp->m); f.t = __ldcg(&rp->t); f.S = __ldcg(&rp->S); f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+            f.m = c.m; f.t = c.t; f.S = c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+            const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
             float x[WL];
-            wterms<BF16, VEC>(sm.exp_tab, sm.stage[w], x, l, c, slot, V, r, f);
+            wload<BF16, VEC>(x, c.rowp, r, nv);
+            wprocess<BF16, VEC>(sm.stage[w], x, l, slot, c.mw, c.entries, r, nv);
+            // the hardware's exp2 decides the bucket, unless the probability lies close to a border
+            const Approx q = approx_of(f);
+            const float eps = (4.0f * fabsf(q.k0) + 200.0f) * 2.384185791015625e-07f;   // (probabilities from 2^-40 on count)
 #pragma unroll
-            for (int j = 0; j < WL; j++) if (x[j] > 0.0f) atomicAdd(&sm.bn[bucket_of(x[j])], 1u);
+            for (int j = 0; j < WL; j++) {
+                float p = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, q.k0));
+                if (bucket_of(p * (1.0f - eps)) != bucket_of(p * (1.0f + eps)) || !(p > 1e-30f)) p = term_of(x[j], 0u, f, sm.exp_tab);
+                if (p > 0.0f) atomicAdd(&sm.bn[bucket_of(p)], 1u);
+            }
         }
         __syncthreads();
         for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT)

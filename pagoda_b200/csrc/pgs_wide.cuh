@@ -29,6 +29,7 @@ struct WideRow {
     float m, S, total;
     uint32_t amax;
     uint32_t cut, n_list;    // entries in buckets >= cut
+    float cut_x;             // rows with a short top-k: the second pass lists the logits from here on (n_list of them)
     uint32_t n_terms;        // segments whose terms are in WideLaunch::terms
     float p_thr;             // kept: p > p_thr, or p == p_thr and id <= id_thr
     uint32_t id_thr, n_kept;
@@ -38,6 +39,7 @@ enum : uint32_t { WS_FIRST = 0u, WS_SUM = 1u, WS_SELECT = 2u, WS_TOTAL = 3u, WS_
 struct WideLaunch {
     WideRow* row;               // [W_CHUNK]
     float2* reg;                // [W_CHUNK][n_regions]: a region's maximum, its plain sum
+    float4* cell;               // [W_CHUNK][n_regions]: the maxima of four parts of the region
     uint2* seg;                 // [W_CHUNK][n_regions]: increments in ulps, binade (0: add term by term)
     float* pre;                 // [W_CHUNK][n_regions]: estimate of the running value at the region's start
     float* terms;               // [W_CHUNK][W_TERMS][W_REGION]: terms of segments that are added one by one
