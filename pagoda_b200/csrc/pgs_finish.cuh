@@ -144,6 +144,16 @@ template <int T, int LIMIT, int E = 1>
 __device__ __forceinline__ void cta_sort_shared(unsigned long long* keys, uint32_t n) {
     if constexpr (T * E < LIMIT)
         if (n > (uint32_t)(T * E)) { cta_sort_shared<T, LIMIT, 2 * E>(keys, n); return; }
+    if (E == 1 && n <= 32u) {   // one warp
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            unsigned long long v1[1] = {threadIdx.x < n ? keys[threadIdx.x] : ~0ull};
+            cta_sort<32, 1>(v1, keys);
+            keys[threadIdx.x] = v1[0];
+        }
+        __syncthreads();
+        return;
+    }
     unsigned long long v[E];
     __syncthreads();
 #pragma unroll

@@ -142,6 +142,7 @@ __device__ __forceinline__ float ex2_approx_ftz(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 #endif
 
 // Monotone map float -> uint32 (larger float = larger key).  Non-finite values get key 0, below

@@ -258,13 +258,15 @@ __device__ __forceinline__ Approx approx_of(const Terms& f) {
     return q;
 }
 // The increment of a term is its value in ulps, rounded: the hardware's exp2 decides that unless it lands close to half an
-// ulp.  The error of its argument is a few 2^-24 of |d * c| and |k|, that of the exp2 below 2^-21; the margin is four times
-// as wide.  Nearly all terms are far below the running value, so that about one of a region's 512 is in doubt and takes the
+// ulp.  Relative errors, with p = d * c and only terms above a quarter of an ulp (|p| <= |k| + 2) of interest: rounding of
+// the argument 4.2e-8 (|k| + 2), of c 5.3e-8 |p|, of the reference's quotient 4.2e-8 |p|, of k and k0 4.2e-8 each, exp2
+// 2.4e-7, the reference's exp and division 1.2e-7; less than eps together.  Nearly all terms are far below the running value, so that about one of a region's 512 is in doubt and takes the
 // exact exponential, which costs ten times as much (64 rows of 151936: 25 us for all of them).
 template <bool BF16, bool VEC>
 __device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id0, const Terms& f, const Approx& q, uint32_t kb, const unsigned long long* tab) {
-    const float k = q.k0 - (float)((int)(kb >> 23) - 127 - 23), eps = (2.0f * fabsf(k) + 2.0f * fabsf(q.k0) + 12.0f) * 2.384185791015625e-07f;
-    const float p_lim = f.filter ? f.p_thr / u2f(kb) * 8388608.0f : 0.0f, slack = 4.0f * eps * p_lim;   // the threshold in ulps
+    const float k = q.k0 - (float)((int)(kb >> 23) - 127 - 23), eps = 2e-7f * fabsf(k) + 1e-7f * fabsf(q.k0) + 1e-6f;
+    const float p_lim = f.filter ? f.p_thr / u2f(kb) * 8388608.0f : 0.0f;   // the threshold in ulps
+    const float slack = (4.0f * eps + 4e-6f) * p_lim;
     uint32_t n = 0u, doubt = 0u;
 #pragma unroll
     for (int j = 0; j < WL; j++) {
@@ -286,10 +288,7 @@ __device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id
             float xj = x[0];
 #pragma unroll
             for (int u = 1; u < WL; u++) if (u == j) xj = x[u];
-            uint32_t o = 0u;
-#pragma unroll
-            for (int u = 0; u < WL; u++) if (u == j) o = WLay<BF16, VEC>::off(threadIdx.x & 31u, u);
-            good &= increment(term_of(xj, id0 + o, f, tab), kb, n);
+            good &= increment(term_of(xj, id0 + WLay<BF16, VEC>::off(threadIdx.x & 31u, (uint32_t)j), f, tab), kb, n);
             doubt &= doubt - 1u;
         }
     }
@@ -341,30 +340,29 @@ __device__ __forceinline__ Runs make_runs(const float (&v)[WL], float R0) {
 // Adds the runs to the exact running value R; one warp, the same result in all lanes.
 __device__ __forceinline__ float add_runs(float R, const Runs& s, const float (&v)[WL]) {
     const uint32_t lane = threadIdx.x & 31, head = s.head & 31u;
+    const bool zero = (s.head >> 31) != 0u;
     uint32_t pos = 0u;
 #pragma unroll 1
     while (pos < 32u) {
+        // The group that begins here, as far as the running value stays in its binade; and what the first lane in which it
+        // does not (or the estimate missed the binade) makes of it: every lane adds its run to the value it would begin with.
         const uint32_t rb = f2u(R), d = (rb & 1u) ? s.c1 : s.c0;
-        // the group that begins here, as far as the running value stays in its binade
-        const bool fits = lane >= pos && head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u;
+        const bool fits = lane >= pos && (zero || (head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u));
+        const uint32_t own = zero ? 0u : d;   // (zeros: the group's increments up to here, which the lane before has too)
         const unsigned ok = __ballot_sync(FULL, fits) >> pos;
-        uint32_t n = ~ok ? __ffs((int)~ok) - 1u : 32u;
-        if (n) {
-            if (n > 32u - pos) n = 32u - pos;
-            R = u2f(rb + __shfl_sync(FULL, d, (int)(pos + n - 1u)));
-            pos += n;
-            continue;
-        }
-        // zeros change nothing; otherwise the running value changes binade in this run, or the estimate missed it
-        const unsigned zero = __ballot_sync(FULL, (s.head >> 31) != 0u) >> pos;
-        if (zero & 1u) { pos += ~zero ? __ffs((int)~zero) - 1u : 32u; continue; }
-        float r = R;
-        if (lane == pos) {
+        const uint32_t n = ~ok ? min((uint32_t)__ffs((int)~ok) - 1u, 32u - pos) : 32u - pos;
+        uint32_t last = __reduce_max_sync(FULL, fits && lane < pos + n ? own : 0u);   // (increments only grow inside a group)
+        float r = u2f(rb + last);
+        pos += n;
+        if (pos < 32u) {
+            if (lane == pos) {
 #pragma unroll
-            for (int j = 0; j < WL; j++) r = fadd(r, v[j]);
+                for (int j = 0; j < WL; j++) r = fadd(r, v[j]);
+            }
+            r = __shfl_sync(FULL, r, (int)pos);
+            pos++;
         }
-        R = __shfl_sync(FULL, r, (int)pos);
-        pos++;
+        R = r;
     }
     return R;
 }
@@ -394,16 +392,20 @@ __device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_
         sm.pre[r] = __ldcg(l.pre + (size_t)slot * l.reg_stride + r);
     }
     __syncthreads();
-    // segments to be added term by term, in order (one warp: there are few)
-    if (w == 0) {
-        uint32_t n = 0u;
-        for (uint32_t r0 = 0; r0 < n_regions; r0 += 32) {
-            const bool s = r0 + lane < n_regions && sm.seg[r0 + lane].y == 0u;
-            const unsigned b = __ballot_sync(FULL, s);
-            if (s) sm.serial[n + __popc(b & ((1u << lane) - 1u))] = r0 + lane;
-            n += __popc(b);
+    // segments to be added term by term, in order
+    {
+        uint32_t before = 0u;
+        for (uint32_t r0 = 0; r0 < n_regions; r0 += W_NT) {
+            const bool is = r0 + tid < n_regions && sm.seg[r0 + tid].y == 0u;
+            const unsigned in_warp = __ballot_sync(FULL, is);
+            if (lane == 0) sm.red_u[w] = __popc(in_warp);
+            __syncthreads();
+            const uint32_t c = sm.red_u[lane], mine = __reduce_add_sync(FULL, lane < w ? c : 0u);
+            if (is) sm.serial[before + mine + __popc(in_warp & ((1u << lane) - 1u))] = r0 + tid;
+            before += __reduce_add_sync(FULL, c);
+            __syncthreads();
         }
-        if (lane == 0) sm.n_serial = n;
+        if (tid == 0) sm.n_serial = before;
     }
     __syncthreads();
     const uint32_t n_serial = sm.n_serial;
@@ -1027,8 +1029,8 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
         for (;;) {
             __syncthreads();
             if (w == 0) {
-                // (four buckets per lane, one where that does not do)
-                for (int per = 4; b >= (int)cut;) {
+                // (eight buckets per lane, one where that does not do)
+                for (int per = 8; b >= (int)cut;) {
                     uint32_t own = 0u, kb = 1u;
                     for (int u = 0; u < per; u++) {
                         const int mine = b - (int)lane * per - u;
@@ -1053,7 +1055,7 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
                     if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
                     if (cnt) R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
                     b -= (int)cnt * per;
-                    if (cnt == 32u) continue;
+                    if (cnt == 32u) { per = 8; continue; }
                     if (per == 1) break;
                     per = 1;
                 }
@@ -1232,6 +1234,11 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
         const uint32_t slot = i / n_regions, r = i - slot * n_regions, nv = min(V - r * W_REGION, (uint32_t)W_REGION);
         const WideRow& c = sm.rows[slot];
         const uint32_t state = c.state;
+        {   // the region after this one, a 128-byte line per lane
+            const uint32_t i1 = i + sm.size * WNW, slot1 = i1 / n_regions, r1 = i1 - slot1 * n_regions;
+            const uint32_t at = r1 * W_REGION + lane * (128u / L::ESZ);
+            if (i1 < n_rows * n_regions && lane < W_REGION * L::ESZ / 128u && at < V) prefetch_l2(sm.rows[slot1].rowp + (size_t)at * L::ESZ);
+        }
         float x[WL];
         if (PHASE == WP_FIRST) {
             if (state != WS_FIRST) continue;
@@ -1326,50 +1333,68 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
             if (lane == 0) *seg = out;
         } else {   // WP_LIST
             const uint32_t cut = c.cut & 0x7fffffffu;
-#pragma unroll
-            for (int j = 0; j < WL; j++) x[j] = term_of(x[j], r * W_REGION + L::off(lane, j), f, sm.exp_tab);
+            // the exact probability only of those that may lie in one of the buckets
+            const Approx q = approx_of(f);
+            const float from = cut ? bucket_floor(cut) * (1.0f - (4.0f * fabsf(q.k0) + 200.0f) * 2.4e-7f) : 0.0f;
+            uint32_t may = 0u;
 #pragma unroll
             for (int j = 0; j < WL; j++)
-                if (x[j] > 0.0f && bucket_of(x[j]) >= cut) {
-                    const uint32_t at = atomicAdd(l.hist + (size_t)slot * W_BUCKETS + bucket_of(x[j]), 1u);
-                    l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
+                if (x[j] > -INFINITY && ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, q.k0)) >= from) may |= 1u << j;
+            while (may) {
+                const uint32_t j = __ffs((int)may) - 1u;
+                may &= may - 1u;
+                float p = x[0];
+#pragma unroll
+                for (int u = 1; u < WL; u++) if ((uint32_t)u == j) p = x[u];
+                p = term_of(p, 0u, f, sm.exp_tab);
+                const uint32_t b = bucket_of(p);
+                if (p > 0.0f && b >= cut) {
+                    const uint32_t at = atomicAdd(l.hist + (size_t)slot * W_BUCKETS + b, 1u);
+                    l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(p) << 32) | (r * W_REGION + L::off(lane, j));
                 }
+            }
         }
     }
 }
 
+// Histogram of the probabilities of the rows that select by them.  Every CTA takes an equal run of the rows' regions, so
+// that most counting happens in shared memory and the buckets are flushed once or twice.
 template <bool BF16, bool VEC>
 __device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
     const uint32_t tid = threadIdx.x, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
-    const uint32_t tiles = (n_regions + WNW - 1) / WNW;
     rows_in(sm, l, n_rows);
-    for (uint32_t i = sm.rank; i < n_rows * tiles; i += sm.size) {   // CTA-uniform
-        const uint32_t slot = i / tiles, r = (i - slot * tiles) * WNW + w;
+    uint32_t n_sel = 0u;
+    for (uint32_t s = 0; s < n_rows; s++) n_sel += sm.rows[s].state == WS_SELECT;
+    const uint32_t per = (n_sel * n_regions + sm.size - 1u) / sm.size, lo = min(sm.rank * per, n_sel * n_regions), hi = min(lo + per, n_sel * n_regions);
+    for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) sm.bn[b] = 0u;
+    uint32_t first = 0u;   // of the row's regions, among all
+    for (uint32_t slot = 0; slot < n_rows; slot++) {   // CTA-uniform
         const WideRow& c = sm.rows[slot];
         if (c.state != WS_SELECT) continue;
-        for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT) sm.bn[b] = 0u;
+        const uint32_t r0 = max(lo, first) - first, r1 = min(hi, first + n_regions) > first ? min(hi, first + n_regions) - first : 0u;
+        first += n_regions;
+        if (r0 >= r1) continue;
         __syncthreads();
-        if (r < n_regions) {
-            Terms f;
-            f.m = c.m; f.t = c.t; f.S = c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+        Terms f;
+        f.m = c.m; f.t = c.t; f.S = c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
+        const Approx q = approx_of(f);
+        const float eps = (4.0f * fabsf(q.k0) + 200.0f) * 2.4e-7f;   // (probabilities from 2^-40 on count)
+        for (uint32_t r = r0 + w; r < r1; r += WNW) {
             const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
             float x[WL];
             wload<BF16, VEC>(x, c.rowp, r, nv);
             wprocess<BF16, VEC>(sm.stage[w], x, l, slot, c.mw, c.entries, r, nv);
             // the hardware's exp2 decides the bucket, unless the probability lies close to a border
-            const Approx q = approx_of(f);
-            const float eps = (4.0f * fabsf(q.k0) + 200.0f) * 2.384185791015625e-07f;   // (probabilities from 2^-40 on count)
 #pragma unroll
             for (int j = 0; j < WL; j++) {
                 float p = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, q.k0));
-                if (bucket_of(p * (1.0f - eps)) != bucket_of(p * (1.0f + eps)) || !(p > 1e-30f)) p = term_of(x[j], 0u, f, sm.exp_tab);
+                if (x[j] > -INFINITY && (bucket_of(p * (1.0f - eps)) != bucket_of(p * (1.0f + eps)) || p < 1e-30f)) p = term_of(x[j], 0u, f, sm.exp_tab);
                 if (p > 0.0f) atomicAdd(&sm.bn[bucket_of(p)], 1u);
             }
         }
         __syncthreads();
         for (uint32_t b = tid; b < (uint32_t)W_BUCKETS; b += W_NT)
-            if (sm.bn[b]) atomicAdd(l.hist + (size_t)slot * W_BUCKETS + b, sm.bn[b]);
-        __syncthreads();
+            if (sm.bn[b]) { atomicAdd(l.hist + (size_t)slot * W_BUCKETS + b, sm.bn[b]); sm.bn[b] = 0u; }
     }
 }
 
