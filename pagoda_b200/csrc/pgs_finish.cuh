@@ -73,11 +73,148 @@ __device__ __forceinline__ int warp_find(const float* pre, int n, int mode, floa
     return -1;
 }
 
-// How many of the n ranked probabilities the top-p walk keeps (sampler.rs:130-150); one warp.  One lane adds, and stops
-// where top-p is reached.
-__device__ __forceinline__ uint32_t warp_top_p(const float* p, uint32_t n, float top_p) {
+constexpr int RUN = 16;   // consecutive terms of a lane
+// 32 runs of terms, one per lane, ready to be added to a running value: lanes whose runs are estimated to begin in one
+// binade form a group, and each lane holds the increments from the group's first lane up to and including its own, for an
+// even and for an odd running value there.
+struct Runs {
+    uint32_t k;         // bits of the estimated binade's lower end (0: none)
+    uint32_t c0, c1;    // SEQ_SAT: leaves the binade
+    uint32_t head;      // first lane of the group; bit 31: nothing but zeros in this lane's run
+};
+
+// v: this lane's run; R0: estimate of the running value at the first lane's run
+__device__ __forceinline__ Runs make_runs(const float (&v)[RUN], float R0) {
+    const uint32_t lane = threadIdx.x & 31;
+    float c = 0.0f;
+#pragma unroll
+    for (int j = 0; j < RUN; j++) c += v[j];
+    float inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    Runs s;
+    s.k = f2u(R0 + (inc - c)) & 0x7f800000u;
+    if (s.k == 0x7f800000u) s.k = 0u;
+    s.c0 = s.c1 = SEQ_SAT;
+    if (c == 0.0f) s.c0 = s.c1 = 0u;
+    else if (s.k) {
+        float a0 = u2f(s.k), a1 = u2f(s.k + 1u);
+#pragma unroll
+        for (int j = 0; j < RUN; j++) { a0 = fadd(a0, v[j]); a1 = fadd(a1, v[j]); }
+        if ((f2u(a0) & 0x7f800000u) == s.k) s.c0 = f2u(a0) - s.k;
+        if ((f2u(a1) & 0x7f800000u) == s.k) s.c1 = f2u(a1) - (s.k + 1u);
+    }
+    const uint32_t before = __shfl_up_sync(FULL, s.k, 1);
+    const unsigned heads = __ballot_sync(FULL, lane == 0u || before != s.k);
+    s.head = 31u - __clz((int)(heads & (0xffffffffu >> (31u - lane))));
+    // compose(left, right)(p) = left_p + right_{(p + left_p) & 1}, inside the group
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t l0 = __shfl_up_sync(FULL, s.c0, o), l1 = __shfl_up_sync(FULL, s.c1, o);
+        if (lane >= s.head + (uint32_t)o) {
+            const uint32_t n0 = l0 + ((l0 & 1u) ? s.c1 : s.c0), n1 = l1 + (((l1 + 1u) & 1u) ? s.c1 : s.c0);
+            s.c0 = (l0 >= SEQ_SAT || n0 >= SEQ_SAT) ? SEQ_SAT : n0;
+            s.c1 = (l1 >= SEQ_SAT || n1 >= SEQ_SAT) ? SEQ_SAT : n1;
+        }
+    }
+    if (c == 0.0f) s.head |= 0x80000000u;
+    return s;
+}
+
+// Adds the runs to the exact running value R; one warp, the same result in all lanes.  ends: the running value behind every
+// run (optional).
+__device__ __forceinline__ float add_runs(float R, const Runs& s, const float (&v)[RUN], float* ends = nullptr) {
+    const uint32_t lane = threadIdx.x & 31, head = s.head & 31u;
+    const bool zero = (s.head >> 31) != 0u;
+    uint32_t pos = 0u;
+#pragma unroll 1
+    while (pos < 32u) {
+        // The group that begins here, as far as the running value stays in its binade; and what the first lane in which it
+        // does not (or the estimate missed the binade) makes of it: every lane adds its run to the value it would begin with.
+        const uint32_t rb = f2u(R), d = (rb & 1u) ? s.c1 : s.c0;
+        const bool fits = lane >= pos && (zero || (head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u));
+        const uint32_t own = zero ? 0u : d;   // (zeros: the group's increments up to here, which the lane before has too)
+        const unsigned ok = __ballot_sync(FULL, fits) >> pos;
+        const uint32_t n = ~ok ? min((uint32_t)__ffs((int)~ok) - 1u, 32u - pos) : 32u - pos;
+        uint32_t last = __reduce_max_sync(FULL, fits && lane < pos + n ? own : 0u);   // (increments only grow inside a group)
+        float r = u2f(rb + last);
+        if (ends) {
+            uint32_t e = fits ? own : 0u;
+            const unsigned zeros = __ballot_sync(FULL, fits && zero);
+            if (zeros) {   // what the runs before come to
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, e, o);
+                    if (lane >= (uint32_t)o) e = umax(e, t);
+                }
+            }
+            if (lane >= pos && lane < pos + n) ends[lane] = u2f(rb + e);
+        }
+        pos += n;
+        if (pos < 32u) {
+            if (lane == pos) {
+#pragma unroll
+                for (int j = 0; j < RUN; j++) r = fadd(r, v[j]);
+            }
+            r = __shfl_sync(FULL, r, (int)pos);
+            if (ends && lane == 0) ends[pos] = r;
+            pos++;
+        }
+        R = r;
+    }
+    return R;
+}
+
+// Exact left fold of n shared-memory floats by one warp, 512 at a time as runs of 16; ends[r]: the running value behind
+// run r (exact).  Stops where the running value reaches `goal`; returns what it has come to.  v: readable up to the next
+// multiple of 4.  (512 terms: the additions one by one take 4000 cycles.)
+__device__ __forceinline__ float warp_fold(const float* v, uint32_t n, float goal, float* ends) {
+    const uint32_t lane = threadIdx.x & 31;
+    float R = 0.0f;
+#pragma unroll 1
+    for (uint32_t base = 0; base < n && !(R >= goal); base += 32u * RUN) {
+        float x[RUN];
+#pragma unroll
+        for (int j = 0; j < RUN; j += 4) {
+            const uint32_t i = base + lane * RUN + j;
+            const float4 q = i < n ? *reinterpret_cast<const float4*>(v + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            x[j] = q.x; x[j + 1] = i + 1 < n ? q.y : 0.0f; x[j + 2] = i + 2 < n ? q.z : 0.0f; x[j + 3] = i + 3 < n ? q.w : 0.0f;
+        }
+        R = add_runs(R, make_runs(x, R), x, ends + base / RUN);
+    }
+    return R;
+}
+// First of the n terms behind which the running value satisfies the predicate, given the running values behind the runs; -1:
+// none.  One warp.
+__device__ __forceinline__ int warp_fold_find(const float* v, uint32_t n, const float* ends, int mode, float target) {
+    const int run = warp_find(ends, (int)((n + RUN - 1) / RUN), mode, target);
+    if (run < 0) return -1;
+    int at = -1;
+    float acc = run ? ends[run - 1] : 0.0f;
+    for (uint32_t j = run * RUN; j < min(n, (uint32_t)(run + 1) * RUN); j++) {
+        acc = fadd(acc, v[j]);
+        if (seq_pred(mode, acc, target)) { at = (int)j; break; }
+    }
+    return at;
+}
+
+// How many of the n ranked probabilities the top-p walk keeps (sampler.rs:130-150); one warp.  Short lists: one lane adds,
+// and stops where top-p is reached (its loads do not wait for the additions).
+constexpr uint32_t F_SERIAL = 160;   // up to here one lane's additions are as fast as the runs, whose code is seldom in the cache
+__device__ __forceinline__ uint32_t warp_top_p(const float* p, uint32_t n, float top_p, float* ends) {
     uint32_t keep = n;
-    if (!(top_p >= 1.0f) && (threadIdx.x & 31) == 0) {
+    if (top_p >= 1.0f) return keep;
+    if (n > F_SERIAL) {
+        const float R = warp_fold(p, n, top_p, ends);
+        __syncwarp();
+        if (R >= top_p) keep = (uint32_t)warp_fold_find(p, n, ends, SEQ_FIND_GE, top_p) + 1u;
+        __syncwarp();
+        return keep;
+    }
+    if ((threadIdx.x & 31) == 0) {
         float acc = 0.0f;
 #pragma unroll 1
         for (uint32_t j0 = 0; j0 < n; j0 += 8) {
@@ -170,9 +307,14 @@ template <class FA>
 __device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, float m, float S, float u01, uint32_t amax,
                                             int status) {
     const int lane = threadIdx.x & 31;
-    const float total = warp_prefix(f.sp, (int)n, f.fp);
+    const bool runs = n > F_SERIAL;
+    const float total = runs ? warp_fold(f.sp, n, INFINITY, f.fp) : warp_prefix(f.sp, (int)n, f.fp);
+    __syncwarp();
     int pick = -1;
-    if (total > 1e-9f) pick = warp_find(f.fp, (int)n, SEQ_FIND_GT, fmul(u01, total));
+    if (total > 1e-9f) {
+        const float target = fmul(u01, total);
+        pick = runs ? warp_fold_find(f.sp, n, f.fp, SEQ_FIND_GT, target) : warp_find(f.fp, (int)n, SEQ_FIND_GT, target);
+    }
     if (lane == 0) {
         uint32_t token = amax;
         int drew = 0;
@@ -226,35 +368,41 @@ __device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint3
     const int lane = threadIdx.x & 31;
     const uint32_t n_live = cta_top_k<T>(f, n, top_k);
     if (threadIdx.x >= 32) return;
-    const uint32_t keep = warp_top_p(f.rp, n_live, top_p);
+    const uint32_t keep = warp_top_p(f.rp, n_live, top_p, f.fp);
     for (uint32_t j = keep + lane; j < n; j += 32) f.sp[f.rpos[j]] = 0.0f;
     __syncwarp();
     warp_finish(f, a, row, V, n, m, S, u01, amax, status);
 }
 
-// Candidates of one row -> token.  Called by every thread of a CTA of T threads (T >= F_QUAD, a multiple of 32)
+// Candidates of one row -> token.  Called by every thread of a CTA of T threads (a multiple of 32)
 // with a barrier in front; cand_id: the row's n <= F_MCAP candidates in any order, prob(j) their probabilities (memory
 // outside of `f`); V: the full vocabulary size (the CDF walk falls through to V - 1, sampler.rs:54).  Ends with the row's
 // outputs written; the caller needs a barrier before it reuses `f` or the candidate arrays.
 template <int T, class FA, class P>
 __device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32_t row, uint32_t V, const uint32_t* cand_id, P prob, uint32_t n,
                                                  float m, float S, uint32_t top_k, float top_p, float u01, uint32_t amax, int status) {
-    static_assert(T >= F_QUAD && T % 32 == 0, "one thread per candidate of a short list");
+    static_assert(T % 32 == 0 && F_QUAD % T == 0 || T > F_QUAD, "whole warps");
     const int tid = threadIdx.x;
     if (tid == 0) f.n_live = 0u;
     if (n <= (uint32_t)F_QUAD) {
         // short list: every candidate counts the candidates in front of it, by id and by (probability descending,
         // id ascending)
-        uint32_t my_id = 0u;
-        float my_p = 0.0f;
-        if ((uint32_t)tid < n) {
-            my_id = cand_id[tid];
-            my_p = prob((uint32_t)tid);
-            f.key[tid] = ((unsigned long long)f2u(my_p) << 32) | (unsigned long long)(0xffffffffu - my_id);   // p >= 0
+        constexpr int U = T >= F_QUAD ? 1 : F_QUAD / T;
+        uint32_t my_id[U];
+        float my_p[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t j = tid + u * T;
+            if (j >= n) continue;
+            my_id[u] = cand_id[j];
+            my_p[u] = prob(j);
+            f.key[j] = ((unsigned long long)f2u(my_p[u]) << 32) | (unsigned long long)(0xffffffffu - my_id[u]);   // p >= 0
         }
         __syncthreads();
-        if ((uint32_t)tid < n) {
-            const unsigned long long kj = f.key[tid];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (tid + u * T >= n) continue;
+            const unsigned long long kj = f.key[tid + u * T];
             uint32_t r_id = 0, r_p = 0;
 #pragma unroll 8
             for (uint32_t o = 0; o < n; o++) {   // broadcast loads, independent of one another
@@ -262,7 +410,7 @@ __device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32
                 r_p += ko > kj;
                 r_id += (uint32_t)ko > (uint32_t)kj;   // larger ~id = smaller id
             }
-            f.sid[r_id] = my_id; f.sp[r_id] = my_p; f.rp[r_p] = my_p; f.rpos[r_p] = r_id;
+            f.sid[r_id] = my_id[u]; f.sp[r_id] = my_p[u]; f.rp[r_p] = my_p[u]; f.rpos[r_p] = r_id;
         }
     } else {
         // long list: sorted by (probability descending, id ascending); what top-k and top-p leave is put into id order, by
@@ -276,18 +424,18 @@ __device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32
         }
         const uint32_t n_live = cta_top_k<T>(f, n, top_k);
         if (tid < 32) {
-            const uint32_t keep = warp_top_p(f.rp, n_live, top_p);
+            const uint32_t keep = warp_top_p(f.rp, n_live, top_p, f.fp);
             if (tid == 0) f.n_live = keep;
         }
         __syncthreads();
         const uint32_t keep = f.n_live;
         if (keep <= (uint32_t)F_QUAD) {
-            if ((uint32_t)tid < keep) {
-                const uint32_t id = f.rpos[tid];
+            for (uint32_t r = tid; r < keep; r += T) {
+                const uint32_t id = f.rpos[r];
                 uint32_t at = 0;
 #pragma unroll 8
                 for (uint32_t o = 0; o < keep; o++) at += f.rpos[o] < id;
-                f.sid[at] = id; f.sp[at] = f.rp[tid];
+                f.sid[at] = id; f.sp[at] = f.rp[r];
             }
             __syncthreads();
         } else {

@@ -64,14 +64,17 @@ __global__ void __launch_bounds__(256) tp_push_kernel(const TpArgs a) {
     }
 }
 
-constexpr int TP_MT = 256;    // threads of the merge kernel
+// Most of a row's time is one warp's: few threads per row, so that an SM holds eight rows (of 256 threads it held four, and
+// 1024 rows of 8 x 64 candidates needed a second wave).
+constexpr int TP_MT = 128;
 constexpr int TP_MCAP = TP_MAX_SHARDS * 128;   // candidates of all shards together (cand <= 128)
 
+template <int CAP>
 struct TpMergeSmem {
-    FinishArraysT<TP_MCAP> fin;
+    FinishArraysT<CAP> fin;
     unsigned long long exp_tab[32];
-    uint32_t cid[TP_MCAP];
-    float cx[TP_MCAP];
+    uint32_t cid[CAP];
+    float cx[CAP];
     float M, S;
     uint32_t amax, n;
     int fault;   // the row's status when it is not ROW_OK
@@ -81,11 +84,14 @@ struct TpMergeSmem {
 };
 
 
-__global__ void __launch_bounds__(TP_MT, 4) tp_merge_kernel(const TpArgs a, const TpOut o) {
+// CAP: candidates of all shards together, at most
+template <int CAP>
+__global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, const TpOut o) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    TpMergeSmem& sm = *reinterpret_cast<TpMergeSmem*>(smem_raw);
+    TpMergeSmem<CAP>& sm = *reinterpret_cast<TpMergeSmem<CAP>*>(smem_raw);
     const int tid = threadIdx.x;
     const uint32_t row = blockIdx.x;
+    cudaGridDependencySynchronize();
     const float temp = a.temperature ? a.temperature[row] : 0.0f;
     const float t = fmaxf(temp, 1e-9f);
     if (tid < 32) sm.exp_tab[tid] = kExp2TableDev[tid];
@@ -118,7 +124,7 @@ __global__ void __launch_bounds__(TP_MT, 4) tp_merge_kernel(const TpArgs a, cons
     // every record slot of the row is requested at once (one trip to memory): the heads by the first threads, the
     // candidate slots one or two per thread; which of the slots are filled is known once the heads are in
     if ((uint32_t)tid < a.n_shards) sm.hd[tid] = *rec(tid);
-    constexpr int SLOTS = (TP_MCAP + TP_MT - 1) / TP_MT;
+    constexpr int SLOTS = (CAP + TP_MT - 1) / TP_MT;
     float gx[SLOTS];
     uint32_t gid[SLOTS];
 #pragma unroll
@@ -132,37 +138,38 @@ __global__ void __launch_bounds__(TP_MT, 4) tp_merge_kernel(const TpArgs a, cons
         }
     }
     __syncthreads();
-    if (tid == 0) {
-        float M = -INFINITY;
+    if (tid < 32) {   // one shard per lane
+        static_assert(TP_MAX_SHARDS <= 32, "one lane per shard");
+        const bool is = (uint32_t)tid < a.n_shards;
+        const float mr = is ? sm.hd[tid].m : -INFINITY;
+        const uint32_t ns = is ? sm.hd[tid].n_status : 0u, st = ns >> 24;
         int fault = (top_k > a.cand) ? ROW_BAD_PARAM : ROW_OK;   // a record holds the shard's `cand` largest, no more
-        bool nonfinite = false, dead = false;
-        for (uint32_t r = 0; r < a.n_shards; r++) {
-            const float mr = sm.hd[r].m;
-            const uint32_t st = sm.hd[r].n_status >> 24;
-            if (st == (uint32_t)ROW_BAD_PARAM) fault = ROW_BAD_PARAM;
-            nonfinite |= st == (uint32_t)ROW_NONFINITE || mr != mr;
-            dead |= st == (uint32_t)ROW_DEAD;
-            if (mr == mr) M = fmaxf(M, mr);
-        }
+        if (__any_sync(FULL, is && st == (uint32_t)ROW_BAD_PARAM)) fault = ROW_BAD_PARAM;
+        const bool nonfinite = __any_sync(FULL, is && (st == (uint32_t)ROW_NONFINITE || mr != mr));
+        const bool dead = __any_sync(FULL, is && st == (uint32_t)ROW_DEAD);
         // the order of engine.rs:1292-1303: parameters, then sanity, then the grammar's dead state
         if (fault == ROW_OK) fault = nonfinite ? ROW_NONFINITE : dead ? ROW_DEAD : ROW_OK;
+        float M = mr == mr ? mr : -INFINITY;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(FULL, M, o));
+        const bool counts = is && fault == ROW_OK && finite_f(mr);
+        const float term = counts ? fmul(sm.hd[tid].s, pgs_expf_tab(fdiv(fsub(mr, M), t), sm.exp_tab)) : 0.0f;
+        // shards are in id order: the first that holds the maximum has the lowest id
+        const unsigned top = __ballot_sync(FULL, counts && mr == M);
+        const uint32_t mine = min(ns & 0xffffffu, a.cand);   // a record can never hold more than `cand` entries
         float S = 0.0f;
-        uint32_t n = 0, amax = 0;
-        float best = -INFINITY;
-        bool have = false;
+        uint32_t before = 0u, n = 0u;
         for (uint32_t r = 0; r < a.n_shards; r++) {
-            const TpRecHead& h = sm.hd[r];
-            if (fault == ROW_OK && finite_f(h.m)) {
-                // shards are in id order, so strict > keeps the lowest id on ties
-                if (!have || h.m > best) { best = h.m; amax = h.argmax; have = true; }
-                S = fadd(S, fmul(h.s, pgs_expf_tab(fdiv(fsub(h.m, M), t), sm.exp_tab)));
-            }
-            sm.start[r] = n;
-            n += min(h.n_status & 0xffffffu, a.cand);   // a record can never hold more than `cand` entries
+            S = fadd(S, __shfl_sync(FULL, term, (int)r));
+            const uint32_t nr = __shfl_sync(FULL, mine, (int)r);
+            if (r < (uint32_t)tid) before += nr;
+            n += nr;
         }
-        sm.start[a.n_shards] = n;
-        sm.M = M; sm.S = S; sm.amax = amax; sm.n = n; sm.fault = fault;
-        sm.unsorted = 0; sm.fin.n_live = 0u;
+        if ((uint32_t)tid <= a.n_shards) sm.start[tid] = before;   // (lane n_shards: all of them)
+        if (tid == 0) {
+            sm.M = M; sm.S = S; sm.amax = top ? sm.hd[__ffs((int)top) - 1].argmax : 0u; sm.n = n; sm.fault = fault;
+            sm.unsorted = 0; sm.fin.n_live = 0u;
+        }
     }
     __syncthreads();
     if (sm.fault) {
@@ -245,6 +252,7 @@ __global__ void __launch_bounds__(TP_MT, 4) tp_merge_kernel(const TpArgs a, cons
 
 __global__ void draft_accept_kernel(const uint32_t* row_argmax, const uint32_t* draft, uint32_t sequences,
                                     uint32_t positions, uint32_t* accepted, uint32_t* next) {
+    cudaGridDependencySynchronize();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= sequences || positions == 0) return;
     uint32_t acc = 0;
@@ -253,36 +261,46 @@ __global__ void draft_accept_kernel(const uint32_t* row_argmax, const uint32_t* 
     next[s] = row_argmax[s * positions + (acc < positions ? acc : positions - 1)];
 }
 
-cudaError_t configure_tp() {
-    cudaError_t e = cudaFuncSetAttribute(tp_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TpMergeSmem));
+template <int CAP>
+static cudaError_t configure_merge() {
+    cudaError_t e = cudaFuncSetAttribute(tp_merge_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TpMergeSmem<CAP>));
     if (e != cudaSuccess) return e;
-    // several rows per SM: most of a row's time is one warp's serial walk
-    return cudaFuncSetAttribute(tp_merge_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(tp_merge_kernel<CAP>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+cudaError_t configure_tp() {
+    const cudaError_t e = configure_merge<TP_MCAP / 2>();
+    return e != cudaSuccess ? e : configure_merge<TP_MCAP>();
 }
 
-cudaError_t launch_tp_push(const TpArgs& a, cudaStream_t stream) {
-    const size_t units = ((size_t)a.rows * a.rec_bytes) / 16 + 1;
+// set up while the kernel before still runs (programmatic stream serialization)
+template <class... A>
+static cudaError_t launch_behind(void (*kernel)(A...), uint32_t grid, uint32_t threads, size_t smem, cudaStream_t stream, A... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((units + 255) / 256 < 64 ? (units + 255) / 256 : 64), 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tp_push_kernel, a);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t launch_tp_push(const TpArgs& a, cudaStream_t stream) {
+    const size_t units = ((size_t)a.rows * a.rec_bytes) / 16 + 1;
+    return launch_behind(tp_push_kernel, (uint32_t)((units + 255) / 256 < 64 ? (units + 255) / 256 : 64), 256u, 0, stream, a);
 }
 
 cudaError_t launch_tp_merge(const TpArgs& a, const TpOut& o, cudaStream_t stream) {
-    tp_merge_kernel<<<a.rows, TP_MT, sizeof(TpMergeSmem), stream>>>(a, o);
-    return cudaGetLastError();
+    // (half the longest list in half the shared memory: eight rows per SM instead of six)
+    if (a.n_shards * a.cand <= (uint32_t)TP_MCAP / 2u) return launch_behind(tp_merge_kernel<TP_MCAP / 2>, a.rows, TP_MT, sizeof(TpMergeSmem<TP_MCAP / 2>), stream, a, o);
+    return launch_behind(tp_merge_kernel<TP_MCAP>, a.rows, TP_MT, sizeof(TpMergeSmem<TP_MCAP>), stream, a, o);
 }
 
 cudaError_t launch_draft_accept(const uint32_t* row_argmax, const uint32_t* draft, uint32_t sequences,
                                 uint32_t positions, uint32_t* accepted, uint32_t* next, cudaStream_t stream) {
-    draft_accept_kernel<<<(sequences + 127) / 128, 128, 0, stream>>>(row_argmax, draft, sequences, positions, accepted,
-                                                                     next);
-    return cudaGetLastError();
+    return launch_behind(draft_accept_kernel, (sequences + 127) / 128, 128u, 0, stream, row_argmax, draft, sequences, positions, accepted, next);
 }
 
 }  // namespace pgs

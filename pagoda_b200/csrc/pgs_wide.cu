@@ -35,18 +35,10 @@ namespace pgs {
 
 constexpr int WNW = W_NT / 32;
 constexpr int WL = W_REGION / 32;        // logits per lane and region
+static_assert(WL == RUN, "a region is a warp's runs");
 constexpr uint32_t W_NIL = 0xffffffffu;
 constexpr uint32_t F_KMAX = F_MCAP / 2;  // top-k up to which the second pass lists the candidates
 constexpr uint32_t W_DUAL = 2u;          // beside a segment's binade: it may also be the next one
-
-// 32 runs of terms, one per lane, ready to be added to a running value: lanes whose runs are estimated to begin in one
-// binade form a group, and each lane holds the increments from the group's first lane up to and including its own, for an
-// even and for an odd running value there.
-struct Runs {
-    uint32_t k;         // bits of the estimated binade's lower end (0: none)
-    uint32_t c0, c1;    // SEQ_SAT: leaves the binade
-    uint32_t head;      // first lane of the group; bit 31: nothing but zeros in this lane's run
-};
 
 struct alignas(16) WideSmem {
     RowArgs a;                           // the launch's arguments, for the phases, which are functions of their own
@@ -294,77 +286,6 @@ __device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id
     }
     if (__any_sync(FULL, !good || n >= 0x01000000u)) return W_TIE;
     return __reduce_add_sync(FULL, n);   // (the table keeps the sum below 2^24 ulps)
-}
-
-// v: this lane's run; R0: estimate of the running value at the first lane's run
-__device__ __forceinline__ Runs make_runs(const float (&v)[WL], float R0) {
-    const uint32_t lane = threadIdx.x & 31;
-    float c = 0.0f;
-#pragma unroll
-    for (int j = 0; j < WL; j++) c += v[j];
-    float inc = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(FULL, inc, o);
-        if (lane >= (uint32_t)o) inc += t;
-    }
-    Runs s;
-    s.k = f2u(R0 + (inc - c)) & 0x7f800000u;
-    if (s.k == 0x7f800000u) s.k = 0u;
-    s.c0 = s.c1 = SEQ_SAT;
-    if (c == 0.0f) s.c0 = s.c1 = 0u;
-    else if (s.k) {
-        float a0 = u2f(s.k), a1 = u2f(s.k + 1u);
-#pragma unroll
-        for (int j = 0; j < WL; j++) { a0 = fadd(a0, v[j]); a1 = fadd(a1, v[j]); }
-        if ((f2u(a0) & 0x7f800000u) == s.k) s.c0 = f2u(a0) - s.k;
-        if ((f2u(a1) & 0x7f800000u) == s.k) s.c1 = f2u(a1) - (s.k + 1u);
-    }
-    const uint32_t before = __shfl_up_sync(FULL, s.k, 1);
-    const unsigned heads = __ballot_sync(FULL, lane == 0u || before != s.k);
-    s.head = 31u - __clz((int)(heads & (0xffffffffu >> (31u - lane))));
-    // compose(left, right)(p) = left_p + right_{(p + left_p) & 1}, inside the group
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t l0 = __shfl_up_sync(FULL, s.c0, o), l1 = __shfl_up_sync(FULL, s.c1, o);
-        if (lane >= s.head + (uint32_t)o) {
-            const uint32_t n0 = l0 + ((l0 & 1u) ? s.c1 : s.c0), n1 = l1 + (((l1 + 1u) & 1u) ? s.c1 : s.c0);
-            s.c0 = (l0 >= SEQ_SAT || n0 >= SEQ_SAT) ? SEQ_SAT : n0;
-            s.c1 = (l1 >= SEQ_SAT || n1 >= SEQ_SAT) ? SEQ_SAT : n1;
-        }
-    }
-    if (c == 0.0f) s.head |= 0x80000000u;
-    return s;
-}
-
-// Adds the runs to the exact running value R; one warp, the same result in all lanes.
-__device__ __forceinline__ float add_runs(float R, const Runs& s, const float (&v)[WL]) {
-    const uint32_t lane = threadIdx.x & 31, head = s.head & 31u;
-    const bool zero = (s.head >> 31) != 0u;
-    uint32_t pos = 0u;
-#pragma unroll 1
-    while (pos < 32u) {
-        // The group that begins here, as far as the running value stays in its binade; and what the first lane in which it
-        // does not (or the estimate missed the binade) makes of it: every lane adds its run to the value it would begin with.
-        const uint32_t rb = f2u(R), d = (rb & 1u) ? s.c1 : s.c0;
-        const bool fits = lane >= pos && (zero || (head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u));
-        const uint32_t own = zero ? 0u : d;   // (zeros: the group's increments up to here, which the lane before has too)
-        const unsigned ok = __ballot_sync(FULL, fits) >> pos;
-        const uint32_t n = ~ok ? min((uint32_t)__ffs((int)~ok) - 1u, 32u - pos) : 32u - pos;
-        uint32_t last = __reduce_max_sync(FULL, fits && lane < pos + n ? own : 0u);   // (increments only grow inside a group)
-        float r = u2f(rb + last);
-        pos += n;
-        if (pos < 32u) {
-            if (lane == pos) {
-#pragma unroll
-                for (int j = 0; j < WL; j++) r = fadd(r, v[j]);
-            }
-            r = __shfl_sync(FULL, r, (int)pos);
-            pos++;
-        }
-        R = r;
-    }
-    return R;
 }
 
 // the warp's terms, as a region holds them, into id order: lane k gets the terms k * WL ..
@@ -1415,7 +1336,9 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     const RowArgs& a = sm.a;
     const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x;
-    if (a_.work_rows) cudaGridDependencySynchronize();   // launched ahead of the end of the kernel that fills the list
+    // Launched ahead of the end of the kernel before, which may fill the list.  (No early trigger for the kernel behind: its
+    // CTAs would crowd on the SMs that this one leaves free, 128 masked rows 50 -> 62 us.)
+    cudaGridDependencySynchronize();
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass
     if (tid == 0) { sm.a = a_; sm.target = 0u; }
@@ -1492,7 +1415,7 @@ cudaError_t configure_wide() {
     return e;
 }
 
-// `grid` CTAs, at most one per SM; a.work_rows: the work-list pass behind another kernel (programmatic stream serialization)
+// `grid` CTAs, at most one per SM; set up while the kernel before still runs (programmatic stream serialization)
 cudaError_t launch_wide(const RowArgs& a, const WideLaunch& l, uint32_t slots, uint32_t grid, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
@@ -1502,7 +1425,7 @@ cudaError_t launch_wide(const RowArgs& a, const WideLaunch& l, uint32_t slots, u
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = a.work_rows ? 1 : 0;
+    cfg.attrs = attr; cfg.numAttrs = 1;
     const uint32_t ge = a.dtype ? 8u : 4u;
     const bool vec = ((uintptr_t)a.logits & 15u) == 0u && a.row_stride % ge == 0u && a.vocab % ge == 0u;
     if (vec) return a.dtype ? cudaLaunchKernelEx(&cfg, wide_kernel<true, true>, a, l, slots) : cudaLaunchKernelEx(&cfg, wide_kernel<false, true>, a, l, slots);
