@@ -106,6 +106,7 @@ struct StreamSmem {
     // cluster mode: one slot per CTA of the cluster, written by that CTA into every CTA's copy (xk .. xflag) or into
     // the first CTA's copy (xs, xam)
     uint32_t xk[8], xlo[8], xfin[8], xflag[8], xam[8];
+    float xb[8];
     double xs[8];
     long long prof_acc[16];
     // Three lives of one area: the id -> count table while the entries are set up, the tables of a row while it streams, and
@@ -122,8 +123,7 @@ struct StreamSmem {
                     uint32_t t_q[SNT];
                     // per warp region of the row (512 consecutive logits): pass 1 leaves the warp's maximum and the plain
                     // sum of its numerators relative to it; then the binade's lower end the fold has there (0 = fold this
-                    // region the careful way) and the estimate of the running value at its start.  While the entries are
-                    // set up, reg_a counts them per region.
+                    // region the careful way) and the estimate of the running value at its start
                     float reg_a[S_MAX_REGIONS], reg_b[S_MAX_REGIONS];
                     // a logit below this adds exactly nothing to the fold in this region; before, the plain sum of the
                     // region's entries relative to the CTA's maximum
@@ -134,7 +134,7 @@ struct StreamSmem {
                     uint16_t rs[S_MAX_REGIONS + 2];
                     uint32_t ent_id[S_ENT];
                     float ent_x[S_ENT];              // before pass 1 is over: the count; ENT_MASKED, ENT_EOS
-                    uint32_t ent_raw[S_ENT];         // the word that holds the raw logit
+                    uint32_t ent_raw[S_ENT];         // the word that holds the raw logit (before pass 1: entries per region)
                     uint32_t bits[S_WORDS];          // one bit per logit: allowed, and no entry
                 };
                 FinishArrays fin;
@@ -680,7 +680,7 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
 // CL: a thread-block cluster of 2, 4 or 8 CTAs shares every row (small batches: a row alone on one CTA is bound by
 // the latency of its own loads and dependent instructions).  CTA k of the cluster takes the pieces k, k + size, ...;
 // the CTAs exchange their maxima, region tables, histograms, candidates and fold shares through distributed shared
-// memory around four cluster barriers per row, and the first CTA finishes the row.  Every decision that ends a row
+// memory around two cluster barriers, and the first CTA finishes the row (a launch has one cluster per row).  Every decision that ends a row
 // early is taken from values all CTAs of the cluster hold alike, so they always meet at the same barriers.
 template <bool BF16, bool CL>
 __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, const StreamLaunch sl) {
@@ -704,7 +704,10 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         for (int i = 0; i < 16; i++) sm.prof_acc[i] = 0;
     constexpr int PREP_TID = SNT - 32;   // lane 0 of the last warp
     uint32_t crank = 0u, csize = 1u;
-    if (CL) { crank = cg::this_cluster().block_rank(); csize = cg::this_cluster().num_blocks(); }
+    if (CL) {
+        crank = cg::this_cluster().block_rank(); csize = cg::this_cluster().num_blocks();
+        cg::this_cluster().barrier_arrive();   // waited for where the first of the others' shared memory is written
+    }
     const uint32_t first_row = CL ? blockIdx.x / csize : blockIdx.x, row_step = CL ? gridDim.x / csize : gridDim.x;
     const uint32_t tail_owner = n_full % csize;   // the CTA that takes the ragged piece
     // set up while the kernel before this one drains; the pass over the work list is set up in the same way behind this one
@@ -792,7 +795,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 // engine.rs:1562; CL: another CTA's piece
                 if (hid[u] >= V || (CL && (hid[u] / S_PIECE) % csize != crank)) hid[u] = S_NIL;
             }
-            uint32_t* rcnt = reinterpret_cast<uint32_t*>(sm.reg_a);
+            uint32_t* rcnt = sm.ent_raw;   // per region, until pass 1
             {
                 const uint32_t whole = V / 32u, words = ((V + S_PIECE - 1) / S_PIECE) * (S_PIECE / 32);
                 const uint32_t* mw = ctl.mw;
@@ -933,12 +936,53 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         if (!greedy && gkey)
             for (uint32_t e = tid; e < n_ent; e += SNT)
                 if (sm.ent_x[e] > -INFINITY) atomicAdd(&sm.reg_t[sm.ent_id[e] / S_REGION], ex2_approx_ftz((sm.ent_x[e] - lm) * sc));
+        // The per-thread maxima are spread over S_NB equal-width buckets between `lo_v` and `top` (a monotone map); with b
+        // the highest bucket such that the buckets b.. hold at least `need` maxima, every logit of bucket b - 1 or higher
+        // counts: at least `need` logits reach the bound returned.  all: over the CTAs of the cluster.
+        const auto kth_bound = [&](uint32_t need, float lo_v, float top, bool all) {
+            const float scb = top > lo_v ? (float)(S_NB - 1) / (top - lo_v) : 0.0f;
+#pragma unroll
+            for (int c = 0; c < S_NCELL; c++) {
+                const float cv = sm.cell[c * SNT + tid];
+                if (finite_f(cv)) atomicAdd(&sm.hist[min((uint32_t)(S_NB - 1), (uint32_t)((cv - lo_v) * scb))], 1u);
+            }
+            __syncthreads();
+            // thread j owns the S_BPT buckets S_NB-1 - j*S_BPT - u; `above` = maxima in higher buckets
+            uint32_t hv[S_BPT], own = 0u;
+            if (CL && all) {
+                cg::cluster_group cluster = cg::this_cluster();
+                cluster.sync();
+#pragma unroll
+                for (int u = 0; u < S_BPT; u++) {
+                    hv[u] = 0u;
+                    for (uint32_t k = 0; k < csize; k++) hv[u] += *cluster.map_shared_rank(&sm.hist[(S_NB - 1) - tid * S_BPT - u], k);
+                    own += hv[u];
+                }
+            } else
+#pragma unroll
+            for (int u = 0; u < S_BPT; u++) { hv[u] = sm.hist[(S_NB - 1) - tid * S_BPT - u]; own += hv[u]; }
+            uint32_t total;
+            uint32_t above = sblock_excl_scan_u32(own, &total, sm.scan_u);
+#pragma unroll
+            for (int u = 0; u < S_BPT; u++) {
+                if (above < need && need <= above + hv[u]) sm.sel_bucket = (uint32_t)((S_NB - 1) - tid * S_BPT - u);
+                above += hv[u];
+            }
+            __syncthreads();
+            const uint32_t bsel = sm.sel_bucket;
+            return (bsel >= 1u && scb > 0.0f) ? lo_v + ((float)bsel - 1.0f) / scb : lo_v;
+        };
+        float bound = NAN;   // CL: at least top_k logits of the row reach it (NaN: not known yet)
         if (CL) {
-            // First barrier: every CTA of the cluster is through its first pass, so nobody still uses the space of the
-            // region table for its history counts, and everybody is done with the row before.  Then every CTA hands its
-            // part of the region table and its four numbers to all the others; second barrier; combine.
+            // Every CTA bounds its own share of the top-k from below, hands that, its part of the region table and its
+            // numbers to all the others, and combines what it gets: one barrier.  (The share: the k / size-th largest, so
+            // that the shares of all CTAs together make k.  A bound over all histograms is tighter, but takes a second
+            // barrier and a trip to every other CTA: 8 rows 28.5 us.)
             cg::cluster_group cluster = cg::this_cluster();
-            cluster.sync();
+            const uint32_t share = (top_k + csize - 1u) / csize;
+            if (!greedy && n_fin >= share) bound = kth_bound(share, key_to_float(lo_key), lm, false);   // CTA-uniform
+            else __syncthreads();   // (the entries' sums are complete)
+            cluster.barrier_wait();   // all of them run
             if (!greedy) {
 #pragma unroll 1
                 for (uint32_t r = tid; r < n_regions; r += SNT) {
@@ -962,13 +1006,18 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 *cluster.map_shared_rank(&sm.xlo[crank], tid) = lo_key;
                 *cluster.map_shared_rank(&sm.xfin[crank], tid) = n_fin;
                 *cluster.map_shared_rank(&sm.xflag[crank], tid) = (nonfinite ? 1u : 0u) | (defer_row ? 2u : 0u);
+                *cluster.map_shared_rank(&sm.xb[crank], tid) = bound;
             }
             cluster.sync();
             gkey = 0u; lo_key = 0xffffffffu; n_fin = 0u; nonfinite = false; defer_row = false;
+            float low = INFINITY;
+            bool known = true;
             for (uint32_t k = 0; k < csize; k++) {
                 gkey = umax(gkey, sm.xk[k]); lo_key = umin(lo_key, sm.xlo[k]); n_fin += sm.xfin[k];
                 nonfinite |= (sm.xflag[k] & 1u) != 0u; defer_row |= (sm.xflag[k] & 2u) != 0u;
+                low = fminf(low, sm.xb[k]); known &= sm.xb[k] == sm.xb[k];
             }
+            bound = known ? low : NAN;
         }
         const bool any = gkey != 0u;
         const float m = any ? key_to_float(gkey) : -INFINITY;
@@ -1043,44 +1092,20 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         }
 
         PGS_STICK(6);   // reductions + argmax
-        // ---- top-k bound.  The per-thread maxima are spread over S_NB equal-width buckets between their
-        // smallest finite value and the row maximum (a monotone map); with b the highest bucket such that the
-        // buckets b.. hold at least top_k maxima, every logit of bucket b - 1 or higher is a candidate.
+        // ---- top-k bound
         const float t = fmaxf(temp, 1e-9f);
         float cut = -INFINITY;
-        if (n_fin >= top_k) {   // CTA-uniform
-            const float lo_v = key_to_float(lo_key);
-            const float scb = m > lo_v ? (float)(S_NB - 1) / (m - lo_v) : 0.0f;
+        if (n_fin >= top_k) {   // CTA-uniform; CL: the same in all CTAs
+            if (!(bound == bound)) {
+                if (CL) {   // some CTA has too few maxima for its share (a mask that leaves its pieces empty)
+                    __syncthreads();
 #pragma unroll
-            for (int c = 0; c < S_NCELL; c++) {
-                const float cv = sm.cell[c * SNT + tid];
-                if (finite_f(cv)) atomicAdd(&sm.hist[min((uint32_t)(S_NB - 1), (uint32_t)((cv - lo_v) * scb))], 1u);
-            }
-            __syncthreads();
-            // thread j owns the S_BPT buckets S_NB-1 - j*S_BPT - u; `above` = maxima in higher buckets
-            uint32_t hv[S_BPT], own = 0u;
-            if (CL) {   // third barrier: the histograms of all CTAs stand; every CTA adds them up for itself
-                cg::cluster_group cluster = cg::this_cluster();
-                cluster.sync();
-#pragma unroll
-                for (int u = 0; u < S_BPT; u++) {
-                    hv[u] = 0u;
-                    for (uint32_t k = 0; k < csize; k++) hv[u] += *cluster.map_shared_rank(&sm.hist[(S_NB - 1) - tid * S_BPT - u], k);
-                    own += hv[u];
+                    for (int u = 0; u < S_BPT; u++) sm.hist[u * SNT + tid] = 0u;
+                    if (tid == 0) sm.sel_bucket = 0u;
+                    __syncthreads();
                 }
-            } else
-#pragma unroll
-            for (int u = 0; u < S_BPT; u++) { hv[u] = sm.hist[(S_NB - 1) - tid * S_BPT - u]; own += hv[u]; }
-            uint32_t total;
-            uint32_t above = sblock_excl_scan_u32(own, &total, sm.scan_u);
-#pragma unroll
-            for (int u = 0; u < S_BPT; u++) {
-                if (above < top_k && top_k <= above + hv[u]) sm.sel_bucket = (uint32_t)((S_NB - 1) - tid * S_BPT - u);
-                above += hv[u];
+                bound = kth_bound(top_k, key_to_float(lo_key), m, true);
             }
-            __syncthreads();
-            const uint32_t bsel = sm.sel_bucket;
-            const float bound = (bsel >= 1u && scb > 0.0f) ? lo_v + ((float)bsel - 1.0f) / scb : lo_v;
             // every logit whose probability could still tie with the k-th one stays above the cut
             const float delta = 4.8e-7f * (fabsf(m - bound) + 4.0f * t) + 4.8e-7f * (fabsf(bound) + fabsf(m));
             cut = bound - delta;
