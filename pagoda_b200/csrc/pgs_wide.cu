@@ -934,9 +934,9 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
             const float p = u2f((uint32_t)(__ldcg(list + j) >> 32));
             if (!(p >= thr_k)) continue;
             const uint32_t b = bucket_of(p), kb = f2u(sm.bs[b]);
-            if (kb == 0u) continue;
+            if (kb == 0u) { sm.bn[b] = f2u(p); continue; }   // (of use where the bucket has one entry)
             const uint32_t i0 = f2u(fadd(u2f(kb), p)) - kb, i1 = f2u(fadd(u2f(kb + 1u), p)) - (kb + 1u);
-            if (i0 != i1 || !(p < u2f(kb))) sm.bs[b] = 0.0f;   // to be added one by one
+            if (i0 != i1 || !(p < u2f(kb))) { sm.bs[b] = 0.0f; sm.bn[b] = f2u(p); }   // to be added one by one
             else atomicAdd(&sm.bn[b], i0);
         }
         // the fold over the buckets, highest first: warp 0 adds whole buckets until it meets one that is not, or the one in
@@ -977,8 +977,14 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
                     if (cnt) R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
                     b -= (int)cnt * per;
                     if (cnt == 32u) { per = 8; continue; }
-                    if (per == 1) break;
-                    per = 1;
+                    if (per == 8) { per = 1; continue; }
+                    // a bucket to be added one by one; a single entry that does not reach top-p needs no sort for that
+                    const uint32_t n1 = ends[b] - (b + 1 < W_BUCKETS ? ends[b + 1] : 0u);
+                    const float R1 = fadd(R, u2f(sm.bn[b]));
+                    if (n1 != 1u || sm.bs[b] != 0.0f || R1 >= sm.row.top_p) break;
+                    R = R1;
+                    b--;
+                    per = 8;
                 }
                 if (lane == 0) sm.last = b >= (int)cut ? (uint32_t)b : W_NIL;
             }
@@ -1083,10 +1089,13 @@ __device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const Wid
             float x[WL], v[WL];
             wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, sm.row, slot, V, r, f);
             to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
-            if (lane == 0) {
-                float acc = sm.start[r];
-                const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
-                for (uint32_t j = 0; j < nv; j++) {
+            add_runs(sm.start[r], make_runs(v, sm.start[r]), v, sm.red_f);
+            __syncwarp();
+            const unsigned over = __ballot_sync(FULL, target < sm.red_f[lane]);
+            if (lane == 0 && over) {
+                const uint32_t run = __ffs((int)over) - 1u;
+                float acc = run ? sm.red_f[run - 1u] : sm.start[r];
+                for (uint32_t j = run * WL; j < (run + 1u) * WL; j++) {
                     acc = fadd(acc, sm.spare[j]);
                     if (target < acc) { token = r * W_REGION + j; break; }
                 }
@@ -1100,7 +1109,8 @@ __device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const Wid
             if (a.total) a.total[row] = total;
         }
     }
-    if (a.n_kept || a.dump_ids || a.dump_probs) {   // diagnostics: the kept set in id order
+    if (tid == 0 && a.n_kept) a.n_kept[row] = sm.row.n_kept;
+    if (a.dump_ids || a.dump_probs) {   // diagnostics: the kept set in id order
         uint32_t done = 0u;
         for (uint32_t r0 = 0; r0 < n_regions; r0 += WNW) {
             __syncthreads();
@@ -1135,7 +1145,6 @@ __device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const Wid
                     }
             }
         }
-        if (tid == 0 && a.n_kept) a.n_kept[row] = done;
     }
 }
 
@@ -1222,6 +1231,17 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
                 }
         }
         if (PHASE == WP_SUM || PHASE == WP_TOTAL) {
+            if (PHASE == WP_TOTAL && !f.filter && a.n_kept) {   // every probability above zero is kept
+                const float c1 = 1.44269504f / f.t, c0 = f.S > 1e-9f ? -log2f(f.S) : 0.0f;
+                uint32_t n = 0u;
+#pragma unroll
+                for (int j = 0; j < WL; j++) {
+                    const float e = __fmaf_rn(fsub(x[j], f.m), c1, c0);   // (a probability below 2^-149 is zero)
+                    n += e > -120.0f || (x[j] > -INFINITY && e > -160.0f && term_of(x[j], 0u, f, sm.exp_tab) > 0.0f);
+                }
+                n = __reduce_add_sync(FULL, n);
+                if (lane == 0 && n) atomicAdd(&l.row[slot].n_kept, n);
+            }
             const uint32_t kb = out.y & ~W_DUAL;
             if (kb) {
                 const Approx q = approx_of(f);
