@@ -5,7 +5,10 @@
 // loads of some overlap the arithmetic of the others, and what a piece costs beyond its logits (addresses, table
 // look-ups, warp reductions, loop control) is paid once per sixteen logits:
 //
-//   pass 1, last piece first, from HBM: sanity, penalties, grammar bitmask, EOS fix; per thread its running
+//   before: the row's entries (distinct history ids, the EOS fix) and one bit per logit that says whether the passes may see
+//           it (the grammar mask without the entries); the entries' logits are copied aside during pass 1 and one thread per
+//           entry adds what the penalties make of them to what the passes find;
+//   pass 1, last piece first, from HBM: sanity, bits; per thread its running
 //           maximum and four more (one per piece number mod 4) that bound the top-k threshold; per warp and piece the
 //           plain sum of the softmax numerators relative to the warp's own maximum;
 //   between: row maximum and argmax (lowest id: the threads that hold the maximum look at that piece again); a bound for the top-k threshold: the k-th largest of the 2048

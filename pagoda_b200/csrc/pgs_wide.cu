@@ -17,6 +17,11 @@
 //   region  increments of the running total over the kept probabilities                  (what has no short list)
 //   row     total and inverse-CDF pick
 //
+// What bounds it: the folds change binade 8 to 16 times a row, and each change is about a microsecond of one warp; a grid
+// barrier is two; a region phase is the latency of one or two regions per warp (mask, history entries and logits are one trip
+// to L2 or HBM each) rather than bandwidth.  Against one CTA per row: 32 rows of 151936 without top-k 8312 -> 231 us, 16 rows
+// in exact mode 383 -> 73, 48 rows of 50257 359 -> 68, scoring of 64 rows 204 -> 84.
+//
 // The fold (pagoda/src/sampler.rs:42, :99-113, :136-144): while the running value stays inside one binade, adding a
 // non-negative term is an integer addition in ulps which depends on the running value only where the term ends exactly on
 // half an ulp.  A region (or bucket) without such a tie whose running value provably stays inside one binade is one
