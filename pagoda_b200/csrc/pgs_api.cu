@@ -148,7 +148,7 @@ int wide_workspace(pgs_handle* h) {
     const uint32_t vocab = h->max_vocab < (uint32_t)W_MAX_VOCAB ? h->max_vocab : (uint32_t)W_MAX_VOCAB;
     const uint32_t regions = (vocab + W_REGION - 1) / W_REGION;
     WideLaunch& l = h->wide;
-    l.reg_stride = regions; l.rs_stride = regions + 1u;
+    l.chunk = (uint32_t)rows; l.reg_stride = regions; l.rs_stride = regions + 1u;
     size_t used = 0;
     auto take = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~size_t(255); return at; };
     const size_t o_sync = take(64), o_left = take(4), zeroed = used;

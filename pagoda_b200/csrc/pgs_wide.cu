@@ -1371,8 +1371,8 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
     bool ok = grid_join(sm, l);
-    for (uint32_t c0 = 0; c0 < n_work && ok; c0 += W_CHUNK) {
-        const uint32_t n = min(n_work - c0, (uint32_t)W_CHUNK);
+    for (uint32_t c0 = 0; c0 < n_work && ok; c0 += l.chunk) {
+        const uint32_t n = min(n_work - c0, l.chunk);
         const auto open = [&](uint32_t s) { open_row<BF16>(sm, a, l, s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
         uint32_t s = sm.rank;
         if (c0 == 0u) {   // (how many take part is not known yet)

@@ -12,7 +12,7 @@ constexpr int W_REGION = 512;           // consecutive logits of one warp
 constexpr int W_MAX_VOCAB = 1 << 20;
 constexpr int W_MAX_REGIONS = W_MAX_VOCAB / W_REGION;
 constexpr int W_MAX_HIST = 2048;
-constexpr int W_CHUNK = 64;             // rows in flight together: what the workspace is sized for
+constexpr int W_CHUNK = 64;             // rows in flight together, at most
 constexpr int W_BUCKETS = 41 * 256;     // probabilities by exponent (2^-40 .. 1) and eight mantissa bits
 constexpr int W_TERMS = 64;             // segments of a row whose terms the region phase leaves for the fold
 constexpr int W_SORT = 4096;            // entries of a bucket that one CTA sorts
@@ -37,18 +37,19 @@ struct WideRow {
 enum : uint32_t { WS_FIRST = 0u, WS_SUM = 1u, WS_SELECT = 2u, WS_TOTAL = 3u, WS_DONE = 4u };
 
 struct WideLaunch {
-    WideRow* row;               // [W_CHUNK]
-    float2* reg;                // [W_CHUNK][n_regions]: a region's maximum, its plain sum
-    float4* cell;               // [W_CHUNK][n_regions]: the maxima of four parts of the region
-    uint2* seg;                 // [W_CHUNK][n_regions]: increments in ulps, binade (0: add term by term)
-    float* pre;                 // [W_CHUNK][n_regions]: estimate of the running value at the region's start
-    float* terms;               // [W_CHUNK][W_TERMS][W_REGION]: terms of segments that are added one by one
-    uint32_t* ent_id;           // [W_CHUNK][W_MAX_HIST + 32]
+    WideRow* row;               // [chunk]
+    float2* reg;                // [chunk][n_regions]: a region's maximum, its plain sum
+    float4* cell;               // [chunk][n_regions]: the maxima of four parts of the region
+    uint2* seg;                 // [chunk][n_regions]: increments in ulps, binade (0: add term by term)
+    float* pre;                 // [chunk][n_regions]: estimate of the running value at the region's start
+    float* terms;               // [chunk][W_TERMS][W_REGION]: terms of segments that are added one by one
+    uint32_t* ent_id;           // [chunk][W_MAX_HIST + 32]
     float* ent_xn;
-    uint32_t* rs;               // [W_CHUNK][n_regions + 1]
-    uint32_t* hist;             // [W_CHUNK][W_BUCKETS]: counts, then list positions
-    unsigned long long* list;   // [W_CHUNK][list_stride] (the general kernel's sort buffer): probability bits and id
+    uint32_t* rs;               // [chunk][n_regions + 1]
+    uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
+    unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
     uint32_t* sync;             // [0] barrier arrivals, [1] lost waits, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    uint32_t chunk;             // rows that the workspace holds (<= W_CHUNK): the launch takes that many at a time
     uint32_t reg_stride, rs_stride, list_stride;
     uint32_t* left_rows;        // rows left to the general kernel
     uint32_t* left_count;

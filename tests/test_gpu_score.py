@@ -40,3 +40,26 @@ def test_log_softmax_matches_oracle(oracle):
         assert status.cpu().numpy().tolist() == [0, 1] and np.isnan(g.cpu().numpy()[1])
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("rows, vocab", [(3, 511), (3, 20001), (64, 50257), (65, 120001), (200, 131072)])
+def test_more_rows_than_the_handle_was_made_for(oracle, rows, vocab):
+    """Scoring has no row limit: the rows of a call beyond what the workspace holds are taken in turn."""
+    import torch
+    import pagoda_b200
+    from pagoda_b200 import synth
+    x = synth.normal_f32(70 + rows, rows * vocab, 3.0).reshape(rows, vocab)
+    ids = np.random.default_rng(rows).integers(0, vocab, rows).astype(np.int32)
+    s = pagoda_b200.Sampler(device=0, max_rows=2, max_vocab=vocab, max_history=1)
+    try:
+        g, full, status = s.log_softmax(torch.from_numpy(x).cuda(), ids=torch.from_numpy(ids).cuda(), full=True,
+                                        stream_ptr=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        full, g = full.cpu().numpy(), g.cpu().numpy()
+        assert (status.cpu().numpy() == 0).all()
+        for r in range(rows):
+            want = oracle.log_softmax(x[r])
+            np.testing.assert_allclose(full[r], want, rtol=0, atol=1e-6 * np.abs(want).max())
+            assert g[r] == full[r][ids[r]]
+    finally:
+        s.close()
