@@ -714,7 +714,8 @@ __device__ __noinline__ void maximum_row(WideSmem& sm, const RowArgs& a, const W
             if (above < k && k <= above + own) sm.last = 1023u - tid;
             __syncthreads();
             const float bound = sm.last >= 1u && scb > 0.0f ? lo_v + ((float)sm.last - 1.0f) / scb : lo_v;
-            if (tid == 0) sm.row.cut_x = bound - 4.8e-7f * (fabsf(m - bound) + 4.0f * sm.row.t) - 4.8e-7f * (fabsf(bound) + fabsf(m));
+            // (finite also where the margin overflows: what is masked, or behind the end of the row, is never a candidate)
+            if (tid == 0) sm.row.cut_x = fmaxf(bound - 4.8e-7f * (fabsf(m - bound) + 4.0f * sm.row.t) - 4.8e-7f * (fabsf(bound) + fabsf(m)), -3.402823466e38f);
         }
     }
     if (sm.row.state == WS_SUM) {
@@ -1232,7 +1233,7 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
             for (int j = 0; j < WL; j++)
                 if (x[j] >= cut) {   // (rare)
                     const uint32_t at = atomicAdd(&l.row[slot].n_list, 1u);
-                    if (at < (uint32_t)F_MCAP) l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
+                    if (at < min((uint32_t)F_MCAP, l.list_stride)) l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
                 }
         }
         if (PHASE == WP_SUM || PHASE == WP_TOTAL) {

@@ -37,3 +37,29 @@ def test_wide_kernel_edges(oracle, rows, vocab, top_k, history):
             assert g[r] == full[r][int(ids[r])]
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("vocab", [3, 4, 513])
+@pytest.mark.parametrize("exact", [True, False])
+def test_top_k_bound_beyond_the_float_range(oracle, vocab, exact):
+    """A bound whose margin overflows (a huge temperature, logits across the whole f32 range) lists finite logits only:
+    what is masked or lies behind the end of a short row stays out of the list."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    rows = 12
+    rng = np.random.default_rng(vocab)
+    x = rng.standard_normal((rows, vocab)).astype(np.float32)
+    x[6:] = x[6:] / np.abs(x[6:]).max(axis=1, keepdims=True) * np.float32(3.0e38)
+    temperature = np.where(np.arange(rows) < 6, np.float32(1e38), np.float32(1.0)).astype(np.float32)
+    words = np.full((2, (vocab + 31) // 32), 0xffffffff, np.uint32)
+    words[1] &= np.uint32(0xaaaaaaab)
+    w = synth.Workload("range", x, temperature, np.resize(np.uint32([1, 2]), rows), np.resize(np.float32([1.0, 0.9]), rows),
+                       np.zeros(rows, np.float32), np.zeros(rows, np.float32), np.ones(rows, np.float32), None, None,
+                       synth.uniform_f32(9, rows), mask_words=words, state_flags=np.zeros(2, np.uint32),
+                       mask_state=np.resize(np.int32([0, 1]), rows))
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    try:
+        s.set_exact(exact)
+        assert_same(*run_both(s, oracle, w), w, exact=exact)
+    finally:
+        s.close()
