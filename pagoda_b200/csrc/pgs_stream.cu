@@ -1095,6 +1095,11 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         }
 
         PGS_STICK(6);   // reductions + argmax
+        // numerators are 2^(x * sc - m * sc) here: where that overflows, the row goes to the kernels that subtract first
+        if (!(fabsf(m) * sc < 1e38f)) {   // CTA-uniform; CL: the same in all CTAs
+            if (writer) sl.work_rows[atomicAdd(sl.work_count, 1u)] = row;
+            continue;
+        }
         // ---- top-k bound
         const float t = fmaxf(temp, 1e-9f);
         float cut = -INFINITY;
