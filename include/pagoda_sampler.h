@@ -41,7 +41,7 @@ enum pgs_error {
     PGS_ERR_CUDA = -2,     /* a CUDA call failed */
     PGS_ERR_NOMEM = -3,
     PGS_ERR_LIMIT = -4,    /* rows / vocab / history beyond what pgs_create was sized for */
-    PGS_ERR_TIMEOUT = -5   /* a bounded device-side wait ran out (peer exchange; pgs_tp_exchange_status) */
+    PGS_ERR_TIMEOUT = -5   /* a bounded device-side wait ran out (pgs_tp_exchange_status) */
 };
 
 /* Per-row outcome.  Maps onto the reference's per-request finish reasons so that a
@@ -52,7 +52,8 @@ enum pgs_row_status {
     PGS_ROW_DEAD = 2,      /* grammar state is a dead end (engine.rs:1299-1303) -> Stop, no token */
     PGS_ROW_EMPTY = 3,     /* nothing finite left after masking; token 0, as sampler.rs:59-70 returns */
     PGS_ROW_BAD_PARAM = 4, /* non-finite parameter, bad mask table/state, history too long */
-    PGS_ROW_LOAD_TIMEOUT = 5 /* a bounded wait for another shard's records ran out; nothing sampled */
+    PGS_ROW_LOAD_TIMEOUT = 5 /* a bounded wait ran out (for another shard's records, or of the wide kernel's CTAs for
+                              * one another); nothing sampled, token 0 */
 };
 
 enum pgs_mem { PGS_MEM_DEVICE = 0, PGS_MEM_HOST = 1 };
@@ -258,9 +259,11 @@ PGS_API int pgs_tp_merge_wait(pgs_handle *h, const pgs_tp_desc *desc, const void
 /* Bound of pgs_tp_merge_wait's wait, in polls of about half a microsecond each (default 2^21: about a second).
  * A serving loop that would rather drop a step than stall sets it to a few thousand. */
 PGS_API int pgs_set_wait_limit(pgs_handle *h, uint32_t polls);
-/* Failure detection for the exchange: waits for the stream of the last pgs_tp_merge_wait and returns
+/* Failure detection for the bounded waits: waits for the stream of the last pgs_tp_merge_wait and returns
  * PGS_ERR_TIMEOUT when rows gave up waiting since the previous call of this function (a peer that never
- * answered), PGS_OK otherwise.  The handle stays usable either way. */
+ * answered, or a step or scoring call finished by then whose wide kernel lost a grid barrier: a wait of a few
+ * seconds, PGS_GRID_POLLS in the environment of pgs_create sets it in polls), PGS_OK otherwise.  The handle stays
+ * usable either way. */
 PGS_API int pgs_tp_exchange_status(pgs_handle *h);
 
 /* Draft verification over per-position argmax ids (pagoda-hf/src/qwen3_5.rs:663-755 produces

@@ -550,7 +550,7 @@ class Sampler:
         self._check(self._lib.pgs_set_wait_limit(self._h, C.c_uint32(polls)))
 
     def tp_exchange_status(self):
-        """Raises SamplerError (code -5) when rows gave up waiting for a shard since the last call."""
+        """Raises SamplerError (code -5) when rows gave up a bounded wait (for a shard, or at a grid barrier) since the last call."""
         self._check(self._lib.pgs_tp_exchange_status(self._h))
 
     def tp_merge_wait(self, records_all, flags, epoch, vocab, n_shards, rank, cand, temperature=None, top_p=None,

@@ -165,6 +165,9 @@ int wide_workspace(pgs_handle* h) {
     l.rs = (uint32_t*)(p + o_rs); l.ent_id = (uint32_t*)(p + o_eid); l.ent_xn = (float*)(p + o_exn); l.hist = (uint32_t*)(p + o_hist);
     l.list = h->sl_key; l.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
     l.terms = (float*)(p + o_terms);
+    l.polls = 1u << 23;
+    if (const char* ev = getenv("PGS_GRID_POLLS")) l.polls = (uint32_t)strtoul(ev, nullptr, 10);
+    l.gave_up = h->tp_timeouts;
     h->wide_vocab = vocab;
     return PGS_OK;
 }
@@ -834,7 +837,7 @@ extern "C" int pgs_tp_exchange_status(pgs_handle* h) {
     if (e != cudaSuccess) return fail(h, PGS_ERR_CUDA, "pgs_tp_exchange_status: %s", cudaGetErrorString(e));
     const unsigned long long fresh = n - h->timeouts_seen;
     h->timeouts_seen = n;
-    if (fresh) return fail(h, PGS_ERR_TIMEOUT, "%llu rows gave up waiting for a shard's records", fresh);
+    if (fresh) return fail(h, PGS_ERR_TIMEOUT, "%llu rows gave up waiting for a shard's records or for the other CTAs of the wide kernel", fresh);
     return PGS_OK;
 }
 

@@ -88,11 +88,11 @@ static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
 // The CTAs that take part are those that run when the first of them closes the list (at most one per SM fits; usually all
 // of the grid, but where another stream's kernel keeps SMs busy the launch does not depend on the rest, which leave at
 // once).  So a barrier never waits for a CTA that has not started, and the launch needs no cooperative attribute, which
-// costs 3 us and keeps the work-list pass from being set up early.  Waits have a limit all the same; when one runs out the
-// launch gives up.
-__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, uint32_t limit) {
+// costs 3 us and keeps the work-list pass from being set up early.  Waits have a limit all the same; when one runs out, or
+// has run out for another CTA, the CTA leaves, and the last one to leave gives the rows without results a status of their own.
+__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, uint32_t limit, const uint32_t* given_up) {
     for (uint32_t i = 0; (int32_t)(*(const volatile uint32_t*)p - target) < 0; i++) {
-        if (i > limit) return false;
+        if (i >= limit || ((i & 63u) == 63u && *(const volatile uint32_t*)given_up)) return false;
         __nanosleep(40);
     }
     return true;
@@ -106,7 +106,8 @@ __device__ __forceinline__ bool grid_join(WideSmem& sm, const WideLaunch& l) {
     return !(sm.rank & W_CLOSED);
 }
 
-__device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l) {
+// open: rows that have no result yet
+__device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l, uint32_t open) {
     __syncthreads();
     if (threadIdx.x == 0) {
         bool good = true;
@@ -114,14 +115,14 @@ __device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l) {
         atomicAdd(l.sync, 1u);
         if (sm.target == 0u) {   // the first barrier: how many take part?
             if (sm.rank == 0u) {
-                wait_for(l.sync + 5, gridDim.x, 64u);
+                wait_for(l.sync + 5, gridDim.x, 64u, l.sync + 1);
                 *(volatile uint32_t*)(l.sync + 6) = atomicOr(l.sync + 5, W_CLOSED);
-            } else good = wait_for(l.sync + 6, 1u, 1u << 23);
+            } else good = wait_for(l.sync + 6, 1u, l.polls, l.sync + 1);
             sm.size = *(volatile uint32_t*)(l.sync + 6);
         }
         sm.target += sm.size;
-        good = good && wait_for(l.sync, sm.target, 1u << 23);
-        if (!good) atomicAdd(l.sync + 1, 1u);
+        good = good && wait_for(l.sync, sm.target, l.polls, l.sync + 1);
+        if (!good) atomicMax(l.sync + 1, open);
         __threadfence();
         sm.ok = good;
     }
@@ -1355,6 +1356,27 @@ __device__ __noinline__ void leftover(WideSmem& sm, const RowArgs& a, const Wide
     general_rows(a, sm.general, sm.rank, slots, n, l.left_rows);
 }
 
+// A barrier was given up: the last `open` rows of the launch, and those still to be done by the general kernel's code, end
+// with a status that says so.
+__device__ __noinline__ void give_up(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_work, uint32_t open) {
+    uint32_t n = 0u;
+    const auto end = [&](uint32_t row) {
+        n++;
+        if (!l.score) { wresult_plain(a, row, ROW_LOAD_TIMEOUT, 0u, -INFINITY); return; }
+        if (a.status) a.status[row] = ROW_LOAD_TIMEOUT;
+        if (l.out_gather) l.out_gather[row] = NAN;
+    };
+    for (uint32_t i = n_work - open + threadIdx.x; i < n_work; i += W_NT) end(a.work_rows ? a.work_rows[i] : i);
+    __syncthreads();
+    const uint32_t n_left = l.score ? 0u : *(volatile uint32_t*)l.left_count;
+    for (uint32_t i = threadIdx.x; i < n_left; i += W_NT) {
+        const uint32_t row = __ldcg(l.left_rows + i);
+        if (__ldcg(a.status + row) != ROW_LOAD_TIMEOUT) end(row);
+    }
+    if (n) atomicAdd(l.gave_up, (unsigned long long)n);
+    __syncthreads();
+}
+
 template <bool BF16, bool VEC>
 __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const WideLaunch l_, uint32_t slots) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1378,53 +1400,59 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         uint32_t s = sm.rank;
         if (c0 == 0u) {   // (how many take part is not known yet)
             if (s < n) open(s);
-            if (!(ok = grid_sync(sm, l))) break;
+            if (!(ok = grid_sync(sm, l, n_work - c0))) break;
             s += sm.size;
         }
         if (c0 || sm.size < n) {
             for (; s < n; s += sm.size) open(s);
-            if (!(ok = grid_sync(sm, l))) break;
+            if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         }
         region_phase<BF16, VEC, WP_FIRST>(sm, a, l, n);
-        if (!(ok = grid_sync(sm, l))) break;
+        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(sm, a, l, s);
         if (sm.rank == 0u && tid == 0) { l.sync[2] = 0u; l.sync[3] = 0u; }
-        if (!(ok = grid_sync(sm, l))) break;
+        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         region_phase<BF16, VEC, WP_SUM>(sm, a, l, n);
-        if (!(ok = grid_sync(sm, l))) break;
+        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         for (uint32_t s = sm.rank; s < n; s += sm.size) sum_row<BF16, VEC>(sm, a, l, s);
-        if (!(ok = grid_sync(sm, l))) break;
+        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         if (l.score) {
             if (l.out_full) region_phase<BF16, VEC, WP_FULL>(sm, a, l, n);
         } else {
             if (*(volatile uint32_t*)(l.sync + 2)) {   // (the same for all CTAs)
                 hist_phase<BF16, VEC>(sm, a, l, n);
-                if (!(ok = grid_sync(sm, l))) break;
+                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) select_row(sm, a, l, s);
-                if (!(ok = grid_sync(sm, l))) break;
+                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
                 region_phase<BF16, VEC, WP_LIST>(sm, a, l, n);
-                if (!(ok = grid_sync(sm, l))) break;
+                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) choose_row(sm, a, l, s);
-                if (!(ok = grid_sync(sm, l))) break;
+                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
             }
             if (*(volatile uint32_t*)(l.sync + 3)) {
                 region_phase<BF16, VEC, WP_TOTAL>(sm, a, l, n);
-                if (!(ok = grid_sync(sm, l))) break;
+                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) total_row<BF16, VEC>(sm, a, l, s);
             }
         }
-        if (!(ok = grid_sync(sm, l))) break;   // the chunk's workspace is free
+        if (!(ok = grid_sync(sm, l, n_work - c0))) break;   // the chunk's workspace is free
     }
     if (ok && !l.score) leftover(sm, a, l, slots);
     // the last CTA of the grid to leave resets the counters and empties the lists
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        if (atomicAdd(l.sync + 4, 1u) == gridDim.x - 1u) {
-            l.sync[0] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
-            *l.left_count = 0u;
-            if (a.work_rows) *a.work_count = 0u;
-        }
+        sm.last = atomicAdd(l.sync + 4, 1u) == gridDim.x - 1u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!sm.last) return;
+    const uint32_t open = *(volatile uint32_t*)(l.sync + 1);
+    if (open) give_up(sm, a, l, n_work, open);
+    if (tid == 0) {
+        l.sync[0] = 0u; l.sync[1] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
+        *l.left_count = 0u;
+        if (a.work_rows) *a.work_count = 0u;
     }
 }
 

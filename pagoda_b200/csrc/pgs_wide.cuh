@@ -48,7 +48,9 @@ struct WideLaunch {
     uint32_t* rs;               // [chunk][n_regions + 1]
     uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
     unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
-    uint32_t* sync;             // [0] barrier arrivals, [1] lost waits, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    uint32_t polls;             // limit of a barrier's wait
+    unsigned long long* gave_up; // rows that ended without results because one ran out
     uint32_t chunk;             // rows that the workspace holds (<= W_CHUNK): the launch takes that many at a time
     uint32_t reg_stride, rs_stride, list_stride;
     uint32_t* left_rows;        // rows left to the general kernel

@@ -63,3 +63,41 @@ def test_top_k_bound_beyond_the_float_range(oracle, vocab, exact):
         assert_same(*run_both(s, oracle, w), w, exact=exact)
     finally:
         s.close()
+
+
+def test_a_barrier_that_gives_up_is_reported(monkeypatch):
+    """With no polls allowed every wait of the grid barrier runs out: each row that the wide kernel had to do gets a status
+    of its own, the counted rows come back as an error code once, and other rows and later calls are not affected."""
+    import torch
+    import pagoda_b200
+    rows, vocab = 6, 65536
+    x = torch.randn(rows, vocab, generator=torch.Generator().manual_seed(1))
+    kw = dict(temperature=np.float32([0.7, 0.0, 0.7, 0.0, 0.7, 0.7]), top_k=np.zeros(rows, np.uint32),
+              top_p=np.full(rows, 0.9, np.float32), uniform=np.full(rows, 0.5, np.float32))
+    good = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    monkeypatch.setenv("PGS_GRID_POLLS", "0")
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    try:
+        want = good.sample_batch(x.numpy(), diagnostics=True, **kw)
+        assert (want.status == 0).all()
+        open_rows = kw["temperature"] > 0
+        for _ in range(2):
+            got = s.sample_batch(x.numpy(), diagnostics=True, **kw)   # the work list: rows without top-k
+            assert got.status.tolist() == np.where(open_rows, 5, 0).tolist()
+            assert (got.token[open_rows] == 0).all() and not got.drew.any()
+            assert (got.token[~open_rows] == want.token[~open_rows]).all()
+            with pytest.raises(pagoda_b200.SamplerError, match="4 rows gave up"):
+                s.tp_exchange_status()
+            s.tp_exchange_status()                                    # reported once
+        s.set_exact(True)
+        assert (s.sample_batch(x.numpy(), **kw).status == 5).all()
+        ids = torch.zeros(rows, dtype=torch.int32).cuda()
+        g, _, status = s.log_softmax(x.cuda(), ids=ids, stream_ptr=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert (status.cpu().numpy() == 5).all() and torch.isnan(g).all()
+        with pytest.raises(pagoda_b200.SamplerError, match="12 rows gave up"):
+            s.tp_exchange_status()
+        good.tp_exchange_status()
+    finally:
+        s.close()
+        good.close()
