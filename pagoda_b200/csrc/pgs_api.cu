@@ -78,9 +78,12 @@ struct pgs_handle {
     uint32_t* work_count = nullptr;   // [2]
     uint32_t* tp_done = nullptr;      // CTAs finished in the current peer-store push
     int exact = 0;
-    // wide kernel: its workspace (one block of device memory)
+    // wide kernel: its workspaces (one block of device memory)
     unsigned char* wide_ws = nullptr;
     pgs::WideLaunch wide = {};
+    pgs::WideLaunch score_wide = {};  // scoring: its own workspace
+    cudaEvent_t ev_score = nullptr;   // behind the last scoring call that used it
+    cudaStream_t score_stream = nullptr;
     uint32_t wide_vocab = 0;          // longest row the workspace holds
     // streaming row kernel: id -> count slots, shared memory and CTAs per SM, the gate's counter
     uint32_t stream_hash = 0, stream_cohort = 0;
@@ -141,33 +144,45 @@ uint32_t pow2_at_least(uint32_t v, uint32_t lo) {
 }  // namespace
 
 namespace {
-// The wide kernel's workspace, sized for W_CHUNK rows (fewer when the handle has fewer) of the handle's vocabulary.
+// The wide kernel's workspaces in one block of device memory.  Steps: W_CHUNK rows of the handle's vocabulary, or as many as
+// the handle has.  Scoring has its own, of W_CHUNK rows: it has no row limit, and is not ordered with the handle's steps.
 int wide_workspace(pgs_handle* h) {
     using namespace pgs;
-    const size_t rows = h->slots < (uint32_t)W_CHUNK ? h->slots : (uint32_t)W_CHUNK;
     const uint32_t vocab = h->max_vocab < (uint32_t)W_MAX_VOCAB ? h->max_vocab : (uint32_t)W_MAX_VOCAB;
     const uint32_t regions = (vocab + W_REGION - 1) / W_REGION;
-    WideLaunch& l = h->wide;
-    l.chunk = (uint32_t)rows; l.reg_stride = regions; l.rs_stride = regions + 1u;
-    size_t used = 0;
-    auto take = [&](size_t bytes) { const size_t at = used; used += (bytes + 255) & ~size_t(255); return at; };
-    const size_t o_sync = take(64), o_left = take(4), zeroed = used;
-    const size_t o_rows = take((size_t)h->max_rows * 4), o_row = take(rows * sizeof(WideRow)), o_reg = take(rows * regions * sizeof(float2)), o_cell = take(rows * regions * sizeof(float4));
-    const size_t o_seg = take(rows * regions * sizeof(uint2)), o_pre = take(rows * regions * 4), o_rs = take(rows * (regions + 1u) * 4);
-    const size_t o_eid = take(rows * (W_MAX_HIST + 32) * 4), o_exn = take(rows * (W_MAX_HIST + 32) * 4);
-    const size_t o_hist = take(rows * W_BUCKETS * 4);
-    const size_t o_terms = take(rows * (size_t)W_TERMS * W_REGION * 4);
+    size_t used = 0, zeroed = 0;
+    unsigned char* base = nullptr;
+    auto take = [&](size_t bytes) { unsigned char* const p = (unsigned char*)((uintptr_t)base + used); used += (bytes + 255) & ~size_t(255); return p; };
+    auto plan = [&]() {
+        used = 0;
+        WideLaunch* const both[2] = {&h->wide, &h->score_wide};
+        for (WideLaunch* l : both) { l->sync = (uint32_t*)take(64); l->left_count = (uint32_t*)take(4); }
+        zeroed = used;
+        for (WideLaunch* l : both) {
+            const size_t rows = l == &h->score_wide || h->slots >= (uint32_t)W_CHUNK ? W_CHUNK : h->slots;
+            l->chunk = (uint32_t)rows; l->reg_stride = regions; l->rs_stride = regions + 1u;
+            l->row = (WideRow*)take(rows * sizeof(WideRow)); l->reg = (float2*)take(rows * regions * sizeof(float2));
+            l->cell = (float4*)take(rows * regions * sizeof(float4)); l->seg = (uint2*)take(rows * regions * sizeof(uint2));
+            l->pre = (float*)take(rows * regions * 4); l->terms = (float*)take(rows * (size_t)W_TERMS * W_REGION * 4);
+        }
+        // steps only
+        WideLaunch& l = h->wide;
+        const size_t rows = l.chunk;
+        l.left_rows = (uint32_t*)take((size_t)h->max_rows * 4); l.rs = (uint32_t*)take(rows * (regions + 1u) * 4);
+        l.ent_id = (uint32_t*)take(rows * (W_MAX_HIST + 32) * 4); l.ent_xn = (float*)take(rows * (W_MAX_HIST + 32) * 4);
+        l.hist = (uint32_t*)take(rows * W_BUCKETS * 4);
+    };
+    plan();
     PGS_CUDA(nullptr, cudaMalloc(&h->wide_ws, used));
     PGS_CUDA(nullptr, cudaMemsetAsync(h->wide_ws, 0, zeroed, h->stream));
-    unsigned char* p = h->wide_ws;
-    l.sync = (uint32_t*)(p + o_sync); l.left_count = (uint32_t*)(p + o_left); l.left_rows = (uint32_t*)(p + o_rows);
-    l.row = (WideRow*)(p + o_row); l.reg = (float2*)(p + o_reg); l.cell = (float4*)(p + o_cell); l.seg = (uint2*)(p + o_seg); l.pre = (float*)(p + o_pre);
-    l.rs = (uint32_t*)(p + o_rs); l.ent_id = (uint32_t*)(p + o_eid); l.ent_xn = (float*)(p + o_exn); l.hist = (uint32_t*)(p + o_hist);
-    l.list = h->sl_key; l.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
-    l.terms = (float*)(p + o_terms);
-    l.polls = 1u << 23;
-    if (const char* ev = getenv("PGS_GRID_POLLS")) l.polls = (uint32_t)strtoul(ev, nullptr, 10);
-    l.gave_up = h->tp_timeouts;
+    base = h->wide_ws;
+    plan();
+    h->wide.list = h->sl_key; h->wide.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
+    h->wide.polls = 1u << 23;
+    if (const char* ev = getenv("PGS_GRID_POLLS")) h->wide.polls = (uint32_t)strtoul(ev, nullptr, 10);
+    h->wide.gave_up = h->tp_timeouts;
+    h->score_wide.polls = h->wide.polls; h->score_wide.gave_up = h->wide.gave_up;
+    h->score_wide.score = 1u;
     h->wide_vocab = vocab;
     return PGS_OK;
 }
@@ -181,6 +196,22 @@ int order_steps(pgs_handle* h, cudaStream_t stream) {
         h->last_stream = stream;
     }
     return PGS_OK;
+}
+
+// Whether a scoring call on `stream` may use the scoring workspace.  Scoring is not ordered with anything but its own stream:
+// while a call on another stream may still be running, or where the call is being captured (a graph may be replayed at any
+// time), it takes the kernel that needs no workspace.  The stream of the call before is only compared, never used.
+bool score_workspace_free(pgs_handle* h, cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (another stream may be capturing; the event is in no capture)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventQuery(h->ev_score);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) return true;
+    cudaGetLastError();
+    // (a wait costs nothing where it is the same stream, and is right where only the handle's value is)
+    return e == cudaErrorNotReady && stream == h->score_stream && cudaStreamWaitEvent(stream, h->ev_score, 0) == cudaSuccess;
 }
 
 // CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid
@@ -209,6 +240,7 @@ static int destroy_impl(pgs_handle* h) {
     cudaFree(h->p1_done); cudaFree(h->faulted); cudaFree(h->wide_ws);
     if (h->aux_host) cudaFreeHost(h->aux_host);
     if (h->ev_step) cudaEventDestroy(h->ev_step);
+    if (h->ev_score) cudaEventDestroy(h->ev_score);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return PGS_OK;
@@ -242,6 +274,7 @@ extern "C" int pgs_create(int device, uint32_t max_rows, uint32_t max_vocab, uin
         h->sm_count = prop.multiProcessorCount;
         PGS_CUDA(nullptr, cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
         PGS_CUDA(nullptr, cudaEventCreateWithFlags(&h->ev_step, cudaEventDisableTiming));
+        PGS_CUDA(nullptr, cudaEventCreateWithFlags(&h->ev_score, cudaEventDisableTiming));
         h->last_stream = h->stream;
         PGS_CUDA(nullptr, pgs::configure_general());
         PGS_CUDA(nullptr, pgs::configure_tp());
@@ -865,16 +898,16 @@ extern "C" int pgs_log_softmax(pgs_handle* h, const float* logits, uint32_t rows
     if (rows == 0) return PGS_OK;
     DeviceGuard g(h->device);
     cudaStream_t stream = cuda_stream ? (cudaStream_t)cuda_stream : h->stream;
-    if (vocab <= h->wide_vocab) {
-        const int rc = order_steps(h, stream);
-        if (rc != PGS_OK) return rc;
+    if (vocab <= h->wide_vocab && score_workspace_free(h, stream)) {
         pgs::RowArgs a;
         memset(&a, 0, sizeof a);
         a.logits = logits; a.rows = rows; a.vocab = vocab; a.row_stride = row_stride; a.status = status; a.eos = -1;
-        pgs::WideLaunch l = h->wide;
-        l.score = 1u; l.ids = ids; l.out_gather = out_gather; l.out_full = out_full;
+        pgs::WideLaunch l = h->score_wide;
+        l.ids = ids; l.out_gather = out_gather; l.out_full = out_full;
         PGS_CUDA(h, pgs::launch_wide(a, l, h->slots, wide_grid(h, rows, vocab), stream));
-    } else {   // longer rows than the handle was made for: one CTA per row, no workspace
+        PGS_CUDA(h, cudaEventRecord(h->ev_score, stream));
+        h->score_stream = stream;
+    } else {   // one CTA per row, no workspace
         pgs::ScoreArgs a{logits, row_stride, rows, vocab, ids, out_gather, out_full, status};
         const uint32_t grid = rows < (uint32_t)h->sm_count ? rows : (uint32_t)h->sm_count;
         PGS_CUDA(h, pgs::launch_log_softmax(a, grid, stream));

@@ -63,3 +63,62 @@ def test_more_rows_than_the_handle_was_made_for(oracle, rows, vocab):
             assert g[r] == full[r][ids[r]]
     finally:
         s.close()
+
+
+def test_scoring_keeps_nothing_of_the_stream_it_ran_on():
+    """Scoring on one stream does not wait for the handle's work on another, can be captured whatever ran before, and the
+    stream may be gone when the handle is used again; every route gives the same bits."""
+    import ctypes
+    import torch
+    import pagoda_b200
+    rows, vocab = 16, 50257
+    x = torch.randn(rows, vocab, generator=torch.Generator().manual_seed(5)).cuda() * 3
+    ids = torch.arange(rows, dtype=torch.int32).cuda() * 3000
+    other, busy = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    token, status = torch.zeros(rows, dtype=torch.int32).cuda(), torch.zeros(rows, dtype=torch.int32).cuda()
+    step = s.make_device_desc(x, token=token, status=status)
+
+    def score(stream):
+        with torch.cuda.stream(stream):
+            g, full, st = s.log_softmax(x, ids=ids, full=True, stream_ptr=stream.cuda_stream)
+            return torch.cat([g[:, None], full], 1), st
+
+    try:
+        want, st = score(other)
+        other.synchronize()
+        assert (st == 0).all()
+        # captured on a stream that is not the handle's last one
+        s.launch_device(step, busy.cuda_stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=other):
+            captured, _ = score(other)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(captured, want)
+        # a step and a scoring call behind a long kernel on one stream, scoring on another
+        with torch.cuda.stream(busy):
+            torch.cuda._sleep(1 << 30)
+        s.launch_device(step, busy.cuda_stream)
+        late, _ = score(busy)
+        again, _ = score(busy)
+        now, _ = score(other)
+        other.synchronize()
+        assert not busy.query()
+        assert torch.equal(now, want)
+        busy.synchronize()
+        assert torch.equal(late, want) and torch.equal(again, want)
+        # a stream that is destroyed afterwards
+        rt, raw = torch.cuda.cudart(), ctypes.c_void_p()
+        assert rt.cudaStreamCreate(ctypes.addressof(raw)) == 0
+        gone, _ = score(torch.cuda.ExternalStream(raw.value))
+        torch.cuda.synchronize()
+        assert rt.cudaStreamDestroy(raw.value) == 0
+        assert torch.equal(gone, want)
+        s.launch_device(step, other.cuda_stream)
+        last, _ = score(busy)
+        torch.cuda.synchronize()
+        assert torch.equal(last, want) and torch.equal(token.long(), x.argmax(1))
+    finally:
+        s.close()
