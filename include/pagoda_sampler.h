@@ -281,8 +281,9 @@ PGS_API int pgs_draft_accept(pgs_handle *h, const uint32_t *row_argmax, const ui
  * only enqueues work on `cuda_stream` (NULL = the handle's stream).  Rows holding a non-finite
  * logit get status PGS_ROW_NONFINITE and NaN.  `rows` has no limit.  Scoring has working storage of its
  * own: it is ordered with nothing but its stream, not with the handle's steps, keeps no use of the stream
- * behind the call, and may be captured (captured calls, calls while another stream's scoring still runs, and
- * rows longer than the handle's vocabulary take a kernel that needs no storage, with the same results). */
+ * behind the call, and may be captured (captured calls, calls while another stream's scoring still runs,
+ * rows longer than the handle's vocabulary, and short rows or many take a kernel that needs no storage, with the
+ * same results). */
 PGS_API int pgs_log_softmax(pgs_handle *h, const float *logits, uint32_t rows, uint32_t vocab,
                             uint64_t row_stride, const uint32_t *ids, float *out_gather, float *out_full,
                             int32_t *status, void *cuda_stream);

@@ -214,6 +214,19 @@ bool score_workspace_free(pgs_handle* h, cudaStream_t stream) {
     return e == cudaErrorNotReady && stream == h->score_stream && cudaStreamWaitEvent(stream, h->ev_score, 0) == cudaSuccess;
 }
 
+// Whether the wide kernel scores a batch faster than one CTA per row does.  One CTA per row: 25 us and 1.2 us per thousand
+// logits (2 us with the whole vector written) for as many rows as there are SMs; wide: 38 us (47) and 4.3 us (10) per million
+// logits for every chunk.  Lines through (us, one CTA per row / wide): 64 x 1000 24 / 39, 64 x 4096 39 / 42, 64 x 16384
+// 53 / 48, 128 x 16384 53 / 85, 128 x 50257 96 / 103, 64 x 151936 199 / 80, 256 x 151936 407 / 307; whole vectors 64 x 1000
+// 25 / 47, 256 x 16384 117 / 205, 256 x 151936 640 / 566.
+bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool full) {
+    const uint32_t sms = (uint32_t)h->sm_count, chunk = h->score_wide.chunk;
+    const double logits = 1e-6 * (rows < chunk ? rows : chunk) * (double)vocab;
+    const double per_row = ((rows - 1u) / sms + 1u) * (25.0 + vocab / (full ? 500.0 : 850.0));
+    const double wide = ((rows - 1u) / chunk + 1u) * (full ? 47.0 + 10.0 * logits : 38.0 + 4.3 * logits);
+    return wide < per_row;
+}
+
 // CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid
 // barriers cost more with more CTAs).
 uint32_t wide_grid(const pgs_handle* h, uint32_t rows, uint32_t vocab) {
@@ -898,7 +911,7 @@ extern "C" int pgs_log_softmax(pgs_handle* h, const float* logits, uint32_t rows
     if (rows == 0) return PGS_OK;
     DeviceGuard g(h->device);
     cudaStream_t stream = cuda_stream ? (cudaStream_t)cuda_stream : h->stream;
-    if (vocab <= h->wide_vocab && score_workspace_free(h, stream)) {
+    if (vocab <= h->wide_vocab && wide_scores_faster(h, rows, vocab, out_full != nullptr) && score_workspace_free(h, stream)) {
         pgs::RowArgs a;
         memset(&a, 0, sizeof a);
         a.logits = logits; a.rows = rows; a.vocab = vocab; a.row_stride = row_stride; a.status = status; a.eos = -1;

@@ -1,0 +1,62 @@
+// Which rows are done by the whole grid (pgs_wide.cu) and which by one CTA each (pgs_general.cuh).  Both give the same bits; the
+// choice is which is quicker for a batch, from what its rows ask for.
+#pragma once
+
+#include "pgs_args.cuh"
+#include "pgs_wide.cuh"
+
+namespace pgs {
+
+// What rows ask for, as far as it decides that; a batch: all of its rows together.
+enum : uint32_t { WK_SAMPLED = 1u, WK_HIST = 2u, WK_OPEN = 4u, WK_SORT = 8u, WK_LONG = 16u };
+constexpr uint32_t WK_ALL = 32u;
+
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t row_kind(const RowArgs& a, uint32_t row) {
+    const float temp = a.temperature ? a.temperature[row] : 0.0f, top_p = a.top_p ? a.top_p[row] : 1.0f;
+    const uint32_t k = a.top_k ? a.top_k[row] : 0u, n_regions = (a.vocab + W_REGION - 1) / W_REGION;
+    const uint32_t nh = a.hist_offsets ? a.hist_offsets[row + 1] - a.hist_offsets[row] : 0u;
+    const uint32_t is_long = nh > (uint32_t)W_MAX_HIST ? WK_LONG : 0u;
+    if (temp < 1e-5f) return is_long;
+    const bool open = k == 0u || k >= a.vocab, big = open || k > (uint32_t)W_KMAX;
+    return WK_SAMPLED | is_long | (big || k > 4u * n_regions ? WK_HIST : 0u) | (open ? WK_OPEN : 0u) | (big && !(top_p >= 1.0f) ? WK_SORT : 0u);
+}
+// the kinds of the first n rows (of the list, or of the batch); `slot`: zero, with a barrier behind it.  A barrier is needed
+// before the result is in `slot`.
+__device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32_t threads, uint32_t* slot) {
+    uint32_t kinds = 0u;
+    for (uint32_t i = threadIdx.x; i < n; i += threads) kinds |= row_kind(a, a.work_rows ? a.work_rows[i] : i);
+    kinds = __reduce_or_sync(0xffffffffu, kinds);
+    if ((threadIdx.x & 31u) == 0u && kinds) atomicOr(slot, kinds);
+}
+#endif
+
+// One bit per combination of kinds: one CTA per row is the quicker way for `n` rows.  Short rows do not pay for the grid's
+// barriers, and batches of many rows go through the grid in chunks of 64 where one CTA per row takes an SM count at a time.
+// us of one row on one CTA: greedy 9 + 0.37 per thousand logits, sampled 47 + 2.2, without top-k 5 more per thousand, with a
+// sort for top-p 75 + 20; of a chunk: greedy 27, sampled 44 (70 where the threshold needs the histogram), 4 per million
+// logits.  Measured (one CTA per row / grid): top-k 50, 1 x 1000 48 / 68, 64 x 4096 64 / 83, 64 x 16384 93 / 54, 128 x 16384
+// 94 / 102, 256 x 50256 338 / 240, 1024 x 16384 576 / 769; greedy 1 x 1000 9 / 27, 64 x 50256 31 / 35, 1 x 151936 64 / 27,
+// 256 x 50256 64 / 126, 256 x 151936 217 / 166; no top-k 16 x 1000 59 / 68, 16 x 16384 160 / 91, with top-p 1 x 1000 76 / 71,
+// 16 x 4096 161 / 78.  Rows with a history beyond the workspace end on one CTA either way (4 of 50256: 187 at once, 239
+// behind the phases).
+inline uint32_t kinds_one_cta_each(uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool long_histories) {
+    const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
+    const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
+    uint32_t mask = 0u;
+    for (uint32_t kinds = 0; kinds < WK_ALL; kinds++) {
+        float row, grid;
+        if (kinds & WK_SAMPLED) {
+            row = kinds & WK_SORT ? 75.0f + 0.02f * v : 47.0f + 0.0022f * v + (kinds & WK_OPEN ? 0.005f * v : 0.0f);
+            grid = (kinds & WK_HIST ? 70.0f : 44.0f) + 4.0f * m;
+        } else {
+            row = 9.0f + 3.7e-4f * v + 1.5e-6f * v * together;
+            grid = 27.0f + 1.65f * m;
+        }
+        if ((kinds & WK_LONG) && !long_histories) row = INFINITY;   // (does not occur)
+        if (waves * row < chunks * grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
+    }
+    return mask;
+}
+
+}  // namespace pgs

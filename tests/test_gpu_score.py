@@ -122,3 +122,25 @@ def test_scoring_keeps_nothing_of_the_stream_it_ran_on():
         assert torch.equal(last, want) and torch.equal(token.long(), x.argmax(1))
     finally:
         s.close()
+
+
+def test_both_kernels_score_alike():
+    """Short rows and batches of many rows are scored by one CTA per row, others by the whole grid: the same row gives the
+    same bits in batches on either side of the line."""
+    import torch
+    import pagoda_b200
+    st = torch.cuda.current_stream().cuda_stream
+    for vocab, many, few in ((16384, 128, 64), (50257, 128, 64), (4096, 64, 1), (20000, 64, 1)):
+        x = torch.randn(many, vocab, generator=torch.Generator().manual_seed(vocab)).cuda() * 3
+        ids = torch.arange(many, dtype=torch.int32).cuda() * 7
+        s = pagoda_b200.Sampler(device=0, max_rows=4, max_vocab=vocab, max_history=1)
+        try:
+            for full in (False, True):
+                a = s.log_softmax(x, ids=ids, full=full, stream_ptr=st)
+                b = s.log_softmax(x[:few], ids=ids[:few], full=full, stream_ptr=st)
+                torch.cuda.synchronize()
+                assert torch.equal(a[0][:few], b[0]) and (a[2] == 0).all()
+                if full:
+                    assert torch.equal(a[1][:few], b[1])
+        finally:
+            s.close()
