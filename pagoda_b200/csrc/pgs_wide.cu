@@ -48,18 +48,18 @@ constexpr uint32_t W_DUAL = 2u;          // beside a segment's binade: it may al
 struct alignas(16) WideSmem {
     RowArgs a;                           // the launch's arguments, for the phases, which are functions of their own
     WideLaunch l;
-    WideRow row;
-    WideRow rows[W_CHUNK];               // region phases: the chunk's rows
+    alignas(16) WideRow row;
+    alignas(16) WideRow rows[W_CHUNK];               // region phases: the chunk's rows
     unsigned long long exp_tab[32];
     uint32_t red_u[WNW], red_v[WNW];
     float red_f[WNW];
     double red_d[WNW];
-    uint32_t last, found, n_serial, ok;
+    uint32_t last, found, n_serial, ok, gave_up;
     uint32_t rank, size, target;         // of the CTA among those that take part; arrivals at the barrier behind this one
     float R;
-    float stage[WNW][W_REGION];          // per warp: a region in id order
-    float spare[W_REGION];
-    Runs runs[WNW][32];
+    alignas(16) float stage[WNW][W_REGION];   // per warp: a region in id order
+    alignas(16) float spare[W_REGION];
+    alignas(16) Runs runs[WNW][32];
     uint32_t serial[W_MAX_REGIONS];      // segments that are added term by term
     union {
         struct {
@@ -88,11 +88,11 @@ static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
 // The CTAs that take part are those that run when the first of them closes the list (at most one per SM fits; usually all
 // of the grid, but where another stream's kernel keeps SMs busy the launch does not depend on the rest, which leave at
 // once).  So a barrier never waits for a CTA that has not started, and the launch needs no cooperative attribute, which
-// costs 3 us and keeps the work-list pass from being set up early.  Waits have a limit all the same; when one runs out, or
-// has run out for another CTA, the CTA leaves, and the last one to leave gives the rows without results a status of their own.
-__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, uint32_t limit, const uint32_t* given_up) {
+// costs 3 us and keeps the work-list pass from being set up early.  Waits have a limit all the same; when one runs out the
+// CTA leaves (and the others when theirs do), and the last one to leave gives the rows without results a status of their own.
+__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t target, uint32_t limit) {
     for (uint32_t i = 0; (int32_t)(*(const volatile uint32_t*)p - target) < 0; i++) {
-        if (i >= limit || ((i & 63u) == 63u && *(const volatile uint32_t*)given_up)) return false;
+        if (i >= limit) return false;
         __nanosleep(40);
     }
     return true;
@@ -115,14 +115,14 @@ __device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l, uin
         atomicAdd(l.sync, 1u);
         if (sm.target == 0u) {   // the first barrier: how many take part?
             if (sm.rank == 0u) {
-                wait_for(l.sync + 5, gridDim.x, 64u, l.sync + 1);
+                wait_for(l.sync + 5, gridDim.x, 64u);
                 *(volatile uint32_t*)(l.sync + 6) = atomicOr(l.sync + 5, W_CLOSED);
-            } else good = wait_for(l.sync + 6, 1u, l.polls, l.sync + 1);
+            } else good = wait_for(l.sync + 6, 1u, l.polls);
             sm.size = *(volatile uint32_t*)(l.sync + 6);
         }
         sm.target += sm.size;
-        good = good && wait_for(l.sync, sm.target, l.polls, l.sync + 1);
-        if (!good) atomicMax(l.sync + 1, open);
+        good = good && wait_for(l.sync, sm.target, l.polls);
+        if (!good) { atomicMax(l.sync + 1, open); sm.gave_up = 1u; }
         __threadfence();
         sm.ok = good;
     }
@@ -1356,9 +1356,9 @@ __device__ __noinline__ void leftover(WideSmem& sm, const RowArgs& a, const Wide
     general_rows(a, sm.general, sm.rank, slots, n, l.left_rows);
 }
 
-// A barrier was given up: the last `open` rows of the launch, and those still to be done by the general kernel's code, end
-// with a status that says so.
-__device__ __noinline__ void give_up(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_work, uint32_t open) {
+// A barrier was given up: the last rows of the launch, and those still to be done by the general kernel's code, end with a
+// status that says so.  One thread.
+__device__ __noinline__ void give_up(const RowArgs& a, const WideLaunch& l, uint32_t n_work) {
     uint32_t n = 0u;
     const auto end = [&](uint32_t row) {
         n++;
@@ -1366,15 +1366,14 @@ __device__ __noinline__ void give_up(WideSmem& sm, const RowArgs& a, const WideL
         if (a.status) a.status[row] = ROW_LOAD_TIMEOUT;
         if (l.out_gather) l.out_gather[row] = NAN;
     };
-    for (uint32_t i = n_work - open + threadIdx.x; i < n_work; i += W_NT) end(a.work_rows ? a.work_rows[i] : i);
-    __syncthreads();
-    const uint32_t n_left = l.score ? 0u : *(volatile uint32_t*)l.left_count;
-    for (uint32_t i = threadIdx.x; i < n_left; i += W_NT) {
+    for (uint32_t i = n_work - __ldcg(l.sync + 1); i < n_work; i++) end(a.work_rows ? a.work_rows[i] : i);
+    const uint32_t n_left = l.score ? 0u : __ldcg(l.left_count);
+    for (uint32_t i = 0; i < n_left; i++) {
         const uint32_t row = __ldcg(l.left_rows + i);
         if (__ldcg(a.status + row) != ROW_LOAD_TIMEOUT) end(row);
     }
-    if (n) atomicAdd(l.gave_up, (unsigned long long)n);
-    __syncthreads();
+    atomicAdd(l.gave_up, (unsigned long long)n);
+    l.sync[1] = 0u;
 }
 
 template <bool BF16, bool VEC>
@@ -1389,7 +1388,7 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     cudaGridDependencySynchronize();
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass
-    if (tid == 0) { sm.a = a_; sm.target = 0u; }
+    if (tid == 0) { sm.a = a_; sm.target = 0u; sm.gave_up = 0u; }
     if (tid == 32u) sm.l = l_;
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
@@ -1438,21 +1437,17 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;   // the chunk's workspace is free
     }
     if (ok && !l.score) leftover(sm, a, l, slots);
-    // the last CTA of the grid to leave resets the counters and empties the lists
+    // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        sm.last = atomicAdd(l.sync + 4, 1u) == gridDim.x - 1u;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!sm.last) return;
-    const uint32_t open = *(volatile uint32_t*)(l.sync + 1);
-    if (open) give_up(sm, a, l, n_work, open);
-    if (tid == 0) {
-        l.sync[0] = 0u; l.sync[1] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
-        *l.left_count = 0u;
-        if (a.work_rows) *a.work_count = 0u;
+        const uint32_t before = atomicAdd(l.sync + 4, sm.gave_up ? 0x10001u : 1u);
+        if ((before & 0xffffu) == gridDim.x - 1u) {
+            if ((before >> 16) || sm.gave_up) { __threadfence(); give_up(a, l, n_work); }
+            l.sync[0] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
+            *l.left_count = 0u;
+            if (a.work_rows) *a.work_count = 0u;
+        }
     }
 }
 
