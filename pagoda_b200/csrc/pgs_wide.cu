@@ -1447,6 +1447,7 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             l.sync[0] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
             *l.left_count = 0u;
             if (a.work_rows) *a.work_count = 0u;
+            if (l.done) { __threadfence(); *(volatile uint32_t*)l.done = l.done_value; }   // (the next launch starts behind this)
         }
     }
 }

@@ -60,6 +60,8 @@ struct WideLaunch {
     const uint32_t* ids;
     float* out_gather;
     float* out_full;
+    uint32_t* done;             // host memory: gets done_value when the launch no longer uses its workspace
+    uint32_t done_value;
 };
 
 }  // namespace pgs
