@@ -4,6 +4,7 @@
 #include "../../include/pagoda_sampler.h"
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -14,6 +15,7 @@
 #include <vector>
 
 #include "pgs_args.cuh"
+#include "pgs_kinds.cuh"
 #include "pgs_stream.cuh"
 #include "pgs_tp.cuh"
 #include "pgs_wide.cuh"
@@ -87,6 +89,7 @@ struct pgs_handle {
     uint32_t score_calls = 0;         // how many there were
     unsigned long long score_stream = 0;   // id of the last one's stream
     uint32_t wide_vocab = 0;          // longest row the workspace holds
+    int wide_route = 0;               // 1: always the grid, 2: always one CTA per row (tests)
     // streaming row kernel: id -> count slots, shared memory and CTAs per SM, the gate's counter
     uint32_t stream_hash = 0, stream_cohort = 0;
     int max_clusters[4] = {0, 0, 0, 0};   // resident clusters of 1 (unused), 2, 4, 8 CTAs of the row kernel
@@ -182,6 +185,7 @@ int wide_workspace(pgs_handle* h) {
     h->wide.list = h->sl_key; h->wide.list_stride = h->sort_pad;   // (free until the launch's own leftovers go to general_rows)
     h->wide.polls = 1u << 23;
     if (const char* ev = getenv("PGS_GRID_POLLS")) h->wide.polls = (uint32_t)strtoul(ev, nullptr, 10);
+    if (const char* ev = getenv("PGS_WIDE_ROUTE")) h->wide_route = atoi(ev);
     h->wide.gave_up = h->tp_timeouts;
     h->score_wide.polls = h->wide.polls; h->score_wide.gave_up = h->wide.gave_up;
     h->score_wide.score = 1u;
@@ -225,6 +229,19 @@ bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool
     const double per_row = ((rows - 1u) / sms + 1u) * (25.0 + vocab / (full ? 500.0 : 850.0));
     const double wide = ((rows - 1u) / chunk + 1u) * (full ? 47.0 + 10.0 * logits : 38.0 + 4.3 * logits);
     return wide < per_row;
+}
+
+// The combinations of kinds that one CTA per row does quicker (*row), and those that the grid does (returned), among those
+// that the handle's rows can have.
+uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row) {
+    using namespace pgs;
+    const bool long_histories = h->max_history > (uint32_t)W_MAX_HIST;
+    uint32_t possible = 0u;
+    for (uint32_t k = 0; k < WK_ALL; k++)
+        if (((k & WK_SAMPLED) || !(k & (WK_HIST | WK_OPEN | WK_SORT))) && ((k & WK_HIST) || !(k & (WK_OPEN | WK_SORT))) && (long_histories || !(k & WK_LONG))) possible |= 1u << k;
+    const uint32_t mask = h->wide_route == 1 ? 0u : h->wide_route == 2 ? ~0u : kinds_one_cta_each(rows, h->wide.chunk, h->slots, vocab, long_histories);
+    *row = mask & possible;
+    return ~mask & possible;
 }
 
 // CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid
@@ -445,9 +462,24 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
     const uint32_t per = a.dtype == 0 ? 4u : 8u;
     const bool aligned = ((uintptr_t)a.logits & 15u) == 0u && a.row_stride % per == 0u && a.vocab % per == 0u;
     if (h->exact || a.vocab > (uint32_t)pgs::S_MAX_VOCAB || (wide && !aligned)) {
-        if (wide) PGS_CUDA(h, pgs::launch_wide(a, h->wide, h->slots, wide_grid(h, rows, a.vocab), stream));
-        else PGS_CUDA(h, pgs::launch_general(a, grid, stream));
-        h->counters.kernel_launches += 1;
+        // What the rows ask for is known on the device only: where both ways are in question, both kernels are launched, and
+        // the one whose batch it is not returns at once.
+        pgs::WideLaunch wl = h->wide;
+        uint32_t grid_kinds = 0u;
+        if (wide) grid_kinds = kinds_for(h, rows, a.vocab, &wl.kinds_front);
+        wl.look = wl.kinds_front;
+        if (!wide || !grid_kinds || wl.kinds_front) {
+            pgs::RowArgs front = a;
+            if (wide && grid_kinds) front.kinds_here = wl.kinds_front;
+            PGS_CUDA(h, pgs::launch_general(front, grid, stream));
+            h->counters.kernel_launches += 1;
+        }
+        if (grid_kinds) {
+            // (both fit on no SM together)
+            const uint32_t want = wide_grid(h, rows, a.vocab), sms = (uint32_t)h->sm_count, room = wl.kinds_front && rows <= sms / 2u ? sms - rows : sms;
+            PGS_CUDA(h, pgs::launch_wide(a, wl, h->slots, want < room ? want : room, stream));
+            h->counters.kernel_launches += 1;
+        }
         return PGS_OK;
     }
     pgs::StreamLaunch sl;
@@ -475,7 +507,11 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         // the pass takes only those, and is in place before the rows are done.
         const uint32_t busy = rows * csize, want = wide_grid(h, rows, a.vocab), sms = (uint32_t)h->sm_count;
         const uint32_t room = csize > 1u && busy <= sms / 2u ? sms - busy : sms;
-        PGS_CUDA(h, pgs::launch_wide(wl, h->wide, h->slots, want < room ? want : room, stream));
+        pgs::WideLaunch l = h->wide;   // (how many rows are listed is known on the device only)
+        kinds_for(h, rows < l.chunk ? rows : l.chunk, a.vocab, &l.kinds_row[0]);
+        if (rows > l.chunk) kinds_for(h, rows, a.vocab, &l.kinds_row[1]);
+        l.look = l.kinds_row[0] | l.kinds_row[1];
+        PGS_CUDA(h, pgs::launch_wide(wl, l, h->slots, want < room ? want : room, stream));
     }
     else PGS_CUDA(h, pgs::launch_general(wl, grid < 32u ? grid : 32u, stream));
     h->counters.kernel_launches += 2;

@@ -70,6 +70,8 @@ struct RowArgs {
     unsigned char* tp_records;      // [rows x tp_rec_bytes]
     uint32_t tp_rec_bytes, tp_cand;
     uint32_t id_base;               // global id of column 0 (0 outside of the sharded mode)
+    // general kernel: where not zero, only a batch whose rows' kinds (pgs_kinds.cuh) have their bit set here is its own
+    uint32_t kinds_here;
 };
 
 // One shard's share of one row.  n_status: candidates in the record (low 24 bits) and the row status the shard

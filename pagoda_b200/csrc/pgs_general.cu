@@ -1,5 +1,6 @@
 // General row kernel: see pgs_general.cuh.
 #include "pgs_general.cuh"
+#include "pgs_kinds.cuh"
 
 namespace pgs {
 
@@ -7,11 +8,18 @@ __global__ void __launch_bounds__(NT, 1) general_row_kernel(const RowArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GeneralSmem& sm = *reinterpret_cast<GeneralSmem*>(smem_raw);
     const int tid = threadIdx.x;
+    if (a.kinds_here) cudaTriggerProgrammaticLaunchCompletion();   // the wide kernel behind this one is set up meanwhile
     if (a.work_rows) cudaGridDependencySynchronize();   // the work-list pass is launched ahead of the end of the kernel that fills the list
     const uint32_t n_work = a.work_rows ? *a.work_count : a.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass: nothing listed, nothing to reset
     if (tid < 32) sm.exp_tab[tid] = kExp2TableDev[tid];
+    if (tid == 0) sm.kinds = 0u;
     __syncthreads();
+    if (a.kinds_here) {   // the wide kernel behind this one does the others
+        batch_kinds(a, n_work, NT, &sm.kinds);
+        __syncthreads();
+        if (!((a.kinds_here >> sm.kinds) & 1u)) return;
+    }
     general_rows(a, sm, blockIdx.x, gridDim.x, n_work, a.work_rows);
     // the last CTA to finish a work list empties it for the next step
     if (a.work_rows && tid == 0) {

@@ -24,6 +24,7 @@ struct GeneralSmem {
     SelectSmem sel;
     unsigned long long sort_tile[SORT_TILE];
     unsigned long long exp_tab[32];
+    uint32_t kinds;
 };
 
 __device__ __forceinline__ float load_logit(const void* base, uint32_t dtype, size_t i) {

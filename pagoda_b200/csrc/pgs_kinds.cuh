@@ -34,7 +34,7 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 // One bit per combination of kinds: one CTA per row is the quicker way for `n` rows.  Short rows do not pay for the grid's
 // barriers, and batches of many rows go through the grid in chunks of 64 where one CTA per row takes an SM count at a time.
 // us of one row on one CTA: greedy 9 + 0.37 per thousand logits, sampled 47 + 2.2, without top-k 5 more per thousand, with a
-// sort for top-p 75 + 20; of a chunk: greedy 27, sampled 44 (70 where the threshold needs the histogram), 4 per million
+// sort for top-p 60 + 18; of a chunk: greedy 27, sampled 44 (70 where the threshold needs the histogram), 4 per million
 // logits.  Measured (one CTA per row / grid): top-k 50, 1 x 1000 48 / 68, 64 x 4096 64 / 83, 64 x 16384 93 / 54, 128 x 16384
 // 94 / 102, 256 x 50256 338 / 240, 1024 x 16384 576 / 769; greedy 1 x 1000 9 / 27, 64 x 50256 31 / 35, 1 x 151936 64 / 27,
 // 256 x 50256 64 / 126, 256 x 151936 217 / 166; no top-k 16 x 1000 59 / 68, 16 x 16384 160 / 91, with top-p 1 x 1000 76 / 71,
@@ -43,11 +43,12 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 inline uint32_t kinds_one_cta_each(uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool long_histories) {
     const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
     const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
+    if (V <= 1024u) return ~0u;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     uint32_t mask = 0u;
     for (uint32_t kinds = 0; kinds < WK_ALL; kinds++) {
         float row, grid;
         if (kinds & WK_SAMPLED) {
-            row = kinds & WK_SORT ? 75.0f + 0.02f * v : 47.0f + 0.0022f * v + (kinds & WK_OPEN ? 0.005f * v : 0.0f);
+            row = kinds & WK_SORT ? 60.0f + 0.018f * v : 47.0f + 0.0022f * v + (kinds & WK_OPEN ? 0.005f * v : 0.0f);
             grid = (kinds & WK_HIST ? 70.0f : 44.0f) + 4.0f * m;
         } else {
             row = 9.0f + 3.7e-4f * v + 1.5e-6f * v * together;

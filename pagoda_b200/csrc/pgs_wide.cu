@@ -34,6 +34,7 @@
 #include "pgs_block.cuh"
 #include "pgs_finish.cuh"
 #include "pgs_general.cuh"
+#include "pgs_kinds.cuh"
 #include "pgs_wide.cuh"
 
 namespace pgs {
@@ -42,7 +43,7 @@ constexpr int WNW = W_NT / 32;
 constexpr int WL = W_REGION / 32;        // logits per lane and region
 static_assert(WL == RUN, "a region is a warp's runs");
 constexpr uint32_t W_NIL = 0xffffffffu;
-constexpr uint32_t F_KMAX = F_MCAP / 2;  // top-k up to which the second pass lists the candidates
+static_assert(W_KMAX <= F_MCAP / 2, "room for the candidates");
 constexpr uint32_t W_DUAL = 2u;          // beside a segment's binade: it may also be the next one
 
 struct alignas(16) WideSmem {
@@ -672,7 +673,7 @@ __device__ __noinline__ void maximum_row(WideSmem& sm, const RowArgs& a, const W
         else c.state = WS_SUM;
     }
     __syncthreads();
-    if (sm.row.state == WS_SUM && sm.row.cut_x == INFINITY && !l.score && sm.row.top_k != 0u && sm.row.top_k < V && sm.row.top_k <= (uint32_t)F_KMAX) {
+    if (sm.row.state == WS_SUM && sm.row.cut_x == INFINITY && !l.score && sm.row.top_k != 0u && sm.row.top_k < V && sm.row.top_k <= (uint32_t)W_KMAX) {
         // A row with a short top-k: the k-th largest of the parts' maxima is reached by at least k logits, so everything
         // from a little below it on (for ties) is a superset of the top-k set, and nearly always a small one.  As in the
         // streaming kernel: buckets of equal width between the smallest finite maximum and the largest.
@@ -1346,14 +1347,28 @@ __device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const Wi
     }
 }
 
-__device__ __noinline__ void leftover(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slots) {
-    const uint32_t n = *(volatile uint32_t*)l.left_count;
-    slots = min(slots, sm.size);
-    if (n == 0u || sm.rank >= slots) return;
+// `n` rows (of the list, or of the batch) one CTA each, by the general kernel's code on `slots` scratch slots
+__device__ __noinline__ void rows_one_cta_each(WideSmem& sm, const RowArgs& a, uint32_t rank, uint32_t slots, uint32_t n, const uint32_t* rows) {
+    if (n == 0u || rank >= slots) return;
     __syncthreads();
     if (threadIdx.x < 32u) sm.general.exp_tab[threadIdx.x] = kExp2TableDev[threadIdx.x];
     __syncthreads();
-    general_rows(a, sm.general, sm.rank, slots, n, l.left_rows);
+    general_rows(a, sm.general, rank, slots, n, rows);
+}
+
+// Whether the batch is done by one CTA per row; it is when this returns true.  (A general kernel for the same rows in front is
+// waited for only here: what the rows ask for stands already.  A function of its own, as the usual launch would fetch the code.)
+__device__ __noinline__ bool look(WideSmem& sm, uint32_t n_work, uint32_t slots) {
+    const WideLaunch& l = sm.l;
+    if (threadIdx.x == 0) sm.found = 0u;
+    __syncthreads();
+    batch_kinds(sm.a, n_work, W_NT, &sm.found);
+    __syncthreads();
+    const bool front = l.kinds_front != 0u;
+    const bool per_row = ((front ? l.kinds_front : n_work > l.chunk ? l.kinds_row[1] : l.kinds_row[0]) >> sm.found) & 1u;
+    if (front) cudaGridDependencySynchronize();
+    else if (per_row) rows_one_cta_each(sm, sm.a, blockIdx.x, min(slots, gridDim.x), n_work, sm.a.work_rows);
+    return per_row;
 }
 
 // A barrier was given up: the last rows of the launch, and those still to be done by the general kernel's code, end with a
@@ -1385,14 +1400,19 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     const uint32_t tid = threadIdx.x;
     // Launched ahead of the end of the kernel before, which may fill the list.  (No early trigger for the kernel behind: its
     // CTAs would crowd on the SMs that this one leaves free, 128 masked rows 50 -> 62 us.)
-    cudaGridDependencySynchronize();
+    if (!l_.kinds_front) cudaGridDependencySynchronize();
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass
     if (tid == 0) { sm.a = a_; sm.target = 0u; sm.gave_up = 0u; }
     if (tid == 32u) sm.l = l_;
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
-    bool ok = grid_join(sm, l);
+    bool ok = true;   // (false for all CTAs, or none)
+    if (l_.look) {
+        ok = !look(sm, n_work, slots);
+        if (!ok && l_.kinds_front) return;
+    }
+    ok = ok && grid_join(sm, l);
     for (uint32_t c0 = 0; c0 < n_work && ok; c0 += l.chunk) {
         const uint32_t n = min(n_work - c0, l.chunk);
         const auto open = [&](uint32_t s) { open_row<BF16>(sm, a, l, s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
@@ -1436,7 +1456,7 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         }
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;   // the chunk's workspace is free
     }
-    if (ok && !l.score) leftover(sm, a, l, slots);
+    if (ok && !l.score) rows_one_cta_each(sm, a, sm.rank, min(slots, sm.size), *(volatile uint32_t*)l.left_count, l.left_rows);
     // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();
     if (tid == 0) {

@@ -15,6 +15,7 @@ constexpr int W_MAX_HIST = 2048;
 constexpr int W_CHUNK = 64;             // rows in flight together, at most
 constexpr int W_BUCKETS = 41 * 256;     // probabilities by exponent (2^-40 .. 1) and eight mantissa bits
 constexpr int W_TERMS = 64;             // segments of a row whose terms the region phase leaves for the fold
+constexpr int W_KMAX = 1024;            // top-k up to which the second pass lists the candidates
 constexpr int W_SORT = 4096;            // entries of a bucket that one CTA sorts
 
 // One row of the chunk.
@@ -49,6 +50,9 @@ struct WideLaunch {
     uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
     unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
     uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    // combinations of kinds (pgs_kinds.cuh) that are done by one CTA per row, here ([0]: at most a chunk of rows, [1]: more)
+    // or by the general kernel in front of this one
+    uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
     uint32_t polls;             // limit of a barrier's wait
     unsigned long long* gave_up; // rows that ended without results because one ran out
     uint32_t chunk;             // rows that the workspace holds (<= W_CHUNK): the launch takes that many at a time

@@ -101,3 +101,30 @@ def test_a_barrier_that_gives_up_is_reported(monkeypatch):
     finally:
         s.close()
         good.close()
+
+
+@pytest.mark.parametrize("route", ["1", "2"])   # the grid on every row; one CTA per row
+@pytest.mark.parametrize("rows, vocab, top_k, history", [
+    (1, 511, 0, 0), (70, 512, 40, 64), (65, 513, 0, 2048), (5, 1025, 1025, 2049), (3, 33025, 0, 300), (200, 1003, 7, 16)])
+def test_both_routes(oracle, monkeypatch, route, rows, vocab, top_k, history):
+    """Short rows and many rows are done by one CTA per row, others by the whole grid: either way, at the edges of both."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    x = synth.normal_f32(17 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    x[:, vocab // 2] = x[:, 0]
+    x[-1, 0] = np.nan if rows > 1 else 0.0
+    w = synth.Workload(
+        "routes", x, np.resize(np.float32([0.7, 0.0, 5.0]), rows), np.full(rows, top_k, np.uint32),
+        np.resize(np.float32([0.95, 1.0, 0.3]), rows), np.full(rows, 0.2, np.float32), np.full(rows, 0.1, np.float32),
+        np.full(rows, 1.1, np.float32), np.arange(rows + 1, dtype=np.uint32) * history if history else None,
+        np.random.default_rng(vocab).integers(0, vocab, rows * history).astype(np.uint32) if history else None,
+        synth.uniform_f32(3, rows))
+    monkeypatch.setenv("PGS_WIDE_ROUTE", route)
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
+    try:
+        s.set_exact(True)
+        assert_same(*run_both(s, oracle, w), w)
+        s.set_exact(False)   # unaligned rows, and the work list
+        assert_same(*run_both(s, oracle, w), w, exact=False)
+    finally:
+        s.close()
