@@ -978,12 +978,15 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         float bound = NAN;   // CL: at least top_k logits of the row reach it (NaN: not known yet)
         if (CL) {
             // Every CTA bounds its own share of the top-k from below, hands that, its part of the region table and its
-            // numbers to all the others, and combines what it gets: one barrier.  (The share: the k / size-th largest, so
-            // that the shares of all CTAs together make k.  A bound over all histograms is tighter, but takes a second
-            // barrier and a trip to every other CTA: 8 rows 28.5 us.)
+            // numbers to all the others, and combines what it gets: one barrier.  (The share: top-k by the CTA's part of the
+            // row's logits, so that the shares of all CTAs together make k.  With equal shares the CTA with the fewest pieces
+            // sets the bound: top-k 1024 of 50256 on four CTAs listed more candidates than there is room for.  A bound over
+            // all histograms is tighter, but takes a second barrier and a trip to every other CTA.)
             cg::cluster_group cluster = cg::this_cluster();
-            const uint32_t share = (top_k + csize - 1u) / csize;
-            if (!greedy && n_fin >= share) bound = kth_bound(share, key_to_float(lo_key), lm, false);   // CTA-uniform
+            const uint32_t mine = (n_full > crank ? (n_full - 1u - crank) / csize + 1u : 0u) * S_PIECE + (my_tail ? V - n_full * S_PIECE : 0u);
+            const uint32_t share = (top_k * mine + V - 1u) / V;   // (top-k is 1024 at most)
+            if (mine == 0u) bound = INFINITY;
+            if (!greedy && mine && n_fin >= share) bound = kth_bound(share, key_to_float(lo_key), lm, false);   // CTA-uniform
             else __syncthreads();   // (the entries' sums are complete)
             cluster.barrier_wait();   // all of them run
             if (!greedy) {

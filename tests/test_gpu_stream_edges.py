@@ -34,3 +34,40 @@ def test_stream_edges(oracle, vocab, top_k, history, crowd, masked, bf16):
         assert_close(*run_both(s, oracle, w), "edges")
     finally:
         s.close()
+
+
+def _batch(rows, vocab, top_k, history, crowd, masked, bf16):
+    from pagoda_b200 import synth
+    rng = np.random.default_rng(vocab + top_k + rows)
+    x = synth.normal_f32(13 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    x[:, rng.integers(0, vocab, 40)] += 6.0
+    x[:, vocab - 1] = x[:, 0]
+    kw = {}
+    if masked:
+        words = rng.integers(0, 1 << 32, (3, (vocab + 31) // 32), dtype=np.uint64).astype(np.uint32)
+        kw = dict(mask_words=words, state_flags=np.array([0, 1, 0], np.uint32),
+                  mask_state=np.resize(np.int32([0, 1, 2, -1, 1, 0]), rows), eos_token_id=vocab - 1)
+    return synth.Workload(
+        "edges", (x.view(np.uint32) >> 16).astype(np.uint16) if bf16 else x, np.resize(np.float32([0.7, 1.3, 0.0]), rows),
+        np.full(rows, top_k, np.uint32), np.resize(np.float32([1.0, 0.9]), rows), np.full(rows, 0.2, np.float32),
+        np.full(rows, 0.1, np.float32), np.full(rows, 1.1, np.float32),
+        np.arange(rows + 1, dtype=np.uint32) * history if history else None,
+        rng.integers(0, crowd, rows * history).astype(np.uint32) if history else None, synth.uniform_f32(5, rows), **kw)
+
+
+# Rows on a cluster of CTAs each, and on one CTA each; 330 rows: more than are resident, so that a CTA takes a second row and
+# its tables and bits are used again.
+@pytest.mark.parametrize("cluster", ["1", "0"])
+@pytest.mark.parametrize("rows, vocab, top_k, history, crowd, masked, bf16", [
+    (330, 8200, 255, 40, 512, False, False), (330, 4096, 40, 2048, 4096, True, True), (330, 1000, 20, 512, 1000, False, False),
+    (24, 8192, 257, 2048, 8192, True, False), (24, 40016, 511, 300, 300, True, True), (16, 50256, 1024, 100, 50256, False, False),
+    (24, 32776, 513, 700, 32776, False, True), (12, 151936, 1024, 1, 1, True, False)])
+def test_stream_edges_on_one_cta_and_on_clusters(oracle, monkeypatch, cluster, rows, vocab, top_k, history, crowd, masked, bf16):
+    import pagoda_b200
+    monkeypatch.setenv("PGS_CLUSTER", cluster)
+    w = _batch(rows, vocab, top_k, history, crowd, masked, bf16)
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=history)
+    try:
+        assert_close(*run_both(s, oracle, w), "edges")
+    finally:
+        s.close()
