@@ -61,13 +61,11 @@ constexpr int SNW = SNT / 32;            // warps per CTA
 constexpr int S_EPT = 16;                // logits per thread and piece
 constexpr int S_PIECE = SNT * S_EPT;     // logits per piece
 constexpr int S_REGION = 32 * S_EPT;     // consecutive logits of one warp in a piece
-constexpr int S_MAX_REGIONS = S_MAX_VOCAB / S_REGION;
 constexpr int S_NCELL = 4;               // running maxima per thread (piece number mod S_NCELL)
 constexpr int S_CELLS = S_NCELL * SNT;   // per-thread maxima that bound the top-k threshold
 constexpr int S_NB = 1024;               // buckets of their histogram
 constexpr int S_BPT = S_NB / SNT;        // buckets per thread
 constexpr int S_ENT = S_MAX_HASH / 2 + 1;   // distinct history ids, and the EOS fix
-constexpr int S_WORDS = S_MAX_VOCAB / 32;
 constexpr uint32_t S_NIL = 0xffffffffu;
 constexpr uint32_t ENT_MASKED = 0x80000000u, ENT_EOS = 0x40000000u;   // beside an entry's count
 static_assert(SNW <= 32, "warp slots are combined by one warp");
@@ -87,6 +85,7 @@ struct SRowCtl {
 enum : uint32_t { PF_REP = 1u, PF_FP = 2u, PF_PRES = 4u };
 struct PassArgs {
     const char* rowp;
+    const uint32_t* mw;     // rows beyond S_SHORT_VOCAB: the grammar mask
     float sc, sc_lo, c_hi, c_lo, cut_f, freq, pres, rep;
     uint32_t V, n_full, n_regions, flags;
     // a row shared by the CTAs of a cluster: this CTA works on the pieces q0, q0 + qstep, ...; the candidates of all of
@@ -97,7 +96,11 @@ struct PassArgs {
     float* cand_x_p;
 };
 
+// LONG: rows beyond S_SHORT_VOCAB, whose bits do not fit beside two CTAs' tables.
+template <bool LONG>
 struct StreamSmem {
+    static constexpr bool IS_LONG = LONG;
+    static constexpr int MAX_REGIONS = (LONG ? S_MAX_VOCAB : S_SHORT_VOCAB) / S_REGION;
     SRowCtl ctl[2];
     PassArgs pa;
     unsigned long long exp_tab[32];
@@ -127,18 +130,18 @@ struct StreamSmem {
                     // per warp region of the row (512 consecutive logits): pass 1 leaves the warp's maximum and the plain
                     // sum of its numerators relative to it; then the binade's lower end the fold has there (0 = fold this
                     // region the careful way) and the estimate of the running value at its start
-                    float reg_a[S_MAX_REGIONS], reg_b[S_MAX_REGIONS];
+                    float reg_a[MAX_REGIONS], reg_b[MAX_REGIONS];
                     // a logit below this adds exactly nothing to the fold in this region; before, the plain sum of the
                     // region's entries relative to the CTA's maximum
-                    float reg_t[S_MAX_REGIONS];
+                    float reg_t[MAX_REGIONS];
                     // The row's entries: the distinct history ids and the EOS fix, those of region r at rs[r] .. rs[r + 1].
                     // The passes leave their logits out (the bits are clear); pass 1 copies them to ent_raw, and one thread
                     // per entry adds what the chain sees there to what the passes find.
-                    uint16_t rs[S_MAX_REGIONS + 2];
+                    uint16_t rs[MAX_REGIONS + 2];
                     uint32_t ent_id[S_ENT];
                     float ent_x[S_ENT];              // before pass 1 is over: the count; ENT_MASKED, ENT_EOS
                     uint32_t ent_raw[S_ENT];         // the word that holds the raw logit (before pass 1: entries per region)
-                    uint32_t bits[S_WORDS];          // one bit per logit: allowed, and no entry
+                    uint32_t bits[LONG ? 1 : S_SHORT_VOCAB / 32];   // one bit per logit: allowed, and no entry
                 };
                 FinishArrays fin;
                 unsigned long long tpkey[SNT];   // vocabulary-sharded mode: one candidate per thread while a record is ranked
@@ -148,8 +151,9 @@ struct StreamSmem {
     };
 };
 
-static_assert(sizeof(StreamSmem) <= 113 * 1024, "two CTAs per SM");
-static_assert(offsetof(StreamSmem, hash) + sizeof(StreamSmem::hash) <= offsetof(StreamSmem, reg_a), "entries are set up while the table stands");
+static_assert(sizeof(StreamSmem<false>) <= 113 * 1024 && sizeof(StreamSmem<true>) <= 113 * 1024, "two CTAs per SM");
+static_assert(offsetof(StreamSmem<false>, hash) + sizeof(StreamSmem<false>::hash) <= offsetof(StreamSmem<false>, reg_a) &&
+              offsetof(StreamSmem<true>, hash) + sizeof(StreamSmem<true>::hash) <= offsetof(StreamSmem<true>, reg_a), "entries are set up while the table stands");
 
 #define PGS_STICK(slot)                                             \
     do {                                                            \
@@ -293,7 +297,8 @@ __device__ __forceinline__ void sprepare_row(const RowArgs& a, const StreamLaunc
 // Vocabulary-sharded mode: the candidates of one row (n <= SNT, one per thread) -> this shard's record: the
 // tp_cand largest by (logit descending, id ascending) behind the head.  Called by every thread; the caller has a
 // barrier in front.
-__device__ __forceinline__ void semit_tp(StreamSmem& sm, const RowArgs& a, uint32_t row, uint32_t n, float m, float S,
+template <class SM>
+__device__ __forceinline__ void semit_tp(SM& sm, const RowArgs& a, uint32_t row, uint32_t n, float m, float S,
                                          uint32_t amax) {
     const int tid = threadIdx.x;
     TpRecHead* head = reinterpret_cast<TpRecHead*>(a.tp_records + (size_t)row * a.tp_rec_bytes);
@@ -361,12 +366,31 @@ __device__ __forceinline__ void raw_unpack(float (&x)[S_EPT], const Raw<BF16>& r
     }
 }
 
+// Rows beyond S_SHORT_VOCAB keep no bits: the first 16 lanes make the region's 16 words from the mask (one 64-byte load, under
+// way together with the logits) and the region's entries.  256 rows of 262208: top-k 103 us, with 512 ids 119, with a mask 112.
+template <bool BITS, class SM>
+__device__ __forceinline__ uint32_t region_word(const SM& sm, uint32_t region) {
+    uint32_t word = 0u;
+    if constexpr (BITS && SM::IS_LONG) {
+        const uint32_t lane = threadIdx.x & 31u, at = region * (S_REGION / 32) + lane, whole = sm.pa.V / 32u;
+        if (lane < S_REGION / 32u) {
+            word = at < whole ? 0xffffffffu : at == whole ? (1u << (sm.pa.V & 31u)) - 1u : 0u;
+            if (sm.pa.mw && word) word &= __ldg(sm.pa.mw + at);
+        }
+        const uint32_t e1 = sm.rs[region + 1];
+        for (uint32_t e = sm.rs[region]; e < e1; e++) {
+            const uint32_t id = sm.ent_id[e];
+            if (((id >> 5) & 15u) == lane) word &= ~(1u << (id & 31u));
+        }
+    }
+    return word;
+}
 // Raw logits of piece q -> the logits of the pass: -inf where the row's bits say so (BITS: grammar mask, entries, end of
 // the row) or behind the end of the row.  The bits come from shared memory, four logits (bf16: eight) of a lane to the
 // load.  (Read from the mask table a piece at a time, every group of the piece waited for L2: 128 masked rows of 151936
 // took 100 us, with the bits 51.)
-template <bool BF16, bool BITS, bool TAIL>
-__device__ __forceinline__ void fix_x(const StreamSmem& sm, float (&x)[S_EPT], uint32_t q) {
+template <bool BF16, bool BITS, bool TAIL, class SM>
+__device__ __forceinline__ void fix_x(const SM& sm, float (&x)[S_EPT], uint32_t q, uint32_t word) {
     constexpr int G = Geo<BF16>::G, GE = Geo<BF16>::GE, GS = Geo<BF16>::GS;
     if (!BITS && !TAIL) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -376,7 +400,8 @@ __device__ __forceinline__ void fix_x(const StreamSmem& sm, float (&x)[S_EPT], u
     for (int h = 0; h < G; h++) {
         const uint32_t idx = e0 + h * GS;
         uint32_t bits = 0xffffffffu;
-        if (BITS) bits = sm.bits[idx >> 5] >> shift;
+        if (BITS && SM::IS_LONG) bits = __shfl_sync(FULL, word, (int)((idx >> 5) & 15u)) >> shift;
+        else if (BITS) bits = sm.bits[idx >> 5] >> shift;
         else if (idx >= sm.pa.V) bits = 0u;
 #pragma unroll
         for (int c = 0; c < GE; c++)
@@ -401,8 +426,8 @@ __device__ __forceinline__ float entry_value(const PassArgs& pa, float v, uint32
 // nothing in the pass waits for these.  (Waited for in the pass, to be part of its maxima and sums, they made pass 1 over
 // 256 rows take 30 us in place of 21; found through a staging area 33 us; gathered before the pass 21 us and 4 us more in
 // front of it.)
-template <bool BF16>
-__device__ __forceinline__ void copy_entries(StreamSmem& sm, uint32_t region) {
+template <bool BF16, class SM>
+__device__ __forceinline__ void copy_entries(SM& sm, uint32_t region) {
     const uint32_t e1 = sm.rs[region + 1];
     for (uint32_t e = sm.rs[region] + (threadIdx.x & 31u); e < e1; e += 32u) {
         const uint32_t id = sm.ent_id[e];
@@ -412,15 +437,16 @@ __device__ __forceinline__ void copy_entries(StreamSmem& sm, uint32_t region) {
 }
 
 // pass 1 on one piece
-template <bool BF16, bool BITS, bool TAIL, bool STOCH>
-__device__ __forceinline__ void p1_piece(StreamSmem& sm, const Raw<BF16>& raw, uint32_t q, float& am, float& tmx, uint32_t& tqx) {
+template <bool BF16, bool BITS, bool TAIL, bool STOCH, class SM>
+__device__ __forceinline__ void p1_piece(SM& sm, const Raw<BF16>& raw, uint32_t q, float& am, float& tmx, uint32_t& tqx) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t region = q * SNW + (uint32_t)w;
     if (BITS) copy_entries<BF16>(sm, region);
+    const uint32_t word = region_word<BITS>(sm, region);
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
     am = absmax_ept_nan(am, x);   // max |raw logit|, NaN-propagating: the sanity check
-    fix_x<BF16, BITS, TAIL>(sm, x, q);
+    fix_x<BF16, BITS, TAIL>(sm, x, q, word);
     const float pm = max_ept(x);
     if (pm >= tmx) { tmx = pm; tqx = q; }   // pieces arrive in descending order: an equal maximum here has the lower id
     if (STOCH) {
@@ -462,8 +488,8 @@ struct FoldAcc {
     }
 };
 
-template <bool CL>
-__device__ __forceinline__ void add_candidate(StreamSmem& sm, uint32_t id, float x) {
+template <bool CL, class SM>
+__device__ __forceinline__ void add_candidate(SM& sm, uint32_t id, float x) {
     uint32_t* n = CL ? sm.pa.cand_n_p : &sm.cand_n;
     const uint32_t at = atomicAdd(n, 1u);
     if (at >= (uint32_t)F_MCAP) return;
@@ -480,8 +506,8 @@ __device__ __forceinline__ float exponent_of(const PassArgs& pa, float x) {
 
 // The entries' part of pass 2: candidates, and what they add to the fold where it stands in their region.  (In a region
 // that is folded the careful way they are added at its start: a rounding there is half an ulp of the running value at most.)
-template <bool BF16, bool CL>
-__device__ __forceinline__ void p2_entries(StreamSmem& sm, uint32_t n_ent) {
+template <bool BF16, bool CL, class SM>
+__device__ __forceinline__ void p2_entries(SM& sm, uint32_t n_ent) {
     if (threadIdx.x / 32u * 32u >= n_ent) return;   // warp-uniform
     double td = 0.0;
     for (uint32_t e = threadIdx.x; e < n_ent; e += SNT) {
@@ -498,14 +524,15 @@ __device__ __forceinline__ void p2_entries(StreamSmem& sm, uint32_t n_ent) {
 }
 
 // pass 2 on one piece
-template <bool BF16, bool BITS, bool TAIL, bool CL = false>
-__device__ __forceinline__ void p2_piece(StreamSmem& sm, const Raw<BF16>& raw, uint32_t q, FoldAcc& fa) {
+template <bool BF16, bool BITS, bool TAIL, bool CL, class SM>
+__device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t q, FoldAcc& fa) {
     constexpr int G = Geo<BF16>::G, GE = Geo<BF16>::GE;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float sc = sm.pa.sc, c_hi = sm.pa.c_hi, c_lo = sm.pa.c_lo, cut_f = sm.pa.cut_f;
+    const uint32_t word = region_word<BITS>(sm, q * SNW + (uint32_t)w);
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
-    fix_x<BF16, BITS, TAIL>(sm, x, q);
+    fix_x<BF16, BITS, TAIL>(sm, x, q, word);
     const float pm = max_ept(x);
     if (pm >= cut_f) {
         const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
@@ -598,8 +625,8 @@ __device__ __forceinline__ void prefetch_piece(const char* warp_piece) {
 }
 
 // pass 1 over the whole pieces n_full-1 .. 0; the thread's results go to sm.t_*[tid]
-template <bool BF16, bool BITS, bool STOCH, bool CL>
-__device__ __noinline__ void pass1_whole(StreamSmem& sm) {
+template <bool BF16, bool BITS, bool STOCH, bool CL, class SM>
+__device__ __noinline__ void pass1_whole(SM& sm) {
     constexpr int PB = S_PIECE * (BF16 ? 2 : 4);
     const uint32_t lane_e0 = (threadIdx.x >> 5) * S_REGION + (threadIdx.x & 31) * Geo<BF16>::GE;
     const uint32_t n = sm.pa.n_full;   // >= 1
@@ -641,8 +668,8 @@ __device__ __noinline__ void pass1_whole(StreamSmem& sm) {
 }
 
 // pass 2 over the whole pieces 0 .. n_full-1; the warp's share of the fold is added to sm.wacc[w]
-template <bool BF16, bool BITS, bool CL>
-__device__ __noinline__ void pass2_whole(StreamSmem& sm) {
+template <bool BF16, bool BITS, bool CL, class SM>
+__device__ __noinline__ void pass2_whole(SM& sm) {
     constexpr int PB = S_PIECE * (BF16 ? 2 : 4);
     const uint32_t lane_e0 = (threadIdx.x >> 5) * S_REGION + (threadIdx.x & 31) * Geo<BF16>::GE;
     const uint32_t n = sm.pa.n_full;   // >= 1
@@ -674,7 +701,7 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
         if (q + (uint32_t)PGS_PF_DIST < n) prefetch_piece<BF16>(wp + (size_t)PGS_PF_DIST * PB);
         Raw<BF16> b;
         raw_load<BF16>(b, p);
-        p2_piece<BF16, BITS, false>(sm, b, q, fa);
+        p2_piece<BF16, BITS, false, false>(sm, b, q, fa);
     }
     fa.flush();
     if ((threadIdx.x & 31) == 0) sm.wacc[threadIdx.x >> 5] += fa.accd;
@@ -685,13 +712,14 @@ __device__ __noinline__ void pass2_whole(StreamSmem& sm) {
 // the CTAs exchange their maxima, region tables, histograms, candidates and fold shares through distributed shared
 // memory around two cluster barriers, and the first CTA finishes the row (a launch has one cluster per row).  Every decision that ends a row
 // early is taken from values all CTAs of the cluster hold alike, so they always meet at the same barriers.
-template <bool BF16, bool CL>
+template <bool BF16, bool CL, bool LONG>
 __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, const StreamLaunch sl) {
     namespace cg = cooperative_groups;
     constexpr int GE = Geo<BF16>::GE;
     constexpr int ESZ = BF16 ? 2 : 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    StreamSmem& sm = *reinterpret_cast<StreamSmem*>(smem_raw);
+    using SM = StreamSmem<LONG>;
+    SM& sm = *reinterpret_cast<SM*>(smem_raw);
     const uint32_t H = sl.hash_slots;
     uint32_t* hkey = sm.hash;
     uint32_t* hcnt = sm.hash + H;
@@ -759,7 +787,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         const bool has_bits = has_mask || pen;
         if (tid == 0) {   // what the pass loops read
             PassArgs& pa = sm.pa;
-            pa.rowp = rowp; pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
+            pa.rowp = rowp; pa.mw = ctl.mw; pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
             pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions;
             pa.q0 = crank; pa.qstep = csize;
             pa.cand_n_p = &sm.cand_n; pa.cand_id_p = sm.cand_id; pa.cand_x_p = sm.cand_x;
@@ -799,9 +827,9 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 if (hid[u] >= V || (CL && (hid[u] / S_PIECE) % csize != crank)) hid[u] = S_NIL;
             }
             uint32_t* rcnt = sm.ent_raw;   // per region, until pass 1
-            {
+            const uint32_t* mw = ctl.mw;
+            if constexpr (!LONG) {
                 const uint32_t whole = V / 32u, words = ((V + S_PIECE - 1) / S_PIECE) * (S_PIECE / 32);
-                const uint32_t* mw = ctl.mw;
 #pragma unroll 4
                 for (uint32_t k = tid; k < words; k += SNT) {
                     uint32_t b = k < whole ? 0xffffffffu : k == whole ? (1u << (V & 31u)) - 1u : 0u;
@@ -809,9 +837,10 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                     sm.bits[k] = b;
                 }
             }
-            static_assert(S_MAX_REGIONS <= SNT, "one thread per region");
-            if (tid < S_MAX_REGIONS) { rcnt[tid] = 0u; sm.rs[tid] = 0; sm.reg_t[tid] = 0.0f; }
-            if (tid < 2) sm.rs[S_MAX_REGIONS + tid] = 0;
+            static_assert(SM::MAX_REGIONS % SNT == 0 && SM::MAX_REGIONS <= S_ENT, "whole regions per thread, their counts in the entries' space");
+#pragma unroll
+            for (int u = 0; u < SM::MAX_REGIONS / SNT; u++) { rcnt[tid + u * SNT] = 0u; sm.rs[tid + u * SNT] = 0; sm.reg_t[tid + u * SNT] = 0.0f; }
+            if (tid < 2) sm.rs[SM::MAX_REGIONS + tid] = 0;
             if (pen || fix) {
 #pragma unroll 1
                 for (uint32_t s = tid; s < 2u * H; s += SNT) sm.hash[s] = s < H ? S_NIL : 0u;
@@ -827,7 +856,8 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                         if (prev == S_NIL || prev == id) {
                             if (prev == S_NIL) {
                                 const uint32_t bit = 1u << (id & 31u);
-                                if (!(atomicAnd(&sm.bits[id >> 5], ~bit) & bit)) n |= ENT_MASKED;
+                                if constexpr (LONG) { if (has_mask && !(__ldg(mw + (id >> 5)) & bit)) n |= ENT_MASKED; }
+                                else if (!(atomicAnd(&sm.bits[id >> 5], ~bit) & bit)) n |= ENT_MASKED;
                                 if (fix && id == (uint32_t)a.eos) n |= ENT_EOS;
                                 atomicAdd(&rcnt[id / S_REGION], 1u);
                             }
@@ -854,10 +884,14 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                     // together.
                     defer_row = true;
                 } else {
-                    const uint32_t own = tid < S_MAX_REGIONS ? rcnt[tid] : 0u;
-                    const uint32_t before = sblock_excl_scan_u32(own, &n_ent, sm.scan_u);
-                    if (tid < S_MAX_REGIONS) { sm.rs[tid] = (uint16_t)before; rcnt[tid] = before; }
-                    if (tid < 2) sm.rs[S_MAX_REGIONS + tid] = (uint16_t)n_ent;
+                    constexpr int RPT = SM::MAX_REGIONS / SNT;   // regions per thread
+                    uint32_t cnt[RPT], own = 0u;
+#pragma unroll
+                    for (int u = 0; u < RPT; u++) { cnt[u] = rcnt[tid * RPT + u]; own += cnt[u]; }
+                    uint32_t before = sblock_excl_scan_u32(own, &n_ent, sm.scan_u);
+#pragma unroll
+                    for (int u = 0; u < RPT; u++) { sm.rs[tid * RPT + u] = (uint16_t)before; rcnt[tid * RPT + u] = before; before += cnt[u]; }
+                    if (tid < 2) sm.rs[SM::MAX_REGIONS + tid] = (uint16_t)n_ent;
                     __syncthreads();
                     const auto entry = [&](uint32_t id, uint32_t s) {
                         if (s & 0x80000000u) return;
@@ -1055,7 +1089,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 raw_load_tail<BF16>(raw, rowp + ((size_t)q * S_PIECE + lane_e0) * ESZ, q * S_PIECE + lane_e0, V);
                 float x[S_EPT];
                 raw_unpack<BF16>(x, raw);
-                if (has_bits) fix_x<BF16, true, true>(sm, x, q); else fix_x<BF16, false, true>(sm, x, q);
+                if (has_bits) fix_x<BF16, true, true>(sm, x, q, region_word<true>(sm, q * SNW + (uint32_t)w)); else fix_x<BF16, false, true>(sm, x, q, 0u);
                 const bool mine = ((pending >> lane) & 1u) && tqx == q;
                 if (mine) {
                     int j0 = 0;
@@ -1238,48 +1272,70 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         for (int i = 0; i < 16; i++) sl.prof[blockIdx.x * 16 + i] += sm.prof_acc[i];
 }
 
-size_t stream_smem_bytes() { return sizeof(StreamSmem); }
+size_t stream_smem_bytes() { return sizeof(StreamSmem<false>); }
 uint32_t stream_threads() { return SNT; }
 
-template <bool BF16, bool CL>
+template <bool BF16, bool CL, bool LONG>
 static cudaError_t configure_one() {
-    cudaError_t e = cudaFuncSetAttribute(stream_row_kernel<BF16, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StreamSmem));
+    cudaError_t e = cudaFuncSetAttribute(stream_row_kernel<BF16, CL, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StreamSmem<LONG>));
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(stream_row_kernel<BF16, CL>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(stream_row_kernel<BF16, CL, LONG>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+template <bool BF16, bool CL>
+static cudaError_t configure_both() {
+    const cudaError_t e = configure_one<BF16, CL, false>();
+    return e != cudaSuccess ? e : configure_one<BF16, CL, true>();
 }
 
 cudaError_t configure_stream() {
-    cudaError_t e = configure_one<false, false>();
-    if (e == cudaSuccess) e = configure_one<true, false>();
-    if (e == cudaSuccess) e = configure_one<false, true>();
-    if (e == cudaSuccess) e = configure_one<true, true>();
+    cudaError_t e = configure_both<false, false>();
+    if (e == cudaSuccess) e = configure_both<true, false>();
+    if (e == cudaSuccess) e = configure_both<false, true>();
+    if (e == cudaSuccess) e = configure_both<true, true>();
     return e;
 }
 
-// CTAs of this kernel that one SM holds
+// CTAs of this kernel that one SM holds (of either length of row)
 cudaError_t stream_ctas_per_sm(int* out) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, stream_row_kernel<false, false>, SNT, sizeof(StreamSmem));
+    int longs = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, stream_row_kernel<false, false, false>, SNT, sizeof(StreamSmem<false>));
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&longs, stream_row_kernel<false, false, true>, SNT, sizeof(StreamSmem<true>));
+    if (longs < *out) *out = longs;
+    return e;
 }
 
 // Clusters of `csize` CTAs of this kernel that the device holds at once (csize 2, 4 or 8)
-cudaError_t stream_max_clusters(int csize, int* out) {
+template <bool LONG>
+static cudaError_t max_clusters(int csize, int* out) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)csize, 1, 1);
     cfg.blockDim = dim3(SNT, 1, 1);
-    cfg.dynamicSmemBytes = sizeof(StreamSmem);
+    cfg.dynamicSmemBytes = sizeof(StreamSmem<LONG>);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)csize; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(out, stream_row_kernel<false, true>, &cfg);
+    return cudaOccupancyMaxActiveClusters(out, stream_row_kernel<false, true, LONG>, &cfg);
+}
+cudaError_t stream_max_clusters(int csize, int* out) {
+    int longs = 0;
+    cudaError_t e = max_clusters<false>(csize, out);
+    if (e == cudaSuccess) e = max_clusters<true>(csize, &longs);
+    if (longs < *out) *out = longs;
+    return e;
 }
 
+template <bool BF16, bool CL>
+static cudaError_t launch_length(const RowArgs& a, const StreamLaunch& sl, cudaLaunchConfig_t& cfg) {
+    const bool is_long = a.vocab > (uint32_t)S_SHORT_VOCAB;
+    cfg.dynamicSmemBytes = is_long ? sizeof(StreamSmem<true>) : sizeof(StreamSmem<false>);
+    return is_long ? cudaLaunchKernelEx(&cfg, stream_row_kernel<BF16, CL, true>, a, sl) : cudaLaunchKernelEx(&cfg, stream_row_kernel<BF16, CL, false>, a, sl);
+}
 // csize == 1: one CTA per row, `grid` CTAs.  csize > 1: `grid` clusters of csize CTAs, one cluster per row at a time.
 cudaError_t launch_stream(const RowArgs& a, const StreamLaunch& sl, uint32_t grid, uint32_t csize, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid * csize, 1, 1);
     cfg.blockDim = dim3(SNT, 1, 1);
-    cfg.dynamicSmemBytes = sizeof(StreamSmem);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1287,12 +1343,8 @@ cudaError_t launch_stream(const RowArgs& a, const StreamLaunch& sl, uint32_t gri
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = csize; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = csize > 1u ? 2 : 1;
-    if (csize > 1u) {
-        if (a.dtype == 0) return cudaLaunchKernelEx(&cfg, stream_row_kernel<false, true>, a, sl);
-        return cudaLaunchKernelEx(&cfg, stream_row_kernel<true, true>, a, sl);
-    }
-    if (a.dtype == 0) return cudaLaunchKernelEx(&cfg, stream_row_kernel<false, false>, a, sl);
-    return cudaLaunchKernelEx(&cfg, stream_row_kernel<true, false>, a, sl);
+    if (csize > 1u) return a.dtype == 0 ? launch_length<false, true>(a, sl, cfg) : launch_length<true, true>(a, sl, cfg);
+    return a.dtype == 0 ? launch_length<false, false>(a, sl, cfg) : launch_length<true, false>(a, sl, cfg);
 }
 
 }  // namespace pgs

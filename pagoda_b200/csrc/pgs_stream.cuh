@@ -7,7 +7,8 @@
 namespace pgs {
 
 constexpr int S_KMAX = 1024;         // largest top-k the streaming kernel serves
-constexpr int S_MAX_VOCAB = 1 << 18;  // longest row the streaming kernel serves (one bit per logit in shared memory)
+constexpr int S_MAX_VOCAB = 1 << 20;  // longest row the streaming kernel serves
+constexpr int S_SHORT_VOCAB = 1 << 18;   // longest row that keeps one bit per logit in shared memory
 constexpr int S_MAX_HASH = 4096;     // id -> count slots (histories of up to 2048 ids)
 
 struct StreamLaunch {

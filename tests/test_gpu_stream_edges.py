@@ -71,3 +71,20 @@ def test_stream_edges_on_one_cta_and_on_clusters(oracle, monkeypatch, cluster, r
         assert_close(*run_both(s, oracle, w), "edges")
     finally:
         s.close()
+
+
+# Rows whose bits do not fit in shared memory, from the first length on to the longest.
+@pytest.mark.parametrize("cluster", ["1", "0"])
+@pytest.mark.parametrize("vocab, top_k, history, crowd, masked, bf16", [
+    (262152, 64, 8, 64, True, True), (262152, 50, 0, 1, False, False), (262148, 1000, 2047, 262148, True, False),
+    (300008, 40, 600, 700, False, True), ((1 << 20) - 4, 20, 2048, 1 << 20, False, False), (1 << 20, 50, 100, 1 << 20, True, True)])
+def test_stream_long_rows(oracle, monkeypatch, cluster, vocab, top_k, history, crowd, masked, bf16):
+    import pagoda_b200
+    monkeypatch.setenv("PGS_CLUSTER", cluster)
+    rows = 9
+    w = _batch(rows, vocab, top_k, history, crowd, masked, bf16)
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
+    try:
+        assert_close(*run_both(s, oracle, w), "long rows")
+    finally:
+        s.close()
