@@ -45,7 +45,7 @@ cudaError_t configure_score();
 cudaError_t launch_log_softmax(const ScoreArgs& a, uint32_t grid, cudaStream_t stream);
 cudaError_t configure_tp();
 cudaError_t launch_tp_push(const TpArgs& a, cudaStream_t stream);
-cudaError_t launch_tp_merge(const TpArgs& a, const TpOut& o, cudaStream_t stream);
+cudaError_t launch_tp_merge(const TpArgs& a, const TpOut& o, uint32_t sms, cudaStream_t stream);
 cudaError_t launch_draft_accept(const uint32_t* row_argmax, const uint32_t* draft, uint32_t sequences,
                                 uint32_t positions, uint32_t* accepted, uint32_t* next, cudaStream_t stream);
 }  // namespace pgs
@@ -786,7 +786,7 @@ extern "C" int pgs_tp_merge(pgs_handle* h, const pgs_tp_desc* d, const void* rec
     DeviceGuard g(h->device);
     a.records = (unsigned char*)records_all;
     pgs::TpOut o{out->token, out->status, out->drew, out->argmax, out->gmax, out->gsum, out->total, out->n_kept};
-    PGS_CUDA(h, pgs::launch_tp_merge(a, o, cuda_stream ? (cudaStream_t)cuda_stream : h->stream));
+    PGS_CUDA(h, pgs::launch_tp_merge(a, o, (uint32_t)h->sm_count, cuda_stream ? (cudaStream_t)cuda_stream : h->stream));
     h->counters.kernel_launches += 1;
     h->counters.rows += a.rows;
     return PGS_OK;
@@ -899,7 +899,7 @@ extern "C" int pgs_tp_merge_wait(pgs_handle* h, const pgs_tp_desc* d, const void
     a.epoch = epoch;
     pgs::TpOut o{out->token, out->status, out->drew, out->argmax, out->gmax, out->gsum, out->total, out->n_kept};
     h->tp_stream = cuda_stream ? (cudaStream_t)cuda_stream : h->stream;
-    PGS_CUDA(h, pgs::launch_tp_merge(a, o, h->tp_stream));
+    PGS_CUDA(h, pgs::launch_tp_merge(a, o, (uint32_t)h->sm_count, h->tp_stream));
     h->counters.kernel_launches += 1;
     h->counters.rows += a.rows;
     return PGS_OK;

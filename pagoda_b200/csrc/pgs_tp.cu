@@ -64,9 +64,10 @@ __global__ void __launch_bounds__(256) tp_push_kernel(const TpArgs a) {
     }
 }
 
-// Most of a row's time is one warp's: few threads per row, so that an SM holds eight rows (of 256 threads it held four, and
-// 1024 rows of 8 x 64 candidates needed a second wave).
-constexpr int TP_MT = 128;
+// Most of a row's time is one warp's: few threads per row, so that an SM holds eight rows (of 256 threads it holds four, and
+// 1024 rows of 8 x 64 candidates need a second wave).  Where all rows are resident either way, long lists take 256
+// threads: 256 rows of 8 x 128 candidates 35 us, with 128 threads 54; of 8 x 64 19 and 27.
+constexpr int TP_FEW = 128, TP_MANY = 256;
 constexpr int TP_MCAP = TP_MAX_SHARDS * 128;   // candidates of all shards together (cand <= 128)
 
 template <int CAP>
@@ -84,9 +85,9 @@ struct TpMergeSmem {
 };
 
 
-// CAP: candidates of all shards together, at most
-template <int CAP>
-__global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, const TpOut o) {
+// T: threads; CAP: candidates of all shards together, at most
+template <int T, int CAP>
+__global__ void __launch_bounds__(T, 1024 / T) tp_merge_kernel(const TpArgs a, const TpOut o) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TpMergeSmem<CAP>& sm = *reinterpret_cast<TpMergeSmem<CAP>*>(smem_raw);
     const int tid = threadIdx.x;
@@ -124,12 +125,12 @@ __global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, cons
     // every record slot of the row is requested at once (one trip to memory): the heads by the first threads, the
     // candidate slots one or two per thread; which of the slots are filled is known once the heads are in
     if ((uint32_t)tid < a.n_shards) sm.hd[tid] = *rec(tid);
-    constexpr int SLOTS = (CAP + TP_MT - 1) / TP_MT;
+    constexpr int SLOTS = (CAP + T - 1) / T;
     float gx[SLOTS];
     uint32_t gid[SLOTS];
 #pragma unroll
     for (int u = 0; u < SLOTS; u++) {
-        const uint32_t c = (uint32_t)tid + u * TP_MT;
+        const uint32_t c = (uint32_t)tid + u * T;
         gx[u] = 0.0f; gid[u] = 0u;
         if (c < a.n_shards * a.cand) {
             const float* rx = reinterpret_cast<const float*>(rec(c / a.cand) + 1);
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, cons
     // the union of the candidates, shard after shard
 #pragma unroll
     for (int u = 0; u < SLOTS; u++) {
-        const uint32_t c = (uint32_t)tid + u * TP_MT;
+        const uint32_t c = (uint32_t)tid + u * T;
         if (c < a.n_shards * a.cand) {
             const uint32_t r = c / a.cand, j = c % a.cand;
             if (j < sm.start[r + 1] - sm.start[r]) { sm.cx[sm.start[r] + j] = gx[u]; sm.cid[sm.start[r] + j] = gid[u]; }
@@ -212,22 +213,22 @@ __global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, cons
     // below) takes the general ranking instead.
     const uint32_t n = sm.n;
     const bool norm = sm.S > 1e-9f;
-    for (uint32_t c = tid; c < n; c += TP_MT) {
+    for (uint32_t c = tid; c < n; c += T) {
         const float e = softmax_num(sm.cx[c], sm.M, t, sm.exp_tab);   // exact expf
         sm.fin.key[c] = ((unsigned long long)f2u(norm ? fdiv(e, sm.S) : e) << 32) | (unsigned long long)(0xffffffffu - sm.cid[c]);
     }
     __syncthreads();
-    for (uint32_t c = tid; c + 1 < n; c += TP_MT) {
+    for (uint32_t c = tid; c + 1 < n; c += T) {
         uint32_t r = 0;
         while (sm.start[r + 1] <= c) r++;
         if (c + 1 < sm.start[r + 1] && !(sm.fin.key[c] > sm.fin.key[c + 1])) sm.unsorted = 1;
     }
     __syncthreads();
     if (sm.unsorted) {   // CTA-uniform
-        cta_finish<TP_MT>(sm.fin, sm.exp_tab, ra, row, a.vocab, sm.cid, sm.cx, n, sm.M, t, sm.S, top_k, top_p, u01, sm.amax, ROW_OK);
+        cta_finish<T>(sm.fin, sm.exp_tab, ra, row, a.vocab, sm.cid, sm.cx, n, sm.M, t, sm.S, top_k, top_p, u01, sm.amax, ROW_OK);
         return;
     }
-    for (uint32_t c = tid; c < n; c += TP_MT) {
+    for (uint32_t c = tid; c < n; c += T) {
         const unsigned long long kc = sm.fin.key[c];
         uint32_t own = 0;
         while (sm.start[own + 1] <= c) own++;
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(TP_MT, 8) tp_merge_kernel(const TpArgs a, cons
         const float pc = u2f((uint32_t)(kc >> 32));
         sm.fin.sid[r_id] = idc; sm.fin.sp[r_id] = pc; sm.fin.rp[r_p] = pc; sm.fin.rpos[r_p] = r_id;
     }
-    cta_finish_ranked<TP_MT>(sm.fin, ra, row, a.vocab, n, sm.M, sm.S, top_k, top_p, u01, sm.amax, ROW_OK);
+    cta_finish_ranked<T>(sm.fin, ra, row, a.vocab, n, sm.M, sm.S, top_k, top_p, u01, sm.amax, ROW_OK);
 }
 
 __global__ void draft_accept_kernel(const uint32_t* row_argmax, const uint32_t* draft, uint32_t sequences,
@@ -261,15 +262,18 @@ __global__ void draft_accept_kernel(const uint32_t* row_argmax, const uint32_t* 
     next[s] = row_argmax[s * positions + (acc < positions ? acc : positions - 1)];
 }
 
-template <int CAP>
+template <int T, int CAP>
 static cudaError_t configure_merge() {
-    cudaError_t e = cudaFuncSetAttribute(tp_merge_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TpMergeSmem<CAP>));
+    cudaError_t e = cudaFuncSetAttribute(tp_merge_kernel<T, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TpMergeSmem<CAP>));
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(tp_merge_kernel<CAP>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(tp_merge_kernel<T, CAP>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 cudaError_t configure_tp() {
-    const cudaError_t e = configure_merge<TP_MCAP / 2>();
-    return e != cudaSuccess ? e : configure_merge<TP_MCAP>();
+    cudaError_t e = configure_merge<TP_FEW, TP_MCAP / 2>();
+    if (e == cudaSuccess) e = configure_merge<TP_FEW, TP_MCAP>();
+    if (e == cudaSuccess) e = configure_merge<TP_MANY, TP_MCAP / 2>();
+    if (e == cudaSuccess) e = configure_merge<TP_MANY, TP_MCAP>();
+    return e;
 }
 
 // set up while the kernel before still runs (programmatic stream serialization)
@@ -292,10 +296,14 @@ cudaError_t launch_tp_push(const TpArgs& a, cudaStream_t stream) {
     return launch_behind(tp_push_kernel, (uint32_t)((units + 255) / 256 < 64 ? (units + 255) / 256 : 64), 256u, 0, stream, a);
 }
 
-cudaError_t launch_tp_merge(const TpArgs& a, const TpOut& o, cudaStream_t stream) {
+template <int T>
+static cudaError_t launch_merge(const TpArgs& a, const TpOut& o, cudaStream_t stream) {
     // (half the longest list in half the shared memory: eight rows per SM instead of six)
-    if (a.n_shards * a.cand <= (uint32_t)TP_MCAP / 2u) return launch_behind(tp_merge_kernel<TP_MCAP / 2>, a.rows, TP_MT, sizeof(TpMergeSmem<TP_MCAP / 2>), stream, a, o);
-    return launch_behind(tp_merge_kernel<TP_MCAP>, a.rows, TP_MT, sizeof(TpMergeSmem<TP_MCAP>), stream, a, o);
+    if (a.n_shards * a.cand <= (uint32_t)TP_MCAP / 2u) return launch_behind(tp_merge_kernel<T, TP_MCAP / 2>, a.rows, T, sizeof(TpMergeSmem<TP_MCAP / 2>), stream, a, o);
+    return launch_behind(tp_merge_kernel<T, TP_MCAP>, a.rows, T, sizeof(TpMergeSmem<TP_MCAP>), stream, a, o);
+}
+cudaError_t launch_tp_merge(const TpArgs& a, const TpOut& o, uint32_t sms, cudaStream_t stream) {
+    return a.n_shards * a.cand > 256u && a.rows <= 4u * sms ? launch_merge<TP_MANY>(a, o, stream) : launch_merge<TP_FEW>(a, o, stream);
 }
 
 cudaError_t launch_draft_accept(const uint32_t* row_argmax, const uint32_t* draft, uint32_t sequences,
