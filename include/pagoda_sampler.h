@@ -158,8 +158,8 @@ PGS_API int pgs_sample_batch(pgs_handle *h, const pgs_batch_desc *desc);
  * Steps of one handle share its per-row working storage, so the library orders them on the GPU:
  * when a step is enqueued on a different stream than the handle's previous step, the new stream
  * first waits (cudaStreamWaitEvent) for the previous step's last kernel.  The caller only has to
- * keep to one host thread per handle at a time, and to keep a stream alive until the steps it
- * carried have finished.  Steps on different handles are independent. */
+ * keep to one host thread per handle at a time, and to keep the stream of the handle's last step
+ * alive until the handle's next step is enqueued or the handle is destroyed.  Steps on different handles are independent. */
 PGS_API int pgs_sample_batch_async(pgs_handle *h, const pgs_batch_desc *desc, void *cuda_stream);
 
 /* Allocation-free variant of pgs_sample_batch_async.  It has no counterpart in the reference
@@ -184,8 +184,9 @@ PGS_API const char *pgs_static_last_error(void);
  * reference, candidate probabilities use the exact expf, and the f32 left-fold sum of
  * temperature_softmax (sampler.rs:99-113) agrees with the reference's to about 1e-6 relative,
  * so a top-p or CDF decision can differ only when it sits that close to its boundary.  With
- * `on` != 0 every row takes the wide kernel, which reproduces that sum -- and therefore
- * every token id -- bit for bit, at a fraction of the speed.  (Environment: PGS_EXACT=1.) */
+ * `on` != 0 every row takes the wide kernel, or one CTA of the general kernel where that is
+ * quicker; both reproduce that sum -- and therefore every token id -- bit for bit, at a fraction
+ * of the speed.  (Environment: PGS_EXACT=1.) */
 PGS_API int pgs_set_exact(pgs_handle *h, int on);
 
 /* ---- vocabulary-sharded sampling (extension; the reference has no multi-GPU code) ----------

@@ -286,7 +286,7 @@ class Sampler:
             raise SamplerError(rc, self._lib.pgs_last_error(self._h).decode())
 
     def set_exact(self, on: bool):
-        """Route every row through the bit-exact wide kernel (see pgs_set_exact)."""
+        """Route every row through the bit-exact kernels (see pgs_set_exact)."""
         self._check(self._lib.pgs_set_exact(self._h, int(on)))
 
     @property

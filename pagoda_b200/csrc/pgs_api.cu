@@ -4,7 +4,6 @@
 #include "../../include/pagoda_sampler.h"
 
 #include <cuda_runtime.h>
-#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -224,6 +223,7 @@ bool score_workspace_free(const pgs_handle* h, cudaStream_t stream, unsigned lon
 // 53 / 48, 128 x 16384 53 / 85, 128 x 50257 96 / 103, 64 x 151936 199 / 80, 256 x 151936 407 / 307; whole vectors 64 x 1000
 // 25 / 47, 256 x 16384 117 / 205, 256 x 151936 640 / 566.
 bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool full) {
+    if (h->wide_route) return h->wide_route == 1;
     const uint32_t sms = (uint32_t)h->sm_count, chunk = h->score_wide.chunk;
     const double logits = 1e-6 * (rows < chunk ? rows : chunk) * (double)vocab;
     const double per_row = ((rows - 1u) / sms + 1u) * (25.0 + vocab / (full ? 500.0 : 850.0));
@@ -235,13 +235,9 @@ bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool
 // that the handle's rows can have.
 uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row) {
     using namespace pgs;
-    const bool long_histories = h->max_history > (uint32_t)W_MAX_HIST;
-    uint32_t possible = 0u;
-    for (uint32_t k = 0; k < WK_ALL; k++)
-        if (((k & WK_SAMPLED) || !(k & (WK_HIST | WK_OPEN | WK_SORT))) && ((k & WK_HIST) || !(k & (WK_OPEN | WK_SORT))) && (long_histories || !(k & WK_LONG))) possible |= 1u << k;
-    const uint32_t mask = h->wide_route == 1 ? 0u : h->wide_route == 2 ? ~0u : kinds_one_cta_each(rows, h->wide.chunk, h->slots, vocab, long_histories);
-    *row = mask & possible;
-    return ~mask & possible;
+    const uint32_t possible = h->max_history > (uint32_t)W_MAX_HIST ? WK_POSSIBLE : WK_SHORT;
+    *row = h->wide_route == 1 ? 0u : h->wide_route == 2 ? possible : kinds_one_cta_each(possible, rows, h->wide.chunk, h->slots, vocab);
+    return possible & ~*row;
 }
 
 // CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid

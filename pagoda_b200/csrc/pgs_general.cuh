@@ -1,7 +1,7 @@
 // One 1024-thread CTA walks a batch row through the whole chain of Engine::advance_with_logits
 // (pagoda/src/engine.rs:1286-1314) with its working copy of the row in a global-memory scratch slot.  It accepts every shape
-// and parameter combination; the wide kernel (pgs_wide.cu) serves nearly all of what the streaming kernel cannot, and this
-// is what is left: vocabularies beyond 2^20, histories beyond 2048 ids, thousands of equal probabilities at a threshold,
+// and parameter combination; the wide kernel (pgs_wide.cu) serves most of what the streaming kernel cannot, and this
+// the rest: short rows and large batches where one CTA per row is quicker (pgs_kinds.cuh), vocabularies beyond 2^20, histories beyond 2048 ids, thousands of equal probabilities at a threshold,
 // shard records in exact mode, and the allocation-free entry point.
 //
 // Order of operations per row, as the reference runs them:

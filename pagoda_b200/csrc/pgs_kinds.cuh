@@ -9,7 +9,10 @@ namespace pgs {
 
 // What rows ask for, as far as it decides that; a batch: all of its rows together.
 enum : uint32_t { WK_SAMPLED = 1u, WK_HIST = 2u, WK_OPEN = 4u, WK_SORT = 8u, WK_LONG = 16u };
-constexpr uint32_t WK_ALL = 32u;
+// the combinations that there are, one bit each: greedy; sampled, and that by the histogram, with top-k off, sort, or both
+constexpr uint32_t WK_SHORT = 1u | 1u << WK_SAMPLED | 1u << (WK_SAMPLED | WK_HIST) | 1u << (WK_SAMPLED | WK_HIST | WK_OPEN) |
+                              1u << (WK_SAMPLED | WK_HIST | WK_SORT) | 1u << (WK_SAMPLED | WK_HIST | WK_OPEN | WK_SORT);
+constexpr uint32_t WK_POSSIBLE = WK_SHORT | WK_SHORT << WK_LONG;
 
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t row_kind(const RowArgs& a, uint32_t row) {
@@ -31,7 +34,7 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 }
 #endif
 
-// One bit per combination of kinds: one CTA per row is the quicker way for `n` rows.  Short rows do not pay for the grid's
+// Those of the combinations `of` for which one CTA per row is the quicker way for `n` rows.  Short rows do not pay for the grid's
 // barriers, and batches of many rows go through the grid in chunks of 64 where one CTA per row takes an SM count at a time.
 // us of one row on one CTA: greedy 9 + 0.37 per thousand logits, sampled 47 + 2.2, without top-k 5 more per thousand, with a
 // sort for top-p 60 + 18; of a chunk: greedy 27, sampled 44 (70 where the threshold needs the histogram), 4 per million
@@ -40,12 +43,13 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 // 256 x 50256 64 / 126, 256 x 151936 217 / 166; no top-k 16 x 1000 59 / 68, 16 x 16384 160 / 91, with top-p 1 x 1000 76 / 71,
 // 16 x 4096 161 / 78.  Rows with a history beyond the workspace end on one CTA either way (4 of 50256: 187 at once, 239
 // behind the phases).
-inline uint32_t kinds_one_cta_each(uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool long_histories) {
+inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V) {
+    if (V <= 1024u) return of;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
     const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
-    if (V <= 1024u) return ~0u;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     uint32_t mask = 0u;
-    for (uint32_t kinds = 0; kinds < WK_ALL; kinds++) {
+    for (uint32_t left = of; left; left &= left - 1u) {
+        const uint32_t kinds = (uint32_t)__builtin_ctz(left);
         float row, grid;
         if (kinds & WK_SAMPLED) {
             row = kinds & WK_SORT ? 60.0f + 0.018f * v : 47.0f + 0.0022f * v + (kinds & WK_OPEN ? 0.005f * v : 0.0f);
@@ -54,7 +58,6 @@ inline uint32_t kinds_one_cta_each(uint32_t n, uint32_t chunk, uint32_t ctas, ui
             row = 9.0f + 3.7e-4f * v + 1.5e-6f * v * together;
             grid = 27.0f + 1.65f * m;
         }
-        if ((kinds & WK_LONG) && !long_histories) row = INFINITY;   // (does not occur)
         if (waves * row < chunks * grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
     }
     return mask;

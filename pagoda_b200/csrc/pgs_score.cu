@@ -3,6 +3,8 @@
 // forward per scored token, log-softmax over the vocabulary, one gather).  Per row:
 //   max over all logits, e_i = exp(x_i - max), the f32 left-fold sum of the e_i (emulated exactly,
 //   see pgs_block.cuh), log_sum = max(ln(sum), f32::MIN_POSITIVE), out_i = ln(e_i) - log_sum.
+// It needs no workspace: it serves short rows and large batches, captured calls, and calls while the wide kernel's scoring
+// workspace is in use; the wide kernel serves the others, with the same bits.
 // exp is the exact expf of pgs_math.cuh; ln is the double-precision logarithm rounded to f32, which
 // equals libm's logf except in rare last-bit cases (the tests allow 1e-6).
 #include <cuda_runtime.h>

@@ -6,8 +6,9 @@
 // look-ups, warp reductions, loop control) is paid once per sixteen logits:
 //
 //   before: the row's entries (distinct history ids, the EOS fix) and one bit per logit that says whether the passes may see
-//           it (the grammar mask without the entries); the entries' logits are copied aside during pass 1 and one thread per
-//           entry adds what the penalties make of them to what the passes find;
+//           it (the grammar mask without the entries; of rows beyond 2^18 logits the passes make them, region by region); the
+//           entries' logits are copied aside during pass 1 and one thread per entry adds what the penalties make of them to
+//           what the passes find;
 //   pass 1, last piece first, from HBM: sanity, bits; per thread its running
 //           maximum and four more (one per piece number mod 4) that bound the top-k threshold; per warp and piece the
 //           plain sum of the softmax numerators relative to the warp's own maximum;
@@ -621,7 +622,7 @@ template <bool BF16>
 __device__ __forceinline__ void prefetch_piece(const char* warp_piece) {
     constexpr int LINES = S_REGION * (BF16 ? 2 : 4) / 128;   // 16 (f32) or 8 (bf16)
     const int lane = threadIdx.x & 31;
-    if (lane < LINES) asm volatile("prefetch.global.L2 [%0];" ::"l"(warp_piece + lane * 128));
+    if (lane < LINES) prefetch_l2(warp_piece + lane * 128);
 }
 
 // pass 1 over the whole pieces n_full-1 .. 0; the thread's results go to sm.t_*[tid]

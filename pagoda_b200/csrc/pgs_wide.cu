@@ -1,6 +1,6 @@
 // Wide kernel: all SMs work on every listed row, bit-exact with the reference's serial folds.  It serves the exact mode, the
 // rows that the streaming kernel cannot (top-k off or > 1024, rows that are not 16-byte aligned, long candidate lists) and
-// log-softmax scoring.
+// log-softmax scoring, as far as one CTA per row is not quicker (pgs_kinds.cuh).
 //
 // A launch is a sequence of phases with a grid barrier between two of them.  In "region" phases the warps of the grid share
 // all regions (512 consecutive logits) of all rows; in "row" phases a CTA does what is left of a row:
@@ -19,8 +19,8 @@
 //
 // What bounds it: the folds change binade 8 to 16 times a row, and each change is about a microsecond of one warp; a grid
 // barrier is two; a region phase is the latency of one or two regions per warp (mask, history entries and logits are one trip
-// to L2 or HBM each) rather than bandwidth.  Against one CTA per row: 32 rows of 151936 without top-k 8312 -> 231 us, 16 rows
-// in exact mode 383 -> 73, 48 rows of 50257 359 -> 68, scoring of 64 rows 204 -> 84.
+// to L2 or HBM each) rather than bandwidth.  Against one CTA per row: 32 rows of 151936 without top-k 8312 -> 222 us, 16 rows
+// in exact mode 377 -> 74, 48 rows of 50257 360 -> 72, scoring of 64 rows 199 -> 82.
 //
 // The fold (pagoda/src/sampler.rs:42, :99-113, :136-144): while the running value stays inside one binade, adding a
 // non-negative term is an integer addition in ulps which depends on the running value only where the term ends exactly on
@@ -54,7 +54,6 @@ struct alignas(16) WideSmem {
     unsigned long long exp_tab[32];
     uint32_t red_u[WNW], red_v[WNW];
     float red_f[WNW];
-    double red_d[WNW];
     uint32_t last, found, n_serial, ok, gave_up;
     uint32_t rank, size, target;         // of the CTA among those that take part; arrivals at the barrier behind this one
     float R;
@@ -1158,10 +1157,9 @@ __device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const Wid
 
 // ------------------------------------------------------------------------------------------------ region phases
 
-enum : int { WP_FIRST = 0, WP_SUM, WP_HIST, WP_LIST, WP_TOTAL, WP_FULL };
+enum : int { WP_FIRST = 0, WP_SUM, WP_LIST, WP_TOTAL, WP_FULL };
 
-// One region phase: the warps of the grid take the regions of all rows of the chunk in turn (the histogram: sixteen regions
-// of a row per half of a CTA's warps, so that most counting happens in shared memory).
+// One region phase: the warps of the grid take the regions of all rows of the chunk in turn.
 template <bool BF16, bool VEC, int PHASE>
 __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
     using L = WLay<BF16, VEC>;

@@ -8,6 +8,14 @@ from .util import assert_same, run_both
 pytestmark = pytest.mark.gpu
 
 
+def check_scores(oracle, x, ids, g, full):
+    g, full = g.cpu().numpy(), full.cpu().numpy()
+    for r in range(len(x)):
+        want = oracle.log_softmax(x[r])
+        np.testing.assert_allclose(full[r], want, rtol=0, atol=1e-6 * max(1.0, np.abs(want).max()))
+        assert g[r] == full[r][ids[r]]
+
+
 @pytest.mark.parametrize("rows, vocab, top_k, history", [
     (1, 511, 0, 0), (70, 512, 40, 64), (65, 513, 0, 2048), (5, 1025, 1025, 2049), (9, 33025, 0, 300), (6, 70001, 2049, 300),
     (2, 1 << 20, 0, 8)])
@@ -32,9 +40,7 @@ def test_wide_kernel_edges(oracle, rows, vocab, top_k, history):
                                         stream_ptr=torch.cuda.current_stream().cuda_stream)
         torch.cuda.synchronize()
         assert (status.cpu().numpy() == 0).all()
-        for r in range(min(rows, 3)):
-            np.testing.assert_allclose(full[r].cpu().numpy(), oracle.log_softmax(x[r]), rtol=0, atol=2e-5)
-            assert g[r] == full[r][int(ids[r])]
+        check_scores(oracle, x, ids, g, full)
     finally:
         s.close()
 
@@ -108,6 +114,7 @@ def test_a_barrier_that_gives_up_is_reported(monkeypatch):
     (1, 511, 0, 0), (70, 512, 40, 64), (65, 513, 0, 2048), (5, 1025, 1025, 2049), (3, 33025, 0, 300), (200, 1003, 7, 16)])
 def test_both_routes(oracle, monkeypatch, route, rows, vocab, top_k, history):
     """Short rows and many rows are done by one CTA per row, others by the whole grid: either way, at the edges of both."""
+    import torch
     import pagoda_b200
     from pagoda_b200 import synth
     x = synth.normal_f32(17 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
@@ -126,5 +133,12 @@ def test_both_routes(oracle, monkeypatch, route, rows, vocab, top_k, history):
         assert_same(*run_both(s, oracle, w), w)
         s.set_exact(False)   # unaligned rows, and the work list
         assert_same(*run_both(s, oracle, w), w, exact=False)
+        clean = np.nan_to_num(x)
+        ids = np.arange(rows, dtype=np.int32) * (vocab - 1) // max(rows - 1, 1)
+        g, full, status = s.log_softmax(torch.from_numpy(clean).cuda(), ids=torch.from_numpy(ids).cuda(), full=True,
+                                        stream_ptr=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert (status.cpu().numpy() == 0).all()
+        check_scores(oracle, clean, ids, g, full)
     finally:
         s.close()
