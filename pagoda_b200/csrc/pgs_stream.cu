@@ -1031,11 +1031,13 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
             // sets the bound: top-k 1024 of 50256 on four CTAs listed more candidates than there is room for.  A bound over
             // all histograms is tighter, but takes a second barrier and a trip to every other CTA.)
             cg::cluster_group cluster = cg::this_cluster();
-            const uint32_t mine = (n_full > crank ? (n_full - 1u - crank) / csize + 1u : 0u) * S_PIECE + (my_tail ? V - n_full * S_PIECE : 0u);
-            const uint32_t share = (top_k * mine + V - 1u) / V;   // (top-k is 1024 at most)
-            if (mine == 0u) bound = INFINITY;
-            if (!greedy && mine && n_fin >= share) bound = kth_bound(share, key_to_float(lo_key), lm, false);   // CTA-uniform
-            else __syncthreads();   // (the entries' sums are complete)
+            if (!greedy) {
+                const uint32_t mine = (n_full > crank ? ((n_full - 1u - crank) >> (__ffs((int)csize) - 1)) + 1u : 0u) * S_PIECE + (my_tail ? V - n_full * S_PIECE : 0u);
+                const uint32_t share = (uint32_t)(__fdividef((float)(top_k * mine), (float)V) * 1.000001f) + 1u;   // (rounded up, whatever the quotient's error; top-k is 1024 at most)
+                if (mine == 0u) bound = INFINITY;
+                if (mine && n_fin >= share) bound = kth_bound(share, key_to_float(lo_key), lm, false);   // CTA-uniform
+                else __syncthreads();   // (the entries' sums are complete)
+            }
             cluster.barrier_wait();   // all of them run
             if (!greedy) {
 #pragma unroll 1
