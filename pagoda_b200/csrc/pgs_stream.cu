@@ -176,6 +176,9 @@ __device__ __forceinline__ float absmax3_nan(float a, float b, float c) {
     asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
     return r;
 }
+// Two exponentials for the packed f32 instructions of sm_100 (two multiply-adds or additions in one issue slot, each rounded
+// as the scalar instruction rounds it): the arithmetic of the passes is issued in pairs.
+__device__ __forceinline__ float2 ex2_pair(float2 e) { return make_float2(ex2_approx_ftz(e.x), ex2_approx_ftz(e.y)); }
 __device__ __forceinline__ float max_ept(const float (&x)[S_EPT]) {
     static_assert(S_EPT % 8 == 0, "eight logits per round");
     float m[S_EPT / 8];
@@ -460,17 +463,16 @@ __device__ __forceinline__ void p1_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
         const uint32_t wkey = __reduce_max_sync(FULL, pb ^ (((uint32_t)((int32_t)pb >> 31)) | 0x80000000u));   // monotone; -inf lowest
         const float wm = u2f((wkey & 0x80000000u) ? (wkey & 0x7fffffffu) : ~wkey);
         const float cc = -wm * sc;
-        float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
+        const float2 sc2 = make_float2(sc, sc), cc2 = make_float2(cc, cc);
+        float2 p01 = make_float2(0.0f, 0.0f), p23 = p01;
 #pragma unroll
         for (int j = 0; j < S_EPT; j += 4) {
-            p0 += ex2_approx_ftz(__fmaf_rn(x[j], sc, cc));
-            p1 += ex2_approx_ftz(__fmaf_rn(x[j + 1], sc, cc));
-            p2 += ex2_approx_ftz(__fmaf_rn(x[j + 2], sc, cc));
-            p3 += ex2_approx_ftz(__fmaf_rn(x[j + 3], sc, cc));
+            p01 = __fadd2_rn(p01, ex2_pair(__ffma2_rn(make_float2(x[j], x[j + 1]), sc2, cc2)));
+            p23 = __fadd2_rn(p23, ex2_pair(__ffma2_rn(make_float2(x[j + 2], x[j + 3]), sc2, cc2)));
         }
         // summed over the warp in fixed point (a lane's sum is at most 16, and an estimate is all that is needed); an
         // all-masked region has NaN here, which converts to 0
-        const uint32_t ws = __reduce_add_sync(FULL, __float2uint_rn(((p0 + p1) + (p2 + p3)) * 1048576.0f));
+        const uint32_t ws = __reduce_add_sync(FULL, __float2uint_rn(((p01.x + p01.y) + (p23.x + p23.y)) * 1048576.0f));
         if (lane == 0) {
             sm.reg_a[region] = wm; sm.reg_b[region] = (float)ws * (1.0f / 1048576.0f);
         }
@@ -545,18 +547,28 @@ __device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
     if (TAIL && region >= sm.pa.n_regions) return;   // warp-uniform: past the end of the row
     // nothing here is large enough to move the running value: the usual case once the sum has grown
     if (__all_sync(FULL, pm < sm.reg_t[region])) return;
+    const float2 sc2 = make_float2(sc, sc), hi2 = make_float2(c_hi, c_hi), lo2 = make_float2(c_lo, c_lo);
     if (BF16) {
         // bf16 rows hold every value thousands of times, and a numerator that is off by 1e-6 in the same direction for
         // all of them moves whole groups of additions across a rounding boundary: scale and constant as two floats
-        const float sc_lo = sm.pa.sc_lo;
+        const float2 sl2 = make_float2(sm.pa.sc_lo, sm.pa.sc_lo);
 #pragma unroll
-        for (int j = 0; j < S_EPT; j++) x[j] = __fmaf_rn(x[j], sc, c_hi) + __fmaf_rn(x[j], sc_lo, c_lo);   // -inf stays -inf
+        for (int j = 0; j < S_EPT; j += 2) {   // -inf stays -inf
+            const float2 v = make_float2(x[j], x[j + 1]), e = __fadd2_rn(__ffma2_rn(v, sc2, hi2), __ffma2_rn(v, sl2, lo2));
+            x[j] = e.x; x[j + 1] = e.y;
+        }
     } else {
 #pragma unroll
-        for (int j = 0; j < S_EPT; j++) x[j] = __fmaf_rn(x[j], sc, c_hi);   // -inf stays -inf
+        for (int j = 0; j < S_EPT; j += 2) {   // -inf stays -inf
+            const float2 e = __ffma2_rn(make_float2(x[j], x[j + 1]), sc2, hi2);
+            x[j] = e.x; x[j + 1] = e.y;
+        }
         if (c_lo != 0.0f) {   // CTA-uniform: the constant needs its second float (cold rows, large maxima)
 #pragma unroll
-            for (int j = 0; j < S_EPT; j++) x[j] += c_lo;
+            for (int j = 0; j < S_EPT; j += 2) {
+                const float2 e = __fadd2_rn(make_float2(x[j], x[j + 1]), lo2);
+                x[j] = e.x; x[j + 1] = e.y;
+            }
         }
     }
 #pragma unroll
@@ -567,13 +579,13 @@ __device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
     if (quick) {
         // every thread from the lower end of the binade the fold is in (the table guarantees that nobody leaves it);
         // four chains: the increments do not depend on the order
-        float ac[4] = {base, base, base, base};
+        float2 a01 = make_float2(base, base), a23 = a01;
 #pragma unroll
-        for (int j = 0; j < S_EPT / 4; j++) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) ac[c] = fadd(ac[c], x[c * (S_EPT / 4) + j]);
+        for (int j = 0; j < S_EPT; j += 4) {
+            a01 = __fadd2_rn(a01, make_float2(x[j], x[j + 1]));
+            a23 = __fadd2_rn(a23, make_float2(x[j + 2], x[j + 3]));
         }
-        const uint32_t ws = __reduce_add_sync(FULL, ((f2u(ac[0]) - bb) + (f2u(ac[1]) - bb)) + ((f2u(ac[2]) - bb) + (f2u(ac[3]) - bb)));   // < 32 * 2^25
+        const uint32_t ws = __reduce_add_sync(FULL, ((f2u(a01.x) - bb) + (f2u(a01.y) - bb)) + ((f2u(a23.x) - bb) + (f2u(a23.y) - bb)));   // < 32 * 2^25
         if (bb != fa.cur_bb) { fa.flush(); fa.cur_bb = bb; }
         fa.cur_n += ws;
     }
