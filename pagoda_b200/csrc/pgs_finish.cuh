@@ -74,96 +74,80 @@ __device__ __forceinline__ int warp_find(const float* pre, int n, int mode, floa
 }
 
 constexpr int RUN = 16;   // consecutive terms of a lane
-// 32 runs of terms, one per lane, ready to be added to a running value: lanes whose runs are estimated to begin in one
-// binade form a group, and each lane holds the increments from the group's first lane up to and including its own, for an
-// even and for an odd running value there.
-struct Runs {
-    uint32_t k;         // bits of the estimated binade's lower end (0: none)
-    uint32_t c0, c1;    // SEQ_SAT: leaves the binade
-    uint32_t head;      // first lane of the group; bit 31: nothing but zeros in this lane's run
-};
-
-// v: this lane's run; R0: estimate of the running value at the first lane's run
-__device__ __forceinline__ Runs make_runs(const float (&v)[RUN], float R0) {
+// What this lane's run adds to a running value in the binade whose lower end has the bits k, in ulps, from an even (c0) and from
+// an odd (c1) value; SEQ_SAT: leaves the binade.
+__device__ __forceinline__ void run_increments(const float (&v)[RUN], uint32_t k, uint32_t& c0, uint32_t& c1) {
+    float2 s = make_float2(u2f(k), u2f(k + 1u));
+#pragma unroll
+    for (int j = 0; j < RUN; j++) s = __fadd2_rn(s, make_float2(v[j], v[j]));
+    c0 = (f2u(s.x) & 0x7f800000u) == k ? f2u(s.x) - k : SEQ_SAT;
+    c1 = (f2u(s.y) & 0x7f800000u) == k ? f2u(s.y) - (k + 1u) : SEQ_SAT;
+}
+// Of c0 and c1, what the lane's run really adds when the first lane's begins with a value of parity `odd`.  A run without a term
+// that ends on half an ulp adds the same either way (tie: ballot of those that do not) and only turns the parity or keeps it;
+// behind a run that ends with one parity whatever it begins with, nothing in front of it matters.  (Three ballots and a few bit
+// operations: composing the pairs of increments lane by lane, five rounds of shuffles and selections, took 511 cycles.)
+__device__ __forceinline__ uint32_t increment_from(uint32_t c0, uint32_t c1, unsigned tie, uint32_t odd) {
+    if (tie) {   // warp-uniform
+        const unsigned m0 = __ballot_sync(FULL, c0 & 1u), m1 = __ballot_sync(FULL, !(c1 & 1u));   // parity behind an even, an odd one
+        const unsigned before = (1u << (threadIdx.x & 31)) - 1u, fixed = ~(m0 ^ m1) & before;
+        const uint32_t from = 32u - __clz((int)fixed);   // the runs in front of this lane that matter begin here (0 .. 31)
+        const uint32_t p = (fixed ? m0 >> (from - 1u) : odd) + __popc(m0 & ~m1 & before & (0xffffffffu << from));
+        if (p & 1u) c0 = c1;
+    }
+    return min(c0, 0x00800000u);   // (2^23 leaves the binade whatever the value)
+}
+__device__ __forceinline__ uint32_t warp_scan_u32(uint32_t v) {   // inclusive
     const uint32_t lane = threadIdx.x & 31;
-    float c = 0.0f;
-#pragma unroll
-    for (int j = 0; j < RUN; j++) c += v[j];
-    float inc = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(FULL, inc, o);
-        if (lane >= (uint32_t)o) inc += t;
+        const uint32_t t = __shfl_up_sync(FULL, v, o);
+        if (lane >= (uint32_t)o) v += t;
     }
-    Runs s;
-    s.k = f2u(R0 + (inc - c)) & 0x7f800000u;
-    if (s.k == 0x7f800000u) s.k = 0u;
-    s.c0 = s.c1 = SEQ_SAT;
-    if (c == 0.0f) s.c0 = s.c1 = 0u;
-    else if (s.k) {
-        float a0 = u2f(s.k), a1 = u2f(s.k + 1u);
-#pragma unroll
-        for (int j = 0; j < RUN; j++) { a0 = fadd(a0, v[j]); a1 = fadd(a1, v[j]); }
-        if ((f2u(a0) & 0x7f800000u) == s.k) s.c0 = f2u(a0) - s.k;
-        if ((f2u(a1) & 0x7f800000u) == s.k) s.c1 = f2u(a1) - (s.k + 1u);
-    }
-    const uint32_t before = __shfl_up_sync(FULL, s.k, 1);
-    const unsigned heads = __ballot_sync(FULL, lane == 0u || before != s.k);
-    s.head = 31u - __clz((int)(heads & (0xffffffffu >> (31u - lane))));
-    // compose(left, right)(p) = left_p + right_{(p + left_p) & 1}, inside the group
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t l0 = __shfl_up_sync(FULL, s.c0, o), l1 = __shfl_up_sync(FULL, s.c1, o);
-        if (lane >= s.head + (uint32_t)o) {
-            const uint32_t n0 = l0 + ((l0 & 1u) ? s.c1 : s.c0), n1 = l1 + (((l1 + 1u) & 1u) ? s.c1 : s.c0);
-            s.c0 = (l0 >= SEQ_SAT || n0 >= SEQ_SAT) ? SEQ_SAT : n0;
-            s.c1 = (l1 >= SEQ_SAT || n1 >= SEQ_SAT) ? SEQ_SAT : n1;
-        }
-    }
-    if (c == 0.0f) s.head |= 0x80000000u;
-    return s;
+    return v;
 }
 
-// Adds the runs to the exact running value R; one warp, the same result in all lanes.  ends: the running value behind every
-// run (optional).
-__device__ __forceinline__ float add_runs(float R, const Runs& s, const float (&v)[RUN], float* ends = nullptr) {
-    const uint32_t lane = threadIdx.x & 31, head = s.head & 31u;
-    const bool zero = (s.head >> 31) != 0u;
-    uint32_t pos = 0u;
+// Adds runs of terms to the exact running value R, those of the lanes pos .. 31 in this order; one warp, the same result in all
+// lanes.  ends: the running value behind every run (optional).  As many runs as keep the running value in its binade at once,
+// then the next one term by term, and on from what that has come to: what the lanes add is looked at anew in every binade, so
+// nothing rests on an estimate.  (With the increments of estimated binades, a crossing that came a run earlier or later than
+// estimated left all runs behind it to be added one by one.)
+__device__ __forceinline__ float add_runs(float R, const float (&v)[RUN], float* ends = nullptr, uint32_t pos = 0u) {
+    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll 1
     while (pos < 32u) {
-        // The group that begins here, as far as the running value stays in its binade; and what the first lane in which it
-        // does not (or the estimate missed the binade) makes of it: every lane adds its run to the value it would begin with.
-        const uint32_t rb = f2u(R), d = (rb & 1u) ? s.c1 : s.c0;
-        const bool fits = lane >= pos && (zero || (head == pos && s.k == (rb & 0x7f800000u) && d < SEQ_SAT && (rb & 0x007fffffu) + d < 0x00800000u));
-        const uint32_t own = zero ? 0u : d;   // (zeros: the group's increments up to here, which the lane before has too)
-        const unsigned ok = __ballot_sync(FULL, fits) >> pos;
-        const uint32_t n = ~ok ? min((uint32_t)__ffs((int)~ok) - 1u, 32u - pos) : 32u - pos;
-        uint32_t last = __reduce_max_sync(FULL, fits && lane < pos + n ? own : 0u);   // (increments only grow inside a group)
-        float r = u2f(rb + last);
-        if (ends) {
-            uint32_t e = fits ? own : 0u;
-            const unsigned zeros = __ballot_sync(FULL, fits && zero);
-            if (zeros) {   // what the runs before come to
+        const uint32_t rb = f2u(R), k = rb & 0x7f800000u, room = 0x00800000u - (rb & 0x007fffffu);
+        uint32_t n, inc = 0u;
+        if (k == 0u) {   // nothing yet: on to the first run with a term
+            uint32_t bits = 0u;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, e, o);
-                    if (lane >= (uint32_t)o) e = umax(e, t);
-                }
+            for (int j = 0; j < RUN; j++) bits |= f2u(v[j]);
+            const unsigned real = __ballot_sync(FULL, bits != 0u) >> pos;
+            n = real ? (uint32_t)__ffs((int)real) - 1u : 32u - pos;
+        } else {
+            uint32_t c0, c1;
+            run_increments(v, k, c0, c1);
+            if (lane < pos) c0 = c1 = 0u;
+            inc = increment_from(c0, c1, __ballot_sync(FULL, c0 != c1), rb);
+            if (!ends) {
+                const uint32_t all = __reduce_add_sync(FULL, inc);
+                if (all < room) return u2f(rb + all);
             }
-            if (lane >= pos && lane < pos + n) ends[lane] = u2f(rb + e);
+            inc = warp_scan_u32(inc);
+            const unsigned ok = __ballot_sync(FULL, inc < room) >> pos;
+            n = ~ok ? min((uint32_t)__ffs((int)~ok) - 1u, 32u - pos) : 32u;
         }
+        if (ends && lane >= pos && lane < pos + n) ends[lane] = u2f(rb + inc);
+        const uint32_t last = __shfl_sync(FULL, inc, (int)(pos + n - 1u) & 31);
+        R = n ? u2f(rb + last) : R;
         pos += n;
         if (pos < 32u) {
-            if (lane == pos) {
 #pragma unroll
-                for (int j = 0; j < RUN; j++) r = fadd(r, v[j]);
-            }
-            r = __shfl_sync(FULL, r, (int)pos);
-            if (ends && lane == 0) ends[pos] = r;
+            for (int j = 0; j < RUN; j++) R = fadd(R, v[j]);   // (every lane its own run)
+            R = __shfl_sync(FULL, R, (int)pos);
+            if (ends && lane == 0) ends[pos] = R;
             pos++;
         }
-        R = r;
     }
     return R;
 }
@@ -183,7 +167,7 @@ __device__ __forceinline__ float warp_fold(const float* v, uint32_t n, float goa
             const float4 q = i < n ? *reinterpret_cast<const float4*>(v + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             x[j] = q.x; x[j + 1] = i + 1 < n ? q.y : 0.0f; x[j + 2] = i + 2 < n ? q.z : 0.0f; x[j + 3] = i + 3 < n ? q.w : 0.0f;
         }
-        R = add_runs(R, make_runs(x, R), x, ends + base / RUN);
+        R = add_runs(R, x, ends + base / RUN);
     }
     return R;
 }

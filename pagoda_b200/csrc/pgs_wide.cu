@@ -26,7 +26,7 @@
 // non-negative term is an integer addition in ulps which depends on the running value only where the term ends exactly on
 // half an ulp.  A region (or bucket) without such a tie whose running value provably stays inside one binade is one
 // integer, whatever the order; the few others are added in order, each lane of a warp a run of terms that is summarised by
-// its increments from an even and from an odd start (as in pgs_block.cuh).  Every summary is checked against the exact
+// its increments from an even and from an odd start.  Every summary is checked against the exact
 // running value before it is used, so the result is bit-identical to the serial fold.
 #include <cuda_runtime.h>
 
@@ -46,6 +46,14 @@ constexpr uint32_t W_NIL = 0xffffffffu;
 static_assert(W_KMAX <= F_MCAP / 2, "room for the candidates");
 constexpr uint32_t W_DUAL = 2u;          // beside a segment's binade: it may also be the next one
 
+// the terms of a fold: softmax numerators (S <= 0), or the probabilities that are kept
+struct Terms {
+    float m, t, S;           // S > 0: probabilities, numerator / S when that is above the reference's epsilon
+    bool filter;
+    float p_thr;
+    uint32_t id_thr;
+};
+
 struct alignas(16) WideSmem {
     RowArgs a;                           // the launch's arguments, for the phases, which are functions of their own
     WideLaunch l;
@@ -54,18 +62,25 @@ struct alignas(16) WideSmem {
     unsigned long long exp_tab[32];
     uint32_t red_u[WNW], red_v[WNW];
     float red_f[WNW];
-    uint32_t last, found, n_serial, ok, gave_up;
+    uint32_t last, found, ok, gave_up;
     uint32_t rank, size, target;         // of the CTA among those that take part; arrivals at the barrier behind this one
     float R;
+    Terms terms;                         // of the fold
+    uint32_t n_ev, at_ev;                // its events, and how many are behind it
     alignas(16) float stage[WNW][W_REGION];   // per warp: a region in id order
     alignas(16) float spare[W_REGION];
-    alignas(16) Runs runs[WNW][32];
+    alignas(16) uint4 runs[WNW][32];     // per warp: a segment that is added term by term (see prepare_segment)
+    uint32_t run_k[WNW];
     uint32_t serial[W_MAX_REGIONS];      // segments that are added term by term
+    unsigned long long red_w[WNW];
     union {
         struct {
             uint2 seg[W_MAX_REGIONS];
             float pre[W_MAX_REGIONS];
             float start[W_MAX_REGIONS];  // exact running value at the segment's start
+            uint4 ev[W_MAX_REGIONS + 1];              // what the fold goes through (see resolve)
+            unsigned long long ev_sum[W_MAX_REGIONS + 1];   // increments of the segments before
+            float ev_R[W_MAX_REGIONS];                // exact running value there; -1: sm.start has it
         };
         uint32_t hash[4 * W_MAX_HIST];   // ids, then counts
         struct {
@@ -82,6 +97,12 @@ struct alignas(16) WideSmem {
     };
 };
 static_assert(sizeof(WideSmem) <= 227 * 1024, "one CTA per SM");
+// (The phases are functions of their own and name the CTA's shared memory themselves: through a reference handed to them every
+// access would be a generic one.)
+__device__ __forceinline__ WideSmem& wide_smem() {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    return *reinterpret_cast<WideSmem*>(smem_raw);
+}
 
 // ------------------------------------------------------------------------------------------------ grid barrier
 
@@ -204,13 +225,6 @@ __device__ __forceinline__ void wprocess(float* buf, float (&x)[WL], const WideL
     }
 }
 
-// the terms of a fold: softmax numerators (S <= 0), or the probabilities that are kept
-struct Terms {
-    float m, t, S;           // S > 0: probabilities, numerator / S when that is above the reference's epsilon
-    bool filter;
-    float p_thr;
-    uint32_t id_thr;
-};
 __device__ __forceinline__ float term_of(float x, uint32_t id, const Terms& f, const unsigned long long* tab) {
     float v = softmax_num(x, f.m, f.t, tab);
     if (f.S >= 0.0f) {
@@ -306,38 +320,245 @@ __device__ __forceinline__ void to_runs(float* buf, float (&v)[WL], const float 
     for (int j = 0; j < WL; j++) v[j] = buf[lane * WL + j];
 }
 
+// A segment that is added term by term, made ready for add_segment by one warp: v, the lanes' runs; pre, the estimate of the
+// running value at its start.  Most such segments are those in which the running value changes binade once.  So per lane, each
+// from an even and from an odd value: the increments up to and including its run in the binade at the start (x, y), and those of
+// its run and all behind it in the next binade (z, w).
+__device__ __forceinline__ void prepare_segment(WideSmem& sm, uint32_t w, const float (&v)[WL], float pre) {
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < WL; j += 4) *reinterpret_cast<float4*>(&sm.stage[w][lane * WL + j]) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    uint32_t k = f2u(pre * 0.9995f) & 0x7f800000u;   // (the estimate is too large, by a few 1e-4, rather than too small)
+    if (k == 0u || k >= 0x7f000000u) k = W_NIL;   // none
+    uint4 s = make_uint4(0u, 0u, 0u, 0u);
+    if (k != W_NIL) {   // warp-uniform
+        uint32_t c0, c1;
+        run_increments(v, k, c0, c1);
+        const unsigned tie = __ballot_sync(FULL, c0 != c1);
+        s.x = warp_scan_u32(increment_from(c0, c1, tie, 0u));
+        s.y = tie ? warp_scan_u32(increment_from(c0, c1, tie, 1u)) : s.x;
+        run_increments(v, k + 0x00800000u, c0, c1);
+        s.z = min(c0, 0x00800000u); s.w = min(c1, 0x00800000u);   // (2^23 leaves the binade whatever else is added)
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {   // (left, right)(p) = left_p + right_{(p + left_p) & 1}
+            const uint32_t r0 = __shfl_down_sync(FULL, s.z, o), r1 = __shfl_down_sync(FULL, s.w, o);
+            if (lane + (uint32_t)o < 32u) { s.z += (s.z & 1u) ? r1 : r0; s.w += (s.w & 1u) ? r0 : r1; }
+        }
+    }
+    sm.runs[w][lane] = s;
+    if (lane == 0) sm.run_k[w] = k;
+}
+// the terms of the runs pos .. n - 1, one after the other
+__device__ __forceinline__ float add_run(float R, const float* terms, uint32_t pos, uint32_t n) {
+    const float4* v = reinterpret_cast<const float4*>(terms + pos * WL);
+    float4 a[WL / 4];
+#pragma unroll
+    for (int j = 0; j < WL / 4; j++) a[j] = v[j];
+#pragma unroll 1
+    for (;;) {
+        pos++;
+        v += pos < n ? WL / 4 : 0;
+#pragma unroll
+        for (int j = 0; j < WL / 4; j++) {   // (the next run is on its way while this one is added)
+            const float4 t = a[j];
+            a[j] = v[j];
+            R = fadd(R, t.x); R = fadd(R, t.y); R = fadd(R, t.z); R = fadd(R, t.w);
+        }
+        if (pos >= n) return R;
+    }
+}
+// Adds the segment that warp q has made ready to the exact running value R, as far as what has been made ready serves for it; one
+// warp.  Returns how many of the 32 runs are done.
+__device__ __forceinline__ uint32_t add_segment(const WideSmem& sm, uint32_t q, float& R) {
+    const uint32_t k = sm.run_k[q], rb = f2u(R);
+    const uint4 s = sm.runs[q][threadIdx.x & 31];
+    if ((rb & 0x7f800000u) != k) return 0u;
+    const uint32_t d = (rb & 1u) ? s.y : s.x;
+    const uint32_t over = ~__ballot_sync(FULL, d < 0x00800000u - (rb & 0x007fffffu));   // (the lanes' increments only grow)
+    const uint32_t n = over ? (uint32_t)__ffs((int)over) - 1u : 32u, inc = __shfl_sync(FULL, d, (int)(n - 1u) & 31);
+    R = u2f(rb + (n ? inc : 0u));
+    if (n == 32u) return 32u;
+    R = add_run(R, sm.stage[q], n, n + 1u);   // the run in which the binade changes
+    if (n == 31u) return 32u;
+    const uint32_t r1 = f2u(R), all = __shfl_sync(FULL, (r1 & 1u) ? s.w : s.z, (int)n + 1);
+    if ((r1 & 0x7f800000u) != k + 0x00800000u || all >= 0x00800000u - (r1 & 0x007fffffu)) return n + 1u;
+    R = u2f(r1 + all);
+    return 32u;
+}
+
+// The segments [pos, stop), for which the estimate was not good enough, added to the exact running value R; one warp.
+template <bool BF16, bool VEC>
+__device__ __noinline__ float add_slowly(uint32_t slot, float R, uint32_t pos, uint32_t stop) {
+    WideSmem& sm = wide_smem();
+    const WideLaunch& l = sm.l;
+    const uint32_t lane = threadIdx.x & 31, V = sm.a.vocab;
+    while (pos < stop) {   // whole segments up to the next one that is not
+        uint2 sg = pos + lane < stop ? sm.seg[pos + lane] : make_uint2(0u, 1u);
+        const uint32_t rb = f2u(R), kb = rb & 0x7f800000u;
+        if ((sg.y & W_DUAL) && kb == sg.y - W_DUAL + 0x00800000u) sg = make_uint2(f2u(sm.pre[pos + lane]), kb);
+        sg.y &= ~W_DUAL;
+        const unsigned not_ok = ~__ballot_sync(FULL, sg.y == 1u || sg.y == kb);
+        uint32_t cnt = not_ok ? __ffs((int)not_ok) - 1u : 32u;
+        uint32_t inc = lane < cnt ? sg.x : 0u;
+        const uint32_t own = inc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, inc, o);
+            if (lane >= (uint32_t)o) inc += t;
+        }
+        const unsigned over = __ballot_sync(FULL, (rb & 0x007fffffu) + inc >= 0x00800000u && own != 0u);
+        if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
+        if (cnt) {
+            if (lane < cnt && pos + lane < stop) sm.start[pos + lane] = u2f(rb + inc - own);
+            R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
+            pos = min(pos + cnt, stop);
+        } else {
+            float x[WL], v[WL];
+            wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, sm.row, slot, V, pos, sm.terms);
+            to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
+            if (lane == 0) sm.start[pos] = R;
+            R = add_runs(R, v);
+            pos++;
+        }
+    }
+    return R;
+}
+
+// Warp 0's way through the events (see resolve) up to the first segment, of those to be added term by term, that is not among
+// the `ready` ones made ready so far (the first of them by warp 0, number q0).  A function of its own, whose inner loop has the
+// usual cases alone: its registers hold nothing else, and nothing is called from there.
+template <bool BF16, bool VEC>
+__device__ __noinline__ float walk(uint32_t slot, float R, uint32_t q0, uint32_t ready) {
+    WideSmem& sm = wide_smem();
+    const uint32_t lane = threadIdx.x & 31, n_ev = sm.n_ev;
+    uint32_t e = sm.at_ev, q = q0;
+    for (;;) {
+        uint32_t done = 32u;   // runs of the segment at which the loop stops; above: not a segment
+        float at_start;
+#pragma unroll 1
+        for (; e < n_ev; e++) {
+            const uint4 x = sm.ev[e];
+            at_start = R;
+            if (x.y == 0u) {
+                if (q == ready) break;
+                done = add_segment(sm, q - q0, R);
+                if (done != 32u) break;
+                q++;
+            } else {
+                const uint32_t rb = f2u(R), kb = rb & 0x7f800000u, k = x.y & ~W_DUAL;
+                const bool second = (x.y & W_DUAL) && kb == k + 0x00800000u;
+                const uint32_t inc = second ? x.w : x.z;
+                if (x.y != 1u && (!(kb == k || second) || inc >= 0x00800000u - (rb & 0x007fffffu))) { done = 33u; break; }
+                R = u2f(rb + inc);   // (zeros: inc is zero)
+            }
+            if (lane == 0) sm.ev_R[e] = at_start;
+        }
+        if (done == 32u) break;
+        if (done < 32u) {
+            const float* terms = sm.stage[q - q0];
+            if (at_start == 0.0f) R = add_run(R, terms, 0u, done = 32u);   // the start of the row: a new binade every few terms
+            else {
+                float v[WL];
+#pragma unroll
+                for (int j = 0; j < WL; j += 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(terms + lane * WL + j);
+                    v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+                }
+                R = add_runs(R, v, nullptr, done);
+            }
+            q++;
+        } else {
+            R = add_slowly<BF16, VEC>(slot, R, sm.ev[e].x, sm.ev[e + 1u].x);
+            at_start = -1.0f;
+        }
+        if (lane == 0) sm.ev_R[e] = at_start;
+        e++;
+    }
+    if (lane == 0) sm.at_ev = e;
+    __syncwarp();
+    return R;
+}
+
 // The exact left fold of a row's terms from the segments that the grid left in l.seg (estimates of the running value in
 // l.pre); the CTA.  Leaves the running value at every region's start in sm.start.
+//
+// One warp goes through the row's events, each from the exact running value: a segment that is added term by term, one that
+// lies in either of two binades, or a run of segments of one binade (or of zeros), whose increments a scan has added up, so that
+// the run is one addition if it stays in the binade.  That walk is the serial part; 64 scored rows of 151936, whose walks have 13
+// such segments and 11 runs on average, us a row on average and at most: 15 and 34 when runs were scanned 32 segments at a time
+// and the runs of terms inside a segment relied on estimated binades, now 8 and 21 (in cycles: a run of segments 70, a segment
+// 300, with a change of binade 500, the first segment of a row 2500).
 template <bool BF16, bool VEC>
-__device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_t slot, uint32_t V, const Terms f) {
+__device__ __noinline__ float resolve(uint32_t slot, uint32_t V, const Terms f) {
+    WideSmem& sm = wide_smem();
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_regions = (V + W_REGION - 1) / W_REGION;
     const WideRow& row = sm.row;
     __syncthreads();
-    if (tid == 0) sm.n_serial = 0u;
     for (uint32_t r = tid; r < n_regions; r += W_NT) {
         sm.seg[r] = __ldcg(l.seg + (size_t)slot * l.reg_stride + r);
         sm.pre[r] = __ldcg(l.pre + (size_t)slot * l.reg_stride + r);
     }
     __syncthreads();
-    // segments to be added term by term, in order
+    // the events: two regions per thread; increments, events and segments to be added term by term in one scan
+    static_assert(W_MAX_REGIONS == 2 * W_NT && W_MAX_REGIONS < 1 << 12, "packed counts");
+    constexpr unsigned long long EVENT = 1ull << 12;
+    unsigned long long own[2], sum;   // increments << 24 | events << 12 | segments
+    uint32_t n_ev, n_serial;
     {
-        uint32_t before = 0u;
-        for (uint32_t r0 = 0; r0 < n_regions; r0 += W_NT) {
-            const bool is = r0 + tid < n_regions && sm.seg[r0 + tid].y == 0u;
-            const unsigned in_warp = __ballot_sync(FULL, is);
-            if (lane == 0) sm.red_u[w] = __popc(in_warp);
-            __syncthreads();
-            const uint32_t c = sm.red_u[lane], mine = __reduce_add_sync(FULL, lane < w ? c : 0u);
-            if (is) sm.serial[before + mine + __popc(in_warp & ((1u << lane) - 1u))] = r0 + tid;
-            before += __reduce_add_sync(FULL, c);
-            __syncthreads();
+        uint32_t yp = tid && 2u * tid <= n_regions ? sm.seg[2u * tid - 1u].y : W_NIL;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t r = 2u * tid + u;
+            own[u] = 0ull;
+            if (r < n_regions) {
+                const uint2 sg = sm.seg[r];
+                const bool single = sg.y == 0u || (sg.y & W_DUAL);
+                if (!single) own[u] = (unsigned long long)min(sg.x, 0x01000000u) << 24;   // (2^23 is too much already)
+                if (single || sg.y != yp) own[u] |= EVENT;
+                own[u] |= sg.y == 0u;
+                yp = sg.y;
+            }
         }
-        if (tid == 0) sm.n_serial = before;
+        unsigned long long inc = own[0] + own[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(FULL, inc, o);
+            if (lane >= (uint32_t)o) inc += t;
+        }
+        if (lane == 31) sm.red_w[w] = inc;
+        __syncthreads();
+        unsigned long long before = sm.red_w[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(FULL, before, o);
+            if (lane >= (uint32_t)o) before += t;
+        }
+        const unsigned long long all = __shfl_sync(FULL, before, 31);
+        before = __shfl_sync(FULL, before, (int)(w + 31u) & 31);
+        sum = (w ? before : 0ull) + inc - own[0] - own[1];   // in front of this thread's regions
+        n_ev = (uint32_t)(all >> 12) & 0xfffu; n_serial = (uint32_t)all & 0xfffu;
+        unsigned long long s = sum;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t e = (uint32_t)(s >> 12) & 0xfffu;
+            if (own[u] & EVENT) { sm.ev[e].x = 2u * tid + u; sm.ev_sum[e] = s >> 24; }
+            if (own[u] & 1ull) sm.serial[(uint32_t)s & 0xfffu] = 2u * tid + u;
+            s += own[u];
+        }
+        if (tid == 0) { sm.ev[n_ev].x = n_regions; sm.ev_sum[n_ev] = all >> 24; sm.n_ev = n_ev; sm.at_ev = 0u; sm.terms = f; }
     }
     __syncthreads();
-    const uint32_t n_serial = sm.n_serial;
+    for (uint32_t e = tid; e < n_ev; e += W_NT) {
+        const uint32_t at = sm.ev[e].x;
+        const uint2 sg = sm.seg[at];
+        const unsigned long long run = sm.ev_sum[e + 1u] - sm.ev_sum[e];
+        sm.ev[e].y = sg.y;
+        sm.ev[e].z = sg.y & W_DUAL ? sg.x : (uint32_t)min(run, 0xffffffffull);
+        sm.ev[e].w = f2u(sm.pre[at]);   // (of a segment in either of two binades: the increments in the second)
+    }
     float R = 0.0f;        // warp 0
-    uint32_t pos = 0u;
     for (uint32_t b = 0; b < n_serial || b == 0u; b += WNW) {
         if (b + w < n_serial) {
             const uint32_t r = sm.serial[b + w], at = sm.seg[r].x;
@@ -346,66 +567,33 @@ __device__ __noinline__ float resolve(WideSmem& sm, const WideLaunch& l, uint32_
                 const float4* t = reinterpret_cast<const float4*>(l.terms + ((size_t)slot * W_TERMS + at - 1u) * W_REGION) + lane * (WL / 4);
 #pragma unroll
                 for (int j = 0; j < WL / 4; j++) {
-                    const float4 q = __ldcg(t + j);
-                    v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+                    const float4 q4 = __ldcg(t + j);
+                    v[4 * j] = q4.x; v[4 * j + 1] = q4.y; v[4 * j + 2] = q4.z; v[4 * j + 3] = q4.w;
                 }
             } else {
                 float x[WL];
                 wterms<BF16, VEC>(sm.exp_tab, sm.stage[w], x, l, row, slot, V, r, f);
                 to_runs<WLay<BF16, VEC>>(sm.stage[w], v, x);
             }
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < WL; j++) sm.stage[w][j * 32 + lane] = v[j];
-            sm.runs[w][lane] = make_runs(v, sm.pre[r]);
+            prepare_segment(sm, w, v, sm.pre[r]);
         }
         __syncthreads();
-        if (w == 0) {
-            const uint32_t n = min(n_serial - min(b, n_serial), (uint32_t)WNW);
-            for (uint32_t q = 0; q <= n; q++) {
-                const uint32_t stop = q < n ? sm.serial[b + q] : b + WNW >= n_serial ? n_regions : pos;
-                while (pos < stop) {   // whole segments up to the next one that is not
-                    uint2 sg = pos + lane < stop ? sm.seg[pos + lane] : make_uint2(0u, 1u);
-                    const uint32_t rb = f2u(R), kb = rb & 0x7f800000u;
-                    if ((sg.y & W_DUAL) && kb == sg.y - W_DUAL + 0x00800000u) sg = make_uint2(f2u(sm.pre[pos + lane]), kb);
-                    sg.y &= ~W_DUAL;
-                    const unsigned not_ok = ~__ballot_sync(FULL, sg.y == 1u || sg.y == kb);
-                    uint32_t cnt = not_ok ? __ffs((int)not_ok) - 1u : 32u;
-                    uint32_t inc = lane < cnt ? sg.x : 0u;
-                    const uint32_t own = inc;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t t = __shfl_up_sync(FULL, inc, o);
-                        if (lane >= (uint32_t)o) inc += t;
-                    }
-                    const unsigned over = __ballot_sync(FULL, (rb & 0x007fffffu) + inc >= 0x00800000u && own != 0u);
-                    if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
-                    if (cnt) {
-                        if (lane < cnt && pos + lane < stop) sm.start[pos + lane] = u2f(rb + inc - own);
-                        R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
-                        pos = min(pos + cnt, stop);
-                    } else {   // the estimate was not good enough for this one
-                        float x[WL], v[WL];
-                        wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, row, slot, V, pos, f);
-                        to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
-                        if (lane == 0) sm.start[pos] = R;
-                        R = add_runs(R, make_runs(v, R), v);
-                        pos++;
-                    }
-                }
-                if (q < n) {
-                    float v[WL];
-#pragma unroll
-                    for (int j = 0; j < WL; j++) v[j] = sm.stage[q][j * 32 + lane];
-                    if (lane == 0) sm.start[pos] = R;
-                    R = add_runs(R, sm.runs[q][lane], v);
-                    pos++;
-                }
-            }
-        }
+        if (w == 0) R = walk<BF16, VEC>(slot, R, b, min(n_serial, b + WNW));
         __syncthreads();
     }
     if (tid == 0) sm.R = R;
+    {
+        unsigned long long s = sum;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const uint32_t r = 2u * tid + u;
+            if (r >= n_regions) break;
+            const uint32_t i = ((uint32_t)((s + own[u]) >> 12) & 0xfffu) - 1u;   // the event that the region belongs to
+            const float at = sm.ev_R[i];
+            if (at >= 0.0f) sm.start[r] = u2f(f2u(at) + (uint32_t)((s >> 24) - sm.ev_sum[i]));
+            s += own[u];
+        }
+    }
     __syncthreads();
     return sm.R;
 }
@@ -507,7 +695,10 @@ __device__ __forceinline__ void row_out(WideSmem& sm, const WideLaunch& l, uint3
 // Parameters (same rules as the other kernels), and the distinct history ids of the row grouped by region with the values
 // the chain sees there.
 template <bool BF16>
-__device__ __noinline__ void open_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot, uint32_t row) {
+__device__ __noinline__ void open_row(uint32_t slot, uint32_t row) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     __syncthreads();
     uint32_t param = 0u;
@@ -625,7 +816,10 @@ __device__ __noinline__ void open_row(WideSmem& sm, const RowArgs& a, const Wide
 
 // Row maximum, argmax, and the table for the fold of the numerators.
 template <bool BF16, bool VEC>
-__device__ __noinline__ void maximum_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+__device__ __noinline__ void maximum_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     row_in(sm, l, slot);
     if (sm.row.state != WS_FIRST) return;
@@ -736,13 +930,16 @@ __device__ __forceinline__ float bucket_floor(uint32_t b) { return b ? u2f((b + 
 
 // The sum of the numerators; rows with top-k or top-p go on to the selection, others to the total.
 template <bool BF16, bool VEC>
-__device__ __noinline__ void sum_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+__device__ __noinline__ void sum_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     row_in(sm, l, slot);
     if (sm.row.state != WS_SUM) return;
     Terms f;
     f.m = sm.row.m; f.t = sm.row.t; f.S = -1.0f; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
-    const float S = resolve<BF16, VEC>(sm, l, slot, V, f);
+    const float S = resolve<BF16, VEC>(slot, V, f);
     if (threadIdx.x == 0) sm.row.n_terms = 0u;
     const bool use_k = sm.row.top_k != 0u && sm.row.top_k < V, use_p = !(sm.row.top_p >= 1.0f);
     __syncthreads();
@@ -789,7 +986,10 @@ __device__ __noinline__ void sum_row(WideSmem& sm, const RowArgs& a, const WideL
 
 // The lowest bucket that can matter: the one with the k-th largest probability, or the one in which the top-p fold ends (a
 // lower bound of the mass above it exceeds top-p by more than the fold can lose).  List positions for the buckets above.
-__device__ __noinline__ void select_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+__device__ __noinline__ void select_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     constexpr int PER = (W_BUCKETS + W_NT - 1) / W_NT;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab;
     row_in(sm, l, slot);
@@ -870,7 +1070,10 @@ __device__ __forceinline__ bool sort_bucket(WideSmem& sm, const WideLaunch& l, u
 
 // Top-k and top-p on the list.  A short list is finished here; a long one leaves the last kept (probability, id) and the
 // table for the fold of the kept probabilities.
-__device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+__device__ __noinline__ void choose_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     row_in(sm, l, slot);
     if (sm.row.state != WS_SELECT) return;
@@ -1010,7 +1213,7 @@ __device__ __noinline__ void choose_row(WideSmem& sm, const RowArgs& a, const Wi
                         const float p = q < nb ? u2f(~(uint32_t)(sm.sort[q] >> 32)) : 0.0f;
                         v[j] = p >= thr_k ? p : 0.0f;
                     }
-                    const float R1 = add_runs(R, make_runs(v, R), v);
+                    const float R1 = add_runs(R, v);
                     if (R1 >= sm.row.top_p) {   // in here: one lane looks for the entry
                         if (lane == 0) {
                             float r = R;
@@ -1075,12 +1278,15 @@ __device__ __forceinline__ Terms kept_terms(const WideRow& c, uint32_t V) {
 
 // Total of the kept probabilities and the inverse-CDF pick.
 template <bool BF16, bool VEC>
-__device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t slot) {
+__device__ __noinline__ void total_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     row_in(sm, l, slot);
     if (sm.row.state != WS_TOTAL) return;
     const Terms f = kept_terms(sm.row, V);
-    const float total = resolve<BF16, VEC>(sm, l, slot, V, f);
+    const float total = resolve<BF16, VEC>(slot, V, f);
     const float target = fmul(sm.row.u01, total);
     if (tid == 0) sm.found = W_NIL;
     __syncthreads();
@@ -1096,7 +1302,7 @@ __device__ __noinline__ void total_row(WideSmem& sm, const RowArgs& a, const Wid
             float x[WL], v[WL];
             wterms<BF16, VEC>(sm.exp_tab, sm.spare, x, l, sm.row, slot, V, r, f);
             to_runs<WLay<BF16, VEC>>(sm.spare, v, x);
-            add_runs(sm.start[r], make_runs(v, sm.start[r]), v, sm.red_f);
+            add_runs(sm.start[r], v, sm.red_f);
             __syncwarp();
             const unsigned over = __ballot_sync(FULL, target < sm.red_f[lane]);
             if (lane == 0 && over) {
@@ -1161,7 +1367,10 @@ enum : int { WP_FIRST = 0, WP_SUM, WP_LIST, WP_TOTAL, WP_FULL };
 
 // One region phase: the warps of the grid take the regions of all rows of the chunk in turn.
 template <bool BF16, bool VEC, int PHASE>
-__device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
+__device__ __noinline__ void region_phase(uint32_t n_rows) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     using L = WLay<BF16, VEC>;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     float* buf = sm.stage[w];
@@ -1307,7 +1516,10 @@ __device__ __noinline__ void region_phase(WideSmem& sm, const RowArgs& a, const 
 // Histogram of the probabilities of the rows that select by them.  Every CTA takes an equal run of the rows' regions, so
 // that most counting happens in shared memory and the buckets are flushed once or twice.
 template <bool BF16, bool VEC>
-__device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const WideLaunch& l, uint32_t n_rows) {
+__device__ __noinline__ void hist_phase(uint32_t n_rows) {
+    WideSmem& sm = wide_smem();
+    const RowArgs& a = sm.a;
+    const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     rows_in(sm, l, n_rows);
     uint32_t n_sel = 0u;
@@ -1346,17 +1558,19 @@ __device__ __noinline__ void hist_phase(WideSmem& sm, const RowArgs& a, const Wi
 }
 
 // `n` rows (of the list, or of the batch) one CTA each, by the general kernel's code on `slots` scratch slots
-__device__ __noinline__ void rows_one_cta_each(WideSmem& sm, const RowArgs& a, uint32_t rank, uint32_t slots, uint32_t n, const uint32_t* rows) {
+__device__ __noinline__ void rows_one_cta_each(uint32_t rank, uint32_t slots, uint32_t n, const uint32_t* rows) {
+    WideSmem& sm = wide_smem();
     if (n == 0u || rank >= slots) return;
     __syncthreads();
     if (threadIdx.x < 32u) sm.general.exp_tab[threadIdx.x] = kExp2TableDev[threadIdx.x];
     __syncthreads();
-    general_rows(a, sm.general, rank, slots, n, rows);
+    general_rows(sm.a, sm.general, rank, slots, n, rows);
 }
 
 // Whether the batch is done by one CTA per row; it is when this returns true.  (A general kernel for the same rows in front is
 // waited for only here: what the rows ask for stands already.  A function of its own, as the usual launch would fetch the code.)
-__device__ __noinline__ bool look(WideSmem& sm, uint32_t n_work, uint32_t slots) {
+__device__ __noinline__ bool look(uint32_t n_work, uint32_t slots) {
+    WideSmem& sm = wide_smem();
     const WideLaunch& l = sm.l;
     if (threadIdx.x == 0) sm.found = 0u;
     __syncthreads();
@@ -1365,7 +1579,7 @@ __device__ __noinline__ bool look(WideSmem& sm, uint32_t n_work, uint32_t slots)
     const bool front = l.kinds_front != 0u;
     const bool per_row = ((front ? l.kinds_front : n_work > l.chunk ? l.kinds_row[1] : l.kinds_row[0]) >> sm.found) & 1u;
     if (front) cudaGridDependencySynchronize();
-    else if (per_row) rows_one_cta_each(sm, sm.a, blockIdx.x, min(slots, gridDim.x), n_work, sm.a.work_rows);
+    else if (per_row) rows_one_cta_each(blockIdx.x, min(slots, gridDim.x), n_work, sm.a.work_rows);
     return per_row;
 }
 
@@ -1391,8 +1605,7 @@ __device__ __noinline__ void give_up(const RowArgs& a, const WideLaunch& l, uint
 
 template <bool BF16, bool VEC>
 __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const WideLaunch l_, uint32_t slots) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    WideSmem& sm = *reinterpret_cast<WideSmem*>(smem_raw);
+    WideSmem& sm = wide_smem();
     const RowArgs& a = sm.a;
     const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x;
@@ -1407,13 +1620,13 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     __syncthreads();
     bool ok = true;   // (false for all CTAs, or none)
     if (l_.look) {
-        ok = !look(sm, n_work, slots);
+        ok = !look(n_work, slots);
         if (!ok && l_.kinds_front) return;
     }
     ok = ok && grid_join(sm, l);
     for (uint32_t c0 = 0; c0 < n_work && ok; c0 += l.chunk) {
         const uint32_t n = min(n_work - c0, l.chunk);
-        const auto open = [&](uint32_t s) { open_row<BF16>(sm, a, l, s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
+        const auto open = [&](uint32_t s) { open_row<BF16>(s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
         uint32_t s = sm.rank;
         if (c0 == 0u) {   // (how many take part is not known yet)
             if (s < n) open(s);
@@ -1424,37 +1637,37 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             for (; s < n; s += sm.size) open(s);
             if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         }
-        region_phase<BF16, VEC, WP_FIRST>(sm, a, l, n);
+        region_phase<BF16, VEC, WP_FIRST>(n);
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(sm, a, l, s);
+        for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(s);
         if (sm.rank == 0u && tid == 0) { l.sync[2] = 0u; l.sync[3] = 0u; }
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        region_phase<BF16, VEC, WP_SUM>(sm, a, l, n);
+        region_phase<BF16, VEC, WP_SUM>(n);
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        for (uint32_t s = sm.rank; s < n; s += sm.size) sum_row<BF16, VEC>(sm, a, l, s);
+        for (uint32_t s = sm.rank; s < n; s += sm.size) sum_row<BF16, VEC>(s);
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;
         if (l.score) {
-            if (l.out_full) region_phase<BF16, VEC, WP_FULL>(sm, a, l, n);
+            if (l.out_full) region_phase<BF16, VEC, WP_FULL>(n);
         } else {
             if (*(volatile uint32_t*)(l.sync + 2)) {   // (the same for all CTAs)
-                hist_phase<BF16, VEC>(sm, a, l, n);
+                hist_phase<BF16, VEC>(n);
                 if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-                for (uint32_t s = sm.rank; s < n; s += sm.size) select_row(sm, a, l, s);
+                for (uint32_t s = sm.rank; s < n; s += sm.size) select_row(s);
                 if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-                region_phase<BF16, VEC, WP_LIST>(sm, a, l, n);
+                region_phase<BF16, VEC, WP_LIST>(n);
                 if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-                for (uint32_t s = sm.rank; s < n; s += sm.size) choose_row(sm, a, l, s);
+                for (uint32_t s = sm.rank; s < n; s += sm.size) choose_row(s);
                 if (!(ok = grid_sync(sm, l, n_work - c0))) break;
             }
             if (*(volatile uint32_t*)(l.sync + 3)) {
-                region_phase<BF16, VEC, WP_TOTAL>(sm, a, l, n);
+                region_phase<BF16, VEC, WP_TOTAL>(n);
                 if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-                for (uint32_t s = sm.rank; s < n; s += sm.size) total_row<BF16, VEC>(sm, a, l, s);
+                for (uint32_t s = sm.rank; s < n; s += sm.size) total_row<BF16, VEC>(s);
             }
         }
         if (!(ok = grid_sync(sm, l, n_work - c0))) break;   // the chunk's workspace is free
     }
-    if (ok && !l.score) rows_one_cta_each(sm, a, sm.rank, min(slots, sm.size), *(volatile uint32_t*)l.left_count, l.left_rows);
+    if (ok && !l.score) rows_one_cta_each(sm.rank, min(slots, sm.size), *(volatile uint32_t*)l.left_count, l.left_rows);
     // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();
     if (tid == 0) {

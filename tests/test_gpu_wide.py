@@ -45,6 +45,41 @@ def test_wide_kernel_edges(oracle, rows, vocab, top_k, history):
         s.close()
 
 
+@pytest.mark.parametrize("vocab", [512 * 33, 512 * 40 + 3])
+@pytest.mark.parametrize("top_k", [0, 40])
+def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k):
+    """The exact fold where its running value changes binade often, in one run of terms, at the edge of a region, or not
+    at all, and where terms end on half an ulp: bit-exact sums, totals, tokens and scores."""
+    import torch
+    import pagoda_b200
+    from pagoda_b200 import synth
+    monkeypatch.setenv("PGS_WIDE_ROUTE", "1")   # on the grid, whatever is quicker
+    i = np.arange(vocab)
+    rng = np.random.default_rng(vocab)
+    noise = rng.standard_normal(vocab)
+    rows = [np.zeros(vocab),                                        # one ulp pattern throughout
+            -40.0 + 40.0 * i / vocab, -40.0 * i / vocab,            # rising: a new binade every few hundred terms; falling
+            -0.6931472 * (i % 24), -0.6931472 * rng.integers(0, 12, vocab),   # powers of two, nearly: ties
+            np.where(i < vocab // 2, -85.0, noise),                 # next to nothing, then everything
+            np.where(i % 512 == 511, 4.0, -3.0) + noise, np.where(i % 512 == 0, 4.0, -3.0) + noise,   # at the regions' edges
+            np.where(i == 777, 20.0, noise), 2.0 * noise]
+    x = np.stack(rows).astype(np.float32) + np.float32(0.0)   # (no -0.0: the kernels report a maximum of zero as +0.0)
+    n = len(x)
+    w = synth.Workload("binades", x, np.resize(np.float32([1.0, 0.7]), n), np.full(n, top_k, np.uint32), np.resize(np.float32([1.0, 0.97, 0.9]), n),
+                       np.zeros(n, np.float32), np.zeros(n, np.float32), np.ones(n, np.float32), None, None, synth.uniform_f32(5, n))
+    s = pagoda_b200.Sampler(device=0, max_rows=n, max_vocab=vocab, max_history=1)
+    try:
+        s.set_exact(True)
+        assert_same(*run_both(s, oracle, w), w)
+        ids = np.full(n, vocab - 1, np.int32)
+        g, full, _ = s.log_softmax(torch.from_numpy(x).cuda(), ids=torch.from_numpy(ids).cuda(), full=True,
+                                   stream_ptr=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        check_scores(oracle, x, ids, g, full)
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("vocab", [3, 4, 513])
 @pytest.mark.parametrize("exact", [True, False])
 def test_top_k_bound_beyond_the_float_range(oracle, vocab, exact):
