@@ -142,6 +142,20 @@ __device__ __forceinline__ float ex2_approx_ftz(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// Two exponentials for the packed f32 instructions of sm_100 (two multiply-adds or additions in one issue slot, each rounded
+// as the scalar instruction rounds it): the arithmetic of the passes is issued in pairs.
+__device__ __forceinline__ float2 ex2_pair(float2 e) { return make_float2(ex2_approx_ftz(e.x), ex2_approx_ftz(e.y)); }
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// max(|a|, |b|, |c|), NaN if any of them is
+__device__ __forceinline__ float absmax3_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
+    return r;
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 #endif
 

@@ -165,20 +165,6 @@ static_assert(offsetof(StreamSmem<false>, hash) + sizeof(StreamSmem<false>::hash
         }                                                           \
     } while (0)
 
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-// max(|a|, |b|, |c|), NaN if any of them is
-__device__ __forceinline__ float absmax3_nan(float a, float b, float c) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
-    return r;
-}
-// Two exponentials for the packed f32 instructions of sm_100 (two multiply-adds or additions in one issue slot, each rounded
-// as the scalar instruction rounds it): the arithmetic of the passes is issued in pairs.
-__device__ __forceinline__ float2 ex2_pair(float2 e) { return make_float2(ex2_approx_ftz(e.x), ex2_approx_ftz(e.y)); }
 __device__ __forceinline__ float max_ept(const float (&x)[S_EPT]) {
     static_assert(S_EPT % 8 == 0, "eight logits per round");
     float m[S_EPT / 8];

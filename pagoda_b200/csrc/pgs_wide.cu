@@ -277,21 +277,32 @@ __device__ __forceinline__ Approx approx_of(const Terms& f) {
 template <bool BF16, bool VEC>
 __device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id0, const Terms& f, const Approx& q, uint32_t kb, const unsigned long long* tab) {
     const float k = q.k0 - (float)((int)(kb >> 23) - 127 - 23), eps = 2e-7f * fabsf(k) + 1e-7f * fabsf(q.k0) + 1e-6f;
-    const float p_lim = f.filter ? f.p_thr / u2f(kb) * 8388608.0f : 0.0f;   // the threshold in ulps
-    const float slack = (4.0f * eps + 4e-6f) * p_lim;
     uint32_t n = 0u, doubt = 0u;
+    if (!f.filter) {   // warp-uniform
+        // With v the term in ulps and d its distance from the nearest integer, |d| + v * eps >= 1/2 implies d * d + v * eps >= 1/4.
+        // (-inf -> 0; beyond 2^23, where d is of no use, v * eps alone is above)
+        const float2 m2 = make_float2(-f.m, -f.m), c2 = make_float2(q.c, q.c), k2 = make_float2(k, k), e2 = make_float2(eps, eps);
+        const float2 one = make_float2(8388608.0f, 8388608.0f), back = make_float2(-8388608.0f, -8388608.0f), minus = make_float2(-1.0f, -1.0f), quarter = make_float2(-0.25f, -0.25f);
 #pragma unroll
-    for (int j = 0; j < WL; j++) {
-        const float v = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, k));   // (-inf -> 0)
-        const float r = fadd(v, 8388608.0f);                                  // (beyond 2^23: in doubt)
-        bool open = !(__fmaf_rn(v, eps, fabsf(fsub(v, fsub(r, 8388608.0f)))) < 0.5f);
-        uint32_t i = f2u(r) - 0x4b000000u;
-        if (f.filter) {   // warp-uniform
+        for (int j = 0; j < WL; j += 2) {
+            const float2 v = ex2_pair(__ffma2_rn(__fadd2_rn(make_float2(x[j], x[j + 1]), m2), c2, k2)), r = __fadd2_rn(v, one);
+            const float2 d = __ffma2_rn(__fadd2_rn(r, back), minus, v), s = __ffma2_rn(d, d, __ffma2_rn(v, e2, quarter));
+            n += (f2u(r.x) - 0x4b000000u) + (f2u(r.y) - 0x4b000000u);
+            doubt = __funnelshift_l(f2u(s.x), doubt, 1);   // the sign bits, one after the other
+            doubt = __funnelshift_l(f2u(s.y), doubt, 1);
+        }
+        doubt = __brev(~doubt << 16);   // bit j: x[j]
+    } else {
+        const float p_lim = f.p_thr / u2f(kb) * 8388608.0f, slack = (4.0f * eps + 4e-6f) * p_lim;   // the threshold in ulps
+#pragma unroll
+        for (int j = 0; j < WL; j++) {
+            const float v = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, k)), r = fadd(v, 8388608.0f);
+            bool open = !(__fmaf_rn(v, eps, fabsf(fsub(v, fsub(r, 8388608.0f)))) < 0.5f);
             open = open && !(v < p_lim - slack);
             open = open || fabsf(v - p_lim) <= slack;
-            if (v < p_lim) i = 0u;
+            if (!(v < p_lim) || open) n += f2u(r) - 0x4b000000u;
+            if (open) doubt |= 1u << j;
         }
-        if (open) doubt |= 1u << j; else n += i;
     }
     bool good = true;
     while (__any_sync(FULL, doubt != 0u)) {
@@ -300,6 +311,7 @@ __device__ __forceinline__ uint32_t increments(const float (&x)[WL], uint32_t id
             float xj = x[0];
 #pragma unroll
             for (int u = 1; u < WL; u++) if (u == j) xj = x[u];
+            n -= f2u(fadd(ex2_approx_ftz(__fmaf_rn(fsub(xj, f.m), q.c, k)), 8388608.0f)) - 0x4b000000u;   // (as above)
             good &= increment(term_of(xj, id0 + WLay<BF16, VEC>::off(threadIdx.x & 31u, (uint32_t)j), f, tab), kb, n);
             doubt &= doubt - 1u;
         }
@@ -1388,13 +1400,14 @@ __device__ __noinline__ void region_phase(uint32_t n_rows) {
         if (PHASE == WP_FIRST) {
             if (state != WS_FIRST) continue;
             wload<BF16, VEC>(x, c.rowp, r, nv);
-            uint32_t bad = 0u;
+            float am = 0.0f;   // max |raw logit|, NaN-propagating
 #pragma unroll
-            for (int j = 0; j < WL; j++) bad |= !finite_f(x[j]);
+            for (int j = 0; j < WL; j += 2) am = absmax3_nan(am, x[j], x[j + 1]);
             wprocess<BF16, VEC>(buf, x, l, slot, c.mw, c.entries, r, nv);
-            float top = -INFINITY;
+            float top = x[0];
 #pragma unroll
-            for (int j = 0; j < WL; j++) top = fmaxf(top, x[j]);
+            for (int j = 1; j + 1 < WL; j += 2) top = max3f(top, x[j], x[j + 1]);
+            top = fmaxf(top, x[WL - 1]);
             float part = top;   // of eight lanes
 #pragma unroll
             for (int o = 4; o; o >>= 1) part = fmaxf(part, __shfl_xor_sync(FULL, part, o));
@@ -1404,12 +1417,18 @@ __device__ __noinline__ void region_phase(uint32_t n_rows) {
             const float wm = u2f((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), sc = 1.44269504f / c.t;
             float s = 0.0f;
             if (wm > -INFINITY) {
+                const float2 m2 = make_float2(-wm, -wm), sc2 = make_float2(sc, sc);
+                float2 a2 = make_float2(0.0f, 0.0f), b2 = a2;
 #pragma unroll
-                for (int j = 0; j < WL; j++) s += ex2_approx_ftz((x[j] - wm) * sc);
+                for (int j = 0; j < WL; j += 4) {
+                    a2 = __fadd2_rn(a2, ex2_pair(__fmul2_rn(__fadd2_rn(make_float2(x[j], x[j + 1]), m2), sc2)));
+                    b2 = __fadd2_rn(b2, ex2_pair(__fmul2_rn(__fadd2_rn(make_float2(x[j + 2], x[j + 3]), m2), sc2)));
+                }
+                s = (a2.x + a2.y) + (b2.x + b2.y);
             }
 #pragma unroll
             for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-            bad = __any_sync(FULL, bad);
+            const uint32_t bad = __any_sync(FULL, !(am < INFINITY));
             if (lane == 0) {
                 l.reg[(size_t)slot * l.reg_stride + r] = make_float2(wm, s);
                 if (bad) l.row[slot].nonfinite = 1u;
