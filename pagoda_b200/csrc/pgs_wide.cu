@@ -68,7 +68,7 @@ struct alignas(16) WideSmem {
     Terms terms;                         // of the fold
     uint32_t n_ev, at_ev;                // its events, and how many are behind it
     alignas(16) float stage[WNW][W_REGION];   // per warp: a region in id order
-    alignas(16) float spare[W_REGION];
+    alignas(16) float spare[W_REGION], spare_too[W_REGION];
     alignas(16) uint4 runs[WNW][32];     // per warp: a segment that is added term by term (see prepare_segment)
     uint32_t run_k[WNW];
     uint32_t serial[W_MAX_REGIONS];      // segments that are added term by term
@@ -437,6 +437,27 @@ __device__ __noinline__ float add_slowly(uint32_t slot, float R, uint32_t pos, u
     return R;
 }
 
+// the lowest id of region r whose processed logit is m; one warp
+template <bool BF16, bool VEC>
+__device__ __forceinline__ uint32_t find_in_region(float* buf, const WideRow& row, const WideLaunch& l, uint32_t slot, uint32_t V, uint32_t r, float m) {
+    float x[WL];
+    const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
+    wload<BF16, VEC>(x, row.rowp, r, nv);
+    wprocess<BF16, VEC>(buf, x, l, slot, row.mw, row.entries, r, nv);
+    uint32_t o = W_NIL;
+#pragma unroll
+    for (int j = WL - 1; j >= 0; j--)
+        if (x[j] == m) o = WLay<BF16, VEC>::off(threadIdx.x & 31, j);   // (a lane's logits are in id order)
+    return r * W_REGION + __reduce_min_sync(FULL, o);
+}
+
+template <bool BF16, bool VEC>
+__device__ __noinline__ void argmax_row(uint32_t slot) {
+    WideSmem& sm = wide_smem();
+    const uint32_t id = find_in_region<BF16, VEC>(sm.spare_too, sm.row, sm.l, slot, sm.a.vocab, sm.row.max_region, sm.row.m);
+    if ((threadIdx.x & 31) == 0) sm.row.amax = id;
+}
+
 // Warp 0's way through the events (see resolve) up to the first segment, of those to be added term by term, that is not among
 // the `ready` ones made ready so far (the first of them by warp 0, number q0).  A function of its own, whose inner loop has the
 // usual cases alone: its registers hold nothing else, and nothing is called from there.
@@ -493,7 +514,8 @@ __device__ __noinline__ float walk(uint32_t slot, float R, uint32_t q0, uint32_t
 }
 
 // The exact left fold of a row's terms from the segments that the grid left in l.seg (estimates of the running value in
-// l.pre); the CTA.  Leaves the running value at every region's start in sm.start.
+// l.pre); the CTA.  Leaves the running value at every region's start in sm.start.  argmax: another warp looks for the row's
+// argmax beside the walk.
 //
 // One warp goes through the row's events, each from the exact running value: a segment that is added term by term, one that
 // lies in either of two binades, or a run of segments of one binade (or of zeros), whose increments a scan has added up, so that
@@ -502,7 +524,7 @@ __device__ __noinline__ float walk(uint32_t slot, float R, uint32_t q0, uint32_t
 // and the runs of terms inside a segment relied on estimated binades, now 8 and 21 (in cycles: a run of segments 70, a segment
 // 300, with a change of binade 500, the first segment of a row 2500).
 template <bool BF16, bool VEC>
-__device__ __noinline__ float resolve(uint32_t slot, uint32_t V, const Terms f) {
+__device__ __noinline__ float resolve(uint32_t slot, uint32_t V, const Terms f, bool argmax) {
     WideSmem& sm = wide_smem();
     const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_regions = (V + W_REGION - 1) / W_REGION;
@@ -591,6 +613,7 @@ __device__ __noinline__ float resolve(uint32_t slot, uint32_t V, const Terms f) 
         }
         __syncthreads();
         if (w == 0) R = walk<BF16, VEC>(slot, R, b, min(n_serial, b + WNW));
+        if (w == 1 && b == 0u && argmax) argmax_row<BF16, VEC>(slot);
         __syncthreads();
     }
     if (tid == 0) sm.R = R;
@@ -849,22 +872,18 @@ __device__ __noinline__ void maximum_row(uint32_t slot) {
     const uint32_t rstar = __reduce_min_sync(FULL, kk == gkey ? sm.red_v[lane] : W_NIL);
     const bool any = gkey != 0u;
     const float m = any ? key_to_float(gkey) : -INFINITY;
-    if (w == 0 && any && !sm.row.nonfinite) {   // the lowest id that holds the maximum
-        float x[WL];
-        const uint32_t nv = min(V - rstar * W_REGION, (uint32_t)W_REGION);
-        wload<BF16, VEC>(x, sm.row.rowp, rstar, nv);
-        wprocess<BF16, VEC>(sm.spare, x, l, slot, sm.row.mw, sm.row.entries, rstar, nv);
-        uint32_t o = W_NIL;
-#pragma unroll
-        for (int j = WL - 1; j >= 0; j--)
-            if (x[j] == m) o = WLay<BF16, VEC>::off(lane, j);   // (a lane's logits are in id order)
-        o = __reduce_min_sync(FULL, o);
-        if (lane == 0) sm.row.amax = rstar * W_REGION + o;
+    // (a row that goes on to be sampled looks for it beside the walk of its fold)
+    const bool ends_here = !l.score && (sm.row.temp < 1e-5f || (sm.row.gflags & 2u));
+    if (w == 0 && any && !sm.row.nonfinite && ends_here) {
+        if (lane == 0) { sm.row.m = m; sm.row.max_region = rstar; }
+        __syncwarp();
+        argmax_row<BF16, VEC>(slot);
     }
     __syncthreads();
     if (tid == 0) {
         WideRow& c = sm.row;
         c.m = m;
+        c.max_region = rstar;
         c.state = WS_DONE;
         if (l.score) {
             if (a.status) a.status[c.row] = c.nonfinite ? ROW_NONFINITE : ROW_OK;
@@ -925,6 +944,8 @@ __device__ __noinline__ void maximum_row(uint32_t slot) {
             if (tid == 0) sm.row.cut_x = fmaxf(bound - 4.8e-7f * (fabsf(m - bound) + 4.0f * sm.row.t) - 4.8e-7f * (fabsf(bound) + fabsf(m)), -3.402823466e38f);
         }
     }
+    if (sm.row.state == WS_SUM && tid == 0 && !l.score && !(sm.row.cut_x < INFINITY))   // (known to all behind the next barrier)
+        atomicAdd(l.sync + ((sm.row.top_k != 0u && sm.row.top_k < V) || !(sm.row.top_p >= 1.0f) ? 2 : 3), 1u);
     if (sm.row.state == WS_SUM) {
         const float sc = 1.44269504f / sm.row.t;
         make_table(sm, l, slot, n_regions, 0.001953125f + 1e-7f * fabsf(m * sc), [&](uint32_t r) {
@@ -951,7 +972,7 @@ __device__ __noinline__ void sum_row(uint32_t slot) {
     if (sm.row.state != WS_SUM) return;
     Terms f;
     f.m = sm.row.m; f.t = sm.row.t; f.S = -1.0f; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
-    const float S = resolve<BF16, VEC>(slot, V, f);
+    const float S = resolve<BF16, VEC>(slot, V, f, !l.score);
     if (threadIdx.x == 0) sm.row.n_terms = 0u;
     const bool use_k = sm.row.top_k != 0u && sm.row.top_k < V, use_p = !(sm.row.top_p >= 1.0f);
     __syncthreads();
@@ -971,8 +992,6 @@ __device__ __noinline__ void sum_row(uint32_t slot) {
                 l.out_gather[c.row] = v;
             }
         } else c.state = c.cut_x < INFINITY && c.n_list <= (uint32_t)F_MCAP ? WS_DONE : use_k || use_p ? WS_SELECT : WS_TOTAL;
-        if (c.state == WS_SELECT) atomicAdd(l.sync + 2, 1u);
-        if (c.state == WS_TOTAL) atomicAdd(l.sync + 3, 1u);
     }
     __syncthreads();
     if (sm.row.state == WS_DONE && !l.score) {   // the second pass has found the candidates
@@ -1298,7 +1317,7 @@ __device__ __noinline__ void total_row(uint32_t slot) {
     row_in(sm, l, slot);
     if (sm.row.state != WS_TOTAL) return;
     const Terms f = kept_terms(sm.row, V);
-    const float total = resolve<BF16, VEC>(slot, V, f);
+    const float total = resolve<BF16, VEC>(slot, V, f, false);
     const float target = fmul(sm.row.u01, total);
     if (tid == 0) sm.found = W_NIL;
     __syncthreads();
@@ -1377,15 +1396,24 @@ __device__ __noinline__ void total_row(uint32_t slot) {
 
 enum : int { WP_FIRST = 0, WP_SUM, WP_LIST, WP_TOTAL, WP_FULL };
 
-// One region phase: the warps of the grid take the regions of all rows of the chunk in turn.
+// One region phase, with the barrier in front of it (open: as there): the warps of the grid take the regions of all rows of the
+// chunk, which begins with row c0, in turn.  False: the barrier was given up.
 template <bool BF16, bool VEC, int PHASE>
-__device__ __noinline__ void region_phase(uint32_t n_rows) {
+__device__ __noinline__ bool region_phase(uint32_t n_rows, uint32_t c0, uint32_t open) {
     WideSmem& sm = wide_smem();
     const RowArgs& a = sm.a;
     const WideLaunch& l = sm.l;
     using L = WLay<BF16, VEC>;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, V = a.vocab, n_regions = (V + W_REGION - 1) / W_REGION;
     float* buf = sm.stage[w];
+    const bool first = sm.target == 0u;   // (how many take part is known behind the first barrier)
+    if (PHASE == WP_FIRST) {   // the warp's first region is on its way while the barrier is waited for
+        const uint32_t i = w * (first ? gridDim.x : sm.size) + sm.rank, slot = i / n_regions, at = (i - slot * n_regions) * W_REGION + lane * (128u / L::ESZ);
+        if (slot < n_rows && lane < W_REGION * L::ESZ / 128u && at < V)
+            prefetch_l2((const char*)a.logits + ((size_t)(a.work_rows ? a.work_rows[c0 + slot] : c0 + slot) * a.row_stride + at) * L::ESZ);
+    }
+    if (!grid_sync(sm, l, open)) return false;
+    if (PHASE == WP_FIRST && first && sm.size < n_rows) return true;   // rows are still to be opened
     rows_in(sm, l, n_rows);
     for (uint32_t i = w * sm.size + sm.rank; i < n_rows * n_regions; i += sm.size * WNW) {
         const uint32_t slot = i / n_regions, r = i - slot * n_regions, nv = min(V - r * W_REGION, (uint32_t)W_REGION);
@@ -1461,6 +1489,7 @@ __device__ __noinline__ void region_phase(uint32_t n_rows) {
             for (int j = 0; j < WL; j++)
                 if (x[j] >= cut) {   // (rare)
                     const uint32_t at = atomicAdd(&l.row[slot].n_list, 1u);
+                    if (at == (uint32_t)F_MCAP) atomicAdd(l.sync + 2, 1u);   // too many: the row selects by the histogram
                     if (at < min((uint32_t)F_MCAP, l.list_stride)) l.list[(size_t)slot * l.list_stride + at] = ((unsigned long long)f2u(x[j]) << 32) | (r * W_REGION + L::off(lane, j));
                 }
         }
@@ -1486,23 +1515,33 @@ __device__ __noinline__ void region_phase(uint32_t n_rows) {
                 else if ((out.y & W_DUAL) && lane == 0) l.pre[(size_t)slot * l.reg_stride + r] = u2f(n1);
             }
             if (out.y == 0u) {   // to be added term by term: the terms are left in id order, as far as there is room
-                bool zeros = true;
+                // (a loop over the staged logits: sixteen copies of the exponential's code, which few regions run through, take
+                // longer to fetch than to execute)
+                float top = x[0];
 #pragma unroll
-                for (int j = 0; j < WL; j++) {
-                    x[j] = term_of(x[j], r * W_REGION + L::off(lane, j), f, sm.exp_tab);
-                    zeros &= x[j] == 0.0f;
+                for (int j = 1; j < WL; j++) top = fmaxf(top, x[j]);
+                bool zeros = true;
+                if (__any_sync(FULL, top > -INFINITY)) {
+                    uint32_t at = 0u;
+                    if (lane == 0) at = atomicAdd(&l.row[slot].n_terms, 1u);
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < WL; j++) buf[L::off(lane, j)] = x[j];
+                    __syncwarp();
+#pragma unroll 4
+                    for (uint32_t o = lane; o < (uint32_t)W_REGION; o += 32u) {
+                        const float t = term_of(buf[o], r * W_REGION + o, f, sm.exp_tab);
+                        zeros &= t == 0.0f;
+                        buf[o] = t;
+                    }
+                    out.x = __shfl_sync(FULL, at, 0) + 1u;
                 }
-                if (__all_sync(FULL, zeros)) {   // nothing but zeros
-                    if (lane == 0) *seg = make_uint2(0u, 1u);
-                    continue;
-                }
-                if (lane == 0) out.x = atomicAdd(&l.row[slot].n_terms, 1u) + 1u;
-                out.x = __shfl_sync(FULL, out.x, 0);
-                if (out.x > (uint32_t)W_TERMS) out.x = 0u;
+                if (__all_sync(FULL, zeros)) out = make_uint2(0u, 1u);   // nothing but zeros
+                else if (out.x > (uint32_t)W_TERMS) out.x = 0u;
                 else {
                     float* t = l.terms + ((size_t)slot * W_TERMS + out.x - 1u) * W_REGION;
 #pragma unroll
-                    for (int j = 0; j < WL; j++) t[L::off(lane, j)] = x[j];
+                    for (int j = 0; j < WL; j++) t[j * 32 + lane] = buf[j * 32 + lane];   // (each lane its own)
                 }
             }
             if (lane == 0) *seg = out;
@@ -1530,6 +1569,7 @@ __device__ __noinline__ void region_phase(uint32_t n_rows) {
             }
         }
     }
+    return true;
 }
 
 // Histogram of the probabilities of the rows that select by them.  Every CTA takes an equal run of the rows' regions, so
@@ -1643,50 +1683,52 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         if (!ok && l_.kinds_front) return;
     }
     ok = ok && grid_join(sm, l);
+    uint32_t n_left = 0u;   // rows left to the general kernel's code
     for (uint32_t c0 = 0; c0 < n_work && ok; c0 += l.chunk) {
-        const uint32_t n = min(n_work - c0, l.chunk);
+        const uint32_t n = min(n_work - c0, l.chunk), to_do = n_work - c0;
         const auto open = [&](uint32_t s) { open_row<BF16>(s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
-        uint32_t s = sm.rank;
-        if (c0 == 0u) {   // (how many take part is not known yet)
-            if (s < n) open(s);
-            if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-            s += sm.size;
-        }
-        if (c0 || sm.size < n) {
-            for (; s < n; s += sm.size) open(s);
-            if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        }
-        region_phase<BF16, VEC, WP_FIRST>(n);
-        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(s);
         if (sm.rank == 0u && tid == 0) { l.sync[2] = 0u; l.sync[3] = 0u; }
-        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-        region_phase<BF16, VEC, WP_SUM>(n);
-        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+        uint32_t s = sm.rank;
+        if (c0 == 0u) { if (s < n) open(s); }   // (how many take part is not known yet)
+        else for (; s < n; s += sm.size) open(s);
+        if (!(ok = region_phase<BF16, VEC, WP_FIRST>(n, c0, to_do))) break;
+        if (c0 == 0u && sm.size < n) {   // not one CTA for every row
+            for (s += sm.size; s < n; s += sm.size) open(s);
+            if (!(ok = region_phase<BF16, VEC, WP_FIRST>(n, c0, to_do))) break;
+        }
+        if (!(ok = grid_sync(sm, l, to_do))) break;
+        for (uint32_t s = sm.rank; s < n; s += sm.size) maximum_row<BF16, VEC>(s);
+        if (!(ok = region_phase<BF16, VEC, WP_SUM>(n, c0, to_do))) break;
+        if (!(ok = grid_sync(sm, l, to_do))) break;
         for (uint32_t s = sm.rank; s < n; s += sm.size) sum_row<BF16, VEC>(s);
-        if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+        // Which phases are still to come is known to all CTAs alike (nothing has been counted since the barrier), and what follows
+        // the last of them needs no barrier.
         if (l.score) {
-            if (l.out_full) region_phase<BF16, VEC, WP_FULL>(n);
+            if (l.out_full && !(ok = region_phase<BF16, VEC, WP_FULL>(n, c0, to_do))) break;
         } else {
-            if (*(volatile uint32_t*)(l.sync + 2)) {   // (the same for all CTAs)
+            uint32_t totals = *(volatile uint32_t*)(l.sync + 3);
+            n_left = *(volatile uint32_t*)l.left_count;
+            if (*(volatile uint32_t*)(l.sync + 2)) {
+                if (!(ok = grid_sync(sm, l, to_do))) break;
                 hist_phase<BF16, VEC>(n);
-                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+                if (!(ok = grid_sync(sm, l, to_do))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) select_row(s);
-                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
-                region_phase<BF16, VEC, WP_LIST>(n);
-                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+                if (!(ok = region_phase<BF16, VEC, WP_LIST>(n, c0, to_do))) break;
+                if (!(ok = grid_sync(sm, l, to_do))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) choose_row(s);
-                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+                if (!(ok = grid_sync(sm, l, to_do))) break;
+                totals = *(volatile uint32_t*)(l.sync + 3);
+                n_left = *(volatile uint32_t*)l.left_count;
             }
-            if (*(volatile uint32_t*)(l.sync + 3)) {
-                region_phase<BF16, VEC, WP_TOTAL>(n);
-                if (!(ok = grid_sync(sm, l, n_work - c0))) break;
+            if (totals) {
+                if (!(ok = region_phase<BF16, VEC, WP_TOTAL>(n, c0, to_do))) break;
+                if (!(ok = grid_sync(sm, l, to_do))) break;
                 for (uint32_t s = sm.rank; s < n; s += sm.size) total_row<BF16, VEC>(s);
             }
         }
-        if (!(ok = grid_sync(sm, l, n_work - c0))) break;   // the chunk's workspace is free
+        if ((to_do > n || n_left) && !(ok = grid_sync(sm, l, to_do))) break;   // the chunk's workspace is free
     }
-    if (ok && !l.score) rows_one_cta_each(sm.rank, min(slots, sm.size), *(volatile uint32_t*)l.left_count, l.left_rows);
+    if (ok && n_left) rows_one_cta_each(sm.rank, min(slots, sm.size), n_left, l.left_rows);
     // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();
     if (tid == 0) {

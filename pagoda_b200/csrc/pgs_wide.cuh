@@ -28,7 +28,7 @@ struct WideRow {
     uint32_t nonfinite;      // set by the first pass
     uint32_t state;          // WS_*
     float m, S, total;
-    uint32_t amax;
+    uint32_t amax, max_region;   // max_region: the first region that holds the maximum
     uint32_t cut, n_list;    // entries in buckets >= cut
     float cut_x;             // rows with a short top-k: the second pass lists the logits from here on (n_list of them)
     uint32_t n_terms;        // segments whose terms are in WideLaunch::terms
@@ -49,7 +49,7 @@ struct WideLaunch {
     uint32_t* rs;               // [chunk][n_regions + 1]
     uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
     unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
-    uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows selecting, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
+    uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows that select by the histogram, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
     // combinations of kinds (pgs_kinds.cuh) that are done by one CTA per row, here ([0]: at most a chunk of rows, [1]: more)
     // or by the general kernel in front of this one
     uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
