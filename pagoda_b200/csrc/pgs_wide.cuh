@@ -53,6 +53,7 @@ struct WideLaunch {
     // combinations of kinds (pgs_kinds.cuh) that are done by one CTA per row, here ([0]: at most a chunk of rows, [1]: more)
     // or by the general kernel in front of this one
     uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
+    uint32_t early;             // the kernel behind may be set up from the start
     uint32_t polls;             // limit of a barrier's wait
     unsigned long long* gave_up; // rows that ended without results because one ran out
     uint32_t chunk;             // rows that the workspace holds (<= W_CHUNK): the launch takes that many at a time
