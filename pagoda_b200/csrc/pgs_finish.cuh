@@ -286,10 +286,10 @@ __device__ __forceinline__ void cta_sort_shared(unsigned long long* keys, uint32
     __syncthreads();
 }
 
-// Total and inverse-CDF pick of the n entries in f.sid / f.sp (id order), and the row's outputs; one warp.
+// Total and inverse-CDF pick of the n entries in f.sid / f.sp (id order; kept_n of them above zero), and the row's outputs; one warp.
 template <class FA>
-__device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, float m, float S, float u01, uint32_t amax,
-                                            int status) {
+__device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t row, uint32_t V, uint32_t n, uint32_t kept_n, float m, float S, float u01,
+                                            uint32_t amax, int status) {
     const int lane = threadIdx.x & 31;
     const bool runs = n > F_SERIAL;
     const float total = runs ? warp_fold(f.sp, n, INFINITY, f.fp) : warp_prefix(f.sp, (int)n, f.fp);
@@ -309,8 +309,9 @@ __device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t ro
         if (a.row_max) a.row_max[row] = m;
         if (a.sumexp) a.sumexp[row] = S;
         if (a.total) a.total[row] = total;
+        if (a.n_kept) a.n_kept[row] = kept_n;
     }
-    if (a.n_kept || a.dump_ids || a.dump_probs) {   // diagnostics: the kept set in id order
+    if (a.dump_ids || a.dump_probs) {   // diagnostics: the kept set in id order
         uint32_t done = 0;
         for (uint32_t base = 0; base < n; base += 32) {
             const uint32_t j = base + lane;
@@ -323,7 +324,6 @@ __device__ __forceinline__ void warp_finish(FA& f, const RowArgs& a, uint32_t ro
             }
             done += __popc(mask);
         }
-        if (lane == 0 && a.n_kept) a.n_kept[row] = done;
     }
 }
 
@@ -355,7 +355,7 @@ __device__ __forceinline__ void cta_finish_ranked(FA& f, const RowArgs& a, uint3
     const uint32_t keep = warp_top_p(f.rp, n_live, top_p, f.fp);
     for (uint32_t j = keep + lane; j < n; j += 32) f.sp[f.rpos[j]] = 0.0f;
     __syncwarp();
-    warp_finish(f, a, row, V, n, m, S, u01, amax, status);
+    warp_finish(f, a, row, V, n, keep, m, S, u01, amax, status);
 }
 
 // Candidates of one row -> token.  Called by every thread of a CTA of T threads (a multiple of 32)
@@ -428,7 +428,7 @@ __device__ __forceinline__ void cta_finish_probs(FA& f, const RowArgs& a, uint32
             for (uint32_t r = tid; r < keep; r += T) { f.sid[r] = (uint32_t)(f.key[r] >> 32); f.sp[r] = u2f((uint32_t)f.key[r]); }
             __syncthreads();
         }
-        if (tid < 32) warp_finish(f, a, row, V, keep, m, S, u01, amax, status);
+        if (tid < 32) warp_finish(f, a, row, V, keep, keep, m, S, u01, amax, status);
         return;
     }
     cta_finish_ranked<T, FA>(f, a, row, V, n, m, S, top_k, top_p, u01, amax, status);

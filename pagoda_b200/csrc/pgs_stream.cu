@@ -89,6 +89,7 @@ struct PassArgs {
     const uint32_t* mw;     // rows beyond S_SHORT_VOCAB: the grammar mask
     float sc, sc_lo, c_hi, c_lo, cut_f, freq, pres, rep;
     uint32_t V, n_full, n_regions, flags;
+    uint32_t few;           // pass 2 meets few candidates (see few_candidates)
     // a row shared by the CTAs of a cluster: this CTA works on the pieces q0, q0 + qstep, ...; the candidates of all of
     // them are collected by the first CTA (pointers into its shared memory)
     uint32_t q0, qstep;
@@ -502,6 +503,18 @@ __device__ __forceinline__ void add_candidate(SM& sm, uint32_t id, float x) {
     (CL ? sm.pa.cand_x_p : sm.cand_x)[at] = x;
 }
 
+// x[j], four selections deep
+__device__ __forceinline__ float pick(const float (&x)[S_EPT], uint32_t j) {
+    float a[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) a[u] = (j & 1u) ? x[2 * u + 1] : x[2 * u];
+#pragma unroll
+    for (int u = 0; u < 4; u++) a[u] = (j & 2u) ? a[2 * u + 1] : a[2 * u];
+#pragma unroll
+    for (int u = 0; u < 2; u++) a[u] = (j & 4u) ? a[2 * u + 1] : a[2 * u];
+    return (j & 8u) ? a[1] : a[0];
+}
+
 // the logarithm (base 2) of a numerator
 template <bool BF16>
 __device__ __forceinline__ float exponent_of(const PassArgs& pa, float x) {
@@ -528,6 +541,14 @@ __device__ __forceinline__ void p2_entries(SM& sm, uint32_t n_ent) {
     if ((threadIdx.x & 31u) == 0u) sm.wacc[threadIdx.x >> 5] += td;
 }
 
+// How pass 2 puts candidates on the list, for f32 rows that a cluster shares: in rounds over the lanes where there are few, in
+// rounds over the sixteen positions of a lane's logits where there are many.  Over the lanes / over the positions, us: 8 rows of
+// 151936 with top-k 40 27.0 / 28.5, 64 with 50 37.9 / 38.5, 64 with 500 49.4 / 50.3, 64 with 1024 68.7 / 68.0.  (One CTA per row, and
+// bf16 rows: over the positions.  Some rows with long lists take half as long again over the lanes, 256 with top-k 500 92 / 80, and
+// both ways in one kernel cost all others 1 %.)
+template <bool BF16, bool CL>
+__device__ __forceinline__ bool few_candidates(uint32_t top_k) { return CL && !BF16 && top_k <= 512u; }
+
 // pass 2 on one piece
 template <bool BF16, bool BITS, bool TAIL, bool CL, class SM>
 __device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t q, FoldAcc& fa) {
@@ -541,9 +562,20 @@ __device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
     const float pm = max_ept(x);
     if (pm >= cut_f) {
         const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
+        if (CL && !BF16 && sm.pa.few) {   // as many rounds as the lane with the most candidates has
+            uint32_t which = 0u;
 #pragma unroll
-        for (int j = 0; j < S_EPT; j++)
-            if (x[j] >= cut_f) add_candidate<CL>(sm, elem_id<BF16>(e0, j), x[j]);
+            for (int j = 0; j < S_EPT; j++) which |= x[j] >= cut_f ? 1u << j : 0u;
+#pragma unroll 1
+            for (; which; which &= which - 1u) {
+                const int j = __ffs((int)which) - 1;
+                add_candidate<CL>(sm, elem_id<BF16>(e0, j), pick(x, (uint32_t)j));
+            }
+        } else {   // one for each of the sixteen positions at which some lane has one
+#pragma unroll
+            for (int j = 0; j < S_EPT; j++)
+                if (x[j] >= cut_f) add_candidate<CL>(sm, elem_id<BF16>(e0, j), x[j]);
+        }
     }
     const uint32_t region = q * SNW + (uint32_t)w;
     if (TAIL && region >= sm.pa.n_regions) return;   // warp-uniform: past the end of the row
@@ -804,7 +836,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         if (tid == 0) {   // what the pass loops read
             PassArgs& pa = sm.pa;
             pa.rowp = rowp; pa.mw = ctl.mw; pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
-            pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions;
+            pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions; pa.few = few_candidates<BF16, CL>(top_k);
             pa.q0 = crank; pa.qstep = csize;
             pa.cand_n_p = &sm.cand_n; pa.cand_id_p = sm.cand_id; pa.cand_x_p = sm.cand_x;
             if (CL) {
