@@ -1015,6 +1015,16 @@ __device__ __noinline__ void sum_row(uint32_t slot) {
     row_out(sm, l, slot);
 }
 
+// The lowest bucket that is counted.  Top-p alone ends where what lies above amounts to top_p (by the lower ends of the buckets,
+// 2^-8 below the probabilities at most, and with the margin of select_row); all V logits below the bucket together are less than
+// what is then left.  A row for which that does not hold, as its sum is not that of its terms, is left to the general kernel.
+// (32 rows of 151936 with top-p 0.95: a quarter of the logits are counted.)
+__device__ __forceinline__ uint32_t lowest_bucket(const WideRow& c, uint32_t V) {
+    if ((c.top_k != 0u && c.top_k < V) || c.top_p >= 1.0f) return 0u;
+    const float left = 0.999f * (1.0f - c.top_p * 1.002f / 0.99609375f);   // (the probabilities' own sum is 1 to within 1e-3)
+    return left > 0.001f ? bucket_of((left - 0.001f) / (float)V) : 0u;
+}
+
 // The lowest bucket that can matter: the one with the k-th largest probability, or the one in which the top-p fold ends (a
 // lower bound of the mass above it exceeds top-p by more than the fold can lose).  List positions for the buckets above.
 __device__ __noinline__ void select_row(uint32_t slot) {
@@ -1070,7 +1080,12 @@ __device__ __noinline__ void select_row(uint32_t slot) {
         }
     }
     __syncthreads();
-    const uint32_t cut = umax(sm.last, sm.found);
+    const uint32_t cut = umax(sm.last, sm.found), low = lowest_bucket(sm.row, V);
+    if (cut < low) {   // CTA-uniform: what is counted does not come to top-p (a sum far from that of its terms)
+        if (tid == 0) { wleave(l, sm.row.row); sm.row.state = WS_DONE; }
+        row_out(sm, l, slot);
+        return;
+    }
     {
         uint32_t above = before;
 #pragma unroll
@@ -1124,6 +1139,17 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
         row_out(sm, l, slot);
         return;
     }
+    // the entries of the list, four of a thread under way at once (one trip to L2 after the other took 20 us for 14000 entries)
+    const auto each = [&](auto what) {
+#pragma unroll 1
+        for (uint32_t j0 = tid; j0 < n; j0 += 4u * W_NT) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = j0 + u * W_NT < n ? __ldcg(list + j0 + u * W_NT) : 0ull;
+#pragma unroll
+            for (int u = 0; u < 4; u++) if (j0 + u * W_NT < n) what(u2f((uint32_t)(v[u] >> 32)), (uint32_t)v[u]);
+        }
+    };
     const uint32_t* hist = l.hist + (size_t)slot * W_BUCKETS;   // where bucket b ends in the list; it begins where b + 1 ends
     float thr_k = 0.0f;
     bool leave = false;
@@ -1147,10 +1173,15 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
         __syncthreads();
         for (uint32_t b = cut + tid; b < (uint32_t)W_BUCKETS; b += W_NT) { sm.bn[b] = 0u; sm.bs[b] = 0.0f; }
         __syncthreads();
-        for (uint32_t j = tid; j < n; j += W_NT) {
-            const float p = u2f((uint32_t)(__ldcg(list + j) >> 32));
-            if (p >= thr_k) atomicAdd(&sm.bs[bucket_of(p)], p);
-        }
+        // (the entries of a bucket share their upper bits: their sum is their number and the sum of the 15 lower bits, whole numbers,
+        // which shared memory adds faster than floats)
+        uint32_t* lower = reinterpret_cast<uint32_t*>(sm.bs);
+        each([&](float p, uint32_t) {
+            if (!(p >= thr_k)) return;
+            const uint32_t b = bucket_of(p);
+            atomicAdd(&sm.bn[b], 1u);
+            atomicAdd(&lower[b], f2u(p) & 0x7fffu);
+        });
         __syncthreads();
         {   // plain sums -> the binade of the running value at each bucket
             constexpr int PER = (W_BUCKETS + W_NT - 1) / W_NT;
@@ -1158,7 +1189,12 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
 #pragma unroll
             for (int u = 0; u < PER; u++) {
                 const int b = W_BUCKETS - 1 - (int)(tid * PER) - u;
-                P[u] = b >= (int)cut ? sm.bs[b] : 0.0f;
+                P[u] = 0.0f;
+                if (b >= (int)cut && sm.bn[b]) {   // (bucket 0: of no account)
+                    const float floor_b = bucket_floor(b);
+                    P[u] = (float)sm.bn[b] * floor_b + (float)lower[b] * (u2f(binade(floor_b)) * 1.1920928955078125e-07f);
+                    sm.bn[b] = 0u;
+                }
                 own += P[u];
             }
             float all;
@@ -1171,65 +1207,123 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
             }
         }
         __syncthreads();
-        for (uint32_t j = tid; j < n; j += W_NT) {
-            const float p = u2f((uint32_t)(__ldcg(list + j) >> 32));
-            if (!(p >= thr_k)) continue;
+        each([&](float p, uint32_t) {
+            if (!(p >= thr_k)) return;
             const uint32_t b = bucket_of(p), kb = f2u(sm.bs[b]);
-            if (kb == 0u) { sm.bn[b] = f2u(p); continue; }   // (of use where the bucket has one entry)
+            if (kb == 0u) { sm.bn[b] = f2u(p); return; }   // (of use where the bucket has one entry)
             const uint32_t i0 = f2u(fadd(u2f(kb), p)) - kb, i1 = f2u(fadd(u2f(kb + 1u), p)) - (kb + 1u);
             if (i0 != i1 || !(p < u2f(kb))) { sm.bs[b] = 0.0f; sm.bn[b] = f2u(p); }   // to be added one by one
             else atomicAdd(&sm.bn[b], i0);
-        }
-        // the fold over the buckets, highest first: warp 0 adds whole buckets until it meets one that is not, or the one in
-        // which top-p is reached; the CTA sorts that bucket and warp 0 adds its entries in order
+        });
+        // The fold over the buckets, highest first, by events as in resolve: a run of buckets of one binade is one addition; a
+        // bucket with several entries that the running value may change binade in, and the one in which top-p is reached, is
+        // sorted by the CTA and its entries are added in order.  (Over the buckets 256 at a time the walk took 27 us a row.)
         uint32_t* ends = reinterpret_cast<uint32_t*>(&sm.stage[0][0]);   // where a bucket ends in the list
-        static_assert(sizeof(sm.stage) >= W_BUCKETS * 4, "one word per bucket");
+        unsigned long long* ev_sum = reinterpret_cast<unsigned long long*>(ends + W_BUCKETS);
+        uint32_t* ev = sm.serial;   // the bucket an event begins with
+        static_assert(sizeof(sm.stage) >= W_BUCKETS * 4 + (W_MAX_REGIONS + 1) * 8 && W_BUCKETS % 2 == 0, "one word per bucket, the events' sums");
         for (uint32_t b = cut + tid; b < (uint32_t)W_BUCKETS; b += W_NT) ends[b] = __ldcg(hist + b);
+        __syncthreads();
+        constexpr int PER = (W_BUCKETS + W_NT - 1) / W_NT;
+        constexpr uint32_t EV_MASK = 0x3fffu;   // events in the lower bits of a sum, increments above
+        static_assert(W_BUCKETS <= 0x3fff, "packed counts");
+        unsigned long long all, before;
+        uint32_t is_event = 0u;   // bit u: this thread's bucket u
+        const auto bucket = [&](int u) { return W_BUCKETS - 1 - (int)(tid * PER) - u; };
+        const auto increment_in = [&](int bb) { return f2u(sm.bs[bb]) ? (unsigned long long)min(sm.bn[bb], 0x01000000u) : 0ull; };   // (2^23 is too much already)
+        const auto empty = [&](int bb) { return bb < (int)cut || ends[bb] == (bb + 1 < W_BUCKETS ? ends[bb + 1] : 0u); };
+        {
+            uint32_t last_y = W_NIL;   // of the thread's buckets that are not empty
+            unsigned long long own = 0ull;
+            for (int u = 0; u < PER; u++) if (!empty(bucket(u))) last_y = f2u(sm.bs[bucket(u)]);
+            const unsigned some = __ballot_sync(FULL, last_y != W_NIL) & ((1u << lane) - 1u);
+            const uint32_t from = __shfl_sync(FULL, last_y, some ? 31 - __clz((int)some) : 0);
+            uint32_t yp = some ? from : W_NIL;   // (an event at the start of every warp's buckets)
+            for (int u = 0; u < PER; u++) {
+                const int bb = bucket(u);
+                if (empty(bb)) continue;
+                const uint32_t y = f2u(sm.bs[bb]);
+                if (y == 0u || y != yp) { is_event |= 1u << u; own++; }
+                own += increment_in(bb) << 14;
+                yp = y;
+            }
+            unsigned long long inc = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= (uint32_t)o) inc += t;
+            }
+            if (lane == 31) sm.red_w[w] = inc;
+            __syncthreads();
+            before = sm.red_w[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(FULL, before, o);
+                if (lane >= (uint32_t)o) before += t;
+            }
+            all = __shfl_sync(FULL, before, 31);
+            before = __shfl_sync(FULL, before, (int)(w + 31u) & 31);
+            before = (w ? before : 0ull) + inc - own;
+        }
+        const uint32_t n_ev = (uint32_t)all & EV_MASK;
+        leave = n_ev > (uint32_t)W_MAX_REGIONS;   // CTA-uniform
+        if (!leave) {
+            unsigned long long at = before;
+            for (int u = 0; u < PER; u++) {
+                const int bb = bucket(u);
+                if (empty(bb)) continue;
+                if ((is_event >> u) & 1u) { ev[(uint32_t)at & EV_MASK] = (uint32_t)bb; ev_sum[(uint32_t)at & EV_MASK] = at >> 14; at++; }
+                at += increment_in(bb) << 14;
+            }
+            if (tid == 0) ev_sum[n_ev] = all >> 14;
+        }
         float R = 0.0f;                              // warp 0
-        int b = W_BUCKETS - 1;
+        uint32_t e = 0u;
         bool found = false;
-        for (;;) {
+        while (!leave) {
             __syncthreads();
             if (w == 0) {
-                // (eight buckets per lane, one where that does not do)
-                for (int per = 8; b >= (int)cut;) {
-                    uint32_t own = 0u, kb = 1u;
-                    for (int u = 0; u < per; u++) {
-                        const int mine = b - (int)lane * per - u;
-                        if (mine < (int)cut || ends[mine] == (mine + 1 < W_BUCKETS ? ends[mine + 1] : 0u)) continue;   // empty
-                        const uint32_t k1 = f2u(sm.bs[mine]);
-                        kb = kb == 1u || kb == k1 ? k1 : 0u;
-                        own += sm.bn[mine];
+                uint32_t need = W_NIL, in_run = 0u;
+#pragma unroll 1
+                for (; e < n_ev && need == W_NIL; e++) {
+                    const uint32_t b = ev[e], k = f2u(sm.bs[b]), rb = f2u(R);
+                    if (k == 0u) {   // (a single entry that does not reach top-p needs no sort)
+                        const float R1 = fadd(R, u2f(sm.bn[b]));
+                        if (ends[b] - (b + 1u < (uint32_t)W_BUCKETS ? ends[b + 1u] : 0u) == 1u && R1 < sm.row.top_p) R = R1; else need = b;
+                    } else {
+                        const unsigned long long run = ev_sum[e + 1u] - ev_sum[e];
+                        if ((rb & 0x7f800000u) != k || run >= 0x00800000u - (rb & 0x007fffffu)) { need = b; in_run = 2u; }   // not as estimated
+                        else if (u2f(rb + (uint32_t)run) >= sm.row.top_p) { need = b; in_run = 1u; }
+                        else R = u2f(rb + (uint32_t)run);
                     }
-                    const bool empty = kb == 1u;
-                    const uint32_t rb = f2u(R);
-                    uint32_t inc = own;
-                    const unsigned bad = __ballot_sync(FULL, !(empty || (kb != 0u && kb == (rb & 0x7f800000u))));
-                    uint32_t cnt = bad ? __ffs((int)bad) - 1u : 32u;
-                    if (lane >= cnt) inc = 0u;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t t = __shfl_up_sync(FULL, inc, o);
-                        if (lane >= (uint32_t)o) inc += t;
-                    }
-                    // (the running value only grows: it reaches top-p in the first bucket behind which it has)
-                    const unsigned over = __ballot_sync(FULL, !empty && lane < cnt && ((rb & 0x007fffffu) + inc >= 0x00800000u || (own != 0u && u2f(rb + inc) >= sm.row.top_p)));
-                    if (over) cnt = min(cnt, (uint32_t)__ffs((int)over) - 1u);
-                    if (cnt) R = u2f(rb + __shfl_sync(FULL, inc, (int)cnt - 1));
-                    b -= (int)cnt * per;
-                    if (cnt == 32u) { per = 8; continue; }
-                    if (per == 8) { per = 1; continue; }
-                    // a bucket to be added one by one; a single entry that does not reach top-p needs no sort for that
-                    const uint32_t n1 = ends[b] - (b + 1 < W_BUCKETS ? ends[b + 1] : 0u);
-                    const float R1 = fadd(R, u2f(sm.bn[b]));
-                    if (n1 != 1u || sm.bs[b] != 0.0f || R1 >= sm.row.top_p) break;
-                    R = R1;
-                    b--;
-                    per = 8;
                 }
-                if (lane == 0) sm.last = b >= (int)cut ? (uint32_t)b : W_NIL;
+                if (lane == 0) { sm.last = need; sm.n_ev = in_run; sm.at_ev = e - 1u; sm.R = R; sm.found = 0u; }
             }
             __syncthreads();
+            if (sm.n_ev == 2u) { leave = true; break; }
+            if (sm.n_ev == 1u) {   // top-p is reached in this run: in its first bucket behind which the running value has come to it
+                const uint32_t rb = f2u(sm.R);
+                const unsigned long long base = ev_sum[sm.at_ev];
+                unsigned long long at = before;
+                for (int u = 0; u < PER; u++) {
+                    const int bb = bucket(u);
+                    if (empty(bb)) continue;
+                    const uint32_t i = ((uint32_t)at & EV_MASK) + ((is_event >> u) & 1u) - 1u;   // the event that the bucket belongs to
+                    at += (increment_in(bb) << 14) + ((is_event >> u) & 1u);
+                    if (i == sm.at_ev && u2f(rb + (uint32_t)((at >> 14) - base)) >= sm.row.top_p) atomicMax(&sm.found, (uint32_t)bb + 1u);
+                }
+                __syncthreads();
+                const uint32_t fb = sm.found - 1u;
+                at = before;
+                for (int u = 0; u < PER; u++) {   // the running value in front of it
+                    const int bb = bucket(u);
+                    if (empty(bb)) continue;
+                    if ((uint32_t)bb == fb) { sm.R = u2f(rb + (uint32_t)((at >> 14) - base)); sm.last = fb; }
+                    at += (increment_in(bb) << 14) + ((is_event >> u) & 1u);
+                }
+                __syncthreads();
+                R = sm.R;
+            }
             const uint32_t sb = sm.last;
             if (sb == W_NIL) break;
             const uint32_t end = ends[sb], at = sb + 1u < (uint32_t)W_BUCKETS ? ends[sb + 1u] : 0u, nb = end - at;
@@ -1270,7 +1364,6 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
                 n_kept = at + sm.found + 1u;
                 break;
             }
-            b--;
         }
         // top-p was not reached although the list ends where it should have been: the list is too short for this row
         if (!found && !leave && cut != 0u && !k_ends) leave = true;
@@ -1283,11 +1376,7 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
     }
     for (uint32_t r = tid; r < n_regions; r += W_NT) sm.start[r] = 0.0f;
     __syncthreads();
-    for (uint32_t j = tid; j < n; j += W_NT) {
-        const unsigned long long v = __ldcg(list + j);
-        const float p = u2f((uint32_t)(v >> 32));
-        if (p > p_thr || (p == p_thr && (uint32_t)v <= id_thr)) atomicAdd(&sm.start[(uint32_t)v / W_REGION], p);
-    }
+    each([&](float p, uint32_t id) { if (p > p_thr || (p == p_thr && id <= id_thr)) atomicAdd(&sm.start[id / W_REGION], p); });
     __syncthreads();
     make_table(sm, l, slot, n_regions, 0.001953125f, [&](uint32_t r) { return sm.start[r]; });
     if (tid == 0) {
@@ -1597,6 +1686,8 @@ __device__ __noinline__ void hist_phase(uint32_t n_rows) {
         f.m = c.m; f.t = c.t; f.S = c.S; f.filter = false; f.p_thr = 0.0f; f.id_thr = 0u;
         const Approx q = approx_of(f);
         const float eps = (4.0f * fabsf(q.k0) + 200.0f) * 2.4e-7f;   // (probabilities from 2^-40 on count)
+        const uint32_t low = lowest_bucket(c, V);
+        const float low_p = low ? bucket_floor(low) * (1.0f - 2.0f * eps) : -1.0f;
         for (uint32_t r = r0 + w; r < r1; r += WNW) {
             const uint32_t nv = min(V - r * W_REGION, (uint32_t)W_REGION);
             float x[WL];
@@ -1606,8 +1697,10 @@ __device__ __noinline__ void hist_phase(uint32_t n_rows) {
 #pragma unroll
             for (int j = 0; j < WL; j++) {
                 float p = ex2_approx_ftz(__fmaf_rn(fsub(x[j], f.m), q.c, q.k0));
+                if (p < low_p) continue;
                 if (x[j] > -INFINITY && (bucket_of(p * (1.0f - eps)) != bucket_of(p * (1.0f + eps)) || p < 1e-30f)) p = term_of(x[j], 0u, f, sm.exp_tab);
-                if (p > 0.0f) atomicAdd(&sm.bn[bucket_of(p)], 1u);
+                const uint32_t b = bucket_of(p);
+                if (p > 0.0f && b >= low) atomicAdd(&sm.bn[b], 1u);
             }
         }
         __syncthreads();
