@@ -88,7 +88,7 @@ struct pgs_handle {
     uint32_t score_calls = 0;         // how many there were
     unsigned long long score_stream = 0;   // id of the last one's stream
     uint32_t wide_vocab = 0;          // longest row the workspace holds
-    int wide_route = 0;               // 1: always the grid, 2: always one CTA per row (tests)
+    int wide_route = 0;               // tests: 1 always the grid, 2 always the general kernel, 3 always the wide kernel's CTA per row
     // streaming row kernel: id -> count slots, shared memory and CTAs per SM, the gate's counter
     uint32_t stream_hash = 0, stream_cohort = 0;
     int max_clusters[4] = {0, 0, 0, 0};   // resident clusters of 1 (unused), 2, 4, 8 CTAs of the row kernel
@@ -161,17 +161,18 @@ int wide_workspace(pgs_handle* h) {
         used = 0;
         WideLaunch* const both[2] = {&h->wide, &h->score_wide};
         for (WideLaunch* l : both) { l->sync = (uint32_t*)take(64); l->left_count = (uint32_t*)take(4); }
+        h->wide.own = (uint32_t*)take((size_t)h->slots * W_OWN * 4);
         zeroed = used;
         for (WideLaunch* l : both) {
-            const size_t rows = l == &h->score_wide || h->slots >= (uint32_t)W_CHUNK ? W_CHUNK : h->slots;
-            l->chunk = (uint32_t)rows; l->reg_stride = regions; l->rs_stride = regions + 1u;
+            const size_t rows = l == &h->score_wide ? W_CHUNK : h->slots;   // (one CTA per row: as many as there are scratch slots)
+            l->chunk = rows < W_CHUNK ? (uint32_t)rows : W_CHUNK; l->reg_stride = regions; l->rs_stride = regions + 1u;
             l->row = (WideRow*)take(rows * sizeof(WideRow)); l->reg = (float2*)take(rows * regions * sizeof(float2));
             l->cell = (float4*)take(rows * regions * sizeof(float4)); l->seg = (uint2*)take(rows * regions * sizeof(uint2));
             l->pre = (float*)take(rows * regions * 4); l->terms = (float*)take(rows * (size_t)W_TERMS * W_REGION * 4);
         }
         // steps only
         WideLaunch& l = h->wide;
-        const size_t rows = l.chunk;
+        const size_t rows = h->slots;
         l.left_rows = (uint32_t*)take((size_t)h->max_rows * 4); l.rs = (uint32_t*)take(rows * (regions + 1u) * 4);
         l.ent_id = (uint32_t*)take(rows * (W_MAX_HIST + 32) * 4); l.ent_xn = (float*)take(rows * (W_MAX_HIST + 32) * 4);
         l.hist = (uint32_t*)take(rows * W_BUCKETS * 4);
@@ -233,11 +234,25 @@ bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool
 
 // The combinations of kinds that one CTA per row does quicker (*row), and those that the grid does (returned), among those
 // that the handle's rows can have.
-uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row) {
+uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row, bool by_rows = false) {
     using namespace pgs;
     const uint32_t possible = h->max_history > (uint32_t)W_MAX_HIST ? WK_POSSIBLE : WK_SHORT;
-    *row = h->wide_route == 1 ? 0u : h->wide_route == 2 ? possible : kinds_one_cta_each(possible, rows, h->wide.chunk, h->slots, vocab);
+    *row = h->wide_route == 1 || h->wide_route == 3 ? 0u : h->wide_route == 2 ? possible : kinds_one_cta_each(possible, rows, h->wide.chunk, h->slots, vocab, by_rows);
     return possible & ~*row;
+}
+
+// Whether the wide kernel takes an exact or unaligned batch one CTA per row, as many at a time as there are SMs, and not with the
+// whole grid on 64 rows at a time: without grid barriers, but with a row's regions on one SM.  Lines through what sampled rows take
+// (us, CTA per row / grid): 1 x 16384 41 / 46, 16 x 50256 53 / 47, 64 x 16384 40 / 48, 64 x 50256 56 / 58, 64 x 100000 70 / 64,
+// 64 x 151936 96 / 88, 48 x 50257 with histories 63 / 59, 148 x 4096 56 / 240, 148 x 50256 59 / 153, 148 x 151936 118 / 226, 256 x 50256 111 / 225, 256 x 151936
+// 187 / 316; without top-k and with top-p 0.9 16 x 16384 65 / 105, 64 x 16384 70 / 126, 256 x 50256 191 / 619; greedy 64 x 50256 21 / 28.
+bool wide_row_by_row(const pgs_handle* h, uint32_t rows, uint32_t vocab) {
+    if (h->wide_route) return h->wide_route == 3;
+    const uint32_t chunk = h->wide.chunk, slots = h->slots;
+    const double v = 1e-6 * vocab;
+    const double by_rows = ((rows - 1u) / slots + 1u) * (36.0 + 400.0 * v + 1.2 * v * (rows < slots ? rows : slots));
+    const double grid = ((rows - 1u) / chunk + 1u) * (44.0 + 4.4 * v * (rows < chunk ? rows : chunk));
+    return by_rows < grid;
 }
 
 // CTAs of the wide kernel for `rows` rows: one per SM, fewer where a CTA would get less than a handful of regions (its grid
@@ -462,7 +477,8 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         // the one whose batch it is not returns at once.
         pgs::WideLaunch wl = h->wide;
         uint32_t grid_kinds = 0u;
-        if (wide) grid_kinds = kinds_for(h, rows, a.vocab, &wl.kinds_front);
+        wl.local = wide && wide_row_by_row(h, rows, a.vocab);
+        if (wide) grid_kinds = kinds_for(h, rows, a.vocab, &wl.kinds_front, wl.local != 0u);
         wl.look = wl.kinds_front;
         if (!wide || !grid_kinds || wl.kinds_front) {
             pgs::RowArgs front = a;
@@ -473,7 +489,7 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         if (grid_kinds) {
             // (both fit on no SM together)
             const uint32_t want = wide_grid(h, rows, a.vocab), sms = (uint32_t)h->sm_count, room = wl.kinds_front && rows <= sms / 2u ? sms - rows : sms;
-            PGS_CUDA(h, pgs::launch_wide(a, wl, h->slots, want < room ? want : room, stream));
+            PGS_CUDA(h, pgs::launch_wide(a, wl, h->slots, wl.local ? grid : want < room ? want : room, stream));
             h->counters.kernel_launches += 1;
         }
         return PGS_OK;

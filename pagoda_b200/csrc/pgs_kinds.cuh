@@ -1,4 +1,4 @@
-// Which rows are done by the whole grid (pgs_wide.cu) and which by one CTA each (pgs_general.cuh).  Both give the same bits; the
+// Which rows are done by the wide kernel (pgs_wide.cu) and which by one CTA each of the general one (pgs_general.cuh).  Both give the same bits; the
 // choice is which is quicker for a batch, from what its rows ask for.
 #pragma once
 
@@ -43,7 +43,11 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 // 256 x 50256 64 / 126, 256 x 151936 217 / 166; no top-k 16 x 1000 59 / 68, 16 x 16384 160 / 91, with top-p 1 x 1000 76 / 71,
 // 16 x 4096 161 / 78.  Rows with a history beyond the workspace end on one CTA either way (4 of 50256: 187 at once, 239
 // behind the phases).
-inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V) {
+//
+// by_rows: the wide kernel takes a CTA per row itself (wide_row_by_row).  us of one row that way, as many at a time as there are
+// SMs: greedy 14 + 0.12 per thousand logits, sampled 36 + 0.3 (55 where the threshold needs the histogram), without top-k 58 + 0.55, with
+// a sort for top-p 60 + 1.
+inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool by_rows) {
     if (V <= 1024u) return of;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
     const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
@@ -58,7 +62,12 @@ inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint
             row = 9.0f + 3.7e-4f * v + 1.5e-6f * v * together;
             grid = 27.0f + 1.65f * m;
         }
-        if (waves * row < chunks * grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
+        if (by_rows) {
+            const float v3 = 1e-3f * v;
+            grid = waves * (!(kinds & WK_SAMPLED) ? 14.0f + 0.12f * v3 : kinds & WK_SORT ? 60.0f + v3 : kinds & WK_OPEN ? 58.0f + 0.55f * v3
+                            : (kinds & WK_HIST ? 55.0f : 36.0f) + 0.3f * v3);
+        } else grid *= chunks;
+        if (waves * row < grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
     }
     return mask;
 }

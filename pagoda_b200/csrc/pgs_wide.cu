@@ -17,10 +17,14 @@
 //   region  increments of the running total over the kept probabilities                  (what has no short list)
 //   row     total and inverse-CDF pick
 //
-// What bounds it: the folds change binade 8 to 16 times a row, and each change is about a microsecond of one warp; a grid
-// barrier is two; a region phase is the latency of one or two regions per warp (mask, history entries and logits are one trip
-// to L2 or HBM each) rather than bandwidth.  Against one CTA per row: 32 rows of 151936 without top-k 8312 -> 222 us, 16 rows
-// in exact mode 377 -> 74, 48 rows of 50257 360 -> 72, scoring of 64 rows 199 -> 82.
+// Batches of many rows, or of short ones, go through the same phases with one CTA per row and a CTA barrier where the grid has
+// its own (WideLaunch::local; the host chooses, wide_row_by_row): 148 exact rows of 50257 153 -> 59 us, 256 rows of 151936 316 -> 187.
+//
+// What bounds it: a row's fold is one warp's (8 us on average and 20 at most of a row of 151936: 500 cycles for each change of binade,
+// of which there are 8 to 16); a grid barrier is two microseconds; a region phase is the latency of one or two regions per
+// warp (mask, history entries and logits are one trip to L2 or HBM each) rather than bandwidth.  Against the general kernel's CTA per
+// row: 32 rows of 151936 without top-k 8312 -> 204 us, 16 rows in exact mode 377 -> 62, 48 rows of 50257 360 -> 59, scoring of 64
+// rows 199 -> 74.
 //
 // The fold (pagoda/src/sampler.rs:42, :99-113, :136-144): while the running value stays inside one binade, adding a
 // non-negative term is an integer addition in ulps which depends on the running value only where the term ends exactly on
@@ -130,6 +134,7 @@ __device__ __forceinline__ bool grid_join(WideSmem& sm, const WideLaunch& l) {
 // open: rows that have no result yet
 __device__ __forceinline__ bool grid_sync(WideSmem& sm, const WideLaunch& l, uint32_t open) {
     __syncthreads();
+    if (l.local) return true;   // one CTA per row: nobody else to wait for
     if (threadIdx.x == 0) {
         bool good = true;
         __threadfence();
@@ -1769,7 +1774,18 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass
     if (tid == 0) { sm.a = a_; sm.target = 0u; sm.gave_up = 0u; }
-    if (tid == 32u) sm.l = l_;
+    if (tid == 32u) {
+        sm.l = l_;
+        if (l_.local) {   // this CTA's part of the workspace
+            WideLaunch& o = sm.l;
+            const size_t at = blockIdx.x;
+            o.row += at; o.reg += at * o.reg_stride; o.cell += at * o.reg_stride; o.seg += at * o.reg_stride; o.pre += at * o.reg_stride;
+            o.terms += at * W_TERMS * W_REGION; o.ent_id += at * (W_MAX_HIST + 32); o.ent_xn += at * (W_MAX_HIST + 32); o.rs += at * o.rs_stride;
+            o.hist += at * W_BUCKETS; o.list += at * o.list_stride;
+            o.sync = o.own + at * W_OWN; o.left_count = o.sync + 8; o.left_rows = o.sync + 9;
+        }
+    }
+    if (l_.local && tid == 0) { sm.rank = 0u; sm.size = 1u; sm.target = 1u; }
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
     bool ok = true;   // (false for all CTAs, or none)
@@ -1777,10 +1793,11 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         ok = !look(n_work, slots);
         if (!ok && l_.kinds_front) return;
     }
-    ok = ok && grid_join(sm, l);
+    const bool local = l_.local != 0u;
+    ok = ok && (local || grid_join(sm, l));
     uint32_t n_left = 0u;   // rows left to the general kernel's code
-    for (uint32_t c0 = 0; c0 < n_work && ok; c0 += l.chunk) {
-        const uint32_t n = min(n_work - c0, l.chunk), to_do = n_work - c0;
+    for (uint32_t c0 = local ? blockIdx.x : 0u; c0 < n_work && ok; c0 += local ? gridDim.x : l.chunk) {
+        const uint32_t n = local ? 1u : min(n_work - c0, l.chunk), to_do = n_work - c0;
         const auto open = [&](uint32_t s) { open_row<BF16>(s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
         if (sm.rank == 0u && tid == 0) { l.sync[2] = 0u; l.sync[3] = 0u; }
         uint32_t s = sm.rank;
@@ -1822,7 +1839,13 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             }
         }
         if ((to_do > n || n_left) && !(ok = grid_sync(sm, l, to_do))) break;   // the chunk's workspace is free
+        if (local && n_left) {   // (the list has one entry; the scratch slot is this CTA's)
+            rows_one_cta_each(blockIdx.x, gridDim.x, blockIdx.x + 1u, l.left_rows - blockIdx.x);
+            __syncthreads();
+            if (tid == 0) *l.left_count = 0u;
+        }
     }
+    if (local) return;
     if (ok && n_left) rows_one_cta_each(sm.rank, min(slots, sm.size), n_left, l.left_rows);
     // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();

@@ -16,6 +16,7 @@ constexpr int W_CHUNK = 64;             // rows in flight together, at most
 constexpr int W_BUCKETS = 41 * 256;     // probabilities by exponent (2^-40 .. 1) and eight mantissa bits
 constexpr int W_TERMS = 64;             // segments of a row whose terms the region phase leaves for the fold
 constexpr int W_KMAX = 1024;            // top-k up to which the second pass lists the candidates
+constexpr int W_OWN = 16;               // words of WideLaunch::own
 constexpr int W_SORT = 4096;            // entries of a bucket that one CTA sorts
 
 // One row of the chunk.
@@ -53,6 +54,8 @@ struct WideLaunch {
     // combinations of kinds (pgs_kinds.cuh) that are done by one CTA per row, here ([0]: at most a chunk of rows, [1]: more)
     // or by the general kernel in front of this one
     uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
+    uint32_t local;             // one CTA per row, with the part of the workspace that has the CTA's number
+    uint32_t* own;              // [CTAs][W_OWN]: what `sync`, `left_count` and `left_rows` are for the grid
     uint32_t early;             // the kernel behind may be set up from the start
     uint32_t polls;             // limit of a barrier's wait
     unsigned long long* gave_up; // rows that ended without results because one ran out

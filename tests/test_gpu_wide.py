@@ -47,13 +47,14 @@ def test_wide_kernel_edges(oracle, rows, vocab, top_k, history):
 
 @pytest.mark.parametrize("vocab", [512 * 33, 512 * 40 + 3])
 @pytest.mark.parametrize("top_k", [0, 40])
-def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k):
+@pytest.mark.parametrize("route", ["1", "3"])
+def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k, route):
     """The exact fold where its running value changes binade often, in one run of terms, at the edge of a region, or not
     at all, and where terms end on half an ulp: bit-exact sums, totals, tokens and scores."""
     import torch
     import pagoda_b200
     from pagoda_b200 import synth
-    monkeypatch.setenv("PGS_WIDE_ROUTE", "1")   # on the grid, whatever is quicker
+    monkeypatch.setenv("PGS_WIDE_ROUTE", route)   # on the grid, or one CTA per row, whatever is quicker
     i = np.arange(vocab)
     rng = np.random.default_rng(vocab)
     noise = rng.standard_normal(vocab)
@@ -76,6 +77,34 @@ def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k):
                                    stream_ptr=torch.cuda.current_stream().cuda_stream)
         torch.cuda.synchronize()
         check_scores(oracle, x, ids, g, full)
+    finally:
+        s.close()
+
+
+@pytest.mark.parametrize("rows, vocab, top_k, history", [(1, 511, 0, 0), (160, 512, 40, 64), (149, 513, 0, 300), (5, 1025, 1025, 2049), (150, 9001, 30, 300),
+                                                         (9, 33025, 0, 300), (3, 70001, 2049, 2100)])
+def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
+    """The wide kernel with one CTA per row: one row, more rows than SMs, rows that go on to the general kernel's code
+    (more history than the workspace holds), short and long lists, a mask that leaves regions empty."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    monkeypatch.setenv("PGS_WIDE_ROUTE", "3")
+    x = synth.normal_f32(11 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    rng = np.random.default_rng(vocab)
+    words = np.full((2, (vocab + 31) // 32), 0xffffffff, np.uint32)
+    words[1, :words.shape[1] // 2] = 0
+    words[1, 0] = 1
+    w = synth.Workload(
+        "rows", x, np.resize(np.float32([0.7, 0.0, 1.3, 5.0]), rows), np.full(rows, top_k, np.uint32), np.resize(np.float32([0.95, 1.0, 0.3]), rows),
+        np.full(rows, 0.2, np.float32), np.full(rows, 0.1, np.float32), np.full(rows, 1.1, np.float32),
+        np.arange(rows + 1, dtype=np.uint32) * history if history else None,
+        rng.integers(0, vocab, rows * history).astype(np.uint32) if history else None, synth.uniform_f32(4, rows),
+        mask_words=words, state_flags=np.zeros(2, np.uint32), mask_state=np.resize(np.int32([-1, 0, 1, -1, 1]), rows))
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
+    try:
+        s.set_exact(True)
+        for _ in range(2):   # (the second time on what the first has left)
+            assert_same(*run_both(s, oracle, w), w)
     finally:
         s.close()
 
