@@ -148,8 +148,9 @@ uint32_t pow2_at_least(uint32_t v, uint32_t lo) {
 }  // namespace
 
 namespace {
-// The wide kernel's workspaces in one block of device memory.  Steps: W_CHUNK rows of the handle's vocabulary, or as many as
-// the handle has.  Scoring has its own, of W_CHUNK rows: it has no row limit, and is not ordered with the handle's steps.
+// The wide kernel's workspaces in one block of device memory.  Steps: as many rows of the handle's vocabulary as there are SMs, or
+// as the handle has (the grid takes W_CHUNK of them at a time).  Scoring has its own, of as many rows as SMs: it has no row
+// limit, and is not ordered with the handle's steps.
 int wide_workspace(pgs_handle* h) {
     using namespace pgs;
     const uint32_t vocab = h->max_vocab < (uint32_t)W_MAX_VOCAB ? h->max_vocab : (uint32_t)W_MAX_VOCAB;
@@ -161,10 +162,10 @@ int wide_workspace(pgs_handle* h) {
         used = 0;
         WideLaunch* const both[2] = {&h->wide, &h->score_wide};
         for (WideLaunch* l : both) { l->sync = (uint32_t*)take(64); l->left_count = (uint32_t*)take(4); }
-        h->wide.own = (uint32_t*)take((size_t)h->slots * W_OWN * 4);
+        h->wide.own = (uint32_t*)take((size_t)h->slots * W_OWN * 4); h->score_wide.own = (uint32_t*)take((size_t)h->sm_count * W_OWN * 4);
         zeroed = used;
         for (WideLaunch* l : both) {
-            const size_t rows = l == &h->score_wide ? W_CHUNK : h->slots;   // (one CTA per row: as many as there are scratch slots)
+            const size_t rows = l == &h->score_wide ? (uint32_t)h->sm_count : h->slots;   // (one CTA per row: as many as there are SMs)
             l->chunk = rows < W_CHUNK ? (uint32_t)rows : W_CHUNK; l->reg_stride = regions; l->rs_stride = regions + 1u;
             l->row = (WideRow*)take(rows * sizeof(WideRow)); l->reg = (float2*)take(rows * regions * sizeof(float2));
             l->cell = (float4*)take(rows * regions * sizeof(float4)); l->seg = (uint2*)take(rows * regions * sizeof(uint2));
@@ -218,18 +219,20 @@ bool score_workspace_free(const pgs_handle* h, cudaStream_t stream, unsigned lon
     return done || *id == h->score_stream;
 }
 
-// Whether the wide kernel scores a batch faster than one CTA per row does.  One CTA per row: 25 us and 1.2 us per thousand
-// logits (2 us with the whole vector written) for as many rows as there are SMs; wide: 38 us (47) and 4.3 us (10) per million
-// logits for every chunk.  Lines through (us, one CTA per row / wide): 64 x 1000 24 / 39, 64 x 4096 39 / 42, 64 x 16384
-// 53 / 48, 128 x 16384 53 / 85, 128 x 50257 96 / 103, 64 x 151936 199 / 80, 256 x 151936 407 / 307; whole vectors 64 x 1000
-// 25 / 47, 256 x 16384 117 / 205, 256 x 151936 640 / 566.
-bool wide_scores_faster(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool full) {
-    if (h->wide_route) return h->wide_route == 1;
+// How a batch is scored: by the kernel that needs no workspace, by the wide kernel's grid, or by its CTA per row.  Lines through
+// (us, without workspace / grid / CTA per row): 1 x 1000 21 / 38 / 41, 64 x 1000 25 / 42 / 33, 64 x 4096 37 / 44 / 36, 64 x 16384
+// 53 / 47 / 42, 148 x 16384 54 / 115 / 41, 16 x 50256 94 / 47 / 56, 64 x 50256 97 / 54 / 55, 256 x 50256 186 / 194 / 106, 64 x 151936
+// 201 / 80 / 86, 256 x 151936 407 / 274 / 174; whole vectors 64 x 1000 26 / 51 / 41, 64 x 16384 64 / 58 / 54, 64 x 50256 128 / 76 / 95,
+// 256 x 50256 256 / 285 / 196, 64 x 151936 305 / 149 / 201.
+enum ScoreRoute { SCORE_PLAIN, SCORE_GRID, SCORE_ROWS };
+ScoreRoute score_route(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool full) {
+    if (h->wide_route) return h->wide_route == 1 ? SCORE_GRID : h->wide_route == 2 ? SCORE_PLAIN : SCORE_ROWS;
     const uint32_t sms = (uint32_t)h->sm_count, chunk = h->score_wide.chunk;
-    const double logits = 1e-6 * (rows < chunk ? rows : chunk) * (double)vocab;
-    const double per_row = ((rows - 1u) / sms + 1u) * (25.0 + vocab / (full ? 500.0 : 850.0));
-    const double wide = ((rows - 1u) / chunk + 1u) * (full ? 47.0 + 10.0 * logits : 38.0 + 4.3 * logits);
-    return wide < per_row;
+    const double v = 1e-6 * vocab, waves = (rows - 1u) / sms + 1u, chunks = (rows - 1u) / chunk + 1u, in_chunk = rows < chunk ? rows : chunk;
+    const double plain = waves * (25.0 + v * (full ? 2000.0 : 1176.0));
+    const double grid = chunks * (full ? 53.0 + 10.0 * v * in_chunk : 43.0 + 3.8 * v * in_chunk);
+    const double by_rows = waves * ((full ? 40.0 + 960.0 * v : 34.0 + 330.0 * v) + 0.9 * v * (rows < sms ? rows : sms));
+    return plain <= grid && plain <= by_rows ? SCORE_PLAIN : grid <= by_rows ? SCORE_GRID : SCORE_ROWS;
 }
 
 // The combinations of kinds that one CTA per row does quicker (*row), and those that the grid does (returned), among those
@@ -524,6 +527,7 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         if (rows > l.chunk) kinds_for(h, rows, a.vocab, &l.kinds_row[1]);
         l.look = l.kinds_row[0] | l.kinds_row[1];
         l.early = csize == 1u && rows > sms;
+        l.local = h->wide_route == 0 ? 2u : h->wide_route == 3 ? 1u : 0u;
         PGS_CUDA(h, pgs::launch_wide(wl, l, h->slots, want < room ? want : room, stream));
     }
     else PGS_CUDA(h, pgs::launch_general(wl, grid < 32u ? grid : 32u, stream));
@@ -963,14 +967,16 @@ extern "C" int pgs_log_softmax(pgs_handle* h, const float* logits, uint32_t rows
     DeviceGuard g(h->device);
     cudaStream_t stream = cuda_stream ? (cudaStream_t)cuda_stream : h->stream;
     unsigned long long id = 0;
-    if (vocab <= h->wide_vocab && wide_scores_faster(h, rows, vocab, out_full != nullptr) && score_workspace_free(h, stream, &id)) {
+    const ScoreRoute route = vocab <= h->wide_vocab ? score_route(h, rows, vocab, out_full != nullptr) : SCORE_PLAIN;
+    if (route != SCORE_PLAIN && score_workspace_free(h, stream, &id)) {
         pgs::RowArgs a;
         memset(&a, 0, sizeof a);
         a.logits = logits; a.rows = rows; a.vocab = vocab; a.row_stride = row_stride; a.status = status; a.eos = -1;
         pgs::WideLaunch l = h->score_wide;
         l.ids = ids; l.out_gather = out_gather; l.out_full = out_full;
         l.done = h->score_done; l.done_value = h->score_calls + 1u;
-        PGS_CUDA(h, pgs::launch_wide(a, l, h->slots, wide_grid(h, rows, vocab), stream));
+        l.local = route == SCORE_ROWS;
+        PGS_CUDA(h, pgs::launch_wide(a, l, h->slots, l.local ? (rows < (uint32_t)h->sm_count ? rows : (uint32_t)h->sm_count) : wide_grid(h, rows, vocab), stream));
         h->score_calls += 1u;
         h->score_stream = id;
     } else {   // one CTA per row, no workspace

@@ -1773,10 +1773,13 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     if (!l_.kinds_front) cudaGridDependencySynchronize();
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass
+    // (how many rows are listed is known here only)
+    const bool local = l_.local == 1u || (l_.local == 2u && listed_one_cta_each(n_work, l_.chunk, slots, a_.vocab));
     if (tid == 0) { sm.a = a_; sm.target = 0u; sm.gave_up = 0u; }
     if (tid == 32u) {
         sm.l = l_;
-        if (l_.local) {   // this CTA's part of the workspace
+        sm.l.local = local ? 1u : 0u;   // (what the barriers go by)
+        if (local) {   // this CTA's part of the workspace
             WideLaunch& o = sm.l;
             const size_t at = blockIdx.x;
             o.row += at; o.reg += at * o.reg_stride; o.cell += at * o.reg_stride; o.seg += at * o.reg_stride; o.pre += at * o.reg_stride;
@@ -1785,15 +1788,14 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             o.sync = o.own + at * W_OWN; o.left_count = o.sync + 8; o.left_rows = o.sync + 9;
         }
     }
-    if (l_.local && tid == 0) { sm.rank = 0u; sm.size = 1u; sm.target = 1u; }
+    if (local && tid == 0) { sm.rank = 0u; sm.size = 1u; sm.target = 1u; }
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
     bool ok = true;   // (false for all CTAs, or none)
-    if (l_.look) {
+    if (l_.look && !(local && l_.local == 2u)) {
         ok = !look(n_work, slots);
         if (!ok && l_.kinds_front) return;
     }
-    const bool local = l_.local != 0u;
     ok = ok && (local || grid_join(sm, l));
     uint32_t n_left = 0u;   // rows left to the general kernel's code
     for (uint32_t c0 = local ? blockIdx.x : 0u; c0 < n_work && ok; c0 += local ? gridDim.x : l.chunk) {
@@ -1843,19 +1845,20 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             rows_one_cta_each(blockIdx.x, gridDim.x, blockIdx.x + 1u, l.left_rows - blockIdx.x);
             __syncthreads();
             if (tid == 0) *l.left_count = 0u;
+            n_left = 0u;
         }
     }
-    if (local) return;
+    if (local && !a.work_rows && !l.done) return;
     if (ok && n_left) rows_one_cta_each(sm.rank, min(slots, sm.size), n_left, l.left_rows);
     // The last CTA of the grid to leave resets the counters and empties the lists; the upper half counts the CTAs that gave up.
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        const uint32_t before = atomicAdd(l.sync + 4, sm.gave_up ? 0x10001u : 1u);
+        const uint32_t before = atomicAdd(l_.sync + 4, sm.gave_up ? 0x10001u : 1u);
         if ((before & 0xffffu) == gridDim.x - 1u) {
             if ((before >> 16) || sm.gave_up) { __threadfence(); give_up(a, l, n_work); }
-            l.sync[0] = 0u; l.sync[4] = 0u; l.sync[5] = 0u; l.sync[6] = 0u;
-            *l.left_count = 0u;
+            l_.sync[0] = 0u; l_.sync[4] = 0u; l_.sync[5] = 0u; l_.sync[6] = 0u;
+            *l_.left_count = 0u;
             if (a.work_rows) *a.work_count = 0u;
             if (l.done) { __threadfence(); *(volatile uint32_t*)l.done = l.done_value; }   // (the next launch starts behind this)
         }

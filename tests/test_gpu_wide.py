@@ -85,7 +85,8 @@ def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k, route):
                                                          (9, 33025, 0, 300), (3, 70001, 2049, 2100)])
 def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
     """The wide kernel with one CTA per row: one row, more rows than SMs, rows that go on to the general kernel's code
-    (more history than the workspace holds), short and long lists, a mask that leaves regions empty."""
+    (more history than the workspace holds), short and long lists, a mask that leaves regions empty; steps, listed rows, scores."""
+    import torch
     import pagoda_b200
     from pagoda_b200 import synth
     monkeypatch.setenv("PGS_WIDE_ROUTE", "3")
@@ -102,9 +103,14 @@ def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
         mask_words=words, state_flags=np.zeros(2, np.uint32), mask_state=np.resize(np.int32([-1, 0, 1, -1, 1]), rows))
     s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
     try:
-        s.set_exact(True)
-        for _ in range(2):   # (the second time on what the first has left)
-            assert_same(*run_both(s, oracle, w), w)
+        for exact in (True, False, True):   # (on what the one before has left; the default mode lists what the row kernel does not do)
+            s.set_exact(exact)
+            assert_same(*run_both(s, oracle, w), w, exact=exact, min_clear=0.0)
+        ids = np.arange(rows, dtype=np.int32) % vocab
+        g, full, _ = s.log_softmax(torch.from_numpy(x).cuda(), ids=torch.from_numpy(ids).cuda(), full=True,
+                                   stream_ptr=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        check_scores(oracle, x, ids, g, full)
     finally:
         s.close()
 
