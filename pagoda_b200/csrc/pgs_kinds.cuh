@@ -57,9 +57,10 @@ __host__ __device__ __forceinline__ bool listed_one_cta_each(uint32_t n, uint32_
 //
 // by_rows: the wide kernel takes a CTA per row itself (wide_row_by_row).  us of one row that way, as many at a time as there are
 // SMs: greedy 14 + 0.12 per thousand logits, sampled 36 + 0.3 (55 where the threshold needs the histogram), without top-k 58 + 0.55, with
-// a sort for top-p 60 + 1.
+// a sort for top-p 60 + 1.  Up to 2048 logits only the last of these is worth it (16 x 1720 111 / 59, others within 5 %), and beyond a
+// chunk of rows not even the look at what the rows ask for (210 x 1719 with top-k 27 100 / 103).
 inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool by_rows) {
-    if (V <= 1024u) return of;   // (the slowest kind is as quick either way, and nothing has to be looked at)
+    if (V <= 1024u || (by_rows && V <= 2048u && n > chunk)) return of;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
     const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
     uint32_t mask = 0u;
@@ -78,6 +79,7 @@ inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint
             grid = waves * (!(kinds & WK_SAMPLED) ? 14.0f + 0.12f * v3 : kinds & WK_SORT ? 60.0f + v3 : kinds & WK_OPEN ? 58.0f + 0.55f * v3
                             : (kinds & WK_HIST ? 55.0f : 36.0f) + 0.3f * v3);
         } else grid *= chunks;
+        if (by_rows && V <= 2048u && !(kinds & WK_SORT)) mask |= 1u << kinds;
         if (waves * row < grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
     }
     return mask;
