@@ -335,6 +335,7 @@ __device__ __forceinline__ void to_runs(float* buf, float (&v)[WL], const float 
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < WL; j++) v[j] = buf[lane * WL + j];
+    __syncwarp();
 }
 
 // A segment that is added term by term, made ready for add_segment by one warp: v, the lanes' runs; pre, the estimate of the
@@ -1637,6 +1638,7 @@ __device__ __noinline__ bool region_phase(uint32_t n_rows, uint32_t c0, uint32_t
 #pragma unroll
                     for (int j = 0; j < WL; j++) t[j * 32 + lane] = buf[j * 32 + lane];   // (each lane its own)
                 }
+                __syncwarp();   // (the next region's entries are staged there by other lanes)
             }
             if (lane == 0) *seg = out;
         } else {   // WP_LIST

@@ -81,6 +81,35 @@ def test_fold_changes_binade(oracle, monkeypatch, vocab, top_k, route):
         s.close()
 
 
+@pytest.mark.parametrize("route", ["1", "3"])
+@pytest.mark.parametrize("top_k", [0, 40])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_terms_and_entries_share_the_staging_buffer(oracle, monkeypatch, route, top_k, bf16):
+    """Rows of which most regions are added term by term, with history entries in every region and no mask: a warp stages one
+    region's terms and the next region's entries in the same buffer.  Bit-exact sums, totals and tokens."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    monkeypatch.setenv("PGS_WIDE_ROUTE", route)
+    n, vocab = 8, 512 * 128
+    i = np.arange(vocab)
+    rng = np.random.default_rng(3)
+    rows = [-40.0 + 40.0 * i / vocab, -0.6931472 * (i % 24), -0.6931472 * rng.integers(0, 12, vocab), 2.0 * rng.standard_normal(vocab)]
+    x = np.stack(rows * 2).astype(np.float32) + np.float32(0.0)
+    if bf16:
+        x = synth.f32_to_bf16_bits(x).reshape(x.shape)
+    ids = np.stack([rng.permutation(np.arange(0, vocab, 512)[:, None] + rng.integers(0, 512, (vocab // 512, 16)), axis=1).ravel()
+                    for _ in range(n)]).astype(np.uint32)   # sixteen in every region
+    w = synth.Workload("staged", x, np.resize(np.float32([1.0, 0.7]), n), np.full(n, top_k, np.uint32),
+                       np.resize(np.float32([1.0, 0.97]), n), np.full(n, 0.2, np.float32), np.full(n, 0.1, np.float32),
+                       np.full(n, 1.1, np.float32), np.arange(n + 1, dtype=np.uint32) * ids.shape[1], ids.ravel(), synth.uniform_f32(5, n))
+    s = pagoda_b200.Sampler(device=0, max_rows=n, max_vocab=vocab, max_history=ids.shape[1])
+    try:
+        s.set_exact(True)
+        assert_same(*run_both(s, oracle, w), w)
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("rows, vocab, top_k, history", [(1, 511, 0, 0), (160, 512, 40, 64), (149, 513, 0, 300), (5, 1025, 1025, 2049), (150, 9001, 30, 300),
                                                          (9, 33025, 0, 300), (3, 70001, 2049, 2100)])
 def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
