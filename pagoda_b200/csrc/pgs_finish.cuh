@@ -153,13 +153,13 @@ __device__ __forceinline__ float add_runs(float R, const float (&v)[RUN], float*
 }
 
 // Exact left fold of n shared-memory floats by one warp, 512 at a time as runs of 16; ends[r]: the running value behind
-// run r (exact).  Stops where the running value reaches `goal`; returns what it has come to.  v: readable up to the next
-// multiple of 4.  (512 terms: the additions one by one take 4000 cycles.)
+// run r (exact).  Stops where the running value reaches `goal`, behind the first 512 at the earliest; returns what it has come
+// to.  v: readable up to the next multiple of 4.  (512 terms: the additions one by one take 4000 cycles.)
 __device__ __forceinline__ float warp_fold(const float* v, uint32_t n, float goal, float* ends) {
     const uint32_t lane = threadIdx.x & 31;
     float R = 0.0f;
 #pragma unroll 1
-    for (uint32_t base = 0; base < n && !(R >= goal); base += 32u * RUN) {
+    for (uint32_t base = 0; base < n && (base == 0u || !(R >= goal)); base += 32u * RUN) {   // (a goal of zero is reached by the first term, not in front of it)
         float x[RUN];
 #pragma unroll
         for (int j = 0; j < RUN; j += 4) {

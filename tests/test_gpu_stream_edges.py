@@ -73,6 +73,34 @@ def test_stream_edges_on_one_cta_and_on_clusters(oracle, monkeypatch, cluster, r
         s.close()
 
 
+# Long candidate lists are folded in runs of sixteen, short ones by one lane.
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("rows, vocab, top_k", [(5, 4096, 160), (5, 40000, 161), (9, 151936, 500), (300, 8192, 700)])
+def test_top_p_of_zero_keeps_the_first_entry(oracle, exact, rows, vocab, top_k):
+    """top_p <= 0 is reached behind the first entry (sampler.rs:136-144), whatever was in shared memory before (the raw logits of
+    the history, which are negative)."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    x = synth.normal_f32(19 + vocab, rows * vocab, 2.0).reshape(rows, vocab) - np.float32(30.0)
+    x[:, vocab // 2] = x[:, 3]
+    w = synth.Workload(
+        "zero", x, np.resize(np.float32([0.7, 1.0, 4.0]), rows), np.full(rows, top_k, np.uint32),
+        np.resize(np.float32([0.0, -1.0, -0.0, -1e30, 1e-30]), rows), np.full(rows, 0.2, np.float32), np.full(rows, 0.1, np.float32),
+        np.ones(rows, np.float32), np.arange(rows + 1, dtype=np.uint32) * 2048,
+        np.stack([np.random.default_rng(r).permutation(vocab)[:2048] for r in range(rows)]).astype(np.uint32).ravel(), synth.uniform_f32(5, rows))
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=2048)
+    try:
+        s.set_exact(exact)
+        for _ in range(2):
+            got, want = run_both(s, oracle, w)
+            assert (want["n_kept"] == 1).all()
+            for name in ("status", "token", "n_kept", "argmax"):
+                np.testing.assert_array_equal(getattr(got, name), want[name], err_msg=name)
+            np.testing.assert_allclose(got.total, want["total"], rtol=1e-5)
+    finally:
+        s.close()
+
+
 # Rows whose bits do not fit in shared memory, from the first length on to the longest.
 @pytest.mark.parametrize("cluster", ["1", "0"])
 @pytest.mark.parametrize("vocab, top_k, history, crowd, masked, bf16", [
