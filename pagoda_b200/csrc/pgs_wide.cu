@@ -1027,7 +1027,7 @@ __device__ __noinline__ void sum_row(uint32_t slot) {
 // (32 rows of 151936 with top-p 0.95: a quarter of the logits are counted.)
 __device__ __forceinline__ uint32_t lowest_bucket(const WideRow& c, uint32_t V) {
     if ((c.top_k != 0u && c.top_k < V) || c.top_p >= 1.0f) return 0u;
-    const float left = 0.999f * (1.0f - c.top_p * 1.002f / 0.99609375f);   // (the probabilities' own sum is 1 to within 1e-3)
+    const float left = 0.999f * (1.0f - fmaxf(c.top_p, 0.0f) * 1.002f / 0.99609375f);   // (the probabilities' own sum is 1 to within 1e-3)
     return left > 0.001f ? bucket_of((left - 0.001f) / (float)V) : 0u;
 }
 
@@ -1070,7 +1070,7 @@ __device__ __noinline__ void select_row(uint32_t slot) {
     __syncthreads();
     const uint32_t x = sm.red_u[lane];
     const uint32_t before = __reduce_add_sync(FULL, lane < w ? x : 0u) + inc - own;
-    const float goal = sm.row.top_p * 1.002f;
+    const float goal = fmaxf(sm.row.top_p * 1.002f, 1.17549435e-38f);   // (top-p of zero or less: the highest bucket with an entry)
     {
         uint32_t above = before;
 #pragma unroll

@@ -241,3 +241,59 @@ def test_both_routes(oracle, monkeypatch, route, rows, vocab, top_k, history):
         check_scores(oracle, clean, ids, g, full)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("route", ["1", "3"])   # the grid, and one CTA per row
+@pytest.mark.parametrize("top_k", [0, 3000])
+@pytest.mark.parametrize("vocab", [16384, 70001])
+def test_open_rows_with_any_top_p(oracle, monkeypatch, route, top_k, vocab):
+    """Top-p from below zero (the first entry) to just below one (all but the last few), over the whole vocabulary."""
+    import pagoda_b200
+    from pagoda_b200 import synth
+    monkeypatch.setenv("PGS_WIDE_ROUTE", route)
+    top_p = np.float32([0.0, -1.0, -0.0, -1e30, 1e-30, 1e-6, 0.5, 0.994, 0.998, 0.9985, 0.999, 0.9999, 0.999999])
+    rows = 2 * len(top_p)
+    x = synth.normal_f32(23 + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    x[:, vocab // 2] = x[:, 3] = x.max(axis=1) + np.float32(0.5)   # a tie at the first entry
+    w = synth.Workload("top-p", x, np.resize(np.float32([1.0, 0.7, 3.0]), rows), np.full(rows, top_k, np.uint32), np.resize(top_p, rows),
+                       np.zeros(rows, np.float32), np.zeros(rows, np.float32), np.ones(rows, np.float32), None, None, synth.uniform_f32(5, rows))
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    try:
+        s.set_exact(True)
+        assert_same(*run_both(s, oracle, w), w)
+    finally:
+        s.close()
+
+
+def _us(sampler, x, temperature, top_p):
+    """A step's time (the best of several) over open rows with one top-p."""
+    import torch
+    rows = x.shape[0]
+    full = lambda v, dt=torch.float32: torch.full((rows,), v, dtype=dt, device=x.device)  # noqa: E731
+    desc = sampler.make_device_desc(x, token=full(0, torch.int32), status=full(0, torch.int32), temperature=full(temperature),
+                                    top_k=full(0, torch.int32), top_p=full(top_p), uniform=full(0.5))
+    stream = torch.cuda.current_stream().cuda_stream
+    best = float("inf")
+    for _ in range(6):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        sampler.launch_device(desc, stream)
+        end.record()
+        end.synchronize()
+        best = min(best, begin.elapsed_time(end) * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("top_p", [0.0, -1.0])
+def test_open_rows_with_top_p_of_zero_stay_in_the_wide_kernel(top_p):
+    """They need no more than rows with a usual top-p (one CTA that sorts the whole row takes a hundred times as long)."""
+    import torch
+    import pagoda_b200
+    rows, vocab = 2, 131072
+    x = 2.0 * torch.randn(rows, vocab, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
+    try:
+        usual = _us(s, x, 1.0, 0.5)
+        assert _us(s, x, 1.0, top_p) < 4.0 * usual
+    finally:
+        s.close()
