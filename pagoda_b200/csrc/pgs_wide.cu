@@ -1222,8 +1222,9 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
             else atomicAdd(&sm.bn[b], i0);
         });
         // The fold over the buckets, highest first, by events as in resolve: a run of buckets of one binade is one addition; a
-        // bucket with several entries that the running value may change binade in, and the one in which top-p is reached, is
-        // sorted by the CTA and its entries are added in order.  (Over the buckets 256 at a time the walk took 27 us a row.)
+        // bucket with several entries that the running value may change binade in, the one in which top-p is reached, and one in
+        // which a run turns out not as estimated, is sorted by the CTA and its entries are added in order.  (Over the buckets 256
+        // at a time the walk took 27 us a row.)
         uint32_t* ends = reinterpret_cast<uint32_t*>(&sm.stage[0][0]);   // where a bucket ends in the list
         unsigned long long* ev_sum = reinterpret_cast<unsigned long long*>(ends + W_BUCKETS);
         uint32_t* ev = sm.serial;   // the bucket an event begins with
@@ -1285,50 +1286,65 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
         }
         float R = 0.0f;                              // warp 0
         uint32_t e = 0u;
+        // A run that does not go by in one addition is cut at a bucket, which is sorted like the others; the run's buckets above
+        // `limit` are behind it then, with the increments up to `from`.
+        uint32_t cut_run = W_NIL, limit = 0u;        // the event that these hold for
+        unsigned long long from = 0ull;
         bool found = false;
         while (!leave) {
             __syncthreads();
             if (w == 0) {
                 uint32_t need = W_NIL, in_run = 0u;
 #pragma unroll 1
-                for (; e < n_ev && need == W_NIL; e++) {
+                for (; e < n_ev; e++) {
                     const uint32_t b = ev[e], k = f2u(sm.bs[b]), rb = f2u(R);
                     if (k == 0u) {   // (a single entry that does not reach top-p needs no sort)
                         const float R1 = fadd(R, u2f(sm.bn[b]));
-                        if (ends[b] - (b + 1u < (uint32_t)W_BUCKETS ? ends[b + 1u] : 0u) == 1u && R1 < sm.row.top_p) R = R1; else need = b;
+                        if (ends[b] - (b + 1u < (uint32_t)W_BUCKETS ? ends[b + 1u] : 0u) == 1u && R1 < sm.row.top_p) R = R1;
+                        else { need = b; e++; break; }
                     } else {
-                        const unsigned long long run = ev_sum[e + 1u] - ev_sum[e];
-                        if ((rb & 0x7f800000u) != k || run >= 0x00800000u - (rb & 0x007fffffu)) { need = b; in_run = 2u; }   // not as estimated
-                        else if (u2f(rb + (uint32_t)run) >= sm.row.top_p) { need = b; in_run = 1u; }
-                        else R = u2f(rb + (uint32_t)run);
+                        const unsigned long long run = ev_sum[e + 1u] - (e == cut_run ? from : ev_sum[e]);
+                        if ((rb & 0x7f800000u) != k || run >= 0x00800000u - (rb & 0x007fffffu) || u2f(rb + (uint32_t)run) >= sm.row.top_p) {
+                            need = b; in_run = 1u;
+                            break;
+                        }
+                        R = u2f(rb + (uint32_t)run);
                     }
                 }
-                if (lane == 0) { sm.last = need; sm.n_ev = in_run; sm.at_ev = e - 1u; sm.R = R; sm.found = 0u; }
+                if (lane == 0) { sm.last = need; sm.n_ev = in_run; sm.at_ev = e; sm.R = R; sm.found = 0u; }
             }
             __syncthreads();
-            if (sm.n_ev == 2u) { leave = true; break; }
-            if (sm.n_ev == 1u) {   // top-p is reached in this run: in its first bucket behind which the running value has come to it
-                const uint32_t rb = f2u(sm.R);
-                const unsigned long long base = ev_sum[sm.at_ev];
+            if (sm.n_ev) {   // the first bucket of the run that top-p is reached in, or that leaves the binade, or any where the estimate missed it
+                const uint32_t run = sm.at_ev, rb = f2u(sm.R), room = 0x00800000u - (rb & 0x007fffffu);
+                const bool other = (rb & 0x7f800000u) != f2u(sm.bs[ev[run]]);
+                if (run != cut_run) { cut_run = run; limit = W_BUCKETS; from = ev_sum[run]; }
                 unsigned long long at = before;
                 for (int u = 0; u < PER; u++) {
                     const int bb = bucket(u);
                     if (empty(bb)) continue;
                     const uint32_t i = ((uint32_t)at & EV_MASK) + ((is_event >> u) & 1u) - 1u;   // the event that the bucket belongs to
                     at += (increment_in(bb) << 14) + ((is_event >> u) & 1u);
-                    if (i == sm.at_ev && u2f(rb + (uint32_t)((at >> 14) - base)) >= sm.row.top_p) atomicMax(&sm.found, (uint32_t)bb + 1u);
+                    if (i != run || (uint32_t)bb >= limit) continue;
+                    const unsigned long long inc = (at >> 14) - from;
+                    if (other || inc >= room || u2f(rb + (uint32_t)inc) >= sm.row.top_p) atomicMax(&sm.found, (uint32_t)bb + 1u);
                 }
                 __syncthreads();
-                const uint32_t fb = sm.found - 1u;
+                if (sm.found == 0u) {   // CTA-uniform: nothing is left of the run
+                    e++;
+                    continue;
+                }
+                limit = sm.found - 1u;
                 at = before;
                 for (int u = 0; u < PER; u++) {   // the running value in front of it
                     const int bb = bucket(u);
                     if (empty(bb)) continue;
-                    if ((uint32_t)bb == fb) { sm.R = u2f(rb + (uint32_t)((at >> 14) - base)); sm.last = fb; }
+                    const unsigned long long in_front = at >> 14;
                     at += (increment_in(bb) << 14) + ((is_event >> u) & 1u);
+                    if ((uint32_t)bb == limit) { sm.R = u2f(rb + (uint32_t)(in_front - from)); sm.red_w[0] = at >> 14; sm.last = limit; }
                 }
                 __syncthreads();
                 R = sm.R;
+                from = sm.red_w[0];
             }
             const uint32_t sb = sm.last;
             if (sb == W_NIL) break;

@@ -297,3 +297,51 @@ def test_open_rows_with_top_p_of_zero_stay_in_the_wide_kernel(top_p):
         assert _us(s, x, 1.0, top_p) < 4.0 * usual
     finally:
         s.close()
+
+
+def _row_below_its_estimate(vocab):
+    """Logits of a row whose running probabilities fall behind their plain sum: four large ones, then values a little less than
+    half an ulp (of a running value below 1/2) above a whole number of ulps, which every addition rounds down.  Where the plain sum
+    passes 1/2 by more than the margin of the estimate the running value is still below it."""
+    rng, ulp = np.random.default_rng(0), 2.0 ** -25
+    parts, mass, m = [np.full(4, 0.065)], 0.26, 44
+    while mass < 0.5036:
+        near = mass > 0.4965   # few to a bucket here
+        n = 1200 if near else min(30000, int((0.497 - mass) / (m + 0.4) / ulp) + 1)
+        parts.append((m + rng.uniform(0.02 if near else 0.3, 0.44, n)) * ulp)
+        mass += parts[-1].sum()
+        m -= 1
+    n = vocab - sum(len(q) for q in parts)
+    parts.append(np.linspace(m + 0.9, 2.0 * (1.0 - mass) / n / ulp - m - 0.9, n) * ulp)
+    p = np.sort(np.concatenate(parts))[::-1]
+    where = rng.permutation(vocab)
+    x, scale = np.zeros(vocab, np.float32), 1.0
+    for _ in range(4):   # (the sum that they are divided by is a fold as well)
+        e = np.minimum(p / p[0] * scale, 1.0)
+        e[:4] = 1.0
+        x[where] = np.log(e)
+        scale = np.add.accumulate(np.exp(x.astype(np.float64)).astype(np.float32), dtype=np.float32)[-1] * p[0]
+    return x
+
+
+def test_top_p_where_the_running_value_is_not_as_estimated(oracle, monkeypatch):
+    """The fold towards top-p goes on behind a run of buckets that turns out to be in another binade: bit-exact, and in a fraction
+    of the time of one CTA that sorts the whole row."""
+    import torch
+    import pagoda_b200
+    from pagoda_b200 import synth
+    vocab = 1 << 20
+    x = np.stack([_row_below_its_estimate(vocab)])
+    w = synth.Workload("estimate", x, np.float32([1.0]), np.uint32([0]), np.float32([0.9]), np.zeros(1, np.float32), np.zeros(1, np.float32),
+                       np.ones(1, np.float32), None, None, synth.uniform_f32(5, 1))
+    us = {}
+    for route in ("1", "2", "3"):
+        monkeypatch.setenv("PGS_WIDE_ROUTE", route)
+        s = pagoda_b200.Sampler(device=0, max_rows=1, max_vocab=vocab, max_history=1)
+        try:
+            s.set_exact(True)
+            assert_same(*run_both(s, oracle, w), w)
+            us[route] = _us(s, torch.from_numpy(x).cuda(), 1.0, 0.9)
+        finally:
+            s.close()
+    assert us["1"] < 0.5 * us["2"] and us["3"] < 0.5 * us["2"], us
