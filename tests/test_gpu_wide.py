@@ -284,9 +284,9 @@ def _us(sampler, x, temperature, top_p):
     return best
 
 
-@pytest.mark.parametrize("top_p", [0.0, -1.0])
-def test_open_rows_with_top_p_of_zero_stay_in_the_wide_kernel(top_p):
-    """They need no more than rows with a usual top-p (one CTA that sorts the whole row takes a hundred times as long)."""
+@pytest.mark.parametrize("top_p, most", [(0.0, 4.0), (-1.0, 4.0), (0.998, 8.0), (0.9995, 8.0)])
+def test_open_rows_with_unusual_top_p_stay_in_the_wide_kernel(top_p, most):
+    """They need not much more than rows with a usual top-p (one CTA that sorts the whole row takes 25 times as long)."""
     import torch
     import pagoda_b200
     rows, vocab = 2, 131072
@@ -294,7 +294,7 @@ def test_open_rows_with_top_p_of_zero_stay_in_the_wide_kernel(top_p):
     s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=1)
     try:
         usual = _us(s, x, 1.0, 0.5)
-        assert _us(s, x, 1.0, top_p) < 4.0 * usual
+        assert _us(s, x, 1.0, top_p) < most * usual
     finally:
         s.close()
 
