@@ -1185,13 +1185,14 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
         for (uint32_t b = cut + tid; b < (uint32_t)W_BUCKETS; b += W_NT) { sm.bn[b] = 0u; sm.bs[b] = 0.0f; }
         __syncthreads();
         // (the entries of a bucket share their upper bits: their sum is their number and the sum of the 15 lower bits, whole numbers,
-        // which shared memory adds faster than floats)
+        // which shared memory adds faster than floats; three bits less, 2^-20 of the sum, so that it fits 32 bits for every row)
+        static_assert((0x7fffu >> 3) <= 0xffffffffu / ((uint32_t)W_MAX_REGIONS * W_REGION), "all logits in one bucket");
         uint32_t* lower = reinterpret_cast<uint32_t*>(sm.bs);
         each([&](float p, uint32_t) {
             if (!(p >= thr_k)) return;
             const uint32_t b = bucket_of(p);
             atomicAdd(&sm.bn[b], 1u);
-            atomicAdd(&lower[b], f2u(p) & 0x7fffu);
+            atomicAdd(&lower[b], (f2u(p) & 0x7fffu) >> 3);
         });
         __syncthreads();
         {   // plain sums -> the binade of the running value at each bucket
@@ -1203,7 +1204,7 @@ __device__ __noinline__ void choose_row(uint32_t slot) {
                 P[u] = 0.0f;
                 if (b >= (int)cut && sm.bn[b]) {   // (bucket 0: of no account)
                     const float floor_b = bucket_floor(b);
-                    P[u] = (float)sm.bn[b] * floor_b + (float)lower[b] * (u2f(binade(floor_b)) * 1.1920928955078125e-07f);
+                    P[u] = (float)sm.bn[b] * floor_b + (float)lower[b] * (u2f(binade(floor_b)) * 9.5367431640625e-07f);
                     sm.bn[b] = 0u;
                 }
                 own += P[u];
