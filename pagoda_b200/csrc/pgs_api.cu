@@ -526,7 +526,6 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         kinds_for(h, rows < l.chunk ? rows : l.chunk, a.vocab, &l.kinds_row[0]);
         if (rows > l.chunk) kinds_for(h, rows, a.vocab, &l.kinds_row[1]);
         l.look = l.kinds_row[0] | l.kinds_row[1];
-        l.early = csize == 1u && rows > sms;
         l.local = h->wide_route == 0 ? 2u : h->wide_route == 3 ? 1u : 0u;
         PGS_CUDA(h, pgs::launch_wide(wl, l, h->slots, want < room ? want : room, stream));
     }

@@ -1790,10 +1790,10 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     const RowArgs& a = sm.a;
     const WideLaunch& l = sm.l;
     const uint32_t tid = threadIdx.x;
-    // Launched ahead of the end of the kernel before, which may fill the list.  The kernel behind is set up ahead as well where
-    // the batch has two CTAs of the row kernel on most SMs (256 mixed bf16 rows 159 -> 154 us, 256 rows of 151936 71.9 -> 71.3);
-    // those of smaller batches would crowd on the SMs that this kernel leaves free (128 masked rows 50 -> 62).
-    if (l_.early) cudaTriggerProgrammaticLaunchCompletion();
+    // Launched ahead of the end of the kernel before, which may fill the list.  (No early trigger for the kernel behind: its
+    // CTAs would crowd on the SMs that this one leaves free, two on an SM while others have none, or those with two rows
+    // together.  us without / with it: 128 masked rows 50 / 62, 149 rows of 151936 66.4 / 69.1, 149 mixed bf16 rows of 256000 129 / 147,
+    // 300 rows of 50256 with 512 ids 58 / 70; 192 to 296 rows within 2 % either way.)
     if (!l_.kinds_front) cudaGridDependencySynchronize();
     const uint32_t n_work = a_.work_rows ? *(volatile uint32_t*)a_.work_count : a_.rows;
     if (n_work == 0u) return;   // the usual case of the work-list pass

@@ -56,7 +56,6 @@ struct WideLaunch {
     uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
     uint32_t local;             // 1: one CTA per row, with the part of the workspace that has the CTA's number; 2: by the number of listed rows
     uint32_t* own;              // [CTAs][W_OWN]: what `sync`, `left_count` and `left_rows` are for the grid
-    uint32_t early;             // the kernel behind may be set up from the start
     uint32_t polls;             // limit of a barrier's wait
     unsigned long long* gave_up; // rows that ended without results because one ran out
     uint32_t chunk;             // rows that the grid takes at a time (<= W_CHUNK, and what the workspace holds)
