@@ -89,13 +89,13 @@ struct PassArgs {
     const uint32_t* mw;     // rows beyond S_SHORT_VOCAB: the grammar mask
     float sc, sc_lo, c_hi, c_lo, cut_f, freq, pres, rep;
     uint32_t V, n_full, n_regions, flags;
-    uint32_t few;           // pass 2 meets few candidates (see few_candidates)
     // a row shared by the CTAs of a cluster: this CTA works on the pieces q0, q0 + qstep, ...; the candidates of all of
     // them are collected by the first CTA (pointers into its shared memory)
     uint32_t q0, qstep;
     uint32_t* cand_n_p;
     uint32_t* cand_id_p;
     float* cand_x_p;
+    uint32_t few;           // pass 2 meets few candidates (see few_candidates)
 };
 
 // LONG: rows beyond S_SHORT_VOCAB, whose bits do not fit beside two CTAs' tables.
@@ -380,11 +380,12 @@ __device__ __forceinline__ uint32_t region_word(const SM& sm, uint32_t region) {
 // Raw logits of piece q -> the logits of the pass: -inf where the row's bits say so (BITS: grammar mask, entries, end of
 // the row) or behind the end of the row.  The bits come from shared memory, four logits (bf16: eight) of a lane to the
 // load.  (Read from the mask table a piece at a time, every group of the piece waited for L2: 128 masked rows of 151936
-// took 100 us, with the bits 51.)  bf16 rows, whose passes are bound by instructions: four bits at a time pick what is added to
-// their logits from a table, two packed additions and a load in place of four tests and four selects (256 mixed rows of 256000
-// 158.5 -> 154.4 us; -0 becomes +0, which compares equal everywhere).  f32 rows wait for the extra load longer than that saves
-// (128 masked rows of 151936 48.5 -> 50.9).
-template <bool BF16, bool BITS, bool TAIL, class SM>
+// took 100 us, with the bits 51.)  bf16 rows of one CTA each, whose passes are bound by instructions: four bits at a time pick what is
+// added to their logits from a table, two packed additions and a load in place of four tests and four selects (256 mixed rows of
+// 256000 158.5 -> 154.4 us; -0 becomes +0, which compares equal everywhere).  f32 rows wait for the extra load longer than that saves
+// (128 masked rows of 151936 48.5 -> 50.9), and so do rows that a cluster shares (bf16, with top-k 1, without / with the
+// table: 16 rows of 1000 17.4 / 18.4, 64 of 16384 19.7 / 20.5, 64 of 128000 with a mask 33.1 / 33.9).
+template <bool BF16, bool BITS, bool TAIL, bool CL, class SM>
 __device__ __forceinline__ void fix_x(const SM& sm, float (&x)[S_EPT], uint32_t q, uint32_t word) {
     constexpr int G = Geo<BF16>::G, GE = Geo<BF16>::GE, GS = Geo<BF16>::GS;
     if (!BITS && !TAIL) return;
@@ -394,7 +395,7 @@ __device__ __forceinline__ void fix_x(const SM& sm, float (&x)[S_EPT], uint32_t 
 #pragma unroll
     for (int h = 0; h < G; h++) {
         const uint32_t idx = e0 + h * GS;
-        if constexpr (BITS && BF16) {
+        if constexpr (BITS && BF16 && !CL) {
             const uint32_t bits = SM::IS_LONG ? __shfl_sync(FULL, word, (int)((idx >> 5) & 15u)) : sm.bits[idx >> 5];
 #pragma unroll
             for (int c = 0; c < GE; c += 4) {
@@ -444,7 +445,7 @@ __device__ __forceinline__ void copy_entries(SM& sm, uint32_t region) {
 }
 
 // pass 1 on one piece
-template <bool BF16, bool BITS, bool TAIL, bool STOCH, class SM>
+template <bool BF16, bool BITS, bool TAIL, bool STOCH, bool CL, class SM>
 __device__ __forceinline__ void p1_piece(SM& sm, const Raw<BF16>& raw, uint32_t q, float& am, float& tmx, uint32_t& tqx) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t region = q * SNW + (uint32_t)w;
@@ -453,7 +454,7 @@ __device__ __forceinline__ void p1_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
     am = absmax_ept_nan(am, x);   // max |raw logit|, NaN-propagating: the sanity check
-    fix_x<BF16, BITS, TAIL>(sm, x, q, word);
+    fix_x<BF16, BITS, TAIL, CL>(sm, x, q, word);
     const float pm = max_ept(x);
     if (pm >= tmx) { tmx = pm; tqx = q; }   // pieces arrive in descending order: an equal maximum here has the lower id
     if (STOCH) {
@@ -558,7 +559,7 @@ __device__ __forceinline__ void p2_piece(SM& sm, const Raw<BF16>& raw, uint32_t 
     const uint32_t word = region_word<BITS>(sm, q * SNW + (uint32_t)w);
     float x[S_EPT];
     raw_unpack<BF16>(x, raw);
-    fix_x<BF16, BITS, TAIL>(sm, x, q, word);
+    fix_x<BF16, BITS, TAIL, CL>(sm, x, q, word);
     const float pm = max_ept(x);
     if (pm >= cut_f) {
         const uint32_t e0 = q * S_PIECE + (uint32_t)w * S_REGION + (uint32_t)lane * GE;
@@ -692,7 +693,7 @@ __device__ __noinline__ void pass1_whole(SM& sm) {
                 if (q - 2 * qs >= q0) prefetch_piece<BF16>(wp - 2 * step);
                 Raw<BF16> b;
                 raw_load<BF16>(b, p);
-                p1_piece<BF16, BITS, false, STOCH>(sm, b, (uint32_t)q, am, tmx, tqx);
+                p1_piece<BF16, BITS, false, STOCH, CL>(sm, b, (uint32_t)q, am, tmx, tqx);
             }
         }
         sm.t_am[threadIdx.x] = am; sm.t_max[threadIdx.x] = tmx; sm.t_q[threadIdx.x] = tqx;
@@ -709,7 +710,7 @@ __device__ __noinline__ void pass1_whole(SM& sm) {
         if (q >= (uint32_t)PGS_PF_DIST) prefetch_piece<BF16>(wp - (size_t)PGS_PF_DIST * PB);
         Raw<BF16> b;
         raw_load<BF16>(b, p);
-        p1_piece<BF16, BITS, false, STOCH>(sm, b, q, am, tmx, tqx);
+        p1_piece<BF16, BITS, false, STOCH, CL>(sm, b, q, am, tmx, tqx);
     }
     sm.t_am[threadIdx.x] = am; sm.t_max[threadIdx.x] = tmx; sm.t_q[threadIdx.x] = tqx;
 }
@@ -777,7 +778,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
     const uint32_t n_regions = (V + S_REGION - 1) / S_REGION;
     const uint32_t lane_e0 = (uint32_t)w * S_REGION + (uint32_t)lane * GE;   // first element of the thread inside a piece
     if (tid < 32) sm.exp_tab[tid] = kExp2TableDev[tid];
-    if (BF16 && tid < 16) sm.bit_tab[tid] = make_float4(tid & 1 ? 0.0f : -INFINITY, tid & 2 ? 0.0f : -INFINITY, tid & 4 ? 0.0f : -INFINITY, tid & 8 ? 0.0f : -INFINITY);
+    if (BF16 && !CL && tid < 16) sm.bit_tab[tid] = make_float4(tid & 1 ? 0.0f : -INFINITY, tid & 2 ? 0.0f : -INFINITY, tid & 4 ? 0.0f : -INFINITY, tid & 8 ? 0.0f : -INFINITY);
     if (tid == 0)
 #pragma unroll 1
         for (int i = 0; i < 16; i++) sm.prof_acc[i] = 0;
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         if (tid == 0) {   // what the pass loops read
             PassArgs& pa = sm.pa;
             pa.rowp = rowp; pa.mw = ctl.mw; pa.freq = ctl.freq; pa.pres = ctl.pres; pa.rep = ctl.rep; pa.sc = sc; pa.sc_lo = ctl.sc_lo; pa.c_hi = 0.0f; pa.c_lo = 0.0f; pa.cut_f = 0.0f;
-            pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions; pa.few = few_candidates<BF16, CL>(top_k);
+            pa.V = V; pa.n_full = n_full; pa.n_regions = n_regions; if (CL && !BF16) pa.few = few_candidates<BF16, CL>(top_k);
             pa.q0 = crank; pa.qstep = csize;
             pa.cand_n_p = &sm.cand_n; pa.cand_id_p = sm.cand_id; pa.cand_x_p = sm.cand_x;
             if (CL) {
@@ -967,8 +968,8 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
         if (my_tail) {
             Raw<BF16> raw;
             raw_load_tail<BF16>(raw, rowp + ((size_t)n_full * S_PIECE + lane_e0) * ESZ, n_full * S_PIECE + lane_e0, V);
-            if (has_bits) { if (greedy) p1_piece<BF16, true, true, false>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, true, true, true>(sm, raw, n_full, am, tmx, tqx); }
-            else { if (greedy) p1_piece<BF16, false, true, false>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, false, true, true>(sm, raw, n_full, am, tmx, tqx); }
+            if (has_bits) { if (greedy) p1_piece<BF16, true, true, false, CL>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, true, true, true, CL>(sm, raw, n_full, am, tmx, tqx); }
+            else { if (greedy) p1_piece<BF16, false, true, false, CL>(sm, raw, n_full, am, tmx, tqx); else p1_piece<BF16, false, true, true, CL>(sm, raw, n_full, am, tmx, tqx); }
         }
         if (n_full > 0u) {
             if (has_bits) { if (greedy) pass1_whole<BF16, true, false, CL>(sm); else pass1_whole<BF16, true, true, CL>(sm); }
@@ -1139,7 +1140,7 @@ __global__ void __launch_bounds__(SNT, 2) stream_row_kernel(const RowArgs a, con
                 raw_load_tail<BF16>(raw, rowp + ((size_t)q * S_PIECE + lane_e0) * ESZ, q * S_PIECE + lane_e0, V);
                 float x[S_EPT];
                 raw_unpack<BF16>(x, raw);
-                if (has_bits) fix_x<BF16, true, true>(sm, x, q, region_word<true>(sm, q * SNW + (uint32_t)w)); else fix_x<BF16, false, true>(sm, x, q, 0u);
+                if (has_bits) fix_x<BF16, true, true, CL>(sm, x, q, region_word<true>(sm, q * SNW + (uint32_t)w)); else fix_x<BF16, false, true, CL>(sm, x, q, 0u);
                 const bool mine = ((pending >> lane) & 1u) && tqx == q;
                 if (mine) {
                     int j0 = 0;
