@@ -80,7 +80,8 @@ inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint
                             : (kinds & WK_HIST ? 55.0f : 36.0f) + 0.3f * v3);
         } else grid *= chunks;
         if (by_rows && V <= 2048u && !(kinds & WK_SORT)) mask |= 1u << kinds;
-        if (waves * row < grid + (kinds & WK_LONG ? row : 0.0f)) mask |= 1u << kinds;
+        // (rows with a history beyond the workspace end in the general kernel's code either way: 200 x 50257 388 at once, 503 otherwise)
+        if (waves * row < grid + (!(kinds & WK_LONG) ? 0.0f : by_rows ? waves * row : row)) mask |= 1u << kinds;
     }
     return mask;
 }

@@ -1822,6 +1822,11 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     }
     ok = ok && (local || grid_join(sm, l));
     uint32_t n_left = 0u;   // rows left to the general kernel's code
+    const auto leave_one = [&]() {   // the CTA's own list has one entry; the scratch slot is the CTA's too
+        rows_one_cta_each(blockIdx.x, gridDim.x, blockIdx.x + 1u, l.left_rows - blockIdx.x);
+        __syncthreads();
+        if (tid == 0) *l.left_count = 0u;
+    };
     for (uint32_t c0 = local ? blockIdx.x : 0u; c0 < n_work && ok; c0 += local ? gridDim.x : l.chunk) {
         const uint32_t n = local ? 1u : min(n_work - c0, l.chunk), to_do = n_work - c0;
         const auto open = [&](uint32_t s) { open_row<BF16>(s, a.work_rows ? a.work_rows[c0 + s] : c0 + s); };
@@ -1829,6 +1834,11 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
         uint32_t s = sm.rank;
         if (c0 == 0u) { if (s < n) open(s); }   // (how many take part is not known yet)
         else for (; s < n; s += sm.size) open(s);
+        if (local && sm.row.state == WS_DONE) {   // CTA-uniform: bad parameters, or left to the general kernel's code
+            __syncthreads();
+            if (*(volatile uint32_t*)l.left_count) leave_one();
+            continue;
+        }
         if (!(ok = region_phase<BF16, VEC, WP_FIRST>(n, c0, to_do))) break;
         if (c0 == 0u && sm.size < n) {   // not one CTA for every row
             for (s += sm.size; s < n; s += sm.size) open(s);
@@ -1865,12 +1875,7 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
             }
         }
         if ((to_do > n || n_left) && !(ok = grid_sync(sm, l, to_do))) break;   // the chunk's workspace is free
-        if (local && n_left) {   // (the list has one entry; the scratch slot is this CTA's)
-            rows_one_cta_each(blockIdx.x, gridDim.x, blockIdx.x + 1u, l.left_rows - blockIdx.x);
-            __syncthreads();
-            if (tid == 0) *l.left_count = 0u;
-            n_left = 0u;
-        }
+        if (local && n_left) { leave_one(); n_left = 0u; }
     }
     if (local && !a.work_rows && !l.done) return;
     if (ok && n_left) rows_one_cta_each(sm.rank, min(slots, sm.size), n_left, l.left_rows);

@@ -144,6 +144,34 @@ def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
         s.close()
 
 
+def _mixed_rows(rows, vocab, top_k, history, greedy, seed=29):
+    from pagoda_b200 import synth
+    x = synth.normal_f32(seed + vocab, rows * vocab, 2.0).reshape(rows, vocab)
+    return synth.Workload(
+        "short rows", x, np.resize(np.float32([0.0] if greedy else [0.7, 1.3, 5.0]), rows), np.full(rows, top_k, np.uint32),
+        np.resize(np.float32([0.95, 1.0, 0.3]), rows), np.full(rows, 0.2, np.float32), np.full(rows, 0.1, np.float32), np.full(rows, 1.1, np.float32),
+        np.arange(rows + 1, dtype=np.uint32) * history if history else None,
+        np.random.default_rng(vocab).integers(0, vocab, rows * history).astype(np.uint32) if history else None, synth.uniform_f32(4, rows))
+
+
+# Aligned rows that the streaming kernel lists for what they ask for: more than SMs, more than are resident, rows that go on to
+# the general kernel's code, and so few and short that they are done by it at once.
+@pytest.mark.parametrize("rows, vocab, top_k, history", [
+    (160, 9000, 0, 0), (320, 2048, 0, 30), (5, 1028, 0, 2049), (40, 4096, 1025, 2100), (1, 1028, 0, 0), (2, 1060, 0, 5), (2, 1796, 0, 0), (3, 1100, 0, 0)])
+def test_listed_rows(oracle, rows, vocab, top_k, history):
+    import pagoda_b200
+    w = _mixed_rows(rows, vocab, top_k, history, False)
+    some = _mixed_rows(rows, vocab, 40, 0, False)   # nothing to list in between
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
+    try:
+        for _ in range(2):
+            got, want = run_both(s, oracle, w)
+            assert_same(got, want, w)   # listed rows are bit-exact in the default mode too
+            assert_same(*run_both(s, oracle, some), some, exact=False, min_clear=0.0)
+    finally:
+        s.close()
+
+
 @pytest.mark.parametrize("vocab", [3, 4, 513])
 @pytest.mark.parametrize("exact", [True, False])
 def test_top_k_bound_beyond_the_float_range(oracle, vocab, exact):
