@@ -237,10 +237,10 @@ ScoreRoute score_route(const pgs_handle* h, uint32_t rows, uint32_t vocab, bool 
 
 // The combinations of kinds that one CTA per row does quicker (*row), and those that the grid does (returned), among those
 // that the handle's rows can have.
-uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row, bool by_rows = false) {
+uint32_t kinds_for(const pgs_handle* h, uint32_t rows, uint32_t vocab, uint32_t* row, pgs::KindsWay way = pgs::WAY_GRID) {
     using namespace pgs;
     const uint32_t possible = h->max_history > (uint32_t)W_MAX_HIST ? WK_POSSIBLE : WK_SHORT;
-    *row = h->wide_route == 1 || h->wide_route == 3 ? 0u : h->wide_route == 2 ? possible : kinds_one_cta_each(possible, rows, h->wide.chunk, h->slots, vocab, by_rows);
+    *row = h->wide_route == 1 || h->wide_route == 3 ? 0u : h->wide_route == 2 ? possible : kinds_one_cta_each(possible, rows, h->wide.chunk, h->slots, vocab, way);
     return possible & ~*row;
 }
 
@@ -477,12 +477,18 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
     const bool aligned = ((uintptr_t)a.logits & 15u) == 0u && a.row_stride % per == 0u && a.vocab % per == 0u;
     if (h->exact || a.vocab > (uint32_t)pgs::S_MAX_VOCAB || (wide && !aligned)) {
         // What the rows ask for is known on the device only: where both ways are in question, both kernels are launched, and
-        // the one whose batch it is not returns at once.
+        // the one whose batch it is not returns at once.  Many short rows (the two kernels share no SM then) are all done by the wide
+        // kernel, which runs the general kernel's code itself.  General kernel alone / both / wide kernel alone, us: 148 x 4096 greedy
+        // 6.2 / 10.3 / 9.4, top-k 5 61 / 42 / 38; 200 x 12000 greedy 14 / 18 / 20, top-k 50 160 / 79 / 73; 16 x 4096 greedy 6.2 / 8.2 / 9.1.
+        // (That code has little L1 there, and long histories want it.)
         pgs::WideLaunch wl = h->wide;
-        uint32_t grid_kinds = 0u;
+        uint32_t grid_kinds = 0u, row_kinds = 0u;
         wl.local = wide && wide_row_by_row(h, rows, a.vocab);
-        if (wide) grid_kinds = kinds_for(h, rows, a.vocab, &wl.kinds_front, wl.local != 0u);
-        wl.look = wl.kinds_front;
+        const bool alone = wl.local && rows > (uint32_t)h->sm_count / 2u && a.vocab < 16384u && h->max_history <= (uint32_t)pgs::W_MAX_HIST;
+        if (wide) grid_kinds = kinds_for(h, rows, a.vocab, &row_kinds, alone ? pgs::WAY_ROWS_ALONE : wl.local ? pgs::WAY_ROWS : pgs::WAY_GRID);
+        if (alone) wl.kinds_row[0] = wl.kinds_row[1] = row_kinds;
+        else wl.kinds_front = row_kinds;
+        wl.look = row_kinds != 0u;
         if (!wide || !grid_kinds || wl.kinds_front) {
             pgs::RowArgs front = a;
             if (wide && grid_kinds) front.kinds_here = wl.kinds_front;
@@ -525,7 +531,9 @@ int launch_step(pgs_handle* h, pgs::RowArgs& a, cudaStream_t stream) {
         pgs::WideLaunch l = h->wide;   // (how many rows are listed is known on the device only)
         kinds_for(h, rows < l.chunk ? rows : l.chunk, a.vocab, &l.kinds_row[0]);
         if (rows > l.chunk) kinds_for(h, rows, a.vocab, &l.kinds_row[1]);
-        l.look = l.kinds_row[0] | l.kinds_row[1];
+        // (one or two short rows without top-k: see listed_one_cta_each)
+        if (a.vocab < 1800u) { kinds_for(h, 1u, a.vocab, &l.kinds_row[2], pgs::WAY_ROWS); kinds_for(h, 2u, a.vocab, &l.kinds_row[3], pgs::WAY_ROWS); }
+        l.look = (l.kinds_row[0] | l.kinds_row[1] ? 1u : 0u) | (l.kinds_row[2] | l.kinds_row[3] ? 2u : 0u);
         l.local = h->wide_route == 0 ? 2u : h->wide_route == 3 ? 1u : 0u;
         PGS_CUDA(h, pgs::launch_wide(wl, l, h->slots, want < room ? want : room, stream));
     }

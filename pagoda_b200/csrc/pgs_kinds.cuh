@@ -55,11 +55,20 @@ __host__ __device__ __forceinline__ bool listed_one_cta_each(uint32_t n, uint32_
 // 16 x 4096 161 / 78.  Rows with a history beyond the workspace end on one CTA either way (4 of 50256: 187 at once, 239
 // behind the phases).
 //
-// by_rows: the wide kernel takes a CTA per row itself (wide_row_by_row).  us of one row that way, as many at a time as there are
-// SMs: greedy 14 + 0.12 per thousand logits, sampled 36 + 0.3 (55 where the threshold needs the histogram), without top-k 58 + 0.55, with
-// a sort for top-p 60 + 1.  Up to 2048 logits only the last of these is worth it (16 x 1720 111 / 59, others within 5 %), and beyond a
-// chunk of rows not even the look at what the rows ask for (210 x 1719 with top-k 27 100 / 103).
-inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, bool by_rows) {
+// WAY_ROWS: the wide kernel takes a CTA per row itself (wide_row_by_row), behind the general kernel; WAY_ROWS_ALONE: it does,
+// and runs the general kernel's code where that is quicker.  us of one row, as many at a time as there are SMs, general /
+// wide, v in thousands of logits: greedy 9 + 0.37 v / 14 + 0.12 v (alone 5 + 0.45 v / 13 + 0.16 v); sampled 48 + 2.9 v (one
+// row 43 + 1.6 v, two 46 + 2.3 v) / 33 + 0.55 v, 57 + 0.3 v (alone 53 + 0.3 v) where the threshold needs the histogram;
+// without top-k 50 + 6 v / 57 + 0.7 v, a sort for top-p 60 + 18 v / 60 + v.  Measured, each on its own: k 50 1 x 1100 43 / 55,
+// 1 x 6000 51 / 57, 51 x 2040 59 / 55, 148 x 4096 64 / 56, 148 x 16385 104 / 43; k 5 1 x 1100 41 / 33, 148 x 3000 60 / 36; no
+// top-k 1 x 1100 35 / 52, 1 x 3000 47 / 52, 2 x 1500 63 / 52, 148 x 3000 93 / 61; with top-p 1 x 1100 65 / 52, 148 x 4096 158
+// / 53; 2100 history ids 148 x 4096 83 / 100, 200 x 50257 388 / 503; greedy 148 x 4096 6.2 / 14.3, 64 x 16385 12.3 / 16.7, 148
+// x 50257 31 / 22.  (The lines for greedy rows end the look at what rows ask for, 4 us with both kernels, where sampled rows
+// need it no more: 64 x 16385 with top-k 42 / 47, 200 x 16385 76 / 82.)  Up to 2048 logits and beyond a chunk of rows the look
+// costs most of them more than it gives (210 x 1719 with top-k 27 100 / 103).
+enum KindsWay { WAY_GRID, WAY_ROWS, WAY_ROWS_ALONE };
+inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint32_t ctas, uint32_t V, KindsWay way) {
+    const bool by_rows = way != WAY_GRID;
     if (V <= 1024u || (by_rows && V <= 2048u && n > chunk)) return of;   // (the slowest kind is as quick either way, and nothing has to be looked at)
     const float v = (float)V, waves = (float)((n - 1u) / ctas + 1u), chunks = (float)((n - 1u) / chunk + 1u);
     const float m = 1e-6f * v * (float)(n < chunk ? n : chunk), together = (float)(n < ctas ? n : ctas);
@@ -76,12 +85,21 @@ inline uint32_t kinds_one_cta_each(uint32_t of, uint32_t n, uint32_t chunk, uint
         }
         if (by_rows) {
             const float v3 = 1e-3f * v;
-            grid = waves * (!(kinds & WK_SAMPLED) ? 14.0f + 0.12f * v3 : kinds & WK_SORT ? 60.0f + v3 : kinds & WK_OPEN ? 58.0f + 0.55f * v3
-                            : (kinds & WK_HIST ? 55.0f : 36.0f) + 0.3f * v3);
+            if (!(kinds & WK_SAMPLED)) {
+                if (way == WAY_ROWS_ALONE) row = 5.0f + 0.45f * v3;
+                grid = way == WAY_ROWS_ALONE ? 13.0f + 0.16f * v3 : 14.0f + 0.12f * v3;
+            } else if (kinds & WK_SORT) grid = 60.0f + v3;
+            else if (kinds & WK_OPEN) {
+                row = n == 1u && V <= 3100u || n == 2u && V < 1100u ? 0.0f : 50.0f + 6.0f * v3;
+                grid = 57.0f + 0.7f * v3;
+            } else {
+                row = n == 1u ? 43.0f + 1.6f * v3 : n == 2u ? 46.0f + 2.3f * v3 : 48.0f + 2.9f * v3;
+                grid = kinds & WK_HIST ? (way == WAY_ROWS_ALONE ? 53.0f : 57.0f) + 0.3f * v3 : 33.0f + 0.55f * v3;
+            }
+            grid *= waves;
         } else grid *= chunks;
-        if (by_rows && V <= 2048u && !(kinds & WK_SORT)) mask |= 1u << kinds;
-        // (rows with a history beyond the workspace end in the general kernel's code either way: 200 x 50257 388 at once, 503 otherwise)
-        if (waves * row < grid + (!(kinds & WK_LONG) ? 0.0f : by_rows ? waves * row : row)) mask |= 1u << kinds;
+        if (kinds & WK_LONG) grid += by_rows ? waves * row : row;   // (ends in the general kernel's code either way)
+        if (waves * row < grid) mask |= 1u << kinds;
     }
     return mask;
 }

@@ -1758,7 +1758,8 @@ __device__ __noinline__ bool look(uint32_t n_work, uint32_t slots) {
     batch_kinds(sm.a, n_work, W_NT, &sm.found);
     __syncthreads();
     const bool front = l.kinds_front != 0u;
-    const bool per_row = ((front ? l.kinds_front : n_work > l.chunk ? l.kinds_row[1] : l.kinds_row[0]) >> sm.found) & 1u;
+    const bool few = l.local && sm.a.work_rows;   // (one or two listed rows, see below)
+    const bool per_row = ((front ? l.kinds_front : l.kinds_row[few ? 1u + n_work : n_work > l.chunk ? 1u : 0u]) >> sm.found) & 1u;
     if (front) cudaGridDependencySynchronize();
     else if (per_row) rows_one_cta_each(blockIdx.x, min(slots, gridDim.x), n_work, sm.a.work_rows);
     return per_row;
@@ -1816,7 +1817,7 @@ __global__ void __launch_bounds__(W_NT, 1) wide_kernel(const RowArgs a_, const W
     if (tid < 32u) sm.exp_tab[tid] = kExp2TableDev[tid];
     __syncthreads();
     bool ok = true;   // (false for all CTAs, or none)
-    if (l_.look && !(local && l_.local == 2u)) {
+    if (local && l_.local == 2u ? (l_.look & 2u) && n_work <= 2u : (l_.look & 1u)) {
         ok = !look(n_work, slots);
         if (!ok && l_.kinds_front) return;
     }

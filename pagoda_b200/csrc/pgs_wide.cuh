@@ -51,9 +51,10 @@ struct WideLaunch {
     uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
     unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
     uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows that select by the histogram, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
-    // combinations of kinds (pgs_kinds.cuh) that are done by one CTA per row, here ([0]: at most a chunk of rows, [1]: more)
-    // or by the general kernel in front of this one
-    uint32_t kinds_row[2], kinds_front, look;   // look: some bit is set
+    // combinations of kinds (pgs_kinds.cuh) that are done by the general kernel's code, one CTA per row: here, where the grid would
+    // do the rows ([0]: at most a chunk of rows, [1]: more) or a CTA each ([2], of the work list: one row, [3]: two), or by the
+    // general kernel in front of this one
+    uint32_t kinds_row[4], kinds_front, look;   // look: bits are set, 1: in kinds_row[0, 1] or kinds_front, 2: in kinds_row[2, 3]
     uint32_t local;             // 1: one CTA per row, with the part of the workspace that has the CTA's number; 2: by the number of listed rows
     uint32_t* own;              // [CTAs][W_OWN]: what `sync`, `left_count` and `left_rows` are for the grid
     uint32_t polls;             // limit of a barrier's wait

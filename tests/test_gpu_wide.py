@@ -154,6 +154,23 @@ def _mixed_rows(rows, vocab, top_k, history, greedy, seed=29):
         np.random.default_rng(vocab).integers(0, vocab, rows * history).astype(np.uint32) if history else None, synth.uniform_f32(4, rows))
 
 
+# Many short rows: one launch that does them one way or the other; where histories may be long, two.
+@pytest.mark.parametrize("max_history", [64, 2049])
+@pytest.mark.parametrize("rows, vocab", [(75, 2049), (148, 2051), (149, 4096), (200, 16383), (330, 2052)])
+@pytest.mark.parametrize("top_k, greedy", [(0, True), (3, False), (200, False), (0, False)])
+def test_many_short_exact_rows(oracle, rows, vocab, top_k, greedy, max_history):
+    import pagoda_b200
+    w = _mixed_rows(rows, vocab, top_k, 40, greedy)
+    w.logits[1, vocab - 1] = np.nan
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max_history)
+    try:
+        s.set_exact(True)
+        for _ in range(2):   # (on what the one before has left)
+            assert_same(*run_both(s, oracle, w), w)
+    finally:
+        s.close()
+
+
 # Aligned rows that the streaming kernel lists for what they ask for: more than SMs, more than are resident, rows that go on to
 # the general kernel's code, and so few and short that they are done by it at once.
 @pytest.mark.parametrize("rows, vocab, top_k, history", [
