@@ -544,9 +544,10 @@ __device__ __forceinline__ void p2_entries(SM& sm, uint32_t n_ent) {
 
 // How pass 2 puts candidates on the list, for f32 rows that a cluster shares: in rounds over the lanes where there are few, in
 // rounds over the sixteen positions of a lane's logits where there are many.  Over the lanes / over the positions, us: 8 rows of
-// 151936 with top-k 40 27.0 / 28.5, 64 with 50 37.9 / 38.5, 64 with 500 49.4 / 50.3, 64 with 1024 68.7 / 68.0.  (One CTA per row, and
-// bf16 rows: over the positions.  Some rows with long lists take half as long again over the lanes, 256 with top-k 500 92 / 80, and
-// both ways in one kernel cost all others 1 %.)
+// 151936 with top-k 40 27.0 / 28.5, 64 with 50 37.9 / 38.5, 64 with 500 49.4 / 50.3, 64 with 1024 68.7 / 68.0; 2048 to 256000
+// logits, 1 to 64 rows and top-k 1 to 512 are within 3 % or quicker.  (One CTA per row, and bf16 rows: over the
+// positions.  Some rows with long lists take half as long again over the lanes, 256 with top-k 500 92 / 80, and both ways in one
+// kernel cost all others 1 %.)
 template <bool BF16, bool CL>
 __device__ __forceinline__ bool few_candidates(uint32_t top_k) { return CL && !BF16 && top_k <= 512u; }
 

@@ -652,9 +652,9 @@ __device__ __forceinline__ uint32_t segment_binade(float pre, float P, float sla
     return kb + 0x00800000u == binade(hi) && binade(pre) == binade(pre + P) ? kb | W_DUAL : 0u;
 }
 // The same for the fold towards top-p, for one binade only.  It ends before the running value is 1, so what may come to 1 or more
-// stays in the binade below as far as the fold goes.  (With 1 as a border like the others, every bucket behind 0.998 was a
-// bucket to be added entry by entry: 32 rows of 151936 with top-p 0.999 took 2.7 ms bucket by bucket and 9.2 on
-// a CTA that sorts the whole row, where there were too many of them for the list of events; now 0.5.)
+// stays in the binade below as far as the fold goes.  (With 1 as a border like the others, every bucket behind 0.998 was to be
+// added entry by entry: 32 rows of 151936 with top-p 0.999 took 2.7 ms bucket by bucket, and 9.2 on a CTA that sorts the whole
+// row, where there were too many of them for the list of events; now 0.5.)
 __device__ __forceinline__ uint32_t top_p_binade(float pre, float P, float slack) {
     constexpr float BELOW_ONE = 0.99999994f;
     const float lo = fminf(pre * (1.0f - slack), BELOW_ONE), hi = fminf((pre + P) * (1.0f + slack), BELOW_ONE);

@@ -39,21 +39,23 @@ struct WideRow {
 enum : uint32_t { WS_FIRST = 0u, WS_SUM = 1u, WS_SELECT = 2u, WS_TOTAL = 3u, WS_DONE = 4u };
 
 struct WideLaunch {
-    WideRow* row;               // [chunk]
-    float2* reg;                // [chunk][n_regions]: a region's maximum, its plain sum
-    float4* cell;               // [chunk][n_regions]: the maxima of four parts of the region
-    uint2* seg;                 // [chunk][n_regions]: increments in ulps, binade (0: add term by term)
-    float* pre;                 // [chunk][n_regions]: estimate of the running value at the region's start
-    float* terms;               // [chunk][W_TERMS][W_REGION]: terms of segments that are added one by one
-    uint32_t* ent_id;           // [chunk][W_MAX_HIST + 32]
+    // The workspace's parts: as many as scratch slots (min(rows of the handle, SMs)) for steps, as SMs for scoring.  The grid uses the
+    // first `chunk` of them, one for every row in flight; with one CTA per row each CTA has the part of its number, so that
+    // min(CTAs, rows) must not be more than there are.
+    WideRow* row;               // [parts]
+    float2* reg;                // [parts][n_regions]: a region's maximum, its plain sum
+    float4* cell;               // [parts][n_regions]: the maxima of four parts of the region
+    uint2* seg;                 // [parts][n_regions]: increments in ulps, binade (0: add term by term)
+    float* pre;                 // [parts][n_regions]: estimate of the running value at the region's start
+    float* terms;               // [parts][W_TERMS][W_REGION]: terms of segments that are added one by one
+    uint32_t* ent_id;           // [parts][W_MAX_HIST + 32]
     float* ent_xn;
-    uint32_t* rs;               // [chunk][n_regions + 1]
-    uint32_t* hist;             // [chunk][W_BUCKETS]: counts, then list positions
-    unsigned long long* list;   // [chunk][list_stride] (the general kernel's sort buffer): probability bits and id
+    uint32_t* rs;               // [parts][n_regions + 1]
+    uint32_t* hist;             // [parts][W_BUCKETS]: counts, then list positions
+    unsigned long long* list;   // [parts][list_stride] (the general kernel's sort buffer): probability bits and id
     uint32_t* sync;             // [0] barrier arrivals, [1] rows without results where a barrier was given up, [2] rows that select by the histogram, [3] rows in the last pass, [4] CTAs that have left, [5] CTAs that have joined, [6] how many take part
-    // combinations of kinds (pgs_kinds.cuh) that are done by the general kernel's code, one CTA per row: here, where the grid would
-    // do the rows ([0]: at most a chunk of rows, [1]: more) or a CTA each ([2], of the work list: one row, [3]: two), or by the
-    // general kernel in front of this one
+    // Combinations of kinds (pgs_kinds.cuh) that are done by the general kernel's code, one CTA per row: here ([0]: at most a chunk of
+    // rows, [1]: more; [2]: one listed row that would have a CTA of its own, [3]: two), or by the general kernel in front of this one.
     uint32_t kinds_row[4], kinds_front, look;   // look: bits are set, 1: in kinds_row[0, 1] or kinds_front, 2: in kinds_row[2, 3]
     uint32_t local;             // 1: one CTA per row, with the part of the workspace that has the CTA's number; 2: by the number of listed rows
     uint32_t* own;              // [CTAs][W_OWN]: what `sync`, `left_count` and `left_rows` are for the grid

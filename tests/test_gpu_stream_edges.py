@@ -73,6 +73,29 @@ def test_stream_edges_on_one_cta_and_on_clusters(oracle, monkeypatch, cluster, r
         s.close()
 
 
+# bf16 rows whose masked logits are the largest by far: one CTA per row adds -inf to them, rows of a cluster and longer ones select.
+@pytest.mark.parametrize("cluster", ["1", "0"])
+@pytest.mark.parametrize("vocab, greedy", [(1000, False), (8200, False), (40016, True), (262152, False)])
+def test_masked_logits_that_are_the_largest(oracle, monkeypatch, cluster, vocab, greedy):
+    import pagoda_b200
+    monkeypatch.setenv("PGS_CLUSTER", cluster)
+    rows = 9
+    w = _batch(rows, vocab, 40, 30, vocab, True, True)
+    x = w.logits_f32().copy()
+    for r, state in enumerate(w.mask_state):
+        if state >= 0:
+            allowed = np.unpackbits(w.mask_words[state].view(np.uint8), bitorder="little")[:vocab].astype(bool)
+            x[r, ~allowed] += 1000.0 * (1 + r)
+    w.logits[...] = (x.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    if greedy:
+        w.temperature[...] = 0.0
+    s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=30)
+    try:
+        assert_close(*run_both(s, oracle, w), "masked", min_clear=0.0)
+    finally:
+        s.close()
+
+
 # Long candidate lists are folded in runs of sixteen, short ones by one lane.
 @pytest.mark.parametrize("exact", [False, True])
 @pytest.mark.parametrize("rows, vocab, top_k", [(5, 4096, 160), (5, 40000, 161), (9, 151936, 500), (300, 8192, 700)])

@@ -114,7 +114,8 @@ def test_terms_and_entries_share_the_staging_buffer(oracle, monkeypatch, route, 
                                                          (9, 33025, 0, 300), (3, 70001, 2049, 2100)])
 def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
     """The wide kernel with one CTA per row: one row, more rows than SMs, rows that go on to the general kernel's code
-    (more history than the workspace holds), short and long lists, a mask that leaves regions empty; steps, listed rows, scores."""
+    (more history than the workspace holds), short and long lists, a mask that leaves regions empty; steps and scores.  (In the
+    default mode the unaligned batches take this way too, the aligned one the streaming kernel: test_listed_rows has what is listed.)"""
     import torch
     import pagoda_b200
     from pagoda_b200 import synth
@@ -132,9 +133,9 @@ def test_one_cta_per_row(oracle, monkeypatch, rows, vocab, top_k, history):
         mask_words=words, state_flags=np.zeros(2, np.uint32), mask_state=np.resize(np.int32([-1, 0, 1, -1, 1]), rows))
     s = pagoda_b200.Sampler(device=0, max_rows=rows, max_vocab=vocab, max_history=max(history, 1))
     try:
-        for exact in (True, False, True):   # (on what the one before has left; the default mode lists what the row kernel does not do)
+        for exact in (True, False, True):   # (on what the one before has left)
             s.set_exact(exact)
-            assert_same(*run_both(s, oracle, w), w, exact=exact, min_clear=0.0)
+            assert_same(*run_both(s, oracle, w), w, exact=exact or vocab % 4 != 0, min_clear=0.0)   # (unaligned rows are bit-exact)
         ids = np.arange(rows, dtype=np.int32) % vocab
         g, full, _ = s.log_softmax(torch.from_numpy(x).cuda(), ids=torch.from_numpy(ids).cuda(), full=True,
                                    stream_ptr=torch.cuda.current_stream().cuda_stream)
