@@ -37,7 +37,8 @@ __device__ __forceinline__ void batch_kinds(const RowArgs& a, uint32_t n, uint32
 // Whether the wide kernel takes n listed rows one CTA each, `parts` at a time, and not with the whole grid on `chunk` at a time.
 // Listed rows have no top-k as a rule, and often top-p.  us with a CTA per row / with the grid, top-p off and 0.9: 1 x 4096 57 / 67,
 // 16 x 16384 64 / 75 and 65 / 105, 64 x 16384 69 / 81 and 70 / 126, 16 x 50256 97 / 82 and 95 / 120, 64 x 50256 96 / 99 and 112 / 167,
-// 64 x 151936 149 / 147 and 223 / 244, 148 x 4096 60 / 212, 256 x 151936 333 / 574 and 464 / 954.
+// 64 x 151936 149 / 147 and 223 / 244, 148 x 4096 60 / 212, 256 x 151936 333 / 574 and 464 / 954.  (The line goes by number and length
+// alone and is drawn for rows without top-p; with it a few that the grid gets would be quicker on a CTA each, 16 x 50256 by 20 %.)
 __host__ __device__ __forceinline__ bool listed_one_cta_each(uint32_t n, uint32_t chunk, uint32_t parts, uint32_t V) {
     const float v = 1e-6f * (float)V;
     const float by_rows = (float)((n - 1u) / parts + 1u) * (58.0f + 800.0f * v + 2.5f * v * (float)(n < parts ? n : parts));
